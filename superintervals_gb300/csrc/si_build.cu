@@ -98,8 +98,7 @@ __global__ void k_decode(const uint32_t* __restrict__ w0, const uint32_t* __rest
 template <typename S>
 __global__ void k_copy_pad(const S* __restrict__ s_in, const S* __restrict__ e_in,
                            const int32_t* __restrict__ d_in, int64_t n, int64_t n_pad,
-                           S* __restrict__ starts, S* __restrict__ ends, int32_t* __restrict__ data,
-                           uint32_t* __restrict__ perm) {
+                           S* __restrict__ starts, S* __restrict__ ends, int32_t* __restrict__ data) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
     if (i >= n) {
@@ -110,7 +109,6 @@ __global__ void k_copy_pad(const S* __restrict__ s_in, const S* __restrict__ e_i
     starts[i] = s_in[i];
     ends[i] = e_in[i];
     data[i] = d_in[i];
-    if (perm) perm[i] = (uint32_t)i;
 }
 
 // out[c] = max(in[32c .. 32c+31]); `in` is padded to a multiple of 32, `out`
@@ -159,6 +157,17 @@ __global__ void k_long_scatter(const S* __restrict__ starts, const S* __restrict
         pos[i] = -1;
         lend[i] = Lim<S>::lo;
     }
+}
+
+// The branch array as contig-local 64-bit positions (-1: none).  One read and one write of HBM per
+// entry, in place of a host loop over the copied array (5 M intervals: arrays back in 8.8 ms with it).
+__global__ void __launch_bounds__(kThreads) k_branch_local(const int32_t* __restrict__ branch,
+                                                           const int64_t* __restrict__ seg, int G, int64_t n,
+                                                           int64_t* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    const int32_t b = branch[i];
+    out[i] = b < 0 ? -1 : (int64_t)b - (G > 1 ? seg[seg_of(seg, G, i)] : 0);
 }
 
 // flag = 1 when a[i] != b[i] for some i < n
@@ -552,11 +561,10 @@ cudaError_t launch_decode(const uint32_t* const* kw, const uint32_t* perm, const
 
 template <typename S>
 cudaError_t launch_copy_pad(const S* s_in, const S* e_in, const int32_t* d_in, int64_t n,
-                            int64_t n_pad, S* starts, S* ends, int32_t* data, uint32_t* perm,
-                            cudaStream_t st) {
+                            int64_t n_pad, S* starts, S* ends, int32_t* data, cudaStream_t st) {
     if (n_pad <= 0) return cudaSuccess;
     k_copy_pad<S><<<blocks_for(n_pad), kThreads, 0, st>>>(s_in, e_in, d_in, n, n_pad, starts, ends,
-                                                         data, perm);
+                                                         data);
     note_launch();
     return cudaGetLastError();
 }
@@ -622,6 +630,14 @@ cudaError_t launch_long_depth(const S* starts, const S* ends, int64_t n, const i
     if (e != cudaSuccess || n <= 0) return e;
     k_long_depth<S><<<(unsigned)std::min<int64_t>(blocks_for(std::max<int64_t>(n, G)), 152 * 4), kThreads, 0, st>>>(
         starts, ends, n, seg, G, X, out);
+    note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_branch_local(const int32_t* branch, const int64_t* seg, int G, int64_t n, int64_t* out,
+                                cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_branch_local<<<blocks_for(n), kThreads, 0, st>>>(branch, seg, G, n, out);
     note_launch();
     return cudaGetLastError();
 }
@@ -730,7 +746,7 @@ cudaError_t launch_branch(const S* ends, int64_t n, int64_t n_pad, Levels<S> L, 
     template cudaError_t launch_decode<S>(const uint32_t* const*, const uint32_t*, const int32_t*, \
                                           int64_t, int64_t, S*, S*, int32_t*, cudaStream_t);     \
     template cudaError_t launch_copy_pad<S>(const S*, const S*, const int32_t*, int64_t, int64_t, \
-                                            S*, S*, int32_t*, uint32_t*, cudaStream_t);          \
+                                            S*, S*, int32_t*, cudaStream_t);                     \
     template cudaError_t launch_pyramid<S>(const S*, const int64_t*, int, S* const*, cudaStream_t); \
     template cudaError_t launch_long_flags<S>(const S*, const S*, int64_t, int64_t, uint32_t*, cudaStream_t); \
     template cudaError_t launch_long_scatter<S>(const S*, const S*, int64_t, int64_t, const int64_t*, int64_t, \

@@ -10,6 +10,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -140,7 +141,7 @@ struct gSuperIntervals {
     int64_t n = 0, n_pad = 0;
     int G = 1, H = 0;
     int64_t lvl_sizes[sig::kMaxLevels + 1] = {0};
-    DevBuf starts, ends, data, branch, seg, perm;
+    DevBuf starts, ends, data, branch, seg;
     DevBuf lvl[sig::kMaxLevels];
     // long-interval list: intervals >= kLongIntervalSplit long, position order, own pyramid
     DevBuf long_pos, long_end, long_seg;
@@ -240,6 +241,27 @@ int check_width(const gSuperIntervals* si) {
     return SI_OK;
 }
 
+// 0, 1, 2, ... as a vector's range: written once, without a pass of zeros before
+struct IotaIt {
+    using iterator_category = std::random_access_iterator_tag;
+    using value_type = int32_t;
+    using difference_type = int64_t;
+    using pointer = const int32_t*;
+    using reference = int32_t;
+    int64_t i = 0;
+    int32_t operator*() const { return (int32_t)i; }
+    IotaIt& operator++() { ++i; return *this; }
+    IotaIt operator++(int) { IotaIt t = *this; ++i; return t; }
+    IotaIt& operator--() { --i; return *this; }
+    IotaIt& operator+=(int64_t d) { i += d; return *this; }
+    IotaIt operator+(int64_t d) const { return IotaIt{i + d}; }
+    int64_t operator-(const IotaIt& o) const { return i - o.i; }
+    int32_t operator[](int64_t d) const { return (int32_t)(i + d); }
+    bool operator==(const IotaIt& o) const { return i == o.i; }
+    bool operator!=(const IotaIt& o) const { return i != o.i; }
+    bool operator<(const IotaIt& o) const { return i < o.i; }
+};
+
 template <typename S>
 int add_many(gSuperIntervals* si, const S* s, const S* e, const int32_t* v, size_t n) {
     SI_TRY(check_width<S>(si));
@@ -252,8 +274,7 @@ int add_many(gSuperIntervals* si, const S* s, const S* e, const int32_t* v, size
     if (v) {
         si->hdata.insert(si->hdata.end(), v, v + n);
     } else {
-        si->hdata.resize(base + n);
-        for (size_t i = 0; i < n; ++i) si->hdata[base + i] = (int32_t)(base + i);
+        si->hdata.insert(si->hdata.end(), IotaIt{(int64_t)base}, IotaIt{(int64_t)(base + n)});
     }
     if (!si->hseg.empty()) si->hseg.back() = (int64_t)staged(si);  // grow the last contig
     si->built = false;
@@ -297,6 +318,19 @@ sig::Levels<S> levels(const gSuperIntervals* si) {
     return L;
 }
 
+// Temporaries cut one after another from one buffer.
+struct TempArena {
+    DevBuf buf;
+    size_t at = 0;
+    static size_t room(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+    template <typename T>
+    T* take(size_t bytes) {
+        T* p = reinterpret_cast<T*>(buf.as<char>() + at);
+        at += room(bytes);
+        return p;
+    }
+};
+
 template <typename S>
 int build_impl(gSuperIntervals* si) {
     SI_TRY(set_dev(si));
@@ -327,7 +361,6 @@ int build_impl(gSuperIntervals* si) {
     SI_TRY(si->ends.reserve(sizeof(S) * n_pad));
     SI_TRY(si->data.reserve(sizeof(int32_t) * n_pad));
     SI_TRY(si->branch.reserve(sizeof(int32_t) * n_pad));
-    SI_TRY(si->perm.reserve(sizeof(uint32_t) * n_pad));
     SI_TRY(si->seg.reserve(sizeof(int64_t) * (G + 1)));
     SI_CK(cudaMemcpyAsync(si->seg.p, segv.data(), sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, st));
     si->H = sig::pyramid_levels(n_pad, si->lvl_sizes);
@@ -337,92 +370,99 @@ int build_impl(gSuperIntervals* si) {
         si->built = true;
         return SI_OK;
     }
-    DevBuf s_in, e_in, d_in, flag, berr;
-    SI_TRY(berr.reserve(sizeof(int)));  // bounded waits of the one-sweep sorts and scans
-    SI_CK(cudaMemsetAsync(berr.p, 0, sizeof(int), st));
-    SI_TRY(s_in.reserve(sizeof(S) * n));
-    SI_TRY(e_in.reserve(sizeof(S) * n));
-    SI_TRY(d_in.reserve(sizeof(int32_t) * n));
-    SI_TRY(flag.reserve(sizeof(int)));
-    SI_CK(cudaMemcpyAsync(s_in.p, hs<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
-    SI_CK(cudaMemcpyAsync(e_in.p, he<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
-    SI_CK(cudaMemcpyAsync(d_in.p, si->hdata.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
-    SI_CK(sig::launch_check_sorted<S>(s_in.as<S>(), e_in.as<S>(), n, si->seg.as<int64_t>(), G,
-                                      flag.as<int>(), st));
+    // Every temporary of the build in one allocation, cut anew for each stage: the stages run one
+    // after the other on the stream, so a stage may overwrite what the one before left.  (One
+    // cudaMalloc / cudaFree instead of some twenty, and no wait between stages to free by: 200 k
+    // intervals built in 1.58 ms before.)
+    const int K = sig::key_words<S>(G), Ke = sig::end_key_words<S>(G);
+    const size_t tb = sig::radix_temp_bytes(n, K), tbe = sig::radix_temp_bytes(n, Ke);
+    const size_t words = TempArena::room(sizeof(uint32_t) * n);
+    const size_t in_bytes = 2 * TempArena::room(sizeof(S) * n) + words + 2 * TempArena::room(256);
+    const size_t stages[4] = {
+        in_bytes + (2 * (size_t)K + 2) * words + TempArena::room(tb),
+        in_bytes + TempArena::room(sig::branch_temp_bytes(n_pad)),
+        in_bytes + words + TempArena::room(sizeof(int64_t) * (n + 1)) + TempArena::room(sig::scan_temp_bytes(n)) +
+            TempArena::room(256),
+        in_bytes + (2 * (size_t)Ke + 2) * words + TempArena::room(tbe)};
+    TempArena arena;
+    SI_TRY(arena.buf.reserve(*std::max_element(stages, stages + 4)));
+    int* berr = arena.take<int>(256);  // bounded waits of the one-sweep sorts and scans
+    int* flag = arena.take<int>(256);
+    S* s_in = arena.take<S>(sizeof(S) * n);
+    S* e_in = arena.take<S>(sizeof(S) * n);
+    int32_t* d_in = arena.take<int32_t>(sizeof(int32_t) * n);
+    const size_t stage0 = arena.at;
+    SI_CK(cudaMemsetAsync(berr, 0, sizeof(int), st));
+    SI_CK(cudaMemcpyAsync(s_in, hs<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
+    SI_CK(cudaMemcpyAsync(e_in, he<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
+    SI_CK(cudaMemcpyAsync(d_in, si->hdata.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
+    SI_CK(sig::launch_check_sorted<S>(s_in, e_in, n, si->seg.as<int64_t>(), G, flag, st));
     int unsorted = 0;
-    SI_CK(cudaMemcpyAsync(&unsorted, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
     si->input_was_sorted = !unsorted;
     si->sort_passes = 0;
+    uint32_t* kp[sig::kMaxKeyWords];
+    uint32_t* ka[sig::kMaxKeyWords];
     if (!unsorted) {
-        SI_CK(sig::launch_copy_pad<S>(s_in.as<S>(), e_in.as<S>(), d_in.as<int32_t>(), n, n_pad,
-                                      si->starts.as<S>(), si->ends.as<S>(), si->data.as<int32_t>(),
-                                      si->perm.as<uint32_t>(), st));
+        SI_CK(sig::launch_copy_pad<S>(s_in, e_in, d_in, n, n_pad, si->starts.as<S>(), si->ends.as<S>(),
+                                      si->data.as<int32_t>(), st));
     } else {
-        const int K = sig::key_words<S>(G);
-        DevBuf kw[sig::kMaxKeyWords], kalt[sig::kMaxKeyWords], pay, palt, tmp;
-        uint32_t* kp[sig::kMaxKeyWords];
-        uint32_t* ka[sig::kMaxKeyWords];
         for (int k = 0; k < K; ++k) {
-            SI_TRY(kw[k].reserve(sizeof(uint32_t) * n));
-            SI_TRY(kalt[k].reserve(sizeof(uint32_t) * n));
-            kp[k] = kw[k].as<uint32_t>();
-            ka[k] = kalt[k].as<uint32_t>();
+            kp[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
+            ka[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
         }
-        SI_TRY(pay.reserve(sizeof(uint32_t) * n));
-        SI_TRY(palt.reserve(sizeof(uint32_t) * n));
-        const size_t tb = sig::radix_temp_bytes(n, K);
-        SI_TRY(tmp.reserve(tb));
-        SI_CK(sig::launch_make_keys<S>(s_in.as<S>(), e_in.as<S>(), n, si->seg.as<int64_t>(), G, kp,
-                                       pay.as<uint32_t>(), st));
+        uint32_t* pay = arena.take<uint32_t>(sizeof(uint32_t) * n);
+        uint32_t* palt = arena.take<uint32_t>(sizeof(uint32_t) * n);
+        void* tmp = arena.take<char>(tb);
+        SI_CK(sig::launch_make_keys<S>(s_in, e_in, n, si->seg.as<int64_t>(), G, kp, pay, st));
         bool in_alt = false;
-        SI_CK(sig::radix_sort(kp, ka, pay.as<uint32_t>(), palt.as<uint32_t>(), K, n, tmp.p, tb,
-                              &in_alt, &si->sort_passes, st, 0, berr.as<int>()));
-        uint32_t* const* res_k = in_alt ? ka : kp;
-        const uint32_t* res_p = in_alt ? palt.as<uint32_t>() : pay.as<uint32_t>();
-        SI_CK(sig::launch_decode<S>(res_k, res_p, d_in.as<int32_t>(), n, n_pad, si->starts.as<S>(),
+        SI_CK(sig::radix_sort(kp, ka, pay, palt, K, n, tmp, tb, &in_alt, &si->sort_passes, st, 0, berr));
+        SI_CK(sig::launch_decode<S>(in_alt ? ka : kp, in_alt ? palt : pay, d_in, n, n_pad, si->starts.as<S>(),
                                     si->ends.as<S>(), si->data.as<int32_t>(), st));
-        SI_CK(cudaMemcpyAsync(si->perm.p, res_p, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
-        SI_CK(cudaStreamSynchronize(st));  // temps are released on scope exit
     }
     const S* ends = si->ends.as<S>();
     S* lp[sig::kMaxLevels];
     for (int h = 0; h < sig::kMaxLevels; ++h) lp[h] = si->lvl[h].as<S>();
     SI_CK(sig::launch_pyramid<S>(ends, si->lvl_sizes, si->H, lp, st));
-    {
-        DevBuf btmp;
-        SI_TRY(btmp.reserve(sig::branch_temp_bytes(n_pad)));
-        SI_CK(sig::launch_branch<S>(ends, n, n_pad, levels<S>(si), si->H, si->seg.as<int64_t>(), G,
-                                    si->branch.as<int32_t>(), st, btmp.p, berr.as<int>()));
-        SI_CK(cudaStreamSynchronize(st));  // the temporary is released on scope exit
-    }
+    arena.at = stage0;
+    SI_CK(sig::launch_branch<S>(ends, n, n_pad, levels<S>(si), si->H, si->seg.as<int64_t>(), G,
+                                si->branch.as<int32_t>(), st, arena.take<char>(sig::branch_temp_bytes(n_pad)), berr));
     // long-interval list of the batched path: intervals at least kLongIntervalSplit long, in
     // position order, with their own max pyramid (a tile reaches them without visiting the
-    // positions in between)
+    // positions in between); and whether some interval has start > end
     {
-        DevBuf flags, offs, tmp;
-        SI_TRY(flags.reserve(sizeof(uint32_t) * n));
-        SI_TRY(offs.reserve(sizeof(int64_t) * (n + 1)));
-        SI_TRY(tmp.reserve(sig::scan_temp_bytes(n)));
-        SI_CK(sig::launch_long_flags<S>(si->starts.as<S>(), ends, n, sig::kLongIntervalSplit, flags.as<uint32_t>(),
-                                        st));
-        SI_CK(sig::exclusive_scan_u32_to_i64(flags.as<uint32_t>(), offs.as<int64_t>(), n, tmp.p, st, berr.as<int>()));
+        arena.at = stage0;
+        uint32_t* flags = arena.take<uint32_t>(sizeof(uint32_t) * n);
+        int64_t* offs = arena.take<int64_t>(sizeof(int64_t) * (n + 1));
+        void* tmp = arena.take<char>(sig::scan_temp_bytes(n));
+        unsigned long long* sums = arena.take<unsigned long long>(256);
+        SI_CK(sig::launch_long_flags<S>(si->starts.as<S>(), ends, n, sig::kLongIntervalSplit, flags, st));
+        SI_CK(sig::exclusive_scan_u32_to_i64(flags, offs, n, tmp, st, berr));
+        SI_CK(sig::launch_any_inverted<S>(view<S>(si), flag, st));
+        SI_CK(sig::launch_long_depth<S>(si->starts.as<S>(), ends, n, si->seg.as<int64_t>(), G,
+                                        sig::kLongIntervalSplit, sums, st));
         int64_t n_long = 0;
-        SI_CK(cudaMemcpyAsync(&n_long, offs.as<int64_t>() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        int f = 0;
+        unsigned long long h[2] = {0, 0};
+        SI_CK(cudaMemcpyAsync(&n_long, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        SI_CK(cudaMemcpyAsync(&f, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        SI_CK(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, st));
         SI_CK(cudaStreamSynchronize(st));
+        si->inverted = f ? 1 : 0;
+        si->long_depth = h[1] > 0 ? (double)h[0] / (double)h[1] : 0.0;
         const int64_t n_long_pad = sig::round_up(std::max<int64_t>(n_long, 1), 32);
         SI_TRY(si->long_pos.reserve(sizeof(int32_t) * n_long_pad));
         SI_TRY(si->long_end.reserve(sizeof(S) * n_long_pad));
         SI_TRY(si->long_seg.reserve(sizeof(int64_t) * (G + 1)));
         si->long_H = sig::pyramid_levels(n_long_pad, si->long_sizes);
-        for (int h = 1; h <= si->long_H; ++h) SI_TRY(si->long_lvl[h - 1].reserve(sizeof(S) * si->long_sizes[h]));
-        SI_CK(sig::launch_long_scatter<S>(si->starts.as<S>(), ends, n, sig::kLongIntervalSplit, offs.as<int64_t>(),
-                                          n_long, n_long_pad, si->seg.as<int64_t>(), G, si->long_pos.as<int32_t>(),
+        for (int h2 = 1; h2 <= si->long_H; ++h2) SI_TRY(si->long_lvl[h2 - 1].reserve(sizeof(S) * si->long_sizes[h2]));
+        SI_CK(sig::launch_long_scatter<S>(si->starts.as<S>(), ends, n, sig::kLongIntervalSplit, offs, n_long,
+                                          n_long_pad, si->seg.as<int64_t>(), G, si->long_pos.as<int32_t>(),
                                           si->long_end.as<S>(), si->long_seg.as<int64_t>(), st));
         S* llv[sig::kMaxLevels];
-        for (int h = 0; h < sig::kMaxLevels; ++h) llv[h] = si->long_lvl[h].as<S>();
+        for (int h2 = 0; h2 < sig::kMaxLevels; ++h2) llv[h2] = si->long_lvl[h2].as<S>();
         SI_CK(sig::launch_pyramid<S>(si->long_end.as<S>(), si->long_sizes, si->long_H, llv, st));
-        SI_CK(cudaStreamSynchronize(st));  // the temporaries are released on scope exit
     }
     si->bws.long_ends = si->long_end.p;
     si->bws.long_pos = si->long_pos.as<int32_t>();
@@ -430,46 +470,23 @@ int build_impl(gSuperIntervals* si) {
     for (int h = 0; h < sig::kMaxLevels; ++h) si->bws.long_lvl[h] = si->long_lvl[h].p;
     si->bws.long_H = si->long_H;
     si->bws.long_split = sig::kLongIntervalSplit;
-    // intervals with start > end; when there are none, each contig's ends in ascending order,
-    // from which the batched path counts short queries (two ranks per query)
-    {
-        DevBuf flag2;
-        SI_TRY(flag2.reserve(8 + 2 * sizeof(unsigned long long)));
-        unsigned long long* sums = reinterpret_cast<unsigned long long*>(flag2.as<char>() + 8);
-        SI_CK(sig::launch_any_inverted<S>(view<S>(si), flag2.as<int>(), st));
-        SI_CK(sig::launch_long_depth<S>(si->starts.as<S>(), si->ends.as<S>(), n, si->seg.as<int64_t>(), G,
-                                         sig::kLongIntervalSplit, sums, st));
-        int f = 0;
-        unsigned long long h[2] = {0, 0};
-        SI_CK(cudaMemcpyAsync(&f, flag2.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-        SI_CK(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, st));
-        SI_CK(cudaStreamSynchronize(st));
-        si->inverted = f ? 1 : 0;
-        si->long_depth = h[1] > 0 ? (double)h[0] / (double)h[1] : 0.0;
-    }
+    // without intervals with start > end: each contig's ends in ascending order, from which the
+    // batched path counts short queries (two ranks per query)
     if (si->inverted == 0) {
-        const int K = sig::end_key_words<S>(G);
-        DevBuf kw[3], kalt[3], pay, palt, tmp;
-        uint32_t* kp[3];
-        uint32_t* ka[3];
-        for (int k = 0; k < K; ++k) {
-            SI_TRY(kw[k].reserve(sizeof(uint32_t) * n));
-            SI_TRY(kalt[k].reserve(sizeof(uint32_t) * n));
-            kp[k] = kw[k].as<uint32_t>();
-            ka[k] = kalt[k].as<uint32_t>();
+        arena.at = stage0;
+        for (int k = 0; k < Ke; ++k) {
+            kp[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
+            ka[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
         }
-        SI_TRY(pay.reserve(sizeof(uint32_t) * n));
-        SI_TRY(palt.reserve(sizeof(uint32_t) * n));
-        const size_t tb = sig::radix_temp_bytes(n, K);
-        SI_TRY(tmp.reserve(tb));
+        uint32_t* pay = arena.take<uint32_t>(sizeof(uint32_t) * n);
+        uint32_t* palt = arena.take<uint32_t>(sizeof(uint32_t) * n);
+        void* tmp = arena.take<char>(tbe);
         SI_CK(sig::launch_end_keys<S>(ends, n, si->seg.as<int64_t>(), G, kp, st));
         bool in_alt = false;
         int passes = 0;
-        SI_CK(sig::radix_sort(kp, ka, pay.as<uint32_t>(), palt.as<uint32_t>(), K, n, tmp.p, tb, &in_alt, &passes,
-                              st, 0, berr.as<int>()));
+        SI_CK(sig::radix_sort(kp, ka, pay, palt, Ke, n, tmp, tbe, &in_alt, &passes, st, 0, berr));
         SI_TRY(si->end_sorted.reserve(sizeof(S) * n_pad));
         SI_CK(sig::launch_end_decode<S>(in_alt ? ka : kp, n, n_pad, si->end_sorted.as<S>(), st));
-        SI_CK(cudaStreamSynchronize(st));  // the temporaries are released on scope exit
         si->bws.end_sorted = si->end_sorted.p;
     }
     SI_TRY(sig::batched_prepare<S>(si->bws, view<S>(si), levels<S>(si), si->H, si->lvl_sizes,
@@ -478,7 +495,7 @@ int build_impl(gSuperIntervals* si) {
     SI_CK(cudaGetLastError());
     {
         int be = 0;
-        SI_CK(cudaMemcpy(&be, berr.p, sizeof(int), cudaMemcpyDeviceToHost));
+        SI_CK(cudaMemcpy(&be, berr, sizeof(int), cudaMemcpyDeviceToHost));
         if (be) return fail(SI_ERR_CUDA, "build: a bounded wait in a sort or scan kernel gave up (%d)", be);
     }
     si->built = true;
@@ -773,17 +790,30 @@ int get_arrays(const gSuperIntervals* si, S* s, S* e, int32_t* d, int64_t* br) {
     if (s) SI_CK(cudaMemcpyAsync(s, si->starts.p, sizeof(S) * n, cudaMemcpyDeviceToHost, st));
     if (e) SI_CK(cudaMemcpyAsync(e, si->ends.p, sizeof(S) * n, cudaMemcpyDeviceToHost, st));
     if (d) SI_CK(cudaMemcpyAsync(d, si->data.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
-    std::vector<int32_t> b32;
-    if (br) {
-        b32.resize(n);
-        SI_CK(cudaMemcpyAsync(b32.data(), si->branch.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    // branch entries as contig-local 64-bit positions: converted on the device, or, without room for
+    // that, in place (the 32-bit entries copied to the buffer's second half and widened from the
+    // first one on)
+    DevBuf b64;
+    const bool wide = br && b64.reserve(sizeof(int64_t) * n) == SI_OK;
+    if (wide) {
+        SI_CK(sig::launch_branch_local(si->branch.as<int32_t>(), si->seg.as<int64_t>(), si->G, n, b64.as<int64_t>(),
+                                       st));
+        SI_CK(cudaMemcpyAsync(br, b64.p, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st));
+    } else if (br) {
+        SI_CK(cudaMemcpyAsync(reinterpret_cast<int32_t*>(br) + n, si->branch.p, sizeof(int32_t) * n,
+                              cudaMemcpyDeviceToHost, st));
     }
     SI_CK(cudaStreamSynchronize(st));
-    if (br) {
+    if (br && !wide) {
         std::vector<int64_t> segv = si->hseg;
         if (segv.empty()) segv = {0, n};
+        const char* src = reinterpret_cast<const char*>(br) + sizeof(int32_t) * n;
         for (int g = 0; g < si->G; ++g)
-            for (int64_t i = segv[g]; i < segv[g + 1]; ++i) br[i] = b32[i] < 0 ? -1 : (int64_t)b32[i] - segv[g];
+            for (int64_t i = segv[g]; i < segv[g + 1]; ++i) {
+                int32_t b;
+                memcpy(&b, src + sizeof(int32_t) * i, sizeof(b));
+                br[i] = b < 0 ? -1 : (int64_t)b - segv[g];
+            }
     }
     return SI_OK;
 }

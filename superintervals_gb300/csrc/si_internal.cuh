@@ -169,8 +169,7 @@ cudaError_t launch_decode(const uint32_t* const* kw, const uint32_t* perm, const
 // Identity build (input already canonical): copy + pad.
 template <typename S>
 cudaError_t launch_copy_pad(const S* s_in, const S* e_in, const int32_t* d_in, int64_t n,
-                            int64_t n_pad, S* starts, S* ends, int32_t* data, uint32_t* perm,
-                            cudaStream_t st);
+                            int64_t n_pad, S* starts, S* ends, int32_t* data, cudaStream_t st);
 // Pyramid sizes: fills sizes[0..H] (sizes[0] = n_pad) and returns H.
 int pyramid_levels(int64_t n_pad, int64_t* sizes);
 template <typename S>
@@ -186,6 +185,9 @@ template <typename S>
 cudaError_t launch_long_scatter(const S* starts, const S* ends, int64_t n, int64_t X, const int64_t* offs,
                                 int64_t n_long, int64_t n_long_pad, const int64_t* seg, int G, int32_t* pos,
                                 S* lend, int64_t* long_seg, cudaStream_t st);
+// out[i] = branch[i] as a contig-local position (-1: none)
+cudaError_t launch_branch_local(const int32_t* branch, const int64_t* seg, int G, int64_t n, int64_t* out,
+                                cudaStream_t st);
 // flag = 1 when a[i] != b[i] for some i < n
 cudaError_t launch_differs_i32(const int32_t* a, const int32_t* b, int64_t n, int* flag, cudaStream_t st);
 // branch array: with temp (branch_temp_bytes(n_pad)) and an error word, one kernel with

@@ -189,6 +189,12 @@ class GpuIndex:
             raise ValueError("contig ids must match the query count")
         return qs, qe, qc
 
+    @staticmethod
+    def _first_capacity(nq: int) -> int:
+        """Result slots offered to the first call: a sparse result then takes one call of the
+        library, a larger one a second call with the size that the first one reported."""
+        return 4 * nq + 1024
+
     def count(self, qs, qe, qc=None) -> np.ndarray:
         qs, qe, qc = self._queries(qs, qe, qc)
         out = np.empty(qs.shape[0], np.uint32)
@@ -211,8 +217,8 @@ class GpuIndex:
         nq = qs.shape[0]
         off = np.empty(nq + 1, np.int64)
         total = C.c_size_t(0)
-        cap = 0
-        out = np.empty(1, np.int32)
+        cap = self._first_capacity(nq)
+        out = np.empty(cap, np.int32)
         for _ in range(2):
             st = self.lib.searchBatchIntoGpu(self.h, _p(qs), _p(qe), _p(qc), nq, int(order),
                                              1 if values else 0, _p(off), _p(out), cap,
@@ -230,8 +236,8 @@ class GpuIndex:
         nq = qs.shape[0]
         off = np.empty(nq + 1, np.int64)
         total = C.c_size_t(0)
-        cap = 0
-        bufs = (np.empty(1, self.dtype), np.empty(1, self.dtype), np.empty(1, np.int32))
+        cap = self._first_capacity(nq)
+        bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
         for _ in range(2):
             args = [self.h, _p(qs), _p(qe), _p(qc), nq, *extra, _p(off), _p(bufs[0]), _p(bufs[1])]
             if want_hits:
@@ -253,8 +259,8 @@ class GpuIndex:
         nq = qs.shape[0]
         off = np.empty(nq + 1, np.int64)
         total = C.c_size_t(0)
-        cap = 0
-        bufs = (np.empty(1, self.dtype), np.empty(1, self.dtype), np.empty(1, np.int32))
+        cap = self._first_capacity(nq)
+        bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
         for _ in range(2):
             st = self.lib.searchKeysBatchGpu(self.h, _p(qs), _p(qe), _p(qc), nq, int(order), _p(off), _p(bufs[0]),
                                              _p(bufs[1]), _p(bufs[2]) if with_data else None, cap,
