@@ -18,6 +18,7 @@
 #include "si_gpu/c_api.h"
 #include "si_internal.cuh"
 #include "si_batched.cuh"
+#include "si_rank.cuh"
 
 namespace {
 
@@ -155,6 +156,12 @@ struct gSuperIntervals {
     DevBuf long_lvl[sig::kMaxLevels];
     int64_t long_sizes[sig::kMaxLevels + 1] = {0};
     int long_H = 0;
+    // rank grids over the starts and, when no interval has start > end, over the sorted ends:
+    // contig records, then t1 and t2 words (si_rank.cuh); without them (no room under the device
+    // budget) the calls that use them take the sorted batch
+    DevBuf grid;
+    bool grid_starts = false, grid_ends = false;
+    size_t grid_at[2][3] = {{0, 0, 0}, {0, 0, 0}};  // byte offsets of [starts | ends][contigs, t1, t2]
     int sort_passes = 0;
     bool input_was_sorted = false;
     // query workspace
@@ -331,6 +338,49 @@ struct TempArena {
     }
 };
 
+// which 0: starts, 1: sorted ends
+template <typename S>
+sig::RankGrid<S> rank_grid(const gSuperIntervals* si, int which) {
+    const char* p = si->grid.as<char>();
+    sig::RankGrid<S> R;
+    R.arr = which ? si->end_sorted.as<S>() : si->starts.as<S>();
+    R.c = reinterpret_cast<const sig::GridContig*>(p + si->grid_at[which][0]);
+    R.t1 = reinterpret_cast<const uint32_t*>(p + si->grid_at[which][1]);
+    R.t2 = reinterpret_cast<const uint32_t*>(p + si->grid_at[which][2]);
+    return R;
+}
+
+// Rank grids of a built index's starts and sorted ends, in one allocation.  Queued on the handle's
+// stream; the caller synchronizes.  No room is no error: the index then works without them.
+template <typename S>
+int build_grids(gSuperIntervals* si, const std::vector<int64_t>& segv, std::vector<uint32_t>& base) {
+    si->grid_starts = si->grid_ends = false;
+    const int G = si->G, arrays = si->inverted == 0 ? 2 : 1;
+    base.resize(G);
+    const int64_t w1 = sig::grid_t1_words(segv.data(), G, base.data()), w2 = sig::grid_t2_words(si->n);
+    size_t at = (sizeof(uint32_t) * (size_t)G + 255) & ~(size_t)255;
+    const size_t parts[3] = {sizeof(sig::GridContig) * (size_t)G, sizeof(uint32_t) * (size_t)w1,
+                             sizeof(uint32_t) * (size_t)w2};
+    for (int a = 0; a < arrays; ++a)
+        for (int k = 0; k < 3; ++k) {
+            si->grid_at[a][k] = at;
+            at += (parts[k] + 255) & ~(size_t)255;
+        }
+    if (si->grid.reserve(at) != SI_OK) return SI_OK;
+    SI_CK(cudaMemcpyAsync(si->grid.p, base.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, si->st));
+    for (int a = 0; a < arrays; ++a) {
+        char* p = si->grid.as<char>();
+        SI_CK(sig::launch_grid_build<S>(rank_grid<S>(si, a).arr, si->n, si->seg.as<int64_t>(), G,
+                                        si->grid.as<uint32_t>(), w1,
+                                        reinterpret_cast<sig::GridContig*>(p + si->grid_at[a][0]),
+                                        reinterpret_cast<uint32_t*>(p + si->grid_at[a][1]),
+                                        reinterpret_cast<uint32_t*>(p + si->grid_at[a][2]), si->st));
+    }
+    si->grid_starts = true;
+    si->grid_ends = arrays == 2;
+    return SI_OK;
+}
+
 template <typename S>
 int build_impl(gSuperIntervals* si) {
     SI_TRY(set_dev(si));
@@ -349,6 +399,7 @@ int build_impl(gSuperIntervals* si) {
     si->bws.end_sorted = nullptr;
     si->cov_ready = false;
     si->rec_ready = false;
+    si->grid_starts = si->grid_ends = false;
     if (si->gexec) {              // a captured graph holds the old buffers
         cudaGraphExecDestroy(si->gexec);
         si->gexec = nullptr;
@@ -489,6 +540,8 @@ int build_impl(gSuperIntervals* si) {
         SI_CK(sig::launch_end_decode<S>(in_alt ? ka : kp, n, n_pad, si->end_sorted.as<S>(), st));
         si->bws.end_sorted = si->end_sorted.p;
     }
+    std::vector<uint32_t> grid_base;
+    SI_TRY(build_grids<S>(si, segv, grid_base));
     SI_TRY(sig::batched_prepare<S>(si->bws, view<S>(si), levels<S>(si), si->H, si->lvl_sizes,
                                    si->ub_mode, st));
     SI_CK(cudaStreamSynchronize(st));
@@ -533,18 +586,26 @@ bool use_batched(const gSuperIntervals* si, int64_t nq, bool emit = false) {
     return nq >= 4096 || (emit && si->long_depth >= kDeepLong);
 }
 
+// The automatic choice for counts, upper bounds and coverage: ranks from the grids, in the batch's
+// own order.  A caller that names the plain or the batched path gets that path.
+bool use_ranks(const gSuperIntervals* si) { return si->grid_ends && si->path == SI_PATH_AUTO; }
+
 // count into d_counts (device) for device-resident queries
 template <typename S>
 int run_count(gSuperIntervals* si, const sig::QueryBatch& q, uint32_t* d_counts, cudaStream_t st,
               bool for_emit = false) {
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
     if (si->n == 0) {
         SI_CK(cudaMemsetAsync(d_counts, 0, sizeof(uint32_t) * std::max<int64_t>(q.nq, 1), st));
         SI_CK(sig::launch_check_contigs(q.qc, q.nq, si->G, si->w_err.as<int>(), st));
         return SI_OK;
     }
-    if (use_batched(si, q.nq, for_emit)) {
+    if (!for_emit && use_ranks(si)) {
+        PhaseTimer pt(si, 0, st);
+        SI_CK(sig::launch_rank_count<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, d_counts,
+                                        si->w_err.as<int>(), st));
+    } else if (use_batched(si, q.nq, for_emit)) {
         {
             PhaseTimer pt(si, 3, st);
             int r = sig::batched_prepare_queries<S>(si->bws, view<S>(si), q, si->w_err.as<int>(), si->ub_mode, st,
@@ -767,7 +828,7 @@ int any_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, s
     if (nq && !out) return fail(SI_ERR_INVALID, "null output");
     sig::QueryBatch q;
     SI_TRY(upload_queries<S>(si, qs, qe, qc, nq, q));
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), si->st));
     if (si->n == 0) {
         memset(out, 0, nq);
@@ -1185,13 +1246,22 @@ extern "C" int upperBoundDeviceGpu(gSuperIntervals* si, const void* d_qe, const 
         return fail(SI_ERR_INVALID, "upper-bound mode %d is not prepared on this handle (current %d)", mode,
                     si->ub_mode);
     cudaStream_t st = stream ? (cudaStream_t)stream : si->st;
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
     if (si->n == 0) {
         if (nq) SI_CK(cudaMemsetAsync(d_out, 0xff, sizeof(int32_t) * nq, st));
         return SI_OK;
     }
     sig::QueryBatch q{d_qe, d_qe, d_qc, (int64_t)nq};
+    if (si->grid_starts && si->path == SI_PATH_AUTO) {
+        if (si->bits == 64)
+            SI_CK(sig::launch_rank_ub<int64_t>(rank_grid<int64_t>(si, 0), si->G, d_qe, d_qc, (int64_t)nq, d_out,
+                                               si->w_err.as<int>(), st));
+        else
+            SI_CK(sig::launch_rank_ub<int32_t>(rank_grid<int32_t>(si, 0), si->G, d_qe, d_qc, (int64_t)nq, d_out,
+                                               si->w_err.as<int>(), st));
+        return SI_OK;
+    }
     // the batched query path sorts the ends first (same answers): see setQueryPathGpu
     const bool sorted = use_batched(si, (int64_t)nq);
     int r = si->bits == 64
@@ -1633,7 +1703,7 @@ extern "C" int searchDeviceGraphGpu(gSuperIntervals* si, const void* d_qs, const
         return SI_OK;
     }
     // workspace first: nothing may be allocated while a capture is open
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * nq));
     SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
     // batched when the handle would take it for this batch and the key packs on the device
@@ -1710,7 +1780,7 @@ int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int orde
         SI_CK(cudaStreamSynchronize(st));
         return SI_OK;
     }
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     if (si->n > 0) {
         SI_TRY(hit_lists<S>(si, q, op == 0 ? order : SI_ORDER_DESC, st));
     } else {
@@ -1888,7 +1958,7 @@ namespace {
 // Hit lists of a device batch (so_hoff / so_hits); an empty index gives empty lists.
 template <typename S>
 int lists_or_empty(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStream_t st, int64_t* P) {
-    SI_TRY(si->w_err.reserve(sizeof(int)));
+    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     if (si->n > 0) {
         SI_TRY(hit_lists<S>(si, q, order, st));
         SI_CK(cudaMemcpyAsync(P, si->so_hoff.as<int64_t>() + q.nq, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -1938,51 +2008,65 @@ int keys_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_
     return SI_OK;
 }
 
+// Prefix sums of the starts and of the sorted ends, made on the first coverage call after a build.
+template <typename S>
+int cov_sums(gSuperIntervals* si, cudaStream_t st) {
+    if (si->cov_ready) return SI_OK;
+    SI_TRY(si->ps_start.reserve(sizeof(uint64_t) * (si->n + 1)));
+    SI_TRY(si->ps_end.reserve(sizeof(uint64_t) * (si->n + 1)));
+    DevBuf tmp;
+    SI_TRY(tmp.reserve(sig::scan_temp_bytes(si->n)));
+    if (sizeof(S) == 4) {
+        SI_CK(sig::exclusive_scan_i32_to_u64((const int32_t*)si->starts.p, si->ps_start.as<uint64_t>(), si->n, tmp.p,
+                                             st));
+        SI_CK(sig::exclusive_scan_i32_to_u64((const int32_t*)si->end_sorted.p, si->ps_end.as<uint64_t>(), si->n,
+                                             tmp.p, st));
+    } else {
+        SI_CK(sig::exclusive_scan_i64_to_u64((const int64_t*)si->starts.p, si->ps_start.as<uint64_t>(), si->n, tmp.p,
+                                             st));
+        SI_CK(sig::exclusive_scan_i64_to_u64((const int64_t*)si->end_sorted.p, si->ps_end.as<uint64_t>(), si->n,
+                                             tmp.p, st));
+    }
+    SI_CK(cudaStreamSynchronize(st));  // tmp is released on scope exit
+    si->cov_ready = true;
+    return SI_OK;
+}
+
 template <typename S>
 int coverage_device(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t* d_count, S* d_cov, cudaStream_t st) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
     if (q.nq && (!q.qs || !q.qe || !d_count || !d_cov)) return fail(SI_ERR_INVALID, "null device buffer");
     if (q.nq == 0) return SI_OK;
-    if (si->n > 0 && si->inverted == 0 && si->bws.end_sorted) {
+    if (si->n > 0 && si->inverted == 0 && si->bws.end_sorted && cov_sums<S>(si, st) == SI_OK) {
         // no interval has start > end: when no query has start > end either, the coverage comes
         // from ranks and prefix sums, without hit lists
-        sig::MapView<S> qv = view<S>(si);
-        qv.starts = static_cast<const S*>(q.qs);
-        qv.ends = static_cast<const S*>(q.qe);
-        qv.n = q.nq;
-        SI_TRY(si->so_flag.reserve(2 * sizeof(int)));
-        SI_CK(sig::launch_any_inverted<S>(qv, si->so_flag.as<int>() + 1, st));
+        SI_TRY(si->w_err.reserve(2 * sizeof(int)));
+        SI_CK(cudaMemsetAsync(si->w_err.p, 0, 2 * sizeof(int), st));
         int inv = 0;
-        SI_CK(cudaMemcpyAsync(&inv, si->so_flag.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        SI_CK(cudaStreamSynchronize(st));
-        if (!inv) {
-            if (!si->cov_ready) {
-                SI_TRY(si->ps_start.reserve(sizeof(uint64_t) * (si->n + 1)));
-                SI_TRY(si->ps_end.reserve(sizeof(uint64_t) * (si->n + 1)));
-                DevBuf tmp;
-                SI_TRY(tmp.reserve(sig::scan_temp_bytes(si->n)));
-                if (sizeof(S) == 4) {
-                    SI_CK(sig::exclusive_scan_i32_to_u64((const int32_t*)si->starts.p, si->ps_start.as<uint64_t>(),
-                                                         si->n, tmp.p, st));
-                    SI_CK(sig::exclusive_scan_i32_to_u64((const int32_t*)si->end_sorted.p,
-                                                         si->ps_end.as<uint64_t>(), si->n, tmp.p, st));
-                } else {
-                    SI_CK(sig::exclusive_scan_i64_to_u64((const int64_t*)si->starts.p, si->ps_start.as<uint64_t>(),
-                                                         si->n, tmp.p, st));
-                    SI_CK(sig::exclusive_scan_i64_to_u64((const int64_t*)si->end_sorted.p,
-                                                         si->ps_end.as<uint64_t>(), si->n, tmp.p, st));
-                }
-                SI_CK(cudaStreamSynchronize(st));  // tmp is released on scope exit
-                si->cov_ready = true;
+        int* d_inv = si->w_err.as<int>() + 1;
+        if (use_ranks(si)) {
+            SI_CK(sig::launch_rank_coverage<S>(rank_grid<S>(si, 0), rank_grid<S>(si, 1), si->G, q,
+                                               si->ps_start.as<uint64_t>(), si->ps_end.as<uint64_t>(), d_count, d_cov,
+                                               si->w_err.as<int>(), d_inv, st));
+            SI_CK(cudaMemcpyAsync(&inv, d_inv, sizeof(int), cudaMemcpyDeviceToHost, st));
+            SI_TRY(read_dev_err(si, st));
+            if (!inv) return SI_OK;  // else some answers are missing: all come from the hit lists
+        } else {
+            sig::MapView<S> qv = view<S>(si);
+            qv.starts = static_cast<const S*>(q.qs);
+            qv.ends = static_cast<const S*>(q.qe);
+            qv.n = q.nq;
+            SI_CK(sig::launch_any_inverted<S>(qv, d_inv, st));
+            SI_CK(cudaMemcpyAsync(&inv, d_inv, sizeof(int), cudaMemcpyDeviceToHost, st));
+            SI_CK(cudaStreamSynchronize(st));
+            if (!inv) {
+                const int r = sig::batched_coverage<S>(si->bws, view<S>(si), q, si->ps_start.as<uint64_t>(),
+                                                       si->ps_end.as<uint64_t>(), d_count, d_cov, si->w_err.as<int>(),
+                                                       si->ub_mode, st);
+                if (r != SI_OK) return fail(r, "coverage from ranks failed (status %d)", r);
+                return read_dev_err(si, st);
             }
-            SI_TRY(si->w_err.reserve(sizeof(int)));
-            SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
-            const int r = sig::batched_coverage<S>(si->bws, view<S>(si), q, si->ps_start.as<uint64_t>(),
-                                                   si->ps_end.as<uint64_t>(), d_count, d_cov, si->w_err.as<int>(),
-                                                   si->ub_mode, st);
-            if (r != SI_OK) return fail(r, "coverage from ranks failed (status %d)", r);
-            return read_dev_err(si, st);
         }
     }
     int64_t P = 0;

@@ -1,0 +1,165 @@
+// si_rank.cuh -- rank grid: the rank of a key in each contig's ascending coordinates in about four
+// dependent reads, for queries in any order.
+//
+// Counts, upper bounds and coverage need only ranks (how many starts / sorted ends lie below a
+// key).  A halving search makes log2(n) dependent reads per rank, and sorting the batch first, so
+// that neighbours share a search window, costs three radix passes, a gather and a scattered write.
+// The grid cuts each contig's coordinate range into power-of-two wide buckets, 4-8 entries each on
+// average (table t1: first position of every bucket), so that a rank is one read of two adjacent
+// table words and a search over the few entries between them.  Where coordinates crowd, a bucket of
+// kGridDense entries or more is cut again, by its own count, in table t2; its words sit at 3/8 of
+// the bucket's first position, so that no second index is needed (a bucket of n entries uses at
+// most n/4 + 1 words).  Any bucket still crowded after that is searched by halving: the answer is
+// exact for every distribution, only the number of reads changes.
+// Memory: 2.5 bytes per entry and array (t1 1, t2 1.5), beside 4 or 8 for the coordinates.
+#pragma once
+#include "si_internal.cuh"
+
+namespace sig {
+
+constexpr uint32_t kGridFill = 4;    // at most n / kGridFill buckets: 4-8 entries a bucket
+constexpr uint32_t kGridDense = 32;  // entries from which a bucket has its own table (>= 24: see above)
+constexpr int kGridSubBits = 10;     // at most 1024 words of t2 per bucket
+
+struct alignas(32) GridContig {
+    int64_t k0;       // smallest key of the contig
+    uint32_t lo, hi;  // its positions
+    uint32_t base;    // its first word in t1 (nb + 1 words: the last one is hi)
+    uint32_t nb;      // buckets (0: empty contig)
+    uint32_t shift;   // bucket width 2^shift
+    uint32_t pad;
+};
+
+template <typename S>
+struct RankGrid {
+    const S* arr = nullptr;          // ascending inside each contig
+    const GridContig* c = nullptr;
+    const uint32_t* t1 = nullptr;
+    const uint32_t* t2 = nullptr;
+};
+
+__device__ __forceinline__ GridContig load_contig(const GridContig* __restrict__ p) {
+    const int4* q = reinterpret_cast<const int4*>(p);
+    const int4 a = __ldg(q), b = __ldg(q + 1);
+    GridContig c;
+    c.k0 = (int64_t)(((uint64_t)(uint32_t)a.y << 32) | (uint32_t)a.x);
+    c.lo = (uint32_t)a.z;
+    c.hi = (uint32_t)a.w;
+    c.base = (uint32_t)b.x;
+    c.nb = (uint32_t)b.y;
+    c.shift = (uint32_t)b.z;
+    c.pad = 0;
+    return c;
+}
+
+// log2 of the sub-buckets of a bucket holding cnt >= kGridDense entries
+__device__ __forceinline__ int grid_sub_bits(uint32_t cnt, uint32_t shift) {
+    const int k = 31 - __clz(cnt >> 2);
+    return min(min(k, (int)shift), kGridSubBits);
+}
+__device__ __forceinline__ uint32_t grid_sub_base(uint32_t first) { return (uint32_t)((3ull * first + 7) >> 3); }
+
+// The positions [a, a + len) among which the first entry >= v of the contig lies (a + len when none
+// of them is): len is 0 where the tables alone give the answer.
+template <typename S>
+__device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridContig& c, S v, uint32_t& a,
+                                             uint32_t& len) {
+    a = c.lo;
+    len = 0;
+    if (c.nb == 0 || (int64_t)v <= c.k0) return;
+    const uint64_t d = (uint64_t)(int64_t)v - (uint64_t)c.k0;
+    const uint64_t b = d >> c.shift;
+    if (b >= c.nb) {
+        a = c.hi;
+        return;
+    }
+    const uint32_t* t = R.t1 + c.base + (uint32_t)b;
+    a = __ldg(t);
+    const uint32_t cnt = __ldg(t + 1) - a;
+    len = cnt;
+    if (cnt >= kGridDense) {
+        const int k = grid_sub_bits(cnt, c.shift);
+        const int ss = (int)c.shift - k;
+        const uint32_t r = (uint32_t)(d >> ss) & ((1u << k) - 1u);
+        const uint32_t* t2 = R.t2 + grid_sub_base(a) + r;
+        a = __ldg(t2);
+        len = __ldg(t2 + 1) - a;
+        if (ss == 0) len = 0;  // one coordinate wide: every entry equals v, the first one is the answer
+    }
+}
+
+// First position of the contig with arr >= v (its end when none).
+template <typename S>
+__device__ __forceinline__ uint32_t grid_first_geq(const RankGrid<S>& R, const GridContig& c, S v) {
+    uint32_t a, len;
+    grid_bracket(R, c, v, a, len);
+    while (len > 0) {
+        const uint32_t half = len >> 1;
+        const bool below = __ldg(R.arr + a + half) < v;
+        a = below ? a + half + 1 : a;
+        len = below ? len - half - 1 : half;
+    }
+    return a;
+}
+
+// First position with arr > v.
+template <typename S>
+__device__ __forceinline__ uint32_t grid_first_gt(const RankGrid<S>& R, const GridContig& c, S v) {
+    return v == Lim<S>::hi ? c.hi : grid_first_geq<S>(R, c, (S)(v + 1));
+}
+
+// first_gt(v1) in one array and first_geq(v2) in another, their reads side by side.
+template <typename S>
+__device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const GridContig& c1, S v1,
+                                               const RankGrid<S>& R2, const GridContig& c2, S v2, uint32_t& r1,
+                                               uint32_t& r2) {
+    uint32_t a1, l1, a2, l2;
+    const bool top = v1 == Lim<S>::hi;
+    const S w1 = top ? v1 : (S)(v1 + 1);
+    grid_bracket(R1, c1, w1, a1, l1);
+    grid_bracket(R2, c2, v2, a2, l2);
+    while ((l1 | l2) != 0u) {
+        const uint32_t h1 = l1 >> 1, h2 = l2 >> 1;
+        S x1 = Lim<S>::hi, x2 = Lim<S>::hi;
+        if (l1) x1 = __ldg(R1.arr + a1 + h1);
+        if (l2) x2 = __ldg(R2.arr + a2 + h2);
+        if (l1) {
+            const bool below = x1 < w1;
+            a1 = below ? a1 + h1 + 1 : a1;
+            l1 = below ? l1 - h1 - 1 : h1;
+        }
+        if (l2) {
+            const bool below = x2 < v2;
+            a2 = below ? a2 + h2 + 1 : a2;
+            l2 = below ? l2 - h2 - 1 : h2;
+        }
+    }
+    r1 = top ? c1.hi : a1;
+    r2 = a2;
+}
+
+// ---------------------------------------------------------------- launchers (si_rank.cu)
+// Words of t1 for contigs of these sizes (fills base[g]), and of t2 for n entries.
+int64_t grid_t1_words(const int64_t* seg, int G, uint32_t* base);
+inline int64_t grid_t2_words(int64_t n) { return (3 * n + 7) / 8 + 8; }
+// Builds the tables over arr (ascending inside each contig): d_base holds grid_t1_words' bases.
+template <typename S>
+cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G, const uint32_t* d_base,
+                              int64_t t1_words, GridContig* c, uint32_t* t1, uint32_t* t2, cudaStream_t st);
+
+// Counts of a batch in its own order, for an index without intervals with start > end.
+template <typename S>
+cudaError_t launch_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, uint32_t* counts,
+                              int* d_err, cudaStream_t st);
+// Contig-local upper bounds (-1: none) of every query end.
+template <typename S>
+cudaError_t launch_rank_ub(RankGrid<S> gs, int G, const void* qe, const int32_t* qc, int64_t nq, int32_t* out,
+                           int* d_err, cudaStream_t st);
+// Coverage from ranks and prefix sums (see launch site); *d_inv is set when a query has start > end
+// (its answer is not written).
+template <typename S>
+cudaError_t launch_rank_coverage(RankGrid<S> gs, RankGrid<S> ge, int G, QueryBatch q, const uint64_t* ps_start,
+                                 const uint64_t* ps_end, uint64_t* count, S* cov, int* d_err, int* d_inv,
+                                 cudaStream_t st);
+
+}  // namespace sig

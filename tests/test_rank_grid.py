@@ -1,0 +1,119 @@
+"""Counts, upper bounds and coverage from the rank grid against numpy ranks, at the shapes where the
+grid's buckets can go wrong: crowded and one-coordinate buckets, huge gaps, type extremes, empty and
+one-interval contigs, keys at and beside every bucket edge, queries with start > end."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api():
+    from superintervals_gb300 import interval_map
+    return interval_map
+
+
+def _starts(rng, kind, n, dt):
+    info = np.iinfo(dt)
+    if kind == "uniform":
+        return rng.integers(0, 50 * n + 1, n)
+    if kind == "duplicates":                    # one-coordinate buckets of many equal keys
+        return rng.choice(np.array([5, 6, 900, 70_000]), n)
+    if kind == "gap":                           # nearly all keys in one bucket, one far away
+        s = rng.integers(0, 200, n)
+        s[0] = info.max - 10
+        return s
+    if kind == "extremes":                      # the whole coordinate range
+        s = rng.integers(info.min // 2, info.max // 2, n)
+        s[: n // 3] = info.min
+        s[n // 3: n // 2] = info.max
+        return s
+    s = rng.integers(0, 10_000_000, n)          # "clustered": sub-tables with entries left to search
+    hot = rng.random(n) < 0.8
+    s[hot] = 4_000_000 + np.rint(rng.standard_normal(int(hot.sum())) * 3000).astype(np.int64)
+    return s
+
+
+def _case(kind, n, dt, seed):
+    rng = np.random.default_rng(seed)
+    info = np.iinfo(dt)
+    s = _starts(rng, kind, n, dt).astype(np.int64)
+    room = np.array([info.max - int(x) for x in s], dtype=np.float64)
+    ln = np.minimum(rng.integers(0, 3000, n), room).astype(np.int64)
+    e = s + ln
+    # contigs: an empty one first, one interval, the rest split in two, an empty one last
+    cut = sorted({0, min(1, n), (n + 1) // 2, n})
+    seg = np.array([0] + cut + [n], dtype=np.int64)
+    G = len(seg) - 1
+    # queries on, beside and between the keys, in every contig, some with start > end
+    near = rng.choice(np.concatenate([s, e]), 3000)
+    qs = np.array([min(max(int(v) + int(d), info.min), info.max) for v, d in zip(near, rng.integers(-2, 3, 3000))])
+    qe = np.array([min(int(v) + int(d), info.max) for v, d in zip(qs, rng.choice([0, 1, 40, 5000], 3000))])
+    qe[:50], qs[:50] = qs[:50].copy(), qe[:50].copy()
+    qs[50:60], qe[50:60] = info.min, info.max
+    qc = rng.integers(0, G, 3000)
+    return s.astype(dt), e.astype(dt), seg, qs.astype(dt), qe.astype(dt), qc.astype(np.int32)
+
+
+def _expected(s, e, seg, qs, qe, qc):
+    ub = np.full(len(qs), -1, np.int64)
+    cnt = np.zeros(len(qs), np.int64)
+    for g in range(len(seg) - 1):
+        a, b = s[seg[g]:seg[g + 1]], e[seg[g]:seg[g + 1]]
+        sel = np.flatnonzero(qc == g)
+        ub[sel] = np.searchsorted(np.sort(a), qe[sel], side="right") - 1
+        cnt[sel] = [int(((a <= y) & (b >= x)).sum()) for x, y in zip(qs[sel], qe[sel])]
+    return ub, cnt
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+@pytest.mark.parametrize("n", [1, 2, 7, 33, 1000, 4097])
+@pytest.mark.parametrize("kind", ["uniform", "duplicates", "gap", "extremes", "clustered"])
+def test_ranks_match_numpy(api, kind, n, dt):
+    s, e, seg, qs, qe, qc = _case(kind, n, dt, seed=n)
+    ub, cnt = _expected(s, e, seg, qs, qe, qc)
+    idx = api.GpuIndex(np.dtype(dt).itemsize * 8)
+    idx.add_arrays(s, e, seg=seg)
+    idx.build()
+    assert np.array_equal(idx.count(qs, qe, qc), cnt)
+    lib, nq = idx.lib, len(qs)
+    d = []
+    for a in (qe, qc, np.zeros(nq, np.int32)):
+        p = C.c_void_p()
+        api.check(lib.deviceMallocGpu(C.byref(p), a.nbytes))
+        api.check(lib.memcpyGpu(p, C.c_void_p(a.ctypes.data), a.nbytes, idx.stream))
+        d.append(p)
+    api.check(lib.upperBoundDeviceGpu(idx.h, d[0], d[1], nq, 0, d[2], None))
+    got = np.empty(nq, np.int32)
+    api.check(lib.memcpyGpu(C.c_void_p(got.ctypes.data), d[2], got.nbytes, idx.stream))
+    api.check(lib.streamSynchronizeGpu(idx.stream))
+    assert np.array_equal(got, ub)
+    for p in d:
+        lib.deviceFreeGpu(p)
+    # coverage, with and without queries that have start > end, in the wrapping coordinate type
+    for sel in (np.flatnonzero(qs <= qe)[:400], np.arange(400)):
+        c2, cov = idx.coverage(qs[sel], qe[sel], qc[sel])
+        assert np.array_equal(c2, cnt[sel])
+        for k, i in enumerate(sel[::13]):
+            a, b = (v[seg[qc[i]]:seg[qc[i] + 1]].astype(object) for v in (s, e))
+            hit = [(x, y) for x, y in zip(a, b) if x <= int(qe[i]) and y >= int(qs[i])]
+            want = sum(min(int(y), int(qe[i])) - max(int(x), int(qs[i])) for x, y in hit)
+            bits = np.dtype(dt).itemsize * 8
+            want = (want + (1 << (bits - 1))) % (1 << bits) - (1 << (bits - 1))
+            assert int(cov[13 * k]) == want
+    idx.close()
+
+
+def test_count_paths_agree(api):
+    s, e, seg, qs, qe, qc = _case("uniform", 4097, np.int32, seed=5)
+    _, cnt = _expected(s, e, seg, qs, qe, qc)
+    idx = api.GpuIndex(32)
+    idx.add_arrays(s, e, seg=seg)
+    idx.build()
+    assert np.array_equal(idx.count(qs, qe, qc), cnt)
+    for path in (api.PATH_PLAIN, api.PATH_BATCHED):
+        idx.set_path(path)
+        assert np.array_equal(idx.count(qs, qe, qc), cnt)
+    idx.close()
