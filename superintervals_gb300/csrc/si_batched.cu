@@ -681,10 +681,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_tiles(TileArgs<S> a) {
                     // a list ending past the output (a replayed graph with too small a capacity,
                     // reported by the caller) is not written
                     q_cap[i] = (o1 - a.out_base <= a.out_cap) ? (int32_t)(o1 - o) : -1;
-                    // queries counted from ranks have no head run from the count pass: the emit
-                    // finds it (-1)
-                    const bool counted_by_rank = a.end_sorted && !code_is_inverted(q_c[i], a.G);
-                    q_h[i] = counted_by_rank ? -1 : a.heads_in[id];
+                    // without intervals with start > end, counts come from ranks and the emit finds
+                    // the head run itself (-1)
+                    q_h[i] = a.end_sorted ? -1 : a.heads_in[id];
                 }
             }
         }
@@ -1549,6 +1548,142 @@ __global__ void __launch_bounds__(kThreads, 6) k_qprep(const uint32_t* __restric
     sq_id[j] = (int32_t)orig;
 }
 
+// ---- sorted records from the queries' upper bounds -------------------------------------
+// With every query's upper bound known (su), its position orders the batch: contigs are laid out
+// one after another, so no contig code and no smallest / largest end are needed, and the number of
+// key bits follows from the sizes alone (no host round trip, the sort runs exactly those passes).
+// Key: class (0 short, 1 long or start > end, 2 no start at or below the query's end) above
+// (position >> shift) + contig, which grows along a contig and differs between contigs, so that the
+// queries of one class and contig stay together.  Also writes (start, su) interleaved and counts
+// the key's `digits` low bytes.
+template <typename S>
+__global__ void __launch_bounds__(kThreads) k_pos_keys(const S* __restrict__ qs, const S* __restrict__ qe,
+                                                       const int32_t* __restrict__ qc,
+                                                       const uint32_t* __restrict__ su, int64_t nq, int64_t long_len,
+                                                       int shift, int pos_bits, int digits,
+                                                       uint32_t* __restrict__ key,
+                                                       uint32_t* __restrict__ pay, S* __restrict__ qpair,
+                                                       uint32_t* __restrict__ ghist) {
+    constexpr int U = 4;
+    __shared__ uint32_t h[4 * 256];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 4 * 256; i += kThreads) h[i] = 0;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * kThreads * U;
+    for (int64_t q0 = (int64_t)blockIdx.x * kThreads * U + tid; q0 < nq; q0 += stride) {
+        S s[U], e[U];
+        uint32_t up[U], g[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t q = q0 + u * kThreads;
+            s[u] = e[u] = 0;
+            up[u] = g[u] = 0;
+            if (q < nq) {
+                s[u] = qs[q];
+                e[u] = qe[q];
+                up[u] = su[q];
+                if (qc) g[u] = (uint32_t)qc[q];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t q = q0 + u * kThreads;
+            if (q >= nq) continue;
+            const bool is_long = s[u] > e[u] || ((double)e[u] - (double)s[u] + 1.0) > (double)long_len;
+            const uint32_t cls = up[u] == 0 ? 2u : is_long ? 1u : 0u;
+            const uint32_t k = (cls << pos_bits) | (up[u] == 0 ? 0u : ((up[u] - 1u) >> shift) + g[u]);
+            key[q] = k;
+            pay[q] = (uint32_t)q;
+            if constexpr (sizeof(S) == 4) {
+                reinterpret_cast<int2*>(qpair)[q] = make_int2((int)s[u], (int)up[u]);
+            } else {
+                reinterpret_cast<longlong2*>(qpair)[q] = make_longlong2((long long)s[u], (long long)up[u]);
+            }
+            for (int d = 0; d < digits; ++d) atomicAdd(&h[256 * d + ((k >> (8 * d)) & 255u)], 1u);
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < 256 * digits; i += kThreads)
+        if (h[i]) atomicAdd(&ghist[i], h[i]);
+}
+
+// The sorted records, in the form of k_qprep's: start, upper bound (-1: none), class code and id;
+// and each block's cut for the tile of its 256 queries.
+template <typename S>
+__global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restrict__ pay,
+                                                       const uint32_t* __restrict__ key, int pos_bits,
+                                                       const S* __restrict__ qpair, int64_t nq, MapView<S> m,
+                                                       RankGrid<S> gs, S* __restrict__ sq_s,
+                                                       int32_t* __restrict__ sq_u, uint32_t* __restrict__ sq_c,
+                                                       int32_t* __restrict__ sq_id, int64_t long_split,
+                                                       const int32_t* __restrict__ long_pos,
+                                                       const int64_t* __restrict__ long_seg,
+                                                       int64_t* __restrict__ blk_cut) {
+    __shared__ S s_mn[kWarpsPerCta];
+    __shared__ uint32_t s_code[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t jb = (int64_t)blockIdx.x * kThreads, j = jb + tid;
+    const int64_t jl = (jb + kThreads < nq ? jb + kThreads : nq) - 1;
+    const bool valid = j < nq;
+    uint32_t code = 0;
+    S vs = Lim<S>::hi;
+    if (valid) {
+        const uint32_t id = pay[j], cls = key[j] >> pos_bits;
+        uint32_t up;
+        if constexpr (sizeof(S) == 4) {
+            const int2 r = reinterpret_cast<const int2*>(qpair)[id];
+            vs = r.x;
+            up = (uint32_t)r.y;
+        } else {
+            const longlong2 r = reinterpret_cast<const longlong2*>(qpair)[id];
+            vs = r.x;
+            up = (uint32_t)r.y;
+        }
+        code = 3u * (uint32_t)m.G;
+        if (cls < 2u) {
+            int g = 0;
+            for (int hi = m.G - 1; g < hi;) {  // largest g with seg[g] < up
+                const int mid = (g + hi + 1) >> 1;
+                if (m.seg[mid] < (int64_t)up) g = mid;
+                else hi = mid - 1;
+            }
+            code = cls * (uint32_t)m.G + (uint32_t)g;
+        }
+        sq_s[j] = vs;
+        sq_u[j] = (int32_t)up - 1;
+        sq_c[j] = code;
+        sq_id[j] = (int32_t)id;
+    }
+    if (!blk_cut) return;
+    // the tile's cut: the first position whose start is within long_split of its smallest query
+    // start, and the first long-list index at or after it
+    S mn = vs;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const S o = __shfl_xor_sync(kFull, mn, d);
+        mn = o < mn ? o : mn;
+    }
+    if (lane == 0) s_mn[warp] = mn;
+    if (j == jb) s_code[0] = code;
+    if (j == jl) s_code[1] = code;
+    __syncthreads();
+    if (warp == 0) {
+        int64_t pc = -1, ch = -1;
+        if (s_code[0] == s_code[1] && s_code[0] < (uint32_t)m.G) {
+            S L = s_mn[0];
+#pragma unroll
+            for (int w = 1; w < kWarpsPerCta; ++w) L = s_mn[w] < L ? s_mn[w] : L;
+            const int g = (int)s_code[0];
+            pc = (int64_t)grid_first_geq<S>(gs, load_contig(gs.c + g), near_threshold<S>(L, long_split));
+            ch = warp_first_pos_geq(long_pos, long_seg[g], long_seg[g + 1], pc, lane);
+        }
+        if (lane == 0) {
+            blk_cut[2 * blockIdx.x] = pc;
+            blk_cut[2 * blockIdx.x + 1] = ch;
+        }
+    }
+}
+
 // First index k in [lo, hi) of the ascending array arr with arr[k] >= key (strict: > key), for
 // every thread's key of a block of 256 sorted queries.  A uniform block (one contig, keys
 // close together) finds the ranks of its smallest and largest key with one warp each, stages
@@ -2107,6 +2242,61 @@ int batched_prepare_queries(BatchedWorkspace& ws, MapView<S> m, const QueryBatch
 }
 
 template <typename S>
+int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>& gs, const QueryBatch& q,
+                           const uint32_t* su, int* d_err, int ub_mode, cudaStream_t st) {
+    const int64_t nq = q.nq;
+    ws.prepared_nq = -1;
+    if (nq <= 0) return SI_OK;
+    if (nq >= (int64_t)INT32_MAX) return SI_ERR_TOO_LARGE;
+    SI_OKR(ws.kw[0].reserve(sizeof(uint32_t) * nq));
+    SI_OKR(ws.kalt[0].reserve(sizeof(uint32_t) * nq));
+    SI_OKR(ws.pay.reserve(sizeof(uint32_t) * nq));
+    SI_OKR(ws.palt.reserve(sizeof(uint32_t) * nq));
+    const size_t tb = radix_temp_bytes(nq, 1);
+    SI_OKR(ws.sort_tmp.reserve(tb));
+    SI_OKR(ws.sq_s.reserve(sizeof(S) * nq));
+    SI_OKR(ws.sq_u.reserve(sizeof(int32_t) * nq));
+    SI_OKR(ws.sq_c.reserve(sizeof(uint32_t) * nq));
+    SI_OKR(ws.sq_id.reserve(sizeof(int32_t) * nq));
+    SI_OKR(ws.qpair.reserve(2 * sizeof(S) * nq));
+    SI_OKR(ws.blk_cut.reserve(2 * sizeof(int64_t) * (size_t)nblk(nq)));
+    // two radix passes (14 position bits) while they leave at most 64 queries on average to a key,
+    // a quarter of a tile; else three (22 bits); four where the contigs alone would fill half of them
+    int digits = nq <= ((int64_t)64 << 14) ? 2 : 3;
+    while (digits < 4 && (int64_t)m.G > ((int64_t)1 << (8 * digits - 3))) ++digits;
+    const int pos_bits = 8 * digits - 2;
+    int shift = 0;
+    while (((m.n - 1) >> shift) + m.G > ((int64_t)1 << pos_bits)) ++shift;
+    uint32_t* kp[1] = {ws.kw[0].as<uint32_t>()};
+    uint32_t* ka[1] = {ws.kalt[0].as<uint32_t>()};
+    SI_CU(cudaMemsetAsync(radix_hist(ws.sort_tmp.p), 0, sizeof(uint32_t) * 4 * 256, st));
+    const int64_t kb = resident_blocks(reinterpret_cast<const void*>(&k_pos_keys<S>), kThreads);
+    k_pos_keys<S><<<(unsigned)std::min<int64_t>(nblk(nq, 4 * kThreads), kb), kThreads, 0, st>>>(
+        static_cast<const S*>(q.qs), static_cast<const S*>(q.qe), q.qc, su, nq, ws.prm.long_len, shift, pos_bits,
+        digits, kp[0],
+        ws.pay.as<uint32_t>(), ws.qpair.as<S>(), radix_hist(ws.sort_tmp.p));
+    note_launch();
+    SI_CU(cudaGetLastError());
+    bool in_alt = false;
+    int passes = 0;
+    SI_CU(radix_sort(kp, ka, ws.pay.as<uint32_t>(), ws.palt.as<uint32_t>(), 1, nq, ws.sort_tmp.p, tb, &in_alt,
+                     &passes, st, (1u << digits) - 1u, d_err, true));
+    k_pos_prep<S><<<nblk(nq), kThreads, 0, st>>>(
+        in_alt ? ws.palt.as<uint32_t>() : ws.pay.as<uint32_t>(), in_alt ? ka[0] : kp[0], pos_bits, ws.qpair.as<S>(),
+        nq, m, gs, ws.sq_s.as<S>(), ws.sq_u.as<int32_t>(), ws.sq_c.as<uint32_t>(), ws.sq_id.as<int32_t>(),
+        ws.long_split, ws.long_pos, ws.long_seg, ws.long_pos ? ws.blk_cut.as<int64_t>() : nullptr);
+    note_launch();
+    SI_CU(cudaGetLastError());
+    ws.launches += 2 + passes + 1;
+    ws.prepared_qs = q.qs;
+    ws.prepared_nq = nq;
+    ws.prepared_mode = ub_mode;
+    ws.n_heads = nq;      // no head runs are kept (the emit finds them)
+    ws.cache_ok = false;  // and no candidate lists
+    return SI_OK;
+}
+
+template <typename S>
 static int run_tiles(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, int64_t nq, bool emit,
                      uint32_t* counts, int32_t* heads, const int32_t* heads_in, const int64_t* offsets,
                      int64_t out_base, int order, bool values, int32_t* out, int* d_err, bool use_cache,
@@ -2297,6 +2487,8 @@ int batched_coverage(BatchedWorkspace& ws, MapView<S> m, const QueryBatch& q, co
                                     cudaStream_t);                                                              \
     template int batched_prepare_queries<S>(BatchedWorkspace&, MapView<S>, const QueryBatch&, int*, int,          \
                                             cudaStream_t, uint32_t*, bool);                                                \
+    template int batched_prepare_ranked<S>(BatchedWorkspace&, MapView<S>, const RankGrid<S>&, const QueryBatch&,  \
+                                           const uint32_t*, int*, int, cudaStream_t);                            \
     template int batched_count<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const QueryBatch&, uint32_t*,   \
                                   int*, cudaStream_t);                                                          \
     template int batched_emit<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const QueryBatch&, int64_t,      \

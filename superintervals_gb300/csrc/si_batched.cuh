@@ -1,6 +1,7 @@
 // si_batched.cuh -- the BATCHED query path (sorted-query tiles).
 #pragma once
 #include "si_internal.cuh"
+#include "si_rank.cuh"
 
 namespace sig {
 
@@ -62,7 +63,8 @@ struct BatchedWorkspace {
     UpperBoundModel ub;
     // query sort
     DBuf kw[3], kalt[3], pay, palt, sort_tmp;
-    DBuf qpair;                  // (start, end) per query, interleaved: one sector per gather
+    DBuf qpair;                  // (start, end) or (start, upper bound) per query, interleaved: one
+                                 // sector per gather
     DBuf blk_cut;                // per 256 sorted queries: (p_cut, long-list end) or -1, for the tiles
     DBuf qminmax;                // smallest and largest query end (key packing)
     // sorted query records
@@ -123,6 +125,11 @@ int batched_prepare(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, cons
 template <typename S>
 int batched_prepare_queries(BatchedWorkspace& ws, MapView<S> m, const QueryBatch& q, int* d_err,
                             int ub_mode, cudaStream_t st, uint32_t* counts = nullptr, bool tile_cuts = true);
+// The same sorted records from the queries' upper bounds (su, launch_rank_scan): sorted by (class,
+// position), without a host round trip.  The batch is counted already; emit it next.
+template <typename S>
+int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>& gs, const QueryBatch& q,
+                           const uint32_t* su, int* d_err, int ub_mode, cudaStream_t st);
 template <typename S>
 int batched_count(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, const QueryBatch& q,
                   uint32_t* counts, int* d_err, cudaStream_t st);

@@ -8,7 +8,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <iterator>
 #include <mutex>
@@ -165,7 +167,9 @@ struct gSuperIntervals {
     int sort_passes = 0;
     bool input_was_sorted = false;
     // query workspace
-    DevBuf wq_s, wq_e, wq_c, w_counts, w_offsets, w_out, w_tmp, w_err;
+    DevBuf wq_s, wq_e, wq_c, w_counts, w_offsets, w_out, w_tmp;
+    DevBuf w_err;    // device error word; the rank searches' whole work record (sig::RankWork)
+    DevBuf w_upper;  // rank searches: each query's upper bound
     // host-buffer searches of several chunks: a second result buffer and a copy stream, so
     // that the emit of one chunk overlaps the device-to-host copy of the previous one
     DevBuf w_out2;
@@ -561,17 +565,21 @@ int check_built(const gSuperIntervals* si) {
     return SI_OK;
 }
 
+int dev_status(const gSuperIntervals* si, int e) {
+    if (e == sig::kDevBadContig) return fail(SI_ERR_INVALID, "a query names a contig outside [0, %d)", si->G);
+    if (e == sig::kDevOverflow) return fail(SI_ERR_CUDA, "internal: emit overran its offsets");
+    if (e == sig::kDevTimeout) return fail(SI_ERR_CUDA, "a bounded wait in a sort or scan kernel gave up");
+    if (e != 0) return fail(SI_ERR_CUDA, "device error word %d", e);
+    return SI_OK;
+}
+
 // Reads the device error word after the work queued on `st` (the handle's stream by default).
 int read_dev_err(gSuperIntervals* si, cudaStream_t st = nullptr) {
     if (!st) st = si->st;
     int e = 0;
     SI_CK(cudaMemcpyAsync(&e, si->w_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
-    if (e == sig::kDevBadContig) return fail(SI_ERR_INVALID, "a query names a contig outside [0, %d)", si->G);
-    if (e == sig::kDevOverflow) return fail(SI_ERR_CUDA, "internal: emit overran its offsets");
-    if (e == sig::kDevTimeout) return fail(SI_ERR_CUDA, "a bounded wait in a sort or scan kernel gave up");
-    if (e != 0) return fail(SI_ERR_CUDA, "device error word %d", e);
-    return SI_OK;
+    return dev_status(si, e);
 }
 
 // The automatic choice: the batched path for batches of 4096+ queries; for smaller ones the plain
@@ -588,7 +596,13 @@ bool use_batched(const gSuperIntervals* si, int64_t nq, bool emit = false) {
 
 // The automatic choice for counts, upper bounds and coverage: ranks from the grids, in the batch's
 // own order.  A caller that names the plain or the batched path gets that path.
-bool use_ranks(const gSuperIntervals* si) { return si->grid_ends && si->path == SI_PATH_AUTO; }
+bool use_ranks(const gSuperIntervals* si, int64_t nq) {
+    return si->grid_ends && si->path == SI_PATH_AUTO && nq < (int64_t)INT32_MAX;
+}
+// Searches count from ranks on the batched path too (the tiles need no counting pass then).
+bool rank_search(const gSuperIntervals* si, int64_t nq) {
+    return si->grid_ends && si->path != SI_PATH_PLAIN && nq < (int64_t)INT32_MAX;
+}
 
 // count into d_counts (device) for device-resident queries
 template <typename S>
@@ -601,7 +615,7 @@ int run_count(gSuperIntervals* si, const sig::QueryBatch& q, uint32_t* d_counts,
         SI_CK(sig::launch_check_contigs(q.qc, q.nq, si->G, si->w_err.as<int>(), st));
         return SI_OK;
     }
-    if (!for_emit && use_ranks(si)) {
+    if (!for_emit && use_ranks(si, q.nq)) {
         PhaseTimer pt(si, 0, st);
         SI_CK(sig::launch_rank_count<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, d_counts,
                                         si->w_err.as<int>(), st));
@@ -640,12 +654,83 @@ int run_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, co
     return SI_OK;
 }
 
-// device-resident queries and outputs
+// ---- searches over ranks (rank_search): counts and offsets in one kernel, then, knowing the result
+// size, either the direct emit or the sorted tiles.
+// Queues counts, upper bounds (w_upper) and offsets; waits for the hit count and the error word.
 template <typename S>
-int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool values,
-                  int64_t* d_offsets, int32_t* d_out, size_t cap, size_t* total, cudaStream_t st) {
-    SI_TRY(check_built(si));
-    SI_TRY(set_dev(si));
+int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, cudaStream_t st,
+                 int64_t* P, int* err) {
+    SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
+    SI_TRY(si->w_upper.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
+    {
+        PhaseTimer pt(si, 0, st);
+        SI_CK(sig::launch_rank_scan<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, pieces,
+                                       si->w_upper.as<uint32_t>(), d_off, si->w_err.as<sig::RankWork>(), st));
+    }
+    struct {
+        int err, inv;
+        unsigned long long total;
+    } h;
+    static_assert(offsetof(sig::RankWork, total) == 8, "read back in one copy");
+    SI_CK(cudaMemcpyAsync(&h, si->w_err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaStreamSynchronize(st));
+    *P = (int64_t)h.total;
+    *err = h.err;
+    return SI_OK;
+}
+
+// The direct emit's lanes per query for a batch of nq queries and P hits, 0 for the sorted tiles.
+// The tiles cost some 100 us (sort, records, tile set-up) and 0.36 ns a query more than the direct
+// emit, which costs some 13 ps a hit more: they pay from about 10 M + 30 hits a query on.  Measured
+// (whole calls, tiles / direct): 3 M queries with 25, 33, 51, 126 hits 1526 / 1313, 1418 / 1130,
+// 1426 / 2703, 2306 / 5551 us; 100 k with 126 and 128 hits 375 / 264, 683 / 390 us; 300 k with 126
+// hits 549 / 690 us.  Where even the smallest tile's candidates (intervals between its queries, and
+// the hits of one) would not fit its lists the direct emit is better at any count (100 k queries
+// with 640 hits over 5 M intervals: 4984 / 2535 us).
+// Lanes: small batches leave lanes idle, so a warp serves one query; large ones fill the device, and
+// few lanes waste less on queries whose hits are few or far apart (3 M queries with 10 far hits: 567
+// us at 2 lanes, 1095 at 8, 2585 at 32), while dense hits want wider chunks (25 hits: 1402, 1313).
+int direct_lanes(const gSuperIntervals* si, int64_t nq, int64_t P) {
+    if (si->path != SI_PATH_AUTO) return 0;
+    const bool fits = 32.0 * (double)si->n / (double)nq + (double)P / (double)nq <= 0.75 * si->bws.prm.cap;
+    if (fits && P > 10000000 + 30 * nq) return 0;
+    const bool far = si->long_depth * (double)nq > 0.5 * (double)P;  // most hits are long intervals, far apart
+    if (nq <= (far ? 4096 : 32768)) return 32;
+    if (nq <= 262144) return 8;
+    return !far && P > 16 * nq ? 8 : 2;
+}
+
+// Sorts the batch into tiles when `lanes` says so; the emits of its parts follow.
+template <typename S>
+int rank_prepare(gSuperIntervals* si, const sig::QueryBatch& q, int lanes, cudaStream_t st) {
+    if (lanes) return SI_OK;
+    PhaseTimer pt(si, 3, st);
+    const int r = sig::batched_prepare_ranked<S>(si->bws, view<S>(si), rank_grid<S>(si, 0), q,
+                                                 si->w_upper.as<uint32_t>(), si->w_err.as<int>(), si->ub_mode, st);
+    return r == SI_OK ? SI_OK : fail(r, "batched query preparation failed (status %d)", r);
+}
+
+// Emits queries [q_offset, q_offset + q.nq) of the batch (P hits in all).
+template <typename S>
+int rank_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, const int64_t* d_off, int64_t out_base,
+              int order, bool values, int32_t* d_out, int lanes, int64_t P, cudaStream_t st) {
+    PhaseTimer pt(si, 2, st);
+    if (lanes) {
+        sig::RankDest<S> d;
+        d.i32 = d_out;
+        SI_CK(sig::launch_rank_emit<S>(view<S>(si), q, si->w_upper.as<uint32_t>() + q_offset, d_off, out_base, order,
+                                       values ? sig::kOutValue : sig::kOutIdx, d, lanes, si->w_err.as<int>(), st));
+        return SI_OK;
+    }
+    const int r = sig::batched_emit<S>(si->bws, view<S>(si), levels<S>(si), si->H, q, q_offset, d_off, out_base, order,
+                                       values, d_out, si->w_err.as<int>(), si->ub_mode, st, P);
+    return r == SI_OK ? SI_OK : fail(r, "batched emit failed (status %d)", r);
+}
+
+// device-resident queries and outputs, counted by the sorted batch or the plain kernels
+template <typename S>
+int search_device_counted(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool values, int64_t* d_offsets,
+                          int32_t* d_out, size_t cap, size_t* total, cudaStream_t st) {
     SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
     SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes(q.nq)));
     SI_TRY(run_count<S>(si, q, si->w_counts.as<uint32_t>(), st, true));
@@ -659,6 +744,26 @@ int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool
     if (total) *total = (size_t)P;
     if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
     SI_TRY(run_emit<S>(si, q, 0, d_offsets, 0, order, values, d_out, st, P));
+    return read_dev_err(si, st);
+}
+
+// device-resident queries and outputs
+template <typename S>
+int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool values,
+                  int64_t* d_offsets, int32_t* d_out, size_t cap, size_t* total, cudaStream_t st) {
+    SI_TRY(check_built(si));
+    SI_TRY(set_dev(si));
+    if (!rank_search(si, q.nq))
+        return search_device_counted<S>(si, q, order, values, d_offsets, d_out, cap, total, st);
+    int64_t P = 0;
+    int err = 0;
+    SI_TRY(rank_offsets<S>(si, q, false, d_offsets, st, &P, &err));
+    if (total) *total = (size_t)P;
+    if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
+    if (err || P == 0) return dev_status(si, err);
+    const int lanes = direct_lanes(si, q.nq, P);
+    SI_TRY(rank_prepare<S>(si, q, lanes, st));
+    SI_TRY(rank_emit<S>(si, q, 0, d_offsets, 0, order, values, d_out, lanes, P, st));
     return read_dev_err(si, st);
 }
 
@@ -706,18 +811,26 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
     }
     sig::QueryBatch q;
     SI_TRY(upload_queries<S>(si, qs, qe, qc, nq, q));
-    SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<size_t>(nq, 1)));
     SI_TRY(si->w_offsets.reserve(sizeof(int64_t) * (nq + 1)));
-    SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
-    SI_TRY(run_count<S>(si, q, si->w_counts.as<uint32_t>(), st, true));
     int64_t* d_off = si->w_offsets.as<int64_t>();
-    {
-        PhaseTimer pt(si, 1, st);
-        SI_CK(sig::exclusive_scan_u32_to_i64(si->w_counts.as<uint32_t>(), d_off, (int64_t)nq, si->w_tmp.p, st, si->w_err.as<int>()));
+    const bool ranks = rank_search(si, q.nq);
+    int64_t P = 0;
+    int err = 0;
+    if (ranks) {
+        SI_TRY(rank_offsets<S>(si, q, false, d_off, st, &P, &err));
+        SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
+    } else {
+        SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<size_t>(nq, 1)));
+        SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
+        SI_TRY(run_count<S>(si, q, si->w_counts.as<uint32_t>(), st, true));
+        {
+            PhaseTimer pt(si, 1, st);
+            SI_CK(sig::exclusive_scan_u32_to_i64(si->w_counts.as<uint32_t>(), d_off, (int64_t)nq, si->w_tmp.p, st, si->w_err.as<int>()));
+        }
+        SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
+        SI_CK(cudaStreamSynchronize(st));
+        P = h_off[nq];
     }
-    SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
-    SI_CK(cudaStreamSynchronize(st));
-    const int64_t P = h_off[nq];
     if (total) *total = (size_t)P;
     if (grow) {
         if (grow->capacity < (size_t)P) {
@@ -729,9 +842,15 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         h_out = grow->values;
         grow->size = (size_t)P;
     } else if ((size_t)P > cap) {
+        if (ranks) SI_CK(cudaStreamSynchronize(st));  // the offsets are the caller's
         return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
     }
-    if (P == 0) return read_dev_err(si);
+    if (P == 0 || err) {
+        SI_TRY(read_dev_err(si));  // waits for the offsets too
+        return dev_status(si, err);
+    }
+    const int lanes = ranks ? direct_lanes(si, q.nq, P) : 0;
+    if (ranks) SI_TRY(rank_prepare<S>(si, q, lanes, st));
     // Results are staged in device memory and copied in bulk: the emit writes every query's
     // list at a scattered place, and such writes over the host link run several times slower
     // than one large copy.  The output is cut into chunks of queries whose lists fit the
@@ -740,7 +859,9 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
     const int64_t budget = std::max<int64_t>((int64_t)(si->out_budget / sizeof(int32_t)), 1 << 20);
     const int64_t buf = std::min<int64_t>(P, budget);
     std::vector<size_t> cuts{0};
-    for (size_t qa = 0; qa < nq;) {
+    if (ranks && P > buf) SI_CK(cudaStreamSynchronize(st));  // the cuts need the offsets
+    if (P <= buf) cuts.push_back(nq);
+    for (size_t qa = P <= buf ? nq : 0; qa < nq;) {
         // largest qb with off[qb] - off[qa] <= buf (at least one query)
         const int64_t limit = h_off[qa] + buf;
         size_t lo = qa + 1, hi = nq;
@@ -753,8 +874,9 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         qa = lo;
     }
     const size_t n_chunks = cuts.size() - 1;
-    int64_t max_need = 1;
-    for (size_t c = 0; c < n_chunks; ++c) max_need = std::max<int64_t>(max_need, h_off[cuts[c + 1]] - h_off[cuts[c]]);
+    int64_t max_need = n_chunks == 1 ? P : 1;
+    for (size_t c = 0; n_chunks > 1 && c < n_chunks; ++c)
+        max_need = std::max<int64_t>(max_need, h_off[cuts[c + 1]] - h_off[cuts[c]]);
     SI_TRY(si->w_out.reserve(sizeof(int32_t) * max_need));
     if (n_chunks > 1) {
         SI_TRY(si->w_out2.reserve(sizeof(int32_t) * max_need));
@@ -766,7 +888,8 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
     }
     auto chunk = [&](size_t c) -> int {
         const size_t qa = cuts[c], qb = cuts[c + 1];
-        const int64_t need = h_off[qb] - h_off[qa];
+        // one chunk: the offsets may still be on their way
+        const int64_t first = n_chunks == 1 ? 0 : h_off[qa], need = n_chunks == 1 ? P : h_off[qb] - first;
         const int b = (int)(c & 1);
         int32_t* dbuf = b ? si->w_out2.as<int32_t>() : si->w_out.as<int32_t>();
         // the buffer's previous copy (chunk c - 2) must be done before the emit overwrites it
@@ -776,17 +899,18 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         sub.qe = static_cast<const S*>(q.qe) + qa;
         sub.qc = q.qc ? q.qc + qa : nullptr;
         sub.nq = (int64_t)(qb - qa);
-        SI_TRY(run_emit<S>(si, sub, (int64_t)qa, d_off + qa, h_off[qa], order, values, dbuf, st, P));
+        if (ranks)
+            SI_TRY(rank_emit<S>(si, sub, (int64_t)qa, d_off + qa, first, order, values, dbuf, lanes, P, st));
+        else
+            SI_TRY(run_emit<S>(si, sub, (int64_t)qa, d_off + qa, first, order, values, dbuf, st, P));
         if (n_chunks == 1) {
-            if (need)
-                SI_CK(cudaMemcpyAsync(h_out + h_off[qa], dbuf, sizeof(int32_t) * need, cudaMemcpyDeviceToHost, st));
+            SI_CK(cudaMemcpyAsync(h_out, dbuf, sizeof(int32_t) * need, cudaMemcpyDeviceToHost, st));
             return SI_OK;
         }
         SI_CK(cudaEventRecord(si->ev_emitted[b], st));
         SI_CK(cudaStreamWaitEvent(si->copy_st, si->ev_emitted[b], 0));
         if (need)
-            SI_CK(cudaMemcpyAsync(h_out + h_off[qa], dbuf, sizeof(int32_t) * need, cudaMemcpyDeviceToHost,
-                                  si->copy_st));
+            SI_CK(cudaMemcpyAsync(h_out + first, dbuf, sizeof(int32_t) * need, cudaMemcpyDeviceToHost, si->copy_st));
         SI_CK(cudaEventRecord(si->ev_copied[b], si->copy_st));
         return SI_OK;
     };
@@ -802,7 +926,6 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
     // the compute stream waits for the last copy (the copy stream runs in order), so later
     // work on it sees the results
     if (n_chunks > 1) SI_CK(cudaStreamWaitEvent(st, si->ev_copied[(n_chunks - 1) & 1], 0));
-    SI_CK(cudaStreamSynchronize(st));
     return read_dev_err(si);
 }
 
@@ -1253,7 +1376,7 @@ extern "C" int upperBoundDeviceGpu(gSuperIntervals* si, const void* d_qe, const 
         return SI_OK;
     }
     sig::QueryBatch q{d_qe, d_qe, d_qc, (int64_t)nq};
-    if (si->grid_starts && si->path == SI_PATH_AUTO) {
+    if (si->grid_starts && si->path == SI_PATH_AUTO && nq < (size_t)INT32_MAX) {
         if (si->bits == 64)
             SI_CK(sig::launch_rank_ub<int64_t>(rank_grid<int64_t>(si, 0), si->G, d_qe, d_qc, (int64_t)nq, d_out,
                                                si->w_err.as<int>(), st));
@@ -1641,7 +1764,7 @@ template <typename S>
 int capture_batched(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_t* d_offsets, int32_t* d_values,
                     size_t capacity, cudaStream_t st) {
     size_t tot = 0;
-    const int r0 = search_device<S>(si, q, order, false, d_offsets, d_values, capacity, &tot, st);
+    const int r0 = search_device_counted<S>(si, q, order, false, d_offsets, d_values, capacity, &tot, st);
     if (r0 != SI_OK && r0 != SI_ERR_CAPACITY) return r0;
     sig::BatchedWorkspace& ws = si->bws;
     const int64_t nq = q.nq;
@@ -1753,6 +1876,19 @@ namespace {
 template <typename S>
 int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStream_t st) {
     SI_TRY(si->so_hoff.reserve(sizeof(int64_t) * (q.nq + 1)));
+    if (rank_search(si, q.nq)) {
+        int64_t P = 0;
+        int err = 0;
+        SI_TRY(rank_offsets<S>(si, q, false, si->so_hoff.as<int64_t>(), st, &P, &err));
+        if (err) return dev_status(si, err);
+        SI_TRY(si->so_hits.reserve(sizeof(int32_t) * std::max<int64_t>(P, 1)));
+        if (P == 0) return SI_OK;
+        const int lanes = direct_lanes(si, q.nq, P);
+        SI_TRY(rank_prepare<S>(si, q, lanes, st));
+        SI_TRY(rank_emit<S>(si, q, 0, si->so_hoff.as<int64_t>(), 0, order, false, si->so_hits.as<int32_t>(), lanes, P,
+                            st));
+        return read_dev_err(si, st);
+    }
     SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
     SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes(q.nq)));
     SI_TRY(run_count<S>(si, q, si->w_counts.as<uint32_t>(), st, true));
@@ -2045,7 +2181,7 @@ int coverage_device(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t* d_c
         SI_CK(cudaMemsetAsync(si->w_err.p, 0, 2 * sizeof(int), st));
         int inv = 0;
         int* d_inv = si->w_err.as<int>() + 1;
-        if (use_ranks(si)) {
+        if (use_ranks(si, q.nq)) {
             SI_CK(sig::launch_rank_coverage<S>(rank_grid<S>(si, 0), rank_grid<S>(si, 1), si->G, q,
                                                si->ps_start.as<uint64_t>(), si->ps_end.as<uint64_t>(), d_count, d_cov,
                                                si->w_err.as<int>(), d_inv, st));

@@ -137,6 +137,49 @@ __device__ uint32_t warp_walk_count(const MapView<S>& m, int64_t lo, int64_t top
     return cnt;
 }
 
+// One query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
+// walked by the whole warp, so every lane of the warp calls it.
+template <typename S>
+__device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid<S>& gs, const RankGrid<S>& ge,
+                                             const S* __restrict__ qs, const S* __restrict__ qe,
+                                             const int32_t* __restrict__ qc, int64_t q, bool live, bool pieces,
+                                             int* d_err, int lane, uint32_t& upper) {
+    bool walk = false;
+    uint32_t cnt = 0, lo = 0, top = 0;
+    S s = 0;
+    upper = 0;
+    if (live) {
+        const int g = qc ? qc[q] : 0;
+        if (g < 0 || g >= m.G) {
+            atomicCAS(d_err, kDevOk, kDevBadContig);
+        } else {
+            s = qs[q];
+            const S e = qe[q];
+            const GridContig c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
+            lo = c1.lo;
+            if (s <= e) {
+                uint32_t r2;
+                grid_two_ranks(gs, c1, e, ge, c2, s, top, r2);
+                cnt = top > r2 ? top - r2 : 0u;
+            } else {
+                top = grid_first_gt<S>(gs, c1, e);
+                walk = !pieces && top > lo;
+            }
+            upper = top > lo ? top : 0u;
+        }
+    }
+    unsigned todo = __ballot_sync(kFull, walk);
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t r = warp_walk_count<S>(m, (int64_t)__shfl_sync(kFull, lo, src),
+                                              (int64_t)__shfl_sync(kFull, top, src) - 1, __shfl_sync(kFull, s, src),
+                                              lane);
+        if (lane == src) cnt = r;
+    }
+    return cnt;
+}
+
 // Counts: no interval has start > end, so an interval that ends before qs starts before qe, and
 // count = #(start <= qe) - #(end < qs) for every query with qs <= qe.  The others (qs > qe) are
 // walked by their warp.
@@ -150,38 +193,8 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
                                                          const int32_t* __restrict__ qc, int64_t nq,
                                                          uint32_t* __restrict__ counts, int* d_err) {
     const int64_t q = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    bool walk = false;
-    uint32_t cnt = 0, lo = 0, top = 0;
-    S s = 0;
-    if (q < nq) {
-        const int g = qc ? qc[q] : 0;
-        if (g < 0 || g >= m.G) {
-            atomicCAS(d_err, kDevOk, kDevBadContig);
-        } else {
-            s = qs[q];
-            const S e = qe[q];
-            const GridContig c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
-            if (s <= e) {
-                uint32_t r1, r2;
-                grid_two_ranks(gs, c1, e, ge, c2, s, r1, r2);
-                cnt = r1 > r2 ? r1 - r2 : 0u;
-            } else {
-                lo = c1.lo;
-                top = grid_first_gt<S>(gs, c1, e);
-                walk = top > lo;
-            }
-        }
-    }
-    unsigned todo = __ballot_sync(kFull, walk);
-    while (todo) {
-        const int src = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const uint32_t r = warp_walk_count<S>(m, (int64_t)__shfl_sync(kFull, lo, src),
-                                              (int64_t)__shfl_sync(kFull, top, src) - 1, __shfl_sync(kFull, s, src),
-                                              lane);
-        if (lane == src) cnt = r;
-    }
+    uint32_t upper;
+    const uint32_t cnt = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, false, d_err, threadIdx.x & 31, upper);
     if (q < nq) counts[q] = cnt;
 }
 
@@ -241,6 +254,211 @@ __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<
     cov[q] = (S)(smin - smax);
 }
 
+// Look-back status of a tile: 2 flag bits over a 62-bit sum.
+constexpr unsigned long long kTileAgg = 1ull << 62;  // the tile's own total
+constexpr unsigned long long kTilePre = 2ull << 62;  // the total of this and all earlier tiles
+constexpr unsigned long long kTileVal = (1ull << 62) - 1ull;
+constexpr int kSpinLimit = 1 << 22;                  // polls of one window before giving up
+
+__device__ __forceinline__ void st_tile(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_tile(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Counts and offsets in one pass: a block takes the next tile of kThreads * R queries from an atomic
+// counter, counts them, publishes the tile's total, and its first warp looks back over the earlier
+// tiles' published totals, 32 at a time, until an inclusive prefix (decoupled look-back; a window
+// that stays unpublished for kSpinLimit polls records kDevTimeout and the walk ends, so the kernel
+// always ends).  Against the count kernel and a scan it saves a launch, a cleared buffer and the
+// counts' way through memory.
+template <typename S, int R>
+__global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
+                                                        const S* __restrict__ qs, const S* __restrict__ qe,
+                                                        const int32_t* __restrict__ qc, int64_t nq, int pieces,
+                                                        uint32_t* __restrict__ su, int64_t* __restrict__ off,
+                                                        RankWork* __restrict__ work) {
+    constexpr int kWarps = kThreads / kWarp;
+    __shared__ int64_t s_warp[kWarps];
+    __shared__ int64_t s_prefix;
+    __shared__ unsigned int s_t;
+    unsigned long long* status = reinterpret_cast<unsigned long long*>(work + 1);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_t = atomicAdd(&work->tiles, 1u);  // tiles in start order: earlier tiles run
+    __syncthreads();
+    const int64_t t = s_t;
+    const int64_t base = t * (kThreads * R) + (int64_t)w * (R * kWarp) + lane;
+    int64_t v[R];
+    int64_t carry = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int64_t q = base + r * kWarp;
+        uint32_t upper;
+        const int64_t x = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, pieces != 0, &work->err, lane, upper);
+        if (q < nq) su[q] = upper;
+        int64_t inc = x;
+#pragma unroll
+        for (int d = 1; d < kWarp; d <<= 1) {
+            const int64_t y = __shfl_up_sync(kFull, inc, d);
+            if (lane >= d) inc += y;
+        }
+        v[r] = carry + inc - x;
+        carry += __shfl_sync(kFull, inc, 31);
+    }
+    if (lane == 0) s_warp[w] = carry;
+    __syncthreads();
+    if (w == 0) {
+        int64_t total = 0;
+#pragma unroll
+        for (int k = 0; k < kWarps; ++k) total += s_warp[k];
+        if (lane == 0) st_tile(status + t, (t == 0 ? kTilePre : kTileAgg) | (unsigned long long)total);
+        int64_t excl = 0;
+        if (t > 0) {
+            int64_t top = t - 1;
+            int spins = 0;
+            while (true) {
+                const int64_t p = top - lane;
+                const unsigned long long s = p >= 0 ? ld_tile(status + p) : kTilePre;
+                const unsigned long long f = s & ~kTileVal;
+                if (__any_sync(kFull, f == 0ull)) {
+                    if (++spins > kSpinLimit) {
+                        if (lane == 0) atomicCAS(&work->err, kDevOk, kDevTimeout);
+                        break;
+                    }
+                    __nanosleep(32);
+                    continue;
+                }
+                spins = 0;
+                const unsigned pm = __ballot_sync(kFull, f == kTilePre);
+                const int first = pm ? __ffs(pm) - 1 : 32;
+                int64_t x = lane <= first ? (int64_t)(s & kTileVal) : 0;
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(kFull, x, d);
+                excl += x;
+                if (pm) break;
+                top -= 32;
+            }
+            if (lane == 0) st_tile(status + t, kTilePre | (unsigned long long)(excl + total));
+        }
+        if (lane == 0) {
+            s_prefix = excl;
+            if ((t + 1) * (kThreads * R) >= nq) {  // the last tile
+                off[nq] = excl + total;
+                work->total = (unsigned long long)(excl + total);
+            }
+        }
+    }
+    __syncthreads();
+    int64_t o = s_prefix;
+    for (int k = 0; k < w; ++k) o += s_warp[k];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int64_t q = base + r * kWarp;
+        if (q < nq) off[q] = v[r] + o;
+    }
+}
+
+// Direct emit: the hits of each query written by W lanes in the batch's own order, from its known
+// upper bound and count.  The lanes look at W positions at a time, downwards; the walk ends with the
+// last hit (the count says which), and goes on below a chunk at the smallest branch of its misses
+// (from a miss at p every position above branch[p] ends before ends[p] < qs).  Neighbouring
+// queries' lists are neighbours in the output, so the writes coalesce across the warp's groups.
+// Right for sparse results: a tile of queries far apart shares nothing, and sorting the batch
+// costs more than the hits.  Bound by the dependent reads of the walk (about 12-16 ps a hit with the
+// device full; lanes per query: see direct_lanes).  Whole calls, before (sorted tiles) and after:
+// 100 k queries with 0.7 hits each 205 -> 57 us, 3 M with 2.7 hits 1290 -> 289 us, 3 M with 33 hits
+// 1418 -> 1130 us; 3 M with 126 hits would go 2306 -> 5551 us.
+template <typename S, int W, int OUT>
+__global__ void __launch_bounds__(kThreads) k_rank_emit(MapView<S> m, const S* __restrict__ qs,
+                                                        const S* __restrict__ qe, const int32_t* __restrict__ qc,
+                                                        int64_t nq, const uint32_t* __restrict__ su,
+                                                        const int64_t* __restrict__ off, int64_t out_base, int order,
+                                                        RankDest<S> dst, int* d_err) {
+    const int lane = threadIdx.x & 31, sub = lane & (W - 1);
+    const unsigned gmask = W == 32 ? kFull : ((1u << (W & 31)) - 1u) << (lane & ~(W - 1));
+    const int64_t q = ((int64_t)blockIdx.x * kThreads + threadIdx.x) / W;
+    int64_t at = 0;
+    int cnt = 0, i = -1, lo = 0;
+    S s = 0, e0 = 0;
+    if (q < nq) {
+        at = off[q];
+        cnt = (int)(off[q + 1] - at);
+        at -= out_base;
+        if (cnt > 0) {
+            i = (int)su[q] - 1;
+            s = qs[q];
+            if (OUT == kOutPieces) e0 = qe[q];
+            const int g = qc ? qc[q] : 0;
+            lo = (int)m.seg[g];
+        }
+    }
+    const bool ascending = order == kOrderIdxsCpp;
+    int done = 0;      // hits written
+    int head = -1;     // length of the head run (ascending order only)
+    while (true) {
+        const bool active = done < cnt && i >= lo;  // group-uniform
+        if (!__any_sync(kFull, active)) break;
+        const int k = i - sub;
+        const bool in = active && k >= lo;
+        S e = 0;
+        if (in) e = m.ends[k];
+        const bool hit = in && s <= e;
+        const unsigned bal = __ballot_sync(kFull, hit);
+        const unsigned mine = (bal & gmask) >> (lane & ~(W - 1));
+        if (ascending && __any_sync(kFull, active && head < 0)) {
+            // the head run: consecutive hits from the upper bound down; it goes on below this chunk
+            // only when the whole chunk hits
+            const unsigned full = W == 32 ? kFull : (1u << (W & 31)) - 1u;
+            bool open = active && head < 0;
+            int h = mine == full ? W : __ffs(~mine) - 1;
+            bool more = open && mine == full && h < cnt;
+            while (__any_sync(kFull, more)) {
+                const int k2 = i - h - sub;
+                const bool hit2 = more && k2 >= lo && s <= m.ends[k2];
+                const unsigned b2 = (__ballot_sync(kFull, hit2) & gmask) >> (lane & ~(W - 1));
+                if (more) {
+                    h += b2 == full ? W : __ffs(~b2) - 1;
+                    more = b2 == full && h < cnt;
+                }
+            }
+            if (open) head = h;
+        }
+        const int rank = done + __popc(mine & ((1u << sub) - 1u));
+        if (hit && rank < cnt) {
+            const int64_t p = at + (rank < head ? head - 1 - rank : rank);
+            if constexpr (OUT == kOutIdx) {
+                dst.i32[p] = k - lo;
+            } else if constexpr (OUT == kOutValue) {
+                dst.i32[p] = m.data[k];
+            } else if constexpr (OUT == kOutKeys) {
+                dst.s[p] = m.starts[k];
+                dst.e[p] = e;
+                if (dst.i32) dst.i32[p] = m.data[k];
+            } else {
+                const S st = m.starts[k];
+                dst.s[p] = st > s ? st : s;
+                dst.e[p] = e < e0 ? e : e0;
+                dst.i32[p] = k - lo;
+            }
+        }
+        done += __popc(mine);
+        // the next chunk, where hits are left
+        int next = i - W;
+        if (__any_sync(kFull, active && done < cnt)) {
+            int br = INT32_MAX;
+            if (in && !hit && done < cnt) br = m.branch[k];
+#pragma unroll
+            for (int d = W / 2; d > 0; d >>= 1) br = min(br, __shfl_xor_sync(kFull, br, d));
+            next = min(next, br);
+        }
+        if (active) i = next;
+    }
+    if (done != cnt && sub == 0) atomicCAS(d_err, kDevOk, kDevOverflow);  // internal: count and walk differ
+}
+
 inline unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, ceil_div(n, kThreads)); }
 
 }  // namespace
@@ -274,6 +492,64 @@ cudaError_t launch_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, Quer
     return cudaGetLastError();
 }
 
+// queries per tile of the count and scan kernel: one per thread while the batch fits the device
+// about once, else four, for fewer look-backs
+constexpr int64_t kScanSmall = 152 * 2048;
+
+size_t rank_work_bytes(int64_t nq) {
+    const int64_t tiles = ceil_div(nq > 0 ? nq : 1, nq <= kScanSmall ? kThreads : 4 * kThreads);
+    return sizeof(RankWork) + sizeof(unsigned long long) * (size_t)tiles;
+}
+
+template <typename S>
+cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, bool pieces, uint32_t* su,
+                             int64_t* off, RankWork* work, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(work, 0, rank_work_bytes(q.nq), st);
+    if (e != cudaSuccess) return e;
+    if (q.nq <= 0) return cudaMemsetAsync(off, 0, sizeof(int64_t), st);
+    const S* qs = static_cast<const S*>(q.qs);
+    const S* qe = static_cast<const S*>(q.qe);
+    if (q.nq <= kScanSmall)
+        k_rank_scan<S, 1><<<blocks_for(q.nq), kThreads, 0, st>>>(m, gs, ge, qs, qe, q.qc, q.nq, pieces, su, off, work);
+    else
+        k_rank_scan<S, 4><<<(unsigned)ceil_div(q.nq, 4 * kThreads), kThreads, 0, st>>>(m, gs, ge, qs, qe, q.qc, q.nq,
+                                                                                      pieces, su, off, work);
+    note_launch();
+    return cudaGetLastError();
+}
+
+template <typename S, int W>
+static cudaError_t rank_emit_w(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
+                               int order, int what, RankDest<S> d, int* d_err, cudaStream_t st) {
+    const unsigned blocks = blocks_for(q.nq * W);
+    const S* qs = static_cast<const S*>(q.qs);
+    const S* qe = static_cast<const S*>(q.qe);
+    switch (what) {
+        case kOutIdx:
+            k_rank_emit<S, W, kOutIdx><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            break;
+        case kOutValue:
+            k_rank_emit<S, W, kOutValue><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            break;
+        case kOutKeys:
+            k_rank_emit<S, W, kOutKeys><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            break;
+        default:
+            k_rank_emit<S, W, kOutPieces><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+    }
+    note_launch();
+    return cudaGetLastError();
+}
+
+template <typename S>
+cudaError_t launch_rank_emit(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
+                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st) {
+    if (q.nq <= 0) return cudaSuccess;
+    if (lanes == 2) return rank_emit_w<S, 2>(m, q, su, off, out_base, order, what, d, d_err, st);
+    if (lanes == 8) return rank_emit_w<S, 8>(m, q, su, off, out_base, order, what, d, d_err, st);
+    return rank_emit_w<S, 32>(m, q, su, off, out_base, order, what, d, d_err, st);
+}
+
 template <typename S>
 cudaError_t launch_rank_ub(RankGrid<S> gs, int G, const void* qe, const int32_t* qc, int64_t nq, int32_t* out,
                            int* d_err, cudaStream_t st) {
@@ -300,6 +576,10 @@ cudaError_t launch_rank_coverage(RankGrid<S> gs, RankGrid<S> ge, int G, QueryBat
                                               GridContig*, uint32_t*, uint32_t*, cudaStream_t);                  \
     template cudaError_t launch_rank_count<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, uint32_t*, int*, \
                                               cudaStream_t);                                                     \
+    template cudaError_t launch_rank_scan<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, bool, uint32_t*,  \
+                                             int64_t*, RankWork*, cudaStream_t);                                 \
+    template cudaError_t launch_rank_emit<S>(MapView<S>, QueryBatch, const uint32_t*, const int64_t*, int64_t,   \
+                                             int, int, RankDest<S>, int, int*, cudaStream_t);                    \
     template cudaError_t launch_rank_ub<S>(RankGrid<S>, int, const void*, const int32_t*, int64_t, int32_t*,     \
                                            int*, cudaStream_t);                                                  \
     template cudaError_t launch_rank_coverage<S>(RankGrid<S>, RankGrid<S>, int, QueryBatch, const uint64_t*,     \

@@ -151,6 +151,34 @@ cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G
 template <typename S>
 cudaError_t launch_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, uint32_t* counts,
                               int* d_err, cudaStream_t st);
+// Counts and their exclusive prefix sums (off, n + 1 entries) in one pass, and each query's upper
+// bound (su: the first position whose start exceeds the query's end, 0 when no start of its contig
+// is at or below it or the contig is outside [0, G)).  work: rank_work_bytes(nq), zeroed by the call.
+// With pieces, a query with start > end counts nothing (it gives no piece of an intersection).
+struct RankWork {
+    int err;                   // device error word
+    int inv;                   // free for the caller
+    unsigned long long total;  // hits of the batch
+    unsigned int tiles;        // tile counter
+    unsigned int pad[11];
+};
+size_t rank_work_bytes(int64_t nq);
+template <typename S>
+cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, bool pieces, uint32_t* su,
+                             int64_t* off, RankWork* work, cudaStream_t st);
+// What the direct emit writes for each hit.
+enum RankOut : int { kOutIdx = 0, kOutValue = 1, kOutKeys = 2, kOutPieces = 3 };
+template <typename S>
+struct RankDest {
+    int32_t* i32 = nullptr;  // positions, payloads or (keys: may be null) payloads
+    S* s = nullptr;          // keys, pieces: starts
+    S* e = nullptr;          // and ends
+};
+// Writes every query's hits at off[q] - out_base, by groups of `lanes` (2, 8 or 32) lanes per query.
+template <typename S>
+cudaError_t launch_rank_emit(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
+                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st);
+
 // Contig-local upper bounds (-1: none) of every query end.
 template <typename S>
 cudaError_t launch_rank_ub(RankGrid<S> gs, int G, const void* qe, const int32_t* qc, int64_t nq, int32_t* out,
