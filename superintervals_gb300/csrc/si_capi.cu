@@ -130,6 +130,13 @@ void dev_release(void** p, size_t* bytes) {
 }
 }  // namespace sig
 
+// Rank grids over one or two arrays of the same contigs: per array the contig records, t1 and t2
+// words (si_rank.cuh), in one allocation.
+struct GridSet {
+    DevBuf buf;
+    size_t at[2][3] = {{0, 0, 0}, {0, 0, 0}};  // byte offsets of [array][contigs, t1, t2]
+};
+
 struct gSuperIntervals {
     int bits = 32;
     int device = 0;
@@ -158,12 +165,16 @@ struct gSuperIntervals {
     DevBuf long_lvl[sig::kMaxLevels];
     int64_t long_sizes[sig::kMaxLevels + 1] = {0};
     int long_H = 0;
-    // rank grids over the starts and, when no interval has start > end, over the sorted ends:
-    // contig records, then t1 and t2 words (si_rank.cuh); without them (no room under the device
-    // budget) the calls that use them take the sorted batch
-    DevBuf grid;
+    // rank grids over the starts and, when no interval has start > end, over the sorted ends;
+    // without them (no room under the device budget) the calls that use them take the sorted batch
+    GridSet grid;
     bool grid_starts = false, grid_ends = false;
-    size_t grid_at[2][3] = {{0, 0, 0}, {0, 0, 0}};  // byte offsets of [starts | ends][contigs, t1, t2]
+    // the stretches of each contig that no interval covers (difference), made by the first such call
+    // after a build: starts, then ends, in one buffer, their contig offsets and their grids
+    DevBuf gaps, gap_seg;
+    GridSet gap_grid;
+    int64_t n_gaps = 0;
+    bool gaps_ready = false;
     int sort_passes = 0;
     bool input_was_sorted = false;
     // query workspace
@@ -342,46 +353,47 @@ struct TempArena {
     }
 };
 
-// which 0: starts, 1: sorted ends
 template <typename S>
-sig::RankGrid<S> rank_grid(const gSuperIntervals* si, int which) {
-    const char* p = si->grid.as<char>();
+sig::RankGrid<S> grid_view(const GridSet& g, const S* arr, int which) {
+    const char* p = g.buf.as<char>();
     sig::RankGrid<S> R;
-    R.arr = which ? si->end_sorted.as<S>() : si->starts.as<S>();
-    R.c = reinterpret_cast<const sig::GridContig*>(p + si->grid_at[which][0]);
-    R.t1 = reinterpret_cast<const uint32_t*>(p + si->grid_at[which][1]);
-    R.t2 = reinterpret_cast<const uint32_t*>(p + si->grid_at[which][2]);
+    R.arr = arr;
+    R.c = reinterpret_cast<const sig::GridContig*>(p + g.at[which][0]);
+    R.t1 = reinterpret_cast<const uint32_t*>(p + g.at[which][1]);
+    R.t2 = reinterpret_cast<const uint32_t*>(p + g.at[which][2]);
     return R;
 }
 
-// Rank grids of a built index's starts and sorted ends, in one allocation.  Queued on the handle's
-// stream; the caller synchronizes.  No room is no error: the index then works without them.
+// which 0: starts, 1: sorted ends
 template <typename S>
-int build_grids(gSuperIntervals* si, const std::vector<int64_t>& segv, std::vector<uint32_t>& base) {
-    si->grid_starts = si->grid_ends = false;
-    const int G = si->G, arrays = si->inverted == 0 ? 2 : 1;
+sig::RankGrid<S> rank_grid(const gSuperIntervals* si, int which) {
+    return grid_view<S>(si->grid, which ? si->end_sorted.as<S>() : si->starts.as<S>(), which);
+}
+
+// Grids over a0 and (unless null) a1, n entries each, ascending inside the contigs segv (d_seg on
+// the device).  Queued on st; `base` must live until the stream is synchronized.
+template <typename S>
+int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vector<int64_t>& segv,
+                const int64_t* d_seg, std::vector<uint32_t>& base, cudaStream_t st) {
+    const int G = (int)segv.size() - 1;
     base.resize(G);
-    const int64_t w1 = sig::grid_t1_words(segv.data(), G, base.data()), w2 = sig::grid_t2_words(si->n);
+    const int64_t w1 = sig::grid_t1_words(segv.data(), G, base.data()), w2 = sig::grid_t2_words(n);
     size_t at = (sizeof(uint32_t) * (size_t)G + 255) & ~(size_t)255;
     const size_t parts[3] = {sizeof(sig::GridContig) * (size_t)G, sizeof(uint32_t) * (size_t)w1,
                              sizeof(uint32_t) * (size_t)w2};
-    for (int a = 0; a < arrays; ++a)
+    for (int a = 0; a < (a1 ? 2 : 1); ++a)
         for (int k = 0; k < 3; ++k) {
-            si->grid_at[a][k] = at;
+            g.at[a][k] = at;
             at += (parts[k] + 255) & ~(size_t)255;
         }
-    if (si->grid.reserve(at) != SI_OK) return SI_OK;
-    SI_CK(cudaMemcpyAsync(si->grid.p, base.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, si->st));
-    for (int a = 0; a < arrays; ++a) {
-        char* p = si->grid.as<char>();
-        SI_CK(sig::launch_grid_build<S>(rank_grid<S>(si, a).arr, si->n, si->seg.as<int64_t>(), G,
-                                        si->grid.as<uint32_t>(), w1,
-                                        reinterpret_cast<sig::GridContig*>(p + si->grid_at[a][0]),
-                                        reinterpret_cast<uint32_t*>(p + si->grid_at[a][1]),
-                                        reinterpret_cast<uint32_t*>(p + si->grid_at[a][2]), si->st));
-    }
-    si->grid_starts = true;
-    si->grid_ends = arrays == 2;
+    SI_TRY(g.buf.reserve(at));
+    char* p = g.buf.as<char>();
+    SI_CK(cudaMemcpyAsync(p, base.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, st));
+    for (int a = 0; a < (a1 ? 2 : 1); ++a)
+        SI_CK(sig::launch_grid_build<S>(a ? a1 : a0, n, d_seg, G, reinterpret_cast<uint32_t*>(p), w1,
+                                        reinterpret_cast<sig::GridContig*>(p + g.at[a][0]),
+                                        reinterpret_cast<uint32_t*>(p + g.at[a][1]),
+                                        reinterpret_cast<uint32_t*>(p + g.at[a][2]), st));
     return SI_OK;
 }
 
@@ -403,6 +415,7 @@ int build_impl(gSuperIntervals* si) {
     si->bws.end_sorted = nullptr;
     si->cov_ready = false;
     si->rec_ready = false;
+    si->gaps_ready = false;
     si->grid_starts = si->grid_ends = false;
     if (si->gexec) {              // a captured graph holds the old buffers
         cudaGraphExecDestroy(si->gexec);
@@ -545,7 +558,13 @@ int build_impl(gSuperIntervals* si) {
         si->bws.end_sorted = si->end_sorted.p;
     }
     std::vector<uint32_t> grid_base;
-    SI_TRY(build_grids<S>(si, segv, grid_base));
+    const bool two = si->inverted == 0;
+    // no room for them is no error: the index then works without
+    const int gr = build_grids<S>(si->grid, si->starts.as<S>(), two ? si->end_sorted.as<S>() : nullptr, n, segv,
+                                  si->seg.as<int64_t>(), grid_base, st);
+    if (gr != SI_OK && gr != SI_ERR_OOM) return gr;
+    si->grid_starts = gr == SI_OK;
+    si->grid_ends = gr == SI_OK && two;
     SI_TRY(sig::batched_prepare<S>(si->bws, view<S>(si), levels<S>(si), si->H, si->lvl_sizes,
                                    si->ub_mode, st));
     SI_CK(cudaStreamSynchronize(st));
@@ -656,6 +675,20 @@ int run_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, co
 
 // ---- searches over ranks (rank_search): counts and offsets in one kernel, then, knowing the result
 // size, either the direct emit or the sorted tiles.
+// The hit count and the error word of launch_rank_scan, in one copy.
+int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err) {
+    struct {
+        int err, inv;
+        unsigned long long total;
+    } h;
+    static_assert(offsetof(sig::RankWork, total) == 8, "read back in one copy");
+    SI_CK(cudaMemcpyAsync(&h, si->w_err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaStreamSynchronize(st));
+    *P = (int64_t)h.total;
+    *err = h.err;
+    return SI_OK;
+}
+
 // Queues counts, upper bounds (w_upper) and offsets; waits for the hit count and the error word.
 template <typename S>
 int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, cudaStream_t st,
@@ -667,16 +700,7 @@ int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int
         SI_CK(sig::launch_rank_scan<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, pieces,
                                        si->w_upper.as<uint32_t>(), d_off, si->w_err.as<sig::RankWork>(), st));
     }
-    struct {
-        int err, inv;
-        unsigned long long total;
-    } h;
-    static_assert(offsetof(sig::RankWork, total) == 8, "read back in one copy");
-    SI_CK(cudaMemcpyAsync(&h, si->w_err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-    SI_CK(cudaStreamSynchronize(st));
-    *P = (int64_t)h.total;
-    *err = h.err;
-    return SI_OK;
+    return read_rank_work(si, st, P, err);
 }
 
 // The direct emit's lanes per query for a batch of nq queries and P hits, 0 for the sorted tiles.
@@ -1902,6 +1926,71 @@ int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStre
     return read_dev_err(si, st);
 }
 
+// The gaps of each contig (no interval has start > end), made on the first difference after a build.
+template <typename S>
+int make_gaps(gSuperIntervals* si, cudaStream_t st) {
+    if (si->gaps_ready) return SI_OK;
+    const int64_t slots = si->n + si->G;
+    if (slots >= (int64_t)INT32_MAX) return SI_ERR_TOO_LARGE;
+    TempArena tmp;
+    const size_t scan = sig::scan_temp_bytes(slots);
+    SI_TRY(tmp.buf.reserve(TempArena::room(sizeof(uint32_t) * slots) + TempArena::room(sizeof(int64_t) * (slots + 1)) +
+                           TempArena::room(scan) + TempArena::room(256)));
+    uint32_t* flags = tmp.take<uint32_t>(sizeof(uint32_t) * slots);
+    int64_t* offs = tmp.take<int64_t>(sizeof(int64_t) * (slots + 1));
+    char* stmp = tmp.take<char>(scan);
+    int* gerr = tmp.take<int>(256);
+    SI_TRY(si->gap_seg.reserve(sizeof(int64_t) * (si->G + 1)));
+    SI_CK(cudaMemsetAsync(gerr, 0, sizeof(int), st));
+    SI_CK(sig::launch_gap_flags<S>(view<S>(si), flags, st));
+    SI_CK(sig::exclusive_scan_u32_to_i64(flags, offs, slots, stmp, st, gerr));
+    SI_CK(sig::launch_gap_seg(offs, si->seg.as<int64_t>(), si->G, si->gap_seg.as<int64_t>(), st));
+    std::vector<int64_t> segv(si->G + 1);
+    int ge = 0;
+    SI_CK(cudaMemcpyAsync(segv.data(), si->gap_seg.p, sizeof(int64_t) * (si->G + 1), cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaMemcpyAsync(&ge, gerr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaStreamSynchronize(st));
+    SI_TRY(dev_status(si, ge));
+    const int64_t M = segv.back();
+    SI_TRY(si->gaps.reserve(2 * sizeof(S) * std::max<int64_t>(M, 1)));
+    S* a0 = si->gaps.as<S>();
+    SI_CK(sig::launch_gap_write<S>(view<S>(si), flags, offs, a0, a0 + M, st));
+    std::vector<uint32_t> base;
+    SI_TRY(build_grids<S>(si->gap_grid, a0, a0 + M, M, segv, si->gap_seg.as<int64_t>(), base, st));
+    SI_CK(cudaStreamSynchronize(st));  // the temporaries are released on scope exit
+    si->n_gaps = M;
+    si->gaps_ready = true;
+    return SI_OK;
+}
+
+template <typename S>
+sig::RankGrid<S> gap_grid(const gSuperIntervals* si, int which) {
+    return grid_view<S>(si->gap_grid, si->gaps.as<S>() + (which ? si->n_gaps : 0), which);
+}
+
+// Difference from the gaps: the pieces of a query are the gaps it meets, so their number is a
+// difference of two ranks, as a search's hits.  Queues offsets and bounds; waits for the total.
+template <typename S>
+int gap_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int64_t* d_off, size_t* total, cudaStream_t st) {
+    SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
+    SI_TRY(si->w_upper.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
+    SI_CK(sig::launch_rank_scan<S>(view<S>(si), gap_grid<S>(si, 0), gap_grid<S>(si, 1), q, true,
+                                   si->w_upper.as<uint32_t>(), d_off, si->w_err.as<sig::RankWork>(), st));
+    int64_t T = 0;
+    int err = 0;
+    SI_TRY(read_rank_work(si, st, &T, &err));
+    SI_TRY(dev_status(si, err));
+    *total = (size_t)T;
+    return SI_OK;
+}
+
+template <typename S>
+int gap_emit(gSuperIntervals* si, const sig::QueryBatch& q, const int64_t* d_off, S* os, S* oe, cudaStream_t st) {
+    const S* a0 = si->gaps.as<S>();
+    SI_CK(sig::launch_gap_emit<S>(a0, a0 + si->n_gaps, q, si->w_upper.as<uint32_t>(), d_off, os, oe, st));
+    return SI_OK;
+}
+
 // op 0: intersection (order = the hit order), op 1: difference.  Pieces go to caller device
 // buffers when they hold `cap` pieces; `total` always receives the piece count.
 template <typename S>
@@ -1915,6 +2004,16 @@ int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int orde
         SI_CK(cudaMemsetAsync(d_off, 0, sizeof(int64_t), st));
         SI_CK(cudaStreamSynchronize(st));
         return SI_OK;
+    }
+    if (op == 1 && use_ranks(si, q.nq) && make_gaps<S>(si, st) == SI_OK) {
+        size_t T = 0;
+        SI_TRY(gap_offsets<S>(si, q, d_off, &T, st));
+        if (total) *total = T;
+        if (T > cap) return fail(SI_ERR_CAPACITY, "output needs %zu pieces, capacity %zu", T, cap);
+        if (T == 0) return SI_OK;
+        if (!d_os || !d_oe) return fail(SI_ERR_INVALID, "null output buffer");
+        SI_TRY(gap_emit<S>(si, q, d_off, d_os, d_oe, st));
+        return read_dev_err(si, st);
     }
     SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     if (si->n > 0) {
@@ -2011,17 +2110,21 @@ int setop_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc,
     SI_TRY(si->so_os.reserve(sizeof(S) * T));
     SI_TRY(si->so_oe.reserve(sizeof(S) * T));
     if (op == 0) SI_TRY(si->so_ob.reserve(sizeof(int32_t) * T));
-    // the hit lists are still in place: emit the pieces only
-    const int64_t* hoff = si->so_hoff.as<int64_t>();
-    const int32_t* hits = si->so_hits.as<int32_t>();
-    sig::MapView<S> rv;
-    SI_TRY(view_rec<S>(si, si->st, &rv));
-    if (op == 0)
-        SI_CK(sig::launch_isect<S>(rv, q, hoff, hits, nullptr, si->so_off.as<int64_t>(), si->so_os.as<S>(),
-                                   si->so_oe.as<S>(), si->so_ob.as<int32_t>(), si->w_err.as<int>(), si->st));
-    else
-        SI_CK(sig::launch_diff<S>(rv, q, hoff, hits, si->inverted == 1, nullptr, si->so_off.as<int64_t>(),
-                                  si->so_os.as<S>(), si->so_oe.as<S>(), si->w_err.as<int>(), si->st));
+    if (op == 1 && use_ranks(si, q.nq) && si->gaps_ready) {
+        SI_TRY(gap_emit<S>(si, q, si->so_off.as<int64_t>(), si->so_os.as<S>(), si->so_oe.as<S>(), si->st));
+    } else {
+        // the hit lists are still in place: emit the pieces only
+        const int64_t* hoff = si->so_hoff.as<int64_t>();
+        const int32_t* hits = si->so_hits.as<int32_t>();
+        sig::MapView<S> rv;
+        SI_TRY(view_rec<S>(si, si->st, &rv));
+        if (op == 0)
+            SI_CK(sig::launch_isect<S>(rv, q, hoff, hits, nullptr, si->so_off.as<int64_t>(), si->so_os.as<S>(),
+                                       si->so_oe.as<S>(), si->so_ob.as<int32_t>(), si->w_err.as<int>(), si->st));
+        else
+            SI_CK(sig::launch_diff<S>(rv, q, hoff, hits, si->inverted == 1, nullptr, si->so_off.as<int64_t>(),
+                                      si->so_os.as<S>(), si->so_oe.as<S>(), si->w_err.as<int>(), si->st));
+    }
     if (!h_os || !h_oe || (op == 0 && !h_ob)) return fail(SI_ERR_INVALID, "null output buffer");
     SI_CK(cudaMemcpyAsync(h_os, si->so_os.p, sizeof(S) * T, cudaMemcpyDeviceToHost, si->st));
     SI_CK(cudaMemcpyAsync(h_oe, si->so_oe.p, sizeof(S) * T, cudaMemcpyDeviceToHost, si->st));

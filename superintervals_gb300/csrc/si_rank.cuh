@@ -179,6 +179,19 @@ template <typename S>
 cudaError_t launch_rank_emit(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
                              int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st);
 
+// Gaps: the stretches of each contig's coordinate range that no interval covers (no interval has
+// start > end).  Slots: contig g's positions, then one after its last; flags mark those with a gap
+// before them, offs are the flags' exclusive prefix sums.
+template <typename S>
+cudaError_t launch_gap_flags(MapView<S> m, uint32_t* flags, cudaStream_t st);
+cudaError_t launch_gap_seg(const int64_t* offs, const int64_t* seg, int G, int64_t* gap_seg, cudaStream_t st);
+template <typename S>
+cudaError_t launch_gap_write(MapView<S> m, const uint32_t* flags, const int64_t* offs, S* gs, S* ge, cudaStream_t st);
+// The gaps that each query meets, clipped to it: the off[q + 1] - off[q] gaps before su[q].
+template <typename S>
+cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32_t* su, const int64_t* off, S* os,
+                            S* oe, cudaStream_t st);
+
 // Contig-local upper bounds (-1: none) of every query end.
 template <typename S>
 cudaError_t launch_rank_ub(RankGrid<S> gs, int G, const void* qe, const int32_t* qc, int64_t nq, int32_t* out,

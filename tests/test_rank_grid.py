@@ -106,6 +106,43 @@ def test_ranks_match_numpy(api, kind, n, dt):
     idx.close()
 
 
+def _uncovered(s, e, lo, hi):
+    """Stretches of [lo, hi] that no interval [s, e] covers, as exact Python ints."""
+    out, cur = [], lo
+    for a, b in sorted(zip(s.tolist(), e.tolist())):
+        if a > hi or b < lo:
+            continue
+        if a > cur:
+            out.append((cur, a - 1))
+        cur = max(cur, b + 1)
+    if cur <= hi:
+        out.append((cur, hi))
+    return out
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+@pytest.mark.parametrize("n", [1, 2, 7, 33, 1000, 4097])
+@pytest.mark.parametrize("kind", ["uniform", "duplicates", "gap", "extremes", "clustered"])
+def test_difference_from_gaps(api, kind, n, dt):
+    s, e, seg, qs, qe, qc = _case(kind, n, dt, seed=n + 1)
+    e = s + np.minimum(e - s, 100).astype(dt)                # leave gaps between the intervals
+    sel = np.concatenate([np.arange(120), np.arange(2500, 2700)])
+    qs, qe, qc = qs[sel], qe[sel], qc[sel]
+    idx = api.GpuIndex(np.dtype(dt).itemsize * 8)
+    idx.add_arrays(s, e, seg=seg)
+    idx.build()
+    off, ps, pe = idx.difference(qs, qe, qc)
+    for i in range(len(qs)):
+        a, b = (v[seg[qc[i]]:seg[qc[i] + 1]] for v in (s, e))
+        want = _uncovered(a, b, int(qs[i]), int(qe[i])) if qs[i] <= qe[i] else []
+        got = list(zip(ps[off[i]:off[i + 1]].tolist(), pe[off[i]:off[i + 1]].tolist()))
+        assert got == want
+    idx.set_path(api.PATH_PLAIN)                             # the hit-list sweep
+    off2, ps2, pe2 = idx.difference(qs, qe, qc)
+    assert np.array_equal(off, off2) and np.array_equal(ps, ps2) and np.array_equal(pe, pe2)
+    idx.close()
+
+
 def test_count_paths_agree(api):
     s, e, seg, qs, qe, qc = _case("uniform", 4097, np.int32, seed=5)
     _, cnt = _expected(s, e, seg, qs, qe, qc)
