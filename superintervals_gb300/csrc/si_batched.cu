@@ -1224,6 +1224,742 @@ __global__ void __launch_bounds__(kThreads, 4) k_tiles(TileArgs<S> a) {
     }
 }
 
+// ---- emit over ranked batches (batched_prepare_ranked) -------------------------------------
+// Tiles of 32-256 neighbouring short queries share their candidates, as in k_tiles, for an index
+// without start > end intervals whose queries are counted already.  What differs is how a tile
+// finds and writes:
+//  * its candidates are read straight from two contiguous stretches (gather_direct), instead of
+//    walking the pyramid level by level;
+//  * the long-interval list's section of its candidates is compacted once per version (below) and
+//    copied whole by each query, 16 bytes a lane, instead of being checked candidate by candidate;
+//  * a query's bounds in the lists are one packed record, and its parts are loops over 32 candidates.
+// Long queries (and the queries of a tile whose candidates overflow its lists) read their own
+// stretches, one warp each.
+
+// One 256-query block of the sorted batch: its tile's stretches and bounds, when all its queries are
+// short and of one contig (ok).
+template <typename S>
+struct TileRec {
+    int64_t pcut;       // first position whose start is within long_split of L
+    int64_t c_hi, c_w;  // long-list entries before pcut that can reach L: [c_w, c_hi)
+    S L, Q;             // smallest and largest query start
+    int32_t umax, ok;   // largest upper bound
+};
+
+template <typename S>
+struct EmitArgs {
+    Pyr<S> P, PL;               // pyramids of the ends and of the long-interval list's ends
+    const S* starts;
+    const int32_t* data;
+    const int64_t* seg;
+    int32_t G;
+    RankGrid<S> gs;
+    const int32_t* long_pos;    // long-interval list: positions, starts (ends: PL.ends)
+    const S* long_start;
+    const int64_t* long_seg;
+    int64_t long_split, long_max, split_len;
+    const TileRec<S>* rec;      // per 256 sorted queries; null: tiles of another size
+    const S* sq_s;
+    const int32_t* sq_u;
+    const uint32_t* sq_c;
+    const int32_t* sq_id;
+    int64_t nq;
+    int tile_q, cap, n_tiles;
+    int* tile_counter;
+    const int64_t* offsets;
+    int64_t id_lo, id_hi, out_base;
+    int order;
+    bool values;
+    const S* qe;                // pieces: query ends, in the batch's order
+    RankDest<S> dst;
+    int* d_err;
+};
+
+constexpr int kDirectBlocks = 128;  // 32-slot blocks of a tile's direct gather
+constexpr int kMaxMiss = 31;        // possible misses up to which a section has versions
+constexpr int kMinSection = 96;     // and its length from which they pay
+
+// One hit at output index p: its position pos with end e and start st.
+template <typename S, int OUT>
+__device__ __forceinline__ void put_hit(const EmitArgs<S>& a, int64_t p, int64_t pos, S e, int64_t lo, S qs, S qe) {
+    if constexpr (OUT == kOutPieces) {
+        const S st = a.starts[pos];
+        a.dst.s[p] = st > qs ? st : qs;
+        a.dst.e[p] = e < qe ? e : qe;
+        a.dst.i32[p] = (int32_t)(pos - lo);
+    } else {
+        a.dst.i32[p] = a.values ? a.data[pos] : (int32_t)(pos - lo);
+    }
+}
+
+// One query by one warp, from its own stretches: the positions from its upper bound u down to the
+// first start within long_split of qs, then the long-interval list's entries below that can reach it.
+// Stretches of more than kScanMax slots are walked over the pyramids instead.  128 slots a round, so
+// that four reads are in flight (the loads of one round do not depend on the last one's hits).
+template <typename S, int OUT>
+__device__ void emit_alone(const EmitArgs<S>& a, S qs, S qe, int64_t u, int g, int64_t out_off, int cnt, int lane) {
+    constexpr int64_t kScanMax = 16384;
+    const int64_t lo = a.seg[g];
+    if (u < lo || cnt <= 0) return;
+    const S* __restrict__ ends = a.P.ends;
+    int h = 0;  // head run, for the ascending order
+    if (a.order == kOrderIdxsCpp) {
+        for (int64_t top = u; top >= lo && h < cnt; top -= 32) {
+            const int64_t p = top - lane;
+            const unsigned m = __ballot_sync(kFull, p >= lo && ends[p] >= qs);
+            const int run = m == kFull ? 32 : __ffs(~m) - 1;
+            h += run;
+            if (run < 32) break;
+        }
+    }
+    const unsigned lt = lanemask_lt();
+    int w = 0;
+    auto put = [&](bool hit, unsigned m, int rank, int64_t pos, S e) {  // rank: place among m's hits
+        if (hit) {
+            const int r = w + rank;
+            if (r < cnt) put_hit<S, OUT>(a, out_off + (r < h ? h - 1 - r : r), pos, e, lo, qs, qe);
+        }
+        w += __popc(m);
+    };
+    const GridContig c = load_contig(a.gs.c + g);
+    const int64_t plo = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(qs, a.long_split));
+    if (u - plo < kScanMax) {
+        for (int64_t top = u; top >= plo; top -= 128) {
+            S e[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int64_t p = top - 32 * k - lane;
+                e[k] = p >= plo ? ends[p] : Lim<S>::lo;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int64_t p = top - 32 * k - lane;
+                const bool hit = p >= plo && e[k] >= qs;
+                const unsigned m = __ballot_sync(kFull, hit);
+                if (m) put(hit, m, __popc(m & lt), p, e[k]);
+            }
+        }
+    } else {
+        scan_desc(a.P, plo, u, qs, lane, [&](int64_t ch, unsigned hm, S e) {
+            put((hm >> lane) & 1u, hm, __popc(hm & above_mask(lane)), (ch << 5) + lane, e);
+            return w < cnt;
+        });
+    }
+    if (w < cnt) {
+        const int64_t below = plo < u + 1 ? plo : u + 1;  // list entries below the window
+        const int64_t c0 = a.long_seg[g];
+        const int64_t ch = warp_first_pos_geq(a.long_pos, c0, a.long_seg[g + 1], below, lane);
+        const int64_t pw = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(qs, a.long_max));
+        const int64_t cw = warp_first_pos_geq(a.long_pos, c0, ch, pw, lane);
+        const S* __restrict__ le = a.PL.ends;
+        if (ch - cw <= kScanMax) {
+            for (int64_t top = ch - 1; top >= cw && w < cnt; top -= 128) {
+                S e[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int64_t p = top - 32 * k - lane;
+                    e[k] = p >= cw ? le[p] : Lim<S>::lo;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int64_t p = top - 32 * k - lane;
+                    const bool hit = p >= cw && e[k] >= qs;
+                    const unsigned m = __ballot_sync(kFull, hit);
+                    if (m) put(hit, m, __popc(m & lt), hit ? (int64_t)a.long_pos[p] : 0, e[k]);
+                }
+            }
+        } else {
+            scan_desc(a.PL, cw, ch - 1, qs, lane, [&](int64_t b, unsigned hm, S e) {
+                const bool hit = (hm >> lane) & 1u;
+                put(hit, hm, __popc(hm & above_mask(lane)), hit ? (int64_t)a.long_pos[(b << 5) + lane] : 0, e);
+                return w < cnt;
+            });
+        }
+    }
+    if (w != cnt && lane == 0) atomicCAS(a.d_err, kDevOk, kDevOverflow);  // internal: count and walk differ
+}
+
+// A tile's candidates: slots [pcut, umax] downwards, then the long-interval list's [c_w, c_hi)
+// downwards.  Kept ones (end >= L) go to (cpos, cend, cstart) in that order, the own ones at least X
+// long also to (lpos, lend), and the list entries ending before Q to the lnu list (candidate index,
+// end).  Two reads of the stretches (the second from cache) around one scan of the 32-slot blocks'
+// counts.  tot: candidates, own candidates, own long ones, lnu entries.  Returns false when more
+// than cap candidates are kept.  Block-uniform; ends synchronized.
+template <typename S>
+__device__ bool gather_direct(const EmitArgs<S>& a, int64_t pcut, int64_t umax, int64_t c_w, int64_t c_hi, S L, S Q,
+                              int64_t X, int32_t* cpos, S* cend, S* cstart, int32_t* lpos, S* lend, uint32_t* s_cnt,
+                              uint32_t* s_sub, int32_t* s_lnu_idx, S* s_lnu_end, int* tot) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_own = umax >= pcut ? (int)(umax - pcut + 1) : 0, n_win = (int)(c_hi - c_w);
+    const int b_own = (n_own + 31) >> 5, nb = b_own + ((n_win + 31) >> 5);
+    const unsigned lt = lanemask_lt();
+    // block b's slots: in the stretch, end and start; sub: own and at least X long, or listed and
+    // ending before Q
+    auto load = [&](int b, S& e, S& st, bool& keep, bool& sub) {
+        const bool own = b < b_own;
+        const int k = ((own ? b : b - b_own) << 5) + lane;
+        const bool in = k < (own ? n_own : n_win);
+        const int64_t at = own ? umax - k : c_hi - 1 - k;
+        e = Lim<S>::lo;
+        st = 0;
+        if (in) {
+            e = (own ? a.P.ends : a.PL.ends)[at];
+            st = (own ? a.starts : a.long_start)[at];
+        }
+        keep = in && e >= L;
+        sub = keep && (own ? is_long_iv<S>(st, e, X) : e < Q);
+    };
+#pragma unroll 4
+    for (int b = warp; b < nb; b += kWarpsPerCta) {
+        S e, st;
+        bool keep, sub;
+        load(b, e, st, keep, sub);
+        const int mc = __popc(__ballot_sync(kFull, keep)), ms = __popc(__ballot_sync(kFull, sub));
+        if (lane == 0) {
+            s_cnt[b] = (uint32_t)mc;
+            s_sub[b] = (uint32_t)ms;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {  // exclusive prefixes; the sub counts start again at the list's first block
+        int run = 0, run_s = 0, own = 0, own_s = 0;
+        for (int b0 = 0; b0 < nb; b0 += 32) {
+            const int b = b0 + lane;
+            const int c = b < nb ? (int)s_cnt[b] : 0, s = b < nb ? (int)s_sub[b] : 0;
+            int ic = c, is = s;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(kFull, ic, d), z = __shfl_up_sync(kFull, is, d);
+                if (lane >= d) {
+                    ic += y;
+                    is += z;
+                }
+            }
+            if (b < nb) {
+                s_cnt[b] = (uint32_t)(run + ic - c);
+                s_sub[b] = (uint32_t)(run_s + is - s);
+            }
+            const unsigned at = __ballot_sync(kFull, b == b_own - 1);  // the last own block
+            if (at) {
+                own = run + __shfl_sync(kFull, ic, __ffs(at) - 1);
+                own_s = run_s + __shfl_sync(kFull, is, __ffs(at) - 1);
+            }
+            run += __shfl_sync(kFull, ic, 31);
+            run_s += __shfl_sync(kFull, is, 31);
+        }
+        if (lane == 0) {
+            tot[0] = run;
+            tot[1] = own;
+            tot[2] = own_s;
+            tot[3] = run_s - own_s;
+        }
+    }
+    __syncthreads();
+    if (tot[0] > a.cap) return false;
+    const int own_s = tot[2];
+#pragma unroll 2
+    for (int b = warp; b < nb; b += kWarpsPerCta) {
+        S e, st;
+        bool keep, sub;
+        load(b, e, st, keep, sub);
+        const unsigned mc = __ballot_sync(kFull, keep), ms = __ballot_sync(kFull, sub);
+        const bool own = b < b_own;
+        if (keep) {
+            const int at = (int)s_cnt[b] + __popc(mc & lt);
+            const int k = ((own ? b : b - b_own) << 5) + lane;
+            const int32_t p = own ? (int32_t)(umax - k) : a.long_pos[c_hi - 1 - k];
+            cpos[at] = p;
+            cend[at] = e;
+            cstart[at] = st;
+            if (sub) {
+                const int slot = (int)s_sub[b] + __popc(ms & lt);
+                if (own) {
+                    lpos[slot] = p;
+                    lend[slot] = e;
+                } else if (slot - own_s < kMaxMiss) {
+                    s_lnu_idx[slot - own_s] = at;
+                    s_lnu_end[slot - own_s] = e;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
+// One warp copies src[0, len) (shared memory, 16-byte aligned, readable to len + 4 rounded up to 4)
+// to dst[0, len) (global memory, 4-byte aligned): up to three values, then 16-byte stores from dst's
+// next 16-byte boundary on (a lane's four values lie in two aligned quads), then up to three values.
+template <int P>
+__device__ __forceinline__ void copy16_body(int4* __restrict__ d4, const int4* __restrict__ s4, int nv, int lane) {
+    for (int j0 = lane; j0 < nv; j0 += 128) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = j0 + 32 * k;
+            if (j < nv) {
+                const int4 x = s4[j];
+                int4 o = x;
+                if constexpr (P != 0) {
+                    const int4 y = s4[j + 1];
+                    if constexpr (P == 1) o = make_int4(x.y, x.z, x.w, y.x);
+                    if constexpr (P == 2) o = make_int4(x.z, x.w, y.x, y.y);
+                    if constexpr (P == 3) o = make_int4(x.w, y.x, y.y, y.z);
+                }
+                d4[j] = o;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void warp_copy16(int32_t* __restrict__ dst, const int32_t* __restrict__ src, int len,
+                                            int lane) {
+    const int p = min((int)((4u - ((uint32_t)(uintptr_t)dst >> 2)) & 3u), len);
+    const int nv = (len - p) >> 2, done = p + 4 * nv;
+    if (lane < p) dst[lane] = src[lane];
+    const int4* __restrict__ s4 = reinterpret_cast<const int4*>(src);
+    int4* __restrict__ d4 = reinterpret_cast<int4*>(dst + p);
+    if (p == 0) copy16_body<0>(d4, s4, nv, lane);
+    else if (p == 1) copy16_body<1>(d4, s4, nv, lane);
+    else if (p == 2) copy16_body<2>(d4, s4, nv, lane);
+    else copy16_body<3>(d4, s4, nv, lane);
+    if (lane < len - done) dst[done + lane] = src[done + lane];
+}
+
+template <typename S, int OUT>
+__global__ void __launch_bounds__(kThreads, 4) k_emit_tiles(EmitArgs<S> a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int cap = a.cap, T = a.tile_q;
+    // candidates: end, start, position (then the value written); own long ones: end, value.  The
+    // pyramid gather's scratch uses lpos, lend and cstart.
+    S* cend = reinterpret_cast<S*>(smem);
+    S* cstart = cend + cap;
+    S* lend = cstart + cap;
+    int64_t* q_off = reinterpret_cast<int64_t*>(lend + cap);
+    S* q_s = reinterpret_cast<S*>(q_off + T);
+    S* q_e = q_s + T;                                          // pieces only
+    uint2* q_pack = reinterpret_cast<uint2*>(q_e + (OUT == kOutPieces ? T : 0));
+    int32_t* q_u = reinterpret_cast<int32_t*>(q_pack + T);
+    uint32_t* q_c = reinterpret_cast<uint32_t*>(q_u + T);      // class word, then (version, order) halves
+    int32_t* q_cap = reinterpret_cast<int32_t*>(q_c + T);
+    int32_t* cpos = q_cap + T;
+    int32_t* lpos = cpos + cap;
+    uint16_t* q_h16 = reinterpret_cast<uint16_t*>(q_c);
+    __shared__ int s_tile, s_n, s_sum, s_next;
+    __shared__ int s_tot[4];
+    __shared__ int64_t s_cut[3];
+    __shared__ int s_wsum[kWarpsPerCta];
+    __shared__ S s_red[kWarpsPerCta], s_red2[kWarpsPerCta];
+    __shared__ int32_t s_red3[kWarpsPerCta];
+    __shared__ uint32_t s_cnt[kMaxBlocks], s_sub[kDirectBlocks];
+    // lnu entries: candidates of the section (the long-interval list's) ending before the run's largest
+    // query start, in candidate order; their ends in ascending order and each one's rank there
+    __shared__ int32_t s_lnu_idx[kMaxMiss + 1];
+    __shared__ S s_lnu_end[kMaxMiss + 1], s_ver_end[kMaxMiss + 1];
+    __shared__ int s_lnu_rank[kMaxMiss + 1], s_ver_at[kMaxMiss + 1], s_ver_first[kMaxMiss + 1];
+    __shared__ unsigned s_ver_used;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // below p_cut only intervals at least long_split long reach a tile: with X at most that, every
+    // candidate of the section is long for every query
+    const int64_t X = a.split_len < a.long_split ? a.split_len : a.long_split;
+    const unsigned lt = lanemask_lt();
+    const bool cpp = a.order == kOrderIdxsCpp;
+    while (true) {
+        if (tid == 0) s_tile = atomicAdd(a.tile_counter, 1);
+        __syncthreads();
+        const int tc = s_tile;
+        if (tc >= a.n_tiles) return;
+        // heaviest first: long queries sort to the end of the batch
+        const int t = a.n_tiles - 1 - tc;
+        const int64_t j0 = (int64_t)t * T;
+        const int nt = (int)((a.nq - j0) < (int64_t)T ? (a.nq - j0) : (int64_t)T);
+        for (int i = tid; i < nt; i += kThreads) {
+            const int32_t id = a.sq_id[j0 + i];
+            q_s[i] = a.sq_s[j0 + i];
+            q_u[i] = a.sq_u[j0 + i];
+            q_c[i] = a.sq_c[j0 + i];
+            if (id < a.id_lo || id >= a.id_hi) {
+                q_off[i] = 0;
+                q_cap[i] = -1;  // outside the emitted window: skipped
+            } else {
+                const int64_t o = a.offsets[id], o1 = a.offsets[id + 1];
+                q_off[i] = o - a.out_base;
+                q_cap[i] = (int32_t)(o1 - o);
+                if (OUT == kOutPieces) q_e[i] = a.qe[id];
+            }
+        }
+        TileRec<S> rec{};
+        if (a.rec) rec = a.rec[t];
+        __syncthreads();
+        int r0 = 0;
+        while (r0 < nt) {
+            // run of equal class/contig words [r0, r1): sorted, so binary search the end
+            const uint32_t cw = q_c[r0];
+            int lo_i = r0 + 1, hi_i = nt;
+            while (lo_i < hi_i) {
+                const int mid = (lo_i + hi_i) >> 1;
+                if (q_c[mid] == cw) lo_i = mid + 1;
+                else hi_i = mid;
+            }
+            const int r1 = lo_i;
+            if (cw >= 3u * (uint32_t)a.G) {  // no start at or below the query: no hits
+                r0 = r1;
+                continue;
+            }
+            const int g = code_contig(cw, a.G);
+            const int64_t lo = a.seg[g];
+            bool alone = code_is_long(cw, a.G);
+            int nc = 0, nco = 0, nl = 0, nlnu = 0;  // candidates, own ones, own long ones, lnu entries
+            if (!alone) {
+                S L = rec.L, Q = rec.Q;
+                int64_t umax = rec.umax, pcut = rec.pcut, c_hi = rec.c_hi, c_w = rec.c_w;
+                if (!rec.ok || r0 != 0 || r1 != nt) {
+                    S mn = Lim<S>::hi, mx = Lim<S>::lo;
+                    int32_t um = INT32_MIN;
+                    for (int i = r0 + tid; i < r1; i += kThreads) {
+                        mn = q_s[i] < mn ? q_s[i] : mn;
+                        mx = q_s[i] > mx ? q_s[i] : mx;
+                        um = q_u[i] > um ? q_u[i] : um;
+                    }
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) {
+                        const S o = __shfl_xor_sync(kFull, mn, d);
+                        mn = o < mn ? o : mn;
+                        const S p = __shfl_xor_sync(kFull, mx, d);
+                        mx = p > mx ? p : mx;
+                        um = max(um, __shfl_xor_sync(kFull, um, d));
+                    }
+                    if (lane == 0) {
+                        s_red[warp] = mn;
+                        s_red2[warp] = mx;
+                        s_red3[warp] = um;
+                    }
+                    __syncthreads();
+                    L = s_red[0];
+                    Q = s_red2[0];
+                    um = s_red3[0];
+#pragma unroll
+                    for (int w = 1; w < kWarpsPerCta; ++w) {
+                        L = s_red[w] < L ? s_red[w] : L;
+                        Q = s_red2[w] > Q ? s_red2[w] : Q;
+                        um = max(um, s_red3[w]);
+                    }
+                    umax = um;
+                    if (warp == 0) {
+                        const GridContig c = load_contig(a.gs.c + g);
+                        const int64_t pc = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(L, a.long_split));
+                        const int64_t pw = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(L, a.long_max));
+                        const int64_t ch = warp_first_pos_geq(a.long_pos, a.long_seg[g], a.long_seg[g + 1], pc, lane);
+                        const int64_t cw2 = warp_first_pos_geq(a.long_pos, a.long_seg[g], ch, pw, lane);
+                        if (lane == 0) {
+                            s_cut[0] = pc;
+                            s_cut[1] = ch;
+                            s_cut[2] = cw2;
+                        }
+                    }
+                    __syncthreads();
+                    pcut = s_cut[0];
+                    c_hi = s_cut[1];
+                    c_w = s_cut[2];
+                }
+                const int64_t slots = (umax >= pcut ? umax - pcut + 1 : 0) + (c_hi - c_w);
+                if (slots <= 32 * (kDirectBlocks - 2)) {
+                    alone = !gather_direct<S>(a, pcut, umax, c_w, c_hi, L, Q, X, cpos, cend, cstart, lpos, lend, s_cnt,
+                                              s_sub, s_lnu_idx, s_lnu_end, s_tot);
+                    if (!alone) {
+                        nc = s_tot[0];
+                        nco = s_tot[1];
+                        nl = s_tot[2];
+                        nlnu = s_tot[3];
+                    }
+                } else {
+                    // sparse or far-reaching stretches: over the pyramids (scratch in cstart and lend)
+                    int32_t* cnt = reinterpret_cast<int32_t*>(lend);
+                    uint32_t* msk = reinterpret_cast<uint32_t*>(cstart);
+                    nco = gather_bfs<S>(a.P, pcut, umax, L, cap, cpos, cend, lpos, cnt, msk, s_wsum, &s_n, &s_sum);
+                    int nw = 0;
+                    if (nco >= 0 && c_hi > c_w)
+                        nw = gather_bfs<S>(a.PL, c_w, c_hi - 1, L, cap - nco, cpos + nco, cend + nco, lpos + nco, cnt,
+                                           msk, s_wsum, &s_n, &s_sum, a.long_pos);
+                    alone = nco < 0 || nw < 0;
+                    if (!alone) {
+                        nc = nco + nw;
+                        __syncthreads();
+                        const int nb = (nco + 31) >> 5;
+                        for (int k = nco + tid; k < nc; k += kThreads) cstart[k] = a.starts[cpos[k]];
+                        for (int b = warp; b < nb; b += kWarpsPerCta) {  // own long ones, in order
+                            const int k = (b << 5) + lane;
+                            bool isl = false;
+                            if (k < nco) {
+                                const S st = a.starts[cpos[k]];
+                                cstart[k] = st;
+                                isl = is_long_iv<S>(st, cend[k], X);
+                            }
+                            const int c = __popc(__ballot_sync(kFull, isl));
+                            if (lane == 0) s_cnt[b] = (uint32_t)c;
+                        }
+                        __syncthreads();
+                        block_excl_scan(reinterpret_cast<int32_t*>(s_cnt), nb, s_wsum, &s_sum);
+                        nl = nb > 0 ? s_sum : 0;
+                        for (int b = warp; b < nb; b += kWarpsPerCta) {
+                            const int k = (b << 5) + lane;
+                            const bool isl = k < nco && is_long_iv<S>(cstart[k], cend[k], X);
+                            const unsigned m = __ballot_sync(kFull, isl);
+                            if (isl) {
+                                const int at = (int)s_cnt[b] + __popc(m & lt);
+                                lpos[at] = cpos[k];
+                                lend[at] = cend[k];
+                            }
+                        }
+                        nlnu = kMaxMiss + 1;  // no versions
+                        __syncthreads();
+                    }
+                }
+            }
+            if (alone) {
+                // their work differs widely in length: warps claim queries one at a time
+                __syncthreads();
+                if (tid == 0) s_next = r0;
+                __syncthreads();
+                while (true) {
+                    int i = 0;
+                    if (lane == 0) i = atomicAdd(&s_next, 1);
+                    i = __shfl_sync(kFull, i, 0);
+                    if (i >= r1) break;
+                    if (q_cap[i] <= 0) continue;  // nothing to write, or outside the emitted window
+                    emit_alone<S, OUT>(a, q_s[i], OUT == kOutPieces ? q_e[i] : (S)0, (int64_t)q_u[i], g, q_off[i],
+                                       q_cap[i], lane);
+                }
+                __syncthreads();
+                r0 = r1;
+                continue;
+            }
+            // The section [nco, nc) is hit by every query of the run but for the lnu entries ending
+            // before its start, and those are nested: a query with v lnu ends below its start misses
+            // exactly the v smallest.  So the run has at most nlnu + 1 different sections (versions);
+            // each is compacted once, and its queries copy it whole.
+            const int sec = nc - nco;
+            const int img0 = (nl + 3) & ~3, stride = (sec + 7) & ~3;  // images: lpos (values), lend (ends)
+            const int slots_v = (cap - img0) / stride;
+            const bool use_ver = nlnu <= kMaxMiss && sec >= kMinSection && slots_v > 0;
+            if (use_ver) {
+                if (warp == 0) {
+                    const S e = lane < nlnu ? s_lnu_end[lane] : Lim<S>::hi;
+                    int r = 0;
+                    for (int j = 0; j < nlnu; ++j) {
+                        const S o = __shfl_sync(kFull, e, j);
+                        r += (o < e || (o == e && j < lane)) ? 1 : 0;
+                    }
+                    if (lane < nlnu) {
+                        s_ver_end[r] = e;
+                        s_lnu_rank[lane] = r;
+                    }
+                    s_ver_at[lane] = 0;
+                }
+                __syncthreads();
+            }
+            // step 1: one query per THREAD finds where its hits lie in the lists: its head run (the
+            // consecutive positions u, u - 1, ... that hit: those down to the last start >= qs always
+            // do), the candidates after it starting at qs - X or later (part A), and its first own
+            // long candidate below those
+            for (int i = r0 + tid; i < r1; i += kThreads) {
+                const S qs = q_s[i];
+                const int32_t u = q_u[i];
+                int h = 0, ta = nc, tsplit = nc, lb = nl, v = 0;
+                if (nc > 0) {
+                    int b0 = 0, b1 = nc;  // first candidate at or below u
+                    while (b0 < b1) {
+                        const int mid = (b0 + b1) >> 1;
+                        if (cpos[mid] > u) b0 = mid + 1;
+                        else b1 = mid;
+                    }
+                    const int t0 = b0;
+                    auto first_start_below = [&](int from, S key) {
+                        int l0 = from, l1 = nc;
+                        while (l0 < l1) {
+                            const int mid = (l0 + l1) >> 1;
+                            if (cstart[mid] >= key) l0 = mid + 1;
+                            else l1 = mid;
+                        }
+                        return l0;
+                    };
+                    int k = first_start_below(t0, qs);
+                    while (k < nc && cpos[k] == u - (k - t0) && cend[k] >= qs) ++k;
+                    h = k - t0;
+                    ta = k;
+                    tsplit = max(ta, first_start_below(ta, near_threshold<S>(qs, X)));
+                    if (tsplit < nco) {
+                        const int32_t pb = cpos[tsplit];
+                        int l0 = 0, l1 = nl;
+                        while (l0 < l1) {
+                            const int mid = (l0 + l1) >> 1;
+                            if (lpos[mid] > pb) l0 = mid + 1;
+                            else l1 = mid;
+                        }
+                        lb = l0;
+                    }
+                    if (use_ver) {  // lnu ends below qs
+                        int v1 = nlnu;
+                        while (v < v1) {
+                            const int mid = (v + v1) >> 1;
+                            if (s_ver_end[mid] < qs) v = mid + 1;
+                            else v1 = mid;
+                        }
+                    }
+                }
+                q_pack[i] = make_uint2((uint32_t)h | ((uint32_t)ta << 16), (uint32_t)tsplit | ((uint32_t)lb << 16));
+                if (use_ver) {
+                    q_h16[2 * i] = (uint16_t)v;
+                    atomicAdd(&s_ver_at[v], 1);
+                }
+            }
+            __syncthreads();
+            if (use_ver && warp == 0) {  // where each version's queries go
+                const int c = s_ver_at[lane];
+                int inc = c;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(kFull, inc, d);
+                    if (lane >= d) inc += y;
+                }
+                const unsigned used = __ballot_sync(kFull, c > 0);
+                s_ver_at[lane] = s_ver_first[lane] = inc - c;
+                if (lane == 0) s_ver_used = used;
+            }
+            // the lists now only feed the writes: positions become the values written
+            for (int k = tid; k < nc; k += kThreads) {
+                const int32_t p = cpos[k];
+                cpos[k] = OUT == kOutIdx && a.values ? a.data[p] : p - (int32_t)lo;
+            }
+            for (int k = tid; k < nl; k += kThreads) {
+                const int32_t p = lpos[k];
+                lpos[k] = OUT == kOutIdx && a.values ? a.data[p] : p - (int32_t)lo;
+            }
+            __syncthreads();
+            if (use_ver) {  // the run's queries ordered by version
+                for (int i = r0 + tid; i < r1; i += kThreads)
+                    q_h16[2 * (r0 + atomicAdd(&s_ver_at[q_h16[2 * i]], 1)) + 1] = (uint16_t)i;
+                __syncthreads();
+            }
+            // step 2: one query per WARP writes its hits.  With versions, as many as fit are compacted
+            // at a time, and their queries written before the next ones.
+            for (unsigned ver = use_ver ? s_ver_used : 1u; ver != 0u;) {
+                unsigned rest = 0u;
+                int first = r0, last = r1;
+                if (use_ver) {
+                    rest = ver;
+                    int v = 0;
+                    for (int slot = 0; slot < slots_v && rest; ++slot) {
+                        v = __ffs(rest) - 1;
+                        rest &= rest - 1;
+                        if ((slot & (kWarpsPerCta - 1)) != warp) continue;
+                        const int img = img0 + slot * stride;
+                        const int gone_at = lane < nlnu && s_lnu_rank[lane] < v ? s_lnu_idx[lane] : INT32_MAX;
+                        for (int k0 = nco; k0 < nc; k0 += 32) {
+                            const int k = k0 + lane;
+                            const int before = __popc(__ballot_sync(kFull, gone_at < k0));
+                            const unsigned in = gone_at >= k0 && gone_at < k0 + 32 ? 1u << (gone_at - k0) : 0u;
+                            const unsigned gone = __reduce_or_sync(kFull, in);
+                            if (k < nc && !((gone >> lane) & 1u)) {
+                                const int at = img + (k - nco) - before - __popc(gone & lt);
+                                lpos[at] = cpos[k];
+                                if (OUT == kOutPieces) lend[at] = cend[k];
+                            }
+                        }
+                    }
+                    first = r0 + s_ver_first[__ffs(ver) - 1];
+                    last = r0 + s_ver_at[v];
+                    __syncthreads();
+                }
+                const unsigned now = ver & ~rest;
+                ver = rest;
+                for (int o = first + warp; o < last; o += kWarpsPerCta) {
+                    const int i = use_ver ? (int)q_h16[2 * o + 1] : o;
+                    const int capq = q_cap[i];
+                    if (capq <= 0) continue;  // nothing to write, or outside the emitted window
+                    const S qs = q_s[i];
+                    const uint2 pk = q_pack[i];
+                    const int64_t off = q_off[i];
+                    const int h = (int)(pk.x & 0xffffu), ta = (int)(pk.x >> 16);
+                    const int tsplit = (int)(pk.y & 0xffffu), lb = (int)(pk.y >> 16);
+                    int32_t* __restrict__ d = a.dst.i32 + off;
+                    S* __restrict__ ds = nullptr;
+                    S* __restrict__ de = nullptr;
+                    S qe = 0;
+                    if (OUT == kOutPieces) {
+                        ds = a.dst.s + off;
+                        de = a.dst.e + off;
+                        qe = q_e[i];
+                    }
+                    int w = h;  // next write
+                    if (h <= capq) {
+                        for (int r = lane; r < h; r += 32) {
+                            const int k = cpp ? ta - 1 - r : ta - h + r;
+                            d[r] = cpos[k];
+                            if (OUT == kOutPieces) {
+                                const S st = cstart[k], e = cend[k];
+                                ds[r] = st > qs ? st : qs;
+                                de[r] = e < qe ? e : qe;
+                            }
+                        }
+                    }
+                    // candidates [from, to) of a list, those reaching qs
+                    auto filter = [&](const int32_t* __restrict__ vals, const S* __restrict__ ends,
+                                      const S* __restrict__ sts, int from, int to) {
+                        for (; from < to && w <= capq; from += 32) {
+                            const int k = from + lane;
+                            const S e = ends[k];
+                            const int32_t val = vals[k];
+                            const bool hit = k < to && e >= qs;
+                            const unsigned m = __ballot_sync(kFull, hit);
+                            const int at = w + __popc(m & lt);
+                            if (hit && at < capq) {
+                                d[at] = val;
+                                if (OUT == kOutPieces) {
+                                    S st = qs;
+                                    if (sts) st = sts[k] > qs ? sts[k] : qs;
+                                    ds[at] = st;
+                                    de[at] = e < qe ? e : qe;
+                                }
+                            }
+                            w += __popc(m);
+                        }
+                    };
+                    filter(cpos, cend, cstart, ta, tsplit);
+                    if (ta <= nco) {
+                        filter(lpos, lend, nullptr, lb, nl);
+                        if (use_ver) {
+                            const int v = (int)q_h16[2 * i], len = sec - v;
+                            const int img = img0 + __popc(now & ((1u << v) - 1u)) * stride;
+                            if (w + len <= capq) {
+                                if (OUT == kOutPieces) {
+                                    for (int k = lane; k < len; k += 32) {
+                                        const S e = lend[img + k];
+                                        d[w + k] = lpos[img + k];
+                                        ds[w + k] = qs;
+                                        de[w + k] = e < qe ? e : qe;
+                                    }
+                                } else {
+                                    warp_copy16(d + w, lpos + img, len, lane);
+                                }
+                            }
+                            w += len;
+                        } else {
+                            filter(cpos, cend, nullptr, nco, nc);
+                        }
+                    } else {  // the head run reached into the section
+                        filter(cpos, cend, cstart, tsplit, nc);
+                    }
+                    if (w != capq && lane == 0) atomicCAS(a.d_err, kDevOk, kDevOverflow);  // internal
+                }
+                if (ver) __syncthreads();  // the images are overwritten next
+            }
+            __syncthreads();
+            r0 = r1;
+        }
+    }
+}
+
 // ---- query keys: (class|contig, end) -------------------------------------------------
 // Smallest and largest query end as offset-binary (unsigned order = signed order).
 template <typename S>
@@ -1608,7 +2344,7 @@ __global__ void __launch_bounds__(kThreads) k_pos_keys(const S* __restrict__ qs,
 }
 
 // The sorted records, in the form of k_qprep's: start, upper bound (-1: none), class code and id;
-// and each block's cut for the tile of its 256 queries.
+// and the record of each block's tile of 256 queries.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restrict__ pay,
                                                        const uint32_t* __restrict__ key, int pos_bits,
@@ -1616,17 +2352,19 @@ __global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restric
                                                        RankGrid<S> gs, S* __restrict__ sq_s,
                                                        int32_t* __restrict__ sq_u, uint32_t* __restrict__ sq_c,
                                                        int32_t* __restrict__ sq_id, int64_t long_split,
-                                                       const int32_t* __restrict__ long_pos,
+                                                       int64_t long_max, const int32_t* __restrict__ long_pos,
                                                        const int64_t* __restrict__ long_seg,
-                                                       int64_t* __restrict__ blk_cut) {
-    __shared__ S s_mn[kWarpsPerCta];
+                                                       TileRec<S>* __restrict__ recs) {
+    __shared__ S s_mn[kWarpsPerCta], s_mx[kWarpsPerCta];
+    __shared__ int32_t s_um[kWarpsPerCta];
     __shared__ uint32_t s_code[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t jb = (int64_t)blockIdx.x * kThreads, j = jb + tid;
     const int64_t jl = (jb + kThreads < nq ? jb + kThreads : nq) - 1;
     const bool valid = j < nq;
     uint32_t code = 0;
-    S vs = Lim<S>::hi;
+    S vs = 0;
+    int32_t um = -1;
     if (valid) {
         const uint32_t id = pay[j], cls = key[j] >> pos_bits;
         uint32_t up;
@@ -1639,6 +2377,7 @@ __global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restric
             vs = r.x;
             up = (uint32_t)r.y;
         }
+        um = (int32_t)up - 1;
         code = 3u * (uint32_t)m.G;
         if (cls < 2u) {
             int g = 0;
@@ -1650,37 +2389,48 @@ __global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restric
             code = cls * (uint32_t)m.G + (uint32_t)g;
         }
         sq_s[j] = vs;
-        sq_u[j] = (int32_t)up - 1;
+        sq_u[j] = um;
         sq_c[j] = code;
         sq_id[j] = (int32_t)id;
     }
-    if (!blk_cut) return;
-    // the tile's cut: the first position whose start is within long_split of its smallest query
-    // start, and the first long-list index at or after it
-    S mn = vs;
+    S mn = valid ? vs : Lim<S>::hi, mx = valid ? vs : Lim<S>::lo;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         const S o = __shfl_xor_sync(kFull, mn, d);
         mn = o < mn ? o : mn;
+        const S p = __shfl_xor_sync(kFull, mx, d);
+        mx = p > mx ? p : mx;
+        um = max(um, __shfl_xor_sync(kFull, um, d));
     }
-    if (lane == 0) s_mn[warp] = mn;
+    if (lane == 0) {
+        s_mn[warp] = mn;
+        s_mx[warp] = mx;
+        s_um[warp] = um;
+    }
     if (j == jb) s_code[0] = code;
     if (j == jl) s_code[1] = code;
     __syncthreads();
     if (warp == 0) {
-        int64_t pc = -1, ch = -1;
-        if (s_code[0] == s_code[1] && s_code[0] < (uint32_t)m.G) {
-            S L = s_mn[0];
+        TileRec<S> r{};
+        if (s_code[0] == s_code[1] && s_code[0] < (uint32_t)m.G) {  // sorted: all short, of one contig
+            r.L = s_mn[0];
+            r.Q = s_mx[0];
+            r.umax = s_um[0];
 #pragma unroll
-            for (int w = 1; w < kWarpsPerCta; ++w) L = s_mn[w] < L ? s_mn[w] : L;
+            for (int w = 1; w < kWarpsPerCta; ++w) {
+                r.L = s_mn[w] < r.L ? s_mn[w] : r.L;
+                r.Q = s_mx[w] > r.Q ? s_mx[w] : r.Q;
+                r.umax = max(r.umax, s_um[w]);
+            }
             const int g = (int)s_code[0];
-            pc = (int64_t)grid_first_geq<S>(gs, load_contig(gs.c + g), near_threshold<S>(L, long_split));
-            ch = warp_first_pos_geq(long_pos, long_seg[g], long_seg[g + 1], pc, lane);
+            const GridContig c = load_contig(gs.c + g);
+            r.pcut = (int64_t)grid_first_geq<S>(gs, c, near_threshold<S>(r.L, long_split));
+            const int64_t pw = (int64_t)grid_first_geq<S>(gs, c, near_threshold<S>(r.L, long_max));
+            r.c_hi = warp_first_pos_geq(long_pos, long_seg[g], long_seg[g + 1], r.pcut, lane);
+            r.c_w = warp_first_pos_geq(long_pos, long_seg[g], r.c_hi, pw, lane);
+            r.ok = 1;
         }
-        if (lane == 0) {
-            blk_cut[2 * blockIdx.x] = pc;
-            blk_cut[2 * blockIdx.x + 1] = ch;
-        }
+        if (lane == 0) recs[blockIdx.x] = r;
     }
 }
 
@@ -2259,7 +3009,7 @@ int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>
     SI_OKR(ws.sq_c.reserve(sizeof(uint32_t) * nq));
     SI_OKR(ws.sq_id.reserve(sizeof(int32_t) * nq));
     SI_OKR(ws.qpair.reserve(2 * sizeof(S) * nq));
-    SI_OKR(ws.blk_cut.reserve(2 * sizeof(int64_t) * (size_t)nblk(nq)));
+    SI_OKR(ws.tile_recs.reserve(sizeof(TileRec<S>) * (size_t)nblk(nq)));
     // two radix passes (14 position bits) while they leave at most 64 queries on average to a key,
     // a quarter of a tile; else three (22 bits); four where the contigs alone would fill half of them
     int digits = nq <= ((int64_t)64 << 14) ? 2 : 3;
@@ -2284,15 +3034,93 @@ int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>
     k_pos_prep<S><<<nblk(nq), kThreads, 0, st>>>(
         in_alt ? ws.palt.as<uint32_t>() : ws.pay.as<uint32_t>(), in_alt ? ka[0] : kp[0], pos_bits, ws.qpair.as<S>(),
         nq, m, gs, ws.sq_s.as<S>(), ws.sq_u.as<int32_t>(), ws.sq_c.as<uint32_t>(), ws.sq_id.as<int32_t>(),
-        ws.long_split, ws.long_pos, ws.long_seg, ws.long_pos ? ws.blk_cut.as<int64_t>() : nullptr);
+        ws.long_split, ws.long_max, ws.long_pos, ws.long_seg, ws.tile_recs.as<TileRec<S>>());
     note_launch();
     SI_CU(cudaGetLastError());
     ws.launches += 2 + passes + 1;
     ws.prepared_qs = q.qs;
     ws.prepared_nq = nq;
     ws.prepared_mode = ub_mode;
-    ws.n_heads = nq;      // no head runs are kept (the emit finds them)
-    ws.cache_ok = false;  // and no candidate lists
+    ws.n_heads = 0;       // no head runs and no candidate lists are kept: batched_emit_ranked only
+    ws.cache_ok = false;
+    return SI_OK;
+}
+
+// Tile size: the largest of 256, 128, 64, 32 queries whose expected candidates, tile * (intervals
+// per query) + hits per query, fill at most 3/4 of the candidate slots (a tile that overflows them
+// emits its queries one by one).
+static int auto_tile(const BatchedParams& prm, int64_t n, int64_t nq, int64_t hits) {
+    if (!prm.auto_tile || hits < 0 || nq <= 0) return prm.tile_q;
+    const double per_q = (double)n / (double)nq, hpq = (double)hits / (double)nq;
+    int tile = kThreads;
+    while (tile > 32 && tile * per_q + hpq > 0.75 * prm.cap) tile >>= 1;
+    return tile;
+}
+
+template <typename S>
+int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, const RankGrid<S>& gs,
+                        const QueryBatch& q, int64_t q_offset, const int64_t* offsets, int64_t out_base, int order,
+                        int what, RankDest<S> dst, int* d_err, cudaStream_t st, int64_t total_hits) {
+    if (q.nq <= 0) return SI_OK;
+    if (q_offset < 0 || ws.prepared_nq < q_offset + q.nq) return SI_ERR_INVALID;
+    SI_OKR(ws.counters.reserve(sizeof(int) * 4));
+    SI_CU(cudaMemsetAsync(ws.counters.p, 0, sizeof(int) * 4, st));
+    EmitArgs<S> a;
+    a.P = make_pyr<S>(m, L, H);
+    a.PL.ends = static_cast<const S*>(ws.long_ends);
+    for (int h = 0; h < kMaxLevels; ++h) a.PL.m[h] = static_cast<const S*>(ws.long_lvl[h]);
+    a.PL.H = ws.long_H;
+    a.starts = m.starts;
+    a.data = m.data;
+    a.seg = m.seg;
+    a.G = m.G;
+    a.gs = gs;
+    a.long_pos = ws.long_pos;
+    a.long_start = static_cast<const S*>(ws.long_starts);
+    a.long_seg = ws.long_seg;
+    a.long_split = ws.long_split;
+    a.long_max = ws.long_max;
+    a.split_len = ws.prm.split_len;
+    a.nq = ws.prepared_nq;
+    a.tile_q = auto_tile(ws.prm, m.n, a.nq, total_hits);
+    a.cap = ws.prm.cap;
+    a.n_tiles = (int)ceil_div(a.nq, a.tile_q);
+    a.rec = a.tile_q == kThreads ? ws.tile_recs.as<TileRec<S>>() : nullptr;
+    a.sq_s = ws.sq_s.as<S>();
+    a.sq_u = ws.sq_u.as<int32_t>();
+    a.sq_c = ws.sq_c.as<uint32_t>();
+    a.sq_id = ws.sq_id.as<int32_t>();
+    a.tile_counter = ws.counters.as<int>();
+    a.offsets = offsets - q_offset;  // by the whole batch's ids
+    a.id_lo = q_offset;
+    a.id_hi = q_offset + q.nq;
+    a.out_base = out_base;
+    a.order = order;
+    a.values = what == kOutValue;
+    a.qe = static_cast<const S*>(q.qe) - q_offset;
+    a.dst = dst;
+    a.d_err = d_err;
+    const bool pieces = what == kOutPieces;
+    const size_t sm = sizeof(S) * 3 * (size_t)a.cap + 8 * (size_t)a.cap +
+                      (size_t)a.tile_q * (sizeof(S) * (pieces ? 2 : 1) + 28) + 256;
+    const void* fn = pieces ? reinterpret_cast<const void*>(&k_emit_tiles<S, kOutPieces>)
+                            : reinterpret_cast<const void*>(&k_emit_tiles<S, kOutIdx>);
+    const int e = pieces ? 3 : 2;
+    if (ws.occ_smem[e] != sm) {
+        int dev = 0, nsm = 152, per_sm = 1;
+        SI_CU(cudaGetDevice(&dev));
+        SI_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        SI_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, sm));
+        ws.occ_blocks[e] = nsm * std::max(per_sm, 1);
+        ws.occ_smem[e] = sm;
+    }
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ws.occ_blocks[e], a.n_tiles));
+    if (pieces) k_emit_tiles<S, kOutPieces><<<grid, kThreads, sm, st>>>(a);
+    else k_emit_tiles<S, kOutIdx><<<grid, kThreads, sm, st>>>(a);
+    note_launch();
+    SI_CU(cudaGetLastError());
+    ws.launches += 1;
     return SI_OK;
 }
 
@@ -2414,12 +3242,8 @@ int batched_emit(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, const Q
     // query, fill at most 3/4 of the candidate slots.  Tiles that overflow fall back to
     // per-query walks, which costs up to 25x at sparse batches.
     const int64_t batch_nq = (same || window) ? ws.prepared_nq : nq;
-    int tile = 0;
-    if (ws.prm.auto_tile && ws.end_sorted && total_hits >= 0 && batch_nq > 0) {
-        const double per_q = (double)m.n / (double)batch_nq, hpq = (double)total_hits / (double)batch_nq;
-        tile = kThreads;
-        while (tile > 32 && tile * per_q + hpq > 0.75 * ws.prm.cap) tile >>= 1;
-    }
+    const int tile = ws.prm.auto_tile && ws.end_sorted && total_hits >= 0 && batch_nq > 0
+                         ? auto_tile(ws.prm, m.n, batch_nq, total_hits) : 0;
     if (window)
         return run_tiles<S>(ws, m, L, H, ws.prepared_nq, true, nullptr, nullptr, ws.heads.as<int32_t>(),
                             offsets - q_offset, out_base, order, values, out, d_err, cache_fits && !tile, st,
@@ -2489,6 +3313,9 @@ int batched_coverage(BatchedWorkspace& ws, MapView<S> m, const QueryBatch& q, co
                                             cudaStream_t, uint32_t*, bool);                                                \
     template int batched_prepare_ranked<S>(BatchedWorkspace&, MapView<S>, const RankGrid<S>&, const QueryBatch&,  \
                                            const uint32_t*, int*, int, cudaStream_t);                            \
+    template int batched_emit_ranked<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const RankGrid<S>&,         \
+                                        const QueryBatch&, int64_t, const int64_t*, int64_t, int, int,            \
+                                        RankDest<S>, int*, cudaStream_t, int64_t);                               \
     template int batched_count<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const QueryBatch&, uint32_t*,   \
                                   int*, cudaStream_t);                                                          \
     template int batched_emit<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const QueryBatch&, int64_t,      \

@@ -66,6 +66,7 @@ struct BatchedWorkspace {
     DBuf qpair;                  // (start, end) or (start, upper bound) per query, interleaved: one
                                  // sector per gather
     DBuf blk_cut;                // per 256 sorted queries: (p_cut, long-list end) or -1, for the tiles
+    DBuf tile_recs;              // per 256 sorted queries of a ranked batch: its tile's record
     DBuf qminmax;                // smallest and largest query end (key packing)
     // sorted query records
     DBuf sq_s, sq_u, sq_c, sq_id;
@@ -84,16 +85,18 @@ struct BatchedWorkspace {
     int cache_prm_tile = 0, cache_prm_cap = 0;
     // tiles kernels (count, emit): dynamic shared memory their attribute was set for, and
     // resident blocks on the device at that size
-    size_t occ_smem[2] = {0, 0};
-    int occ_blocks[2] = {0, 0};
-    // long-interval list: global positions and ends of the intervals at least long_split long,
+    size_t occ_smem[4] = {0, 0, 0, 0};  // count, emit, ranked emit, ranked pieces
+    int occ_blocks[4] = {0, 0, 0, 0};
+    // long-interval list: global positions, starts and ends of the intervals at least long_split long,
     // in position order, its max pyramid (long_H levels) and each contig's first list index
     const void* long_ends = nullptr;
+    const void* long_starts = nullptr;
     const int32_t* long_pos = nullptr;
     const int64_t* long_seg = nullptr;
     const void* long_lvl[kMaxLevels] = {nullptr};
     int long_H = 0;
     int64_t long_split = 0;
+    int64_t long_max = 0;        // the longest interval's end - start, 64 bits read as unsigned
     // each contig's ends in ascending order (positions as the index), when no interval has
     // start > end: short queries are then counted from two ranks instead of the tile lists
     const void* end_sorted = nullptr;
@@ -130,6 +133,12 @@ int batched_prepare_queries(BatchedWorkspace& ws, MapView<S> m, const QueryBatch
 template <typename S>
 int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>& gs, const QueryBatch& q,
                            const uint32_t* su, int* d_err, int ub_mode, cudaStream_t st);
+// Emits queries [q_offset, q_offset + q.nq) of the batch prepared last by batched_prepare_ranked;
+// `what` is a RankOut other than keys.
+template <typename S>
+int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, const RankGrid<S>& gs,
+                        const QueryBatch& q, int64_t q_offset, const int64_t* offsets, int64_t out_base, int order,
+                        int what, RankDest<S> dst, int* d_err, cudaStream_t st, int64_t total_hits);
 template <typename S>
 int batched_count(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, const QueryBatch& q,
                   uint32_t* counts, int* d_err, cudaStream_t st);

@@ -146,11 +146,12 @@ __global__ void k_long_flags(const S* __restrict__ starts, const S* __restrict__
 template <typename S>
 __global__ void k_long_scatter(const S* __restrict__ starts, const S* __restrict__ ends, int64_t n, int64_t X,
                                const int64_t* __restrict__ offs, int64_t n_long, int64_t n_long_pad,
-                               int32_t* __restrict__ pos, S* __restrict__ lend) {
+                               int32_t* __restrict__ pos, S* __restrict__ lstart, S* __restrict__ lend) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n && long_iv(starts[i], ends[i], X)) {
         const int64_t k = offs[i];
         pos[k] = (int32_t)i;
+        lstart[k] = starts[i];
         lend[k] = ends[i];
     }
     if (i >= n_long && i < n_long_pad) {
@@ -182,20 +183,22 @@ __global__ void k_differs_i32(const int32_t* __restrict__ a, const int32_t* __re
 // out[0] += total length of the intervals at least X long; out[1] += the contigs' extents (last
 // start - first start + 1 over the sorted starts).  Their ratio is the depth of long intervals.
 // Integer sums (a length is clamped to 2^40, which leaves room for 2^23 such intervals per
-// block before the 64-bit total could wrap; the ratio only steers a path choice).
+// block before the 64-bit total could wrap; the ratio only steers a path choice).  out[2] = the
+// largest end - start of an interval with start <= end.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_long_depth(const S* __restrict__ starts, const S* __restrict__ ends,
                                                          int64_t n, const int64_t* __restrict__ seg, int G,
                                                          int64_t X, unsigned long long* __restrict__ out) {
     __shared__ unsigned long long red[kThreads / 32];
     constexpr unsigned long long kClamp = 1ull << 40;
-    unsigned long long a = 0, b = 0;
+    unsigned long long a = 0, b = 0, longest = 0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const int64_t s0 = (int64_t)starts[i], e0 = (int64_t)ends[i];
         const unsigned long long d = (unsigned long long)e0 - (unsigned long long)s0;  // e - s when e >= s
         if (e0 >= s0 && d >= (unsigned long long)(X - 1))                                 // length >= X
             a += d < kClamp ? d + 1ull : kClamp;
+        if (e0 >= s0 && d > longest) longest = d;
     }
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G; g += stride)
         if (seg[g + 1] > seg[g]) {
@@ -215,6 +218,11 @@ __global__ void __launch_bounds__(kThreads) k_long_depth(const S* __restrict__ s
         }
         __syncthreads();
     }
+    for (int d = 16; d > 0; d >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFull, longest, d);
+        longest = o > longest ? o : longest;
+    }
+    if ((threadIdx.x & 31) == 0 && longest) atomicMax(&out[2], longest);
 }
 
 // out[g] = offs[seg[g]]: first long-list index of each contig (g = 0..G)
@@ -612,10 +620,11 @@ cudaError_t launch_long_flags(const S* starts, const S* ends, int64_t n, int64_t
 template <typename S>
 cudaError_t launch_long_scatter(const S* starts, const S* ends, int64_t n, int64_t X, const int64_t* offs,
                                 int64_t n_long, int64_t n_long_pad, const int64_t* seg, int G, int32_t* pos,
-                                S* lend, int64_t* long_seg, cudaStream_t st) {
+                                S* lstart, S* lend, int64_t* long_seg, cudaStream_t st) {
     const int64_t m = std::max(n, n_long_pad);
     if (m > 0) {
-        k_long_scatter<S><<<blocks_for(m), kThreads, 0, st>>>(starts, ends, n, X, offs, n_long, n_long_pad, pos, lend);
+        k_long_scatter<S><<<blocks_for(m), kThreads, 0, st>>>(starts, ends, n, X, offs, n_long, n_long_pad, pos, lstart,
+                                                               lend);
         note_launch();
     }
     k_long_seg<<<blocks_for(G + 1), kThreads, 0, st>>>(offs, seg, G, long_seg);
@@ -626,7 +635,7 @@ cudaError_t launch_long_scatter(const S* starts, const S* ends, int64_t n, int64
 template <typename S>
 cudaError_t launch_long_depth(const S* starts, const S* ends, int64_t n, const int64_t* seg, int G, int64_t X,
                               unsigned long long* out, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), st);
+    cudaError_t e = cudaMemsetAsync(out, 0, 3 * sizeof(unsigned long long), st);
     if (e != cudaSuccess || n <= 0) return e;
     k_long_depth<S><<<(unsigned)std::min<int64_t>(blocks_for(std::max<int64_t>(n, G)), 152 * 4), kThreads, 0, st>>>(
         starts, ends, n, seg, G, X, out);
@@ -750,7 +759,7 @@ cudaError_t launch_branch(const S* ends, int64_t n, int64_t n_pad, Levels<S> L, 
     template cudaError_t launch_pyramid<S>(const S*, const int64_t*, int, S* const*, cudaStream_t); \
     template cudaError_t launch_long_flags<S>(const S*, const S*, int64_t, int64_t, uint32_t*, cudaStream_t); \
     template cudaError_t launch_long_scatter<S>(const S*, const S*, int64_t, int64_t, const int64_t*, int64_t, \
-                                                int64_t, const int64_t*, int, int32_t*, S*, int64_t*,        \
+                                                int64_t, const int64_t*, int, int32_t*, S*, S*, int64_t*,    \
                                                 cudaStream_t);                                               \
     template cudaError_t launch_branch<S>(const S*, int64_t, int64_t, Levels<S>, int,           \
                                           const int64_t*, int, int32_t*, cudaStream_t, void*, int*); \

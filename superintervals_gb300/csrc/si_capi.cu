@@ -154,7 +154,7 @@ struct gSuperIntervals {
     DevBuf starts, ends, data, branch, seg;
     DevBuf lvl[sig::kMaxLevels];
     // long-interval list: intervals >= kLongIntervalSplit long, position order, own pyramid
-    DevBuf long_pos, long_end, long_seg;
+    DevBuf long_pos, long_start, long_end, long_seg;
     DevBuf end_sorted;  // each contig's ends ascending (built when no interval has start > end)
     // exclusive prefix sums (mod 2^64) of the starts and of the sorted ends, for coverage from
     // ranks; built by the first such call after a build
@@ -512,26 +512,30 @@ int build_impl(gSuperIntervals* si) {
                                         sig::kLongIntervalSplit, sums, st));
         int64_t n_long = 0;
         int f = 0;
-        unsigned long long h[2] = {0, 0};
+        unsigned long long h[3] = {0, 0, 0};
         SI_CK(cudaMemcpyAsync(&n_long, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         SI_CK(cudaMemcpyAsync(&f, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
         SI_CK(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, st));
         SI_CK(cudaStreamSynchronize(st));
         si->inverted = f ? 1 : 0;
+        si->bws.long_max = (int64_t)h[2];  // as 64 unsigned bits
         si->long_depth = h[1] > 0 ? (double)h[0] / (double)h[1] : 0.0;
         const int64_t n_long_pad = sig::round_up(std::max<int64_t>(n_long, 1), 32);
         SI_TRY(si->long_pos.reserve(sizeof(int32_t) * n_long_pad));
+        SI_TRY(si->long_start.reserve(sizeof(S) * n_long_pad));
         SI_TRY(si->long_end.reserve(sizeof(S) * n_long_pad));
         SI_TRY(si->long_seg.reserve(sizeof(int64_t) * (G + 1)));
         si->long_H = sig::pyramid_levels(n_long_pad, si->long_sizes);
         for (int h2 = 1; h2 <= si->long_H; ++h2) SI_TRY(si->long_lvl[h2 - 1].reserve(sizeof(S) * si->long_sizes[h2]));
         SI_CK(sig::launch_long_scatter<S>(si->starts.as<S>(), ends, n, sig::kLongIntervalSplit, offs, n_long,
                                           n_long_pad, si->seg.as<int64_t>(), G, si->long_pos.as<int32_t>(),
-                                          si->long_end.as<S>(), si->long_seg.as<int64_t>(), st));
+                                          si->long_start.as<S>(), si->long_end.as<S>(), si->long_seg.as<int64_t>(),
+                                          st));
         S* llv[sig::kMaxLevels];
         for (int h2 = 0; h2 < sig::kMaxLevels; ++h2) llv[h2] = si->long_lvl[h2].as<S>();
         SI_CK(sig::launch_pyramid<S>(si->long_end.as<S>(), si->long_sizes, si->long_H, llv, st));
     }
+    si->bws.long_starts = si->long_start.p;
     si->bws.long_ends = si->long_end.p;
     si->bws.long_pos = si->long_pos.as<int32_t>();
     si->bws.long_seg = si->long_seg.as<int64_t>();
@@ -739,15 +743,16 @@ template <typename S>
 int rank_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, const int64_t* d_off, int64_t out_base,
               int order, bool values, int32_t* d_out, int lanes, int64_t P, cudaStream_t st) {
     PhaseTimer pt(si, 2, st);
+    sig::RankDest<S> d;
+    d.i32 = d_out;
+    const int what = values ? sig::kOutValue : sig::kOutIdx;
     if (lanes) {
-        sig::RankDest<S> d;
-        d.i32 = d_out;
         SI_CK(sig::launch_rank_emit<S>(view<S>(si), q, si->w_upper.as<uint32_t>() + q_offset, d_off, out_base, order,
-                                       values ? sig::kOutValue : sig::kOutIdx, d, lanes, si->w_err.as<int>(), st));
+                                       what, d, lanes, si->w_err.as<int>(), st));
         return SI_OK;
     }
-    const int r = sig::batched_emit<S>(si->bws, view<S>(si), levels<S>(si), si->H, q, q_offset, d_off, out_base, order,
-                                       values, d_out, si->w_err.as<int>(), si->ub_mode, st, P);
+    const int r = sig::batched_emit_ranked<S>(si->bws, view<S>(si), levels<S>(si), si->H, rank_grid<S>(si, 0), q,
+                                              q_offset, d_off, out_base, order, what, d, si->w_err.as<int>(), st, P);
     return r == SI_OK ? SI_OK : fail(r, "batched emit failed (status %d)", r);
 }
 

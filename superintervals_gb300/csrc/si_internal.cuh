@@ -176,7 +176,7 @@ template <typename S>
 cudaError_t launch_pyramid(const S* ends, const int64_t* sizes, int H, S* const* lvl,
                            cudaStream_t st);
 // long-interval list (end - start >= X) in position order: flags per interval; then, with
-// offs = exclusive scan of the flags (n + 1 entries), the positions and ends of the n_long
+// offs = exclusive scan of the flags (n + 1 entries), the positions, starts and ends of the n_long
 // long intervals padded to n_long_pad, and each contig's first list index (G + 1 entries)
 template <typename S>
 cudaError_t launch_long_flags(const S* starts, const S* ends, int64_t n, int64_t X, uint32_t* flags,
@@ -184,7 +184,7 @@ cudaError_t launch_long_flags(const S* starts, const S* ends, int64_t n, int64_t
 template <typename S>
 cudaError_t launch_long_scatter(const S* starts, const S* ends, int64_t n, int64_t X, const int64_t* offs,
                                 int64_t n_long, int64_t n_long_pad, const int64_t* seg, int G, int32_t* pos,
-                                S* lend, int64_t* long_seg, cudaStream_t st);
+                                S* lstart, S* lend, int64_t* long_seg, cudaStream_t st);
 // out[i] = branch[i] as a contig-local position (-1: none)
 cudaError_t launch_branch_local(const int32_t* branch, const int64_t* seg, int G, int64_t n, int64_t* out,
                                 cudaStream_t st);
@@ -206,7 +206,8 @@ cudaError_t launch_end_keys(const S* ends, int64_t n, const int64_t* seg, int G,
                             cudaStream_t st);
 template <typename S>
 cudaError_t launch_end_decode(const uint32_t* const* kw, int64_t n, int64_t n_pad, S* out, cudaStream_t st);
-// out[0] = total length of intervals at least X long, out[1] = total contig extent (sorted starts)
+// out[0] = total length of intervals at least X long, out[1] = total contig extent (sorted starts),
+// out[2] = the largest end - start
 template <typename S>
 cudaError_t launch_long_depth(const S* starts, const S* ends, int64_t n, const int64_t* seg, int G, int64_t X,
                               unsigned long long* out, cudaStream_t st);
