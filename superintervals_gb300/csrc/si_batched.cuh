@@ -96,6 +96,7 @@ struct BatchedWorkspace {
     const void* long_lvl[kMaxLevels] = {nullptr};
     int long_H = 0;
     int64_t long_split = 0;
+    double density = 0.0;        // intervals per coordinate over the contigs' extents
     int64_t long_max = 0;        // the longest interval's end - start, 64 bits read as unsigned
     // each contig's ends in ascending order (positions as the index), when no interval has
     // start > end: short queries are then counted from two ranks instead of the tile lists

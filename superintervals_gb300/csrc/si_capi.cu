@@ -519,6 +519,7 @@ int build_impl(gSuperIntervals* si) {
         SI_CK(cudaStreamSynchronize(st));
         si->inverted = f ? 1 : 0;
         si->bws.long_max = (int64_t)h[2];  // as 64 unsigned bits
+        si->bws.density = h[1] > 0 ? (double)n / (double)h[1] : 0.0;
         si->long_depth = h[1] > 0 ? (double)h[0] / (double)h[1] : 0.0;
         const int64_t n_long_pad = sig::round_up(std::max<int64_t>(n_long, 1), 32);
         SI_TRY(si->long_pos.reserve(sizeof(int32_t) * n_long_pad));

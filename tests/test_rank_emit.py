@@ -30,12 +30,16 @@ def _intervals(kind, n, rng):
     else:                                      # "far": a few intervals over everything
         ln = rng.integers(1, 60, n)
         ln[rng.random(n) < 0.002] = span
+    if kind == "deep":                         # sections of some 250 long intervals, few of them missed
+        ln = rng.integers(1, 60, n)
+        deep = rng.random(n) < 0.05
+        ln[deep] = rng.integers(100_000, 300_000, int(deep.sum()))
     return s, s + ln - 1, span
 
 
 @pytest.mark.parametrize("dt", [np.int32, np.int64])
-@pytest.mark.parametrize("kind", ["sparse", "runs", "far"])
-@pytest.mark.parametrize("nq", [1, 33, 4097, 32769, 262145])
+@pytest.mark.parametrize("kind,nq", [(k, q) for k in ("sparse", "runs", "far") for q in (1, 33, 4097, 32769, 262145)]
+                         + [("deep", q) for q in (1, 255, 4097, 32769)])
 def test_direct_emit_matches_oracle(api, oracle, kind, nq, dt):
     rng = np.random.default_rng(nq)
     n = 20_001
