@@ -1932,6 +1932,44 @@ int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStre
     return read_dev_err(si, st);
 }
 
+// Intersections and keys of a rank search: every hit gives one piece (a query with start > end none),
+// or one key, so the hits' offsets are the result's, and the emit writes the fields itself instead of
+// a hit list for a second pass.  Queues offsets and bounds; waits for the total.
+template <typename S>
+int field_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool keys, int64_t* d_off, cudaStream_t st,
+                  int64_t* P) {
+    int err = 0;
+    SI_TRY(rank_offsets<S>(si, q, !keys, d_off, st, P, &err));
+    return dev_status(si, err);
+}
+
+// The P pieces or keys of the batch counted last by field_offsets.  Dense keys go through hit lists:
+// a tile holds no start and payload of its candidates.
+template <typename S>
+int field_emit(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool keys, const int64_t* d_off,
+               sig::RankDest<S> d, int64_t P, cudaStream_t st) {
+    const int lanes = direct_lanes(si, q.nq, P);
+    const uint32_t* su = si->w_upper.as<uint32_t>();
+    int* err = si->w_err.as<int>();
+    if (lanes) {
+        SI_CK(sig::launch_rank_emit<S>(view<S>(si), q, su, d_off, 0, order, keys ? sig::kOutKeys : sig::kOutPieces, d,
+                                       lanes, err, st));
+        return SI_OK;
+    }
+    SI_TRY(rank_prepare<S>(si, q, lanes, st));
+    if (!keys) {
+        const int r = sig::batched_emit_ranked<S>(si->bws, view<S>(si), levels<S>(si), si->H, rank_grid<S>(si, 0), q, 0,
+                                                  d_off, 0, order, sig::kOutPieces, d, err, st, P);
+        return r == SI_OK ? SI_OK : fail(r, "batched emit failed (status %d)", r);
+    }
+    SI_TRY(si->so_hits.reserve(sizeof(int32_t) * std::max<int64_t>(P, 1)));
+    SI_TRY(rank_emit<S>(si, q, 0, d_off, 0, order, false, si->so_hits.as<int32_t>(), lanes, P, st));
+    sig::MapView<S> rv;
+    SI_TRY(view_rec<S>(si, st, &rv));
+    SI_CK(sig::launch_keys<S>(rv, q, d_off, si->so_hits.as<int32_t>(), d.s, d.e, d.i32, st));
+    return SI_OK;
+}
+
 // The gaps of each contig (no interval has start > end), made on the first difference after a build.
 template <typename S>
 int make_gaps(gSuperIntervals* si, cudaStream_t st) {
@@ -2019,6 +2057,16 @@ int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int orde
         if (T == 0) return SI_OK;
         if (!d_os || !d_oe) return fail(SI_ERR_INVALID, "null output buffer");
         SI_TRY(gap_emit<S>(si, q, d_off, d_os, d_oe, st));
+        return read_dev_err(si, st);
+    }
+    if (op == 0 && rank_search(si, q.nq)) {
+        int64_t P = 0;
+        SI_TRY(field_offsets<S>(si, q, false, d_off, st, &P));
+        if (total) *total = (size_t)P;
+        if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld pieces, capacity %zu", (long long)P, cap);
+        if (P == 0) return SI_OK;
+        if (!d_os || !d_oe || !d_ob) return fail(SI_ERR_INVALID, "null output buffer");
+        SI_TRY(field_emit<S>(si, q, order, false, d_off, {d_ob, d_os, d_oe}, P, st));
         return read_dev_err(si, st);
     }
     SI_TRY(si->w_err.reserve(2 * sizeof(int)));
@@ -2118,6 +2166,10 @@ int setop_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc,
     if (op == 0) SI_TRY(si->so_ob.reserve(sizeof(int32_t) * T));
     if (op == 1 && use_ranks(si, q.nq) && si->gaps_ready) {
         SI_TRY(gap_emit<S>(si, q, si->so_off.as<int64_t>(), si->so_os.as<S>(), si->so_oe.as<S>(), si->st));
+    } else if (op == 0 && rank_search(si, q.nq)) {
+        SI_TRY(field_emit<S>(si, q, order, false, si->so_off.as<int64_t>(),
+                             {si->so_ob.as<int32_t>(), si->so_os.as<S>(), si->so_oe.as<S>()}, (int64_t)T, si->st));
+        SI_TRY(read_dev_err(si));
     } else {
         // the hit lists are still in place: emit the pieces only
         const int64_t* hoff = si->so_hoff.as<int64_t>();
@@ -2234,6 +2286,15 @@ int keys_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_
         return SI_OK;
     }
     int64_t P = 0;
+    if (rank_search(si, q.nq)) {
+        SI_TRY(field_offsets<S>(si, q, true, d_off, st, &P));
+        if (total) *total = (size_t)P;
+        if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld keys, capacity %zu", (long long)P, cap);
+        if (P == 0) return SI_OK;
+        if (!d_s || !d_e) return fail(SI_ERR_INVALID, "null output buffer");
+        SI_TRY(field_emit<S>(si, q, order, true, d_off, {d_d, d_s, d_e}, P, st));
+        return read_dev_err(si, st);
+    }
     SI_TRY(lists_or_empty<S>(si, q, order, st, &P));
     SI_CK(cudaMemcpyAsync(d_off, si->so_hoff.p, sizeof(int64_t) * (q.nq + 1), cudaMemcpyDeviceToDevice, st));
     if (total) *total = (size_t)P;
@@ -2367,19 +2428,29 @@ extern "C" int searchKeysBatchGpu(gSuperIntervals* si, const void* qs, const voi
     SI_TRY(si->so_os.reserve(sb * T));
     SI_TRY(si->so_oe.reserve(sb * T));
     if (data) SI_TRY(si->so_ob.reserve(sizeof(int32_t) * T));
-    // the hit lists are still in place: gather only
-    sig::MapView<int64_t> rv64;
-    sig::MapView<int32_t> rv32;
-    if (si->bits == 64) SI_TRY(view_rec<int64_t>(si, si->st, &rv64));
-    else SI_TRY(view_rec<int32_t>(si, si->st, &rv32));
-    if (si->bits == 64)
-        SI_CK(sig::launch_keys<int64_t>(rv64, q, si->so_hoff.as<int64_t>(), si->so_hits.as<int32_t>(),
-                                        si->so_os.as<int64_t>(), si->so_oe.as<int64_t>(),
-                                        data ? si->so_ob.as<int32_t>() : nullptr, si->st));
-    else
-        SI_CK(sig::launch_keys<int32_t>(rv32, q, si->so_hoff.as<int64_t>(), si->so_hits.as<int32_t>(),
-                                        si->so_os.as<int32_t>(), si->so_oe.as<int32_t>(),
-                                        data ? si->so_ob.as<int32_t>() : nullptr, si->st));
+    if (rank_search(si, q.nq)) {  // counted and bounded: emit only
+        int32_t* od = data ? si->so_ob.as<int32_t>() : nullptr;
+        r = si->bits == 64 ? field_emit<int64_t>(si, q, order, true, si->so_off.as<int64_t>(),
+                                                 {od, si->so_os.as<int64_t>(), si->so_oe.as<int64_t>()}, (int64_t)T, si->st)
+                           : field_emit<int32_t>(si, q, order, true, si->so_off.as<int64_t>(),
+                                                 {od, si->so_os.as<int32_t>(), si->so_oe.as<int32_t>()}, (int64_t)T, si->st);
+        SI_TRY(r);
+        SI_TRY(read_dev_err(si));
+    } else {
+        // the hit lists are still in place: gather only
+        sig::MapView<int64_t> rv64;
+        sig::MapView<int32_t> rv32;
+        if (si->bits == 64) SI_TRY(view_rec<int64_t>(si, si->st, &rv64));
+        else SI_TRY(view_rec<int32_t>(si, si->st, &rv32));
+        if (si->bits == 64)
+            SI_CK(sig::launch_keys<int64_t>(rv64, q, si->so_hoff.as<int64_t>(), si->so_hits.as<int32_t>(),
+                                            si->so_os.as<int64_t>(), si->so_oe.as<int64_t>(),
+                                            data ? si->so_ob.as<int32_t>() : nullptr, si->st));
+        else
+            SI_CK(sig::launch_keys<int32_t>(rv32, q, si->so_hoff.as<int64_t>(), si->so_hits.as<int32_t>(),
+                                            si->so_os.as<int32_t>(), si->so_oe.as<int32_t>(),
+                                            data ? si->so_ob.as<int32_t>() : nullptr, si->st));
+    }
     SI_CK(cudaMemcpyAsync(starts, si->so_os.p, sb * T, cudaMemcpyDeviceToHost, si->st));
     SI_CK(cudaMemcpyAsync(ends, si->so_oe.p, sb * T, cudaMemcpyDeviceToHost, si->st));
     if (data) SI_CK(cudaMemcpyAsync(data, si->so_ob.p, sizeof(int32_t) * T, cudaMemcpyDeviceToHost, si->st));

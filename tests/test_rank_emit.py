@@ -67,6 +67,23 @@ def test_direct_emit_matches_oracle(api, oracle, kind, nq, dt):
                 _, _, data, _ = idx.arrays()
                 want = data[want + np.repeat(seg[qc], np.diff(want_off))]
             assert np.array_equal(out, want)
+    # the fields written by the emit itself: pieces (none for start > end) and keys
+    sorted_s, sorted_e, data, _ = idx.arrays()
+    for path in (api.PATH_AUTO, api.PATH_BATCHED):
+        idx.set_path(path)
+        for order in (0, 1):
+            want_off, want = oracle.search_batch(m, qs, qe, qc, order=order, nthreads=8)
+            at = want + np.repeat(seg[qc], np.diff(want_off))
+            off, ks, ke, kd = idx.search_keys(qs, qe, qc, order=order, with_data=True)
+            assert np.array_equal(off, want_off) and np.array_equal(kd, data[at])
+            assert np.array_equal(ks, sorted_s[at]) and np.array_equal(ke, sorted_e[at])
+            owner = np.repeat(np.arange(nq), np.diff(want_off))
+            keep = (qs <= qe)[owner]
+            off, ps, pe, ph = idx.intersect(qs, qe, qc, order=order)
+            assert np.array_equal(off, np.concatenate([[0], np.cumsum(np.bincount(owner[keep], minlength=nq))]))
+            assert np.array_equal(ph, want[keep])
+            assert np.array_equal(ps, np.maximum(qs[owner], sorted_s[at])[keep])
+            assert np.array_equal(pe, np.minimum(qe[owner], sorted_e[at])[keep])
     idx.set_path(api.PATH_AUTO)
     want_off, want = oracle.search_batch(m, qs, qe, qc, order=0, nthreads=8)
     idx.set_output_budget(1 << 20)                            # host results in chunks
