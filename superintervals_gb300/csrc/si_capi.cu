@@ -709,22 +709,22 @@ int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int
 }
 
 // The direct emit's lanes per query for a batch of nq queries and P hits, 0 for the sorted tiles.
-// The tiles cost some 100 us (sort, records, tile set-up) and 0.36 ns a query more than the direct
-// emit, which costs some 13 ps a hit more: they pay from about 10 M + 30 hits a query on.  Measured
-// (whole calls, tiles / direct): 3 M queries with 25, 33, 51, 126 hits 1526 / 1313, 1418 / 1130,
-// 1426 / 2703, 2306 / 5551 us; 100 k with 126 and 128 hits 375 / 264, 683 / 390 us; 300 k with 126
-// hits 549 / 690 us.  Where even the smallest tile's candidates (intervals between its queries, and
-// the hits of one) would not fit its lists the direct emit is better at any count (100 k queries
-// with 640 hits over 5 M intervals: 4984 / 2535 us).
+// The tiles cost some 75 us (sort, records, tile set-up), 0.19 ns a query and 20 ps an interval (each
+// is gathered by some tile) more than the direct emit; that costs 11 ps a hit more, or 20 where most
+// hits are long intervals lying far apart, each a step of the walk.  Measured (whole calls of 3 M
+// queries, tiles / direct): 10, 25, 126 near hits 1106 / 706, 1122 / 1317, 1841 / 5541 us; 10, 51
+// far ones 952 / 569, 1158 / 2701 us; 300 k queries over 12 M intervals with 79 near hits 590 / 375 us.
+// A query of many far hits is a long chain of dependent reads whatever the batch: 100 queries with
+// 639 of them 202 / 516 us.
 // Lanes: small batches leave lanes idle, so a warp serves one query; large ones fill the device, and
-// few lanes waste less on queries whose hits are few or far apart (3 M queries with 10 far hits: 567
-// us at 2 lanes, 1095 at 8, 2585 at 32), while dense hits want wider chunks (25 hits: 1402, 1313).
+// few lanes waste less on queries whose hits are few or far apart (3 M queries with 10 far hits: 569
+// us at 2 lanes, 1097 at 8, 2589 at 32), while dense hits want wider chunks (25 hits: 1403, 1317;
+// 300 k queries with 79 hits: 803, 468, 375).
 int direct_lanes(const gSuperIntervals* si, int64_t nq, int64_t P) {
     if (si->path != SI_PATH_AUTO) return 0;
-    const bool fits = 32.0 * (double)si->n / (double)nq + (double)P / (double)nq <= 0.75 * si->bws.prm.cap;
-    if (fits && P > 10000000 + 30 * nq) return 0;
-    const bool far = si->long_depth * (double)nq > 0.5 * (double)P;  // most hits are long intervals, far apart
-    if (nq <= (far ? 4096 : 32768)) return 32;
+    const bool far = si->long_depth * (double)nq > 0.5 * (double)P;
+    if (far ? P > 4000000 + 10 * nq + si->n || P > 160 * nq : P > 7000000 + 17 * nq + 9 * si->n / 5) return 0;
+    if (nq <= (far ? 4096 : P > 30 * nq ? 524288 : 32768)) return 32;
     if (nq <= 262144) return 8;
     return !far && P > 16 * nq ? 8 : 2;
 }
