@@ -1703,7 +1703,7 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_emit_tiles(EmitArgs<S> a) 
                     }
                     umax = um;
                     if (warp == 0) {
-                        const GridContig c = load_contig(a.gs.c + g);
+                        const GridContig<S> c = load_contig(a.gs.c + g);
                         const int64_t pc = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(L, a.long_split));
                         const int64_t pw = (int64_t)grid_first_geq<S>(a.gs, c, near_threshold<S>(L, a.long_max));
                         const int64_t ch = warp_first_pos_geq(a.long_pos, a.long_seg[g], a.long_seg[g + 1], pc, lane);
@@ -1782,7 +1782,7 @@ __global__ void __launch_bounds__(kThreads, BLOCKS) k_emit_tiles(EmitArgs<S> a) 
                 // a warp takes some queries at a time and finds their stretches one query per LANE
                 // (a handful of dependent reads each), then writes them one after another
                 const int per = min(32, (r1 - r0 + kWarpsPerCta - 1) / kWarpsPerCta);
-                const GridContig c = load_contig(a.gs.c + g);
+                const GridContig<S> c = load_contig(a.gs.c + g);
                 const int64_t l0 = a.long_seg[g], l1 = a.long_seg[g + 1];
                 for (int b = r0 + warp * per; b < r1; b += kWarpsPerCta * per) {
                     const int mine = b + lane, nb = min(per, r1 - b);
@@ -2505,7 +2505,7 @@ __global__ void __launch_bounds__(kThreads) k_pos_prep(const uint32_t* __restric
                 r.umax = max(r.umax, s_um[w]);
             }
             const int g = (int)s_code[0];
-            const GridContig c = load_contig(gs.c + g);
+            const GridContig<S> c = load_contig(gs.c + g);
             r.pcut = (int64_t)grid_first_geq<S>(gs, c, near_threshold<S>(r.L, long_split));
             const int64_t pw = (int64_t)grid_first_geq<S>(gs, c, near_threshold<S>(r.L, long_max));
             r.c_hi = warp_first_pos_geq(long_pos, long_seg[g], long_seg[g + 1], r.pcut, lane);

@@ -131,10 +131,10 @@ void dev_release(void** p, size_t* bytes) {
 }  // namespace sig
 
 // Rank grids over one or two arrays of the same contigs: per array the contig records, t1 and t2
-// words (si_rank.cuh), in one allocation.
+// words and offsets (si_rank.cuh), in one allocation.
 struct GridSet {
     DevBuf buf;
-    size_t at[2][3] = {{0, 0, 0}, {0, 0, 0}};  // byte offsets of [array][contigs, t1, t2]
+    size_t at[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};  // byte offsets of [array][contigs, t1, t2, offsets]
 };
 
 struct gSuperIntervals {
@@ -358,9 +358,10 @@ sig::RankGrid<S> grid_view(const GridSet& g, const S* arr, int which) {
     const char* p = g.buf.as<char>();
     sig::RankGrid<S> R;
     R.arr = arr;
-    R.c = reinterpret_cast<const sig::GridContig*>(p + g.at[which][0]);
+    R.c = reinterpret_cast<const sig::GridContig<S>*>(p + g.at[which][0]);
     R.t1 = reinterpret_cast<const uint32_t*>(p + g.at[which][1]);
     R.t2 = reinterpret_cast<const uint32_t*>(p + g.at[which][2]);
+    R.lo = reinterpret_cast<const uint16_t*>(p + g.at[which][3]);
     return R;
 }
 
@@ -379,10 +380,10 @@ int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vect
     base.resize(G);
     const int64_t w1 = sig::grid_t1_words(segv.data(), G, base.data()), w2 = sig::grid_t2_words(n);
     size_t at = (sizeof(uint32_t) * (size_t)G + 255) & ~(size_t)255;
-    const size_t parts[3] = {sizeof(sig::GridContig) * (size_t)G, sizeof(uint32_t) * (size_t)w1,
-                             sizeof(uint32_t) * (size_t)w2};
+    const size_t parts[4] = {sizeof(sig::GridContig<S>) * (size_t)G, sizeof(uint32_t) * (size_t)w1,
+                             sizeof(uint32_t) * (size_t)w2, sizeof(uint16_t) * (size_t)(n + 16)};
     for (int a = 0; a < (a1 ? 2 : 1); ++a)
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 4; ++k) {
             g.at[a][k] = at;
             at += (parts[k] + 255) & ~(size_t)255;
         }
@@ -391,9 +392,10 @@ int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vect
     SI_CK(cudaMemcpyAsync(p, base.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, st));
     for (int a = 0; a < (a1 ? 2 : 1); ++a)
         SI_CK(sig::launch_grid_build<S>(a ? a1 : a0, n, d_seg, G, reinterpret_cast<uint32_t*>(p), w1,
-                                        reinterpret_cast<sig::GridContig*>(p + g.at[a][0]),
+                                        reinterpret_cast<sig::GridContig<S>*>(p + g.at[a][0]),
                                         reinterpret_cast<uint32_t*>(p + g.at[a][1]),
-                                        reinterpret_cast<uint32_t*>(p + g.at[a][2]), st));
+                                        reinterpret_cast<uint32_t*>(p + g.at[a][2]),
+                                        reinterpret_cast<uint16_t*>(p + g.at[a][3]), st));
     return SI_OK;
 }
 

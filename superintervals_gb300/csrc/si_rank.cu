@@ -30,17 +30,15 @@ __host__ __device__ __forceinline__ uint32_t grid_cap(int64_t n) {
 
 template <typename S>
 __global__ void k_grid_params(const S* __restrict__ arr, const int64_t* __restrict__ seg, int G,
-                              const uint32_t* __restrict__ base, GridContig* __restrict__ out) {
+                              const uint32_t* __restrict__ base, GridContig<S>* __restrict__ out) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G) return;
     const int64_t lo = seg[g], hi = seg[g + 1];
-    GridContig c{};
-    c.lo = (uint32_t)lo;
-    c.hi = (uint32_t)hi;
+    GridContig<S> c{};
     c.base = base[g];
     if (hi > lo) {
-        c.k0 = (int64_t)arr[lo];
-        const uint64_t span = (uint64_t)(int64_t)arr[hi - 1] - (uint64_t)c.k0;
+        c.k0 = arr[lo];
+        const uint64_t span = (uint64_t)(int64_t)arr[hi - 1] - (uint64_t)(int64_t)arr[lo];
         const uint32_t cap = grid_cap(hi - lo);
         uint32_t sh = 0;
         while ((span >> sh) >= cap) ++sh;  // at most 63: span >> 63 is below cap
@@ -50,14 +48,13 @@ __global__ void k_grid_params(const S* __restrict__ arr, const int64_t* __restri
     out[g] = c;
 }
 
-// First position in [a, b) with arr >= v, as offset keys (key - k0, unsigned).
+// First position in [a, b) with arr >= k0 + off.
 template <typename S>
-__device__ __forceinline__ uint32_t first_off(const S* __restrict__ arr, uint32_t a, uint32_t b, int64_t k0,
-                                              uint64_t off) {
+__device__ __forceinline__ uint32_t first_off(const S* __restrict__ arr, uint32_t a, uint32_t b, S k0, uint64_t off) {
     uint32_t len = b - a;
     while (len > 0) {
         const uint32_t half = len >> 1;
-        const bool below = (uint64_t)(int64_t)arr[a + half] - (uint64_t)k0 < off;
+        const bool below = (uint64_t)(int64_t)arr[a + half] - (uint64_t)(int64_t)k0 < off;
         a = below ? a + half + 1 : a;
         len = below ? len - half - 1 : half;
     }
@@ -67,26 +64,29 @@ __device__ __forceinline__ uint32_t first_off(const S* __restrict__ arr, uint32_
 // t1: one thread per bucket word, a halving search each.  Neighbouring threads search for
 // neighbouring keys, so their reads fall on the same lines.
 template <typename S>
-__global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ arr, int G,
-                                                        const uint32_t* __restrict__ base,
-                                                        const GridContig* __restrict__ cs, uint32_t words,
+__global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ arr, const int64_t* __restrict__ seg,
+                                                        int G, const uint32_t* __restrict__ base,
+                                                        const GridContig<S>* __restrict__ cs, uint32_t words,
                                                         uint32_t* __restrict__ t1) {
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= words) return;
-    const GridContig c = cs[owner(base, G, i)];
+    const int g = owner(base, G, i);
+    const GridContig<S> c = cs[g];
     const uint32_t j = i - c.base;
     if (j > c.nb) return;
-    t1[i] = j == 0 ? c.lo : j == c.nb ? c.hi : first_off(arr, c.lo, c.hi, c.k0, (uint64_t)j << c.shift);
+    const uint32_t lo = (uint32_t)seg[g], hi = (uint32_t)seg[g + 1];
+    t1[i] = j == 0 ? lo : j == c.nb ? hi : first_off(arr, lo, hi, c.k0, (uint64_t)j << c.shift);
 }
 
-// t2: one thread per position.  A position of a crowded bucket writes itself to the words of the
+// Offsets and t2: one thread per position.  A position of a crowded bucket writes itself to the words of the
 // sub-buckets after its predecessor's up to its own (at most 1024), the bucket's last position also
 // the rest.  Coalesced reads and no search: 20 M clustered 64-bit keys took 7.6 ms with a warp per
 // bucket searching every word.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr, const int64_t* __restrict__ seg,
-                                                       int G, int64_t n, const GridContig* __restrict__ cs,
-                                                       const uint32_t* __restrict__ t1, uint32_t* __restrict__ t2) {
+                                                       int G, int64_t n, const GridContig<S>* __restrict__ cs,
+                                                       const uint32_t* __restrict__ t1, uint32_t* __restrict__ t2,
+                                                       uint16_t* __restrict__ lo) {
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     int g = 0;
@@ -95,8 +95,9 @@ __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr
         if (seg[mid] <= i) g = mid;
         else hi = mid - 1;
     }
-    const GridContig c = cs[g];
-    const uint64_t d = (uint64_t)(int64_t)arr[i] - (uint64_t)c.k0;
+    const GridContig<S> c = cs[g];
+    const uint64_t d = (uint64_t)(int64_t)arr[i] - (uint64_t)(int64_t)c.k0;
+    lo[i] = (uint16_t)((uint32_t)d & ((1u << min(c.shift, 16u)) - 1u));
     const uint32_t* t = t1 + c.base + (uint32_t)(d >> c.shift);
     const uint32_t a = t[0], e = t[1], cnt = e - a;
     if (cnt < kGridDense) return;
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr
     const uint32_t r = (uint32_t)(d >> ss) & last;
     uint32_t from = 0;
     if ((uint32_t)i > a) {
-        const uint64_t dp = (uint64_t)(int64_t)arr[i - 1] - (uint64_t)c.k0;
+        const uint64_t dp = (uint64_t)(int64_t)arr[i - 1] - (uint64_t)(int64_t)c.k0;
         from = ((uint32_t)(dp >> ss) & last) + 1u;
     }
     uint32_t* __restrict__ w = t2 + grid_sub_base(a);
@@ -155,17 +156,18 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
         } else {
             s = qs[q];
             const S e = qe[q];
-            const GridContig c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
-            lo = c1.lo;
+            const GridContig<S> c1 = load_contig(gs.c + g);
+            const bool any = c1.nb != 0 && e >= c1.k0;  // some start at or below the query's end
             if (s <= e) {
                 uint32_t r2;
-                grid_two_ranks(gs, c1, e, ge, c2, s, top, r2);
+                grid_two_ranks(gs, c1, e, ge, load_contig(ge.c + g), s, top, r2);
                 cnt = top > r2 ? top - r2 : 0u;
             } else {
                 top = grid_first_gt<S>(gs, c1, e);
-                walk = !pieces && top > lo;
+                walk = !pieces && any;
+                lo = walk ? (uint32_t)m.seg[g] : 0u;
             }
-            upper = top > lo && (s <= e || !pieces) ? top : 0u;
+            upper = any && (s <= e || !pieces) ? top : 0u;
         }
     }
     unsigned todo = __ballot_sync(kFull, walk);
@@ -185,8 +187,10 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
 // walked by their warp.
 // Bound by random sector reads (ncu at 12.5 M x 12.5 M int32: L2 75%, DRAM 63% of peak, 5.0 TB/s;
 // issue 23%).  One query per thread keeps 92% of the warps resident to cover the four dependent
-// reads.  12.5 M random queries: 372 us; 990 us through the sorted batch (sort, gather and
-// scattered count write).  2-4 or 8-16 entries a bucket instead of 4-8: 408 and 409 us.
+// reads.  12.5 M random queries: 267 us (371 us halving over the coordinates instead of packed
+// offsets); 990 us through the sorted batch (sort, gather and scattered count write).  2-4 or 8-16
+// entries a bucket instead of 4-8: 296 and 287 us.  A word pair per bucket, so that both table words
+// come in one read: 319 us (twice the table).  Contig records in shared memory: 352 us.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
                                                          const S* __restrict__ qs, const S* __restrict__ qe,
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
     if (q < nq) counts[q] = cnt;
 }
 
-// 20 M random 64-bit queries over 20 M keys, 70% of both in hotspots: 267 us; 2.31 ms through the
+// 20 M random 64-bit queries over 20 M keys, 70% of both in hotspots: 218 us; 2.31 ms through the
 // sorted batch, whose search windows a hotspot overflows.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, const S* __restrict__ qe,
@@ -212,8 +216,9 @@ __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, con
         out[q] = -1;
         return;
     }
-    const GridContig c = load_contig(gs.c + g);
-    out[q] = (int32_t)(grid_first_gt<S>(gs, c, qe[q]) - c.lo) - 1;
+    const GridContig<S> c = load_contig(gs.c + g);
+    const uint32_t r = grid_first_gt<S>(gs, c, qe[q]);
+    out[q] = (int32_t)(r - (qc ? __ldg(gs.t1 + c.base) : 0u)) - 1;  // without contig ids: contig 0
 }
 
 // Coverage of a query with qs <= qe, over the hits {start <= qe} minus {end < qs}:
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, con
 // with a_u the first start > qe, r_qs / r_qe the first sorted ends >= qs / > qe, ls the first
 // start >= qs, and PS / PE the exclusive prefix sums (mod 2^64) of the starts and of the sorted
 // ends.  The coverage, sum min - sum max, wraps as the coordinate type does.
-// 5 M x 5 M: 374 us for the call; 853 us through the sorted batch and three block searches.
+// 5 M x 5 M: 288 us for the call; 853 us through the sorted batch and three block searches.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<S> ge, int G,
                                                        const S* __restrict__ qs, const S* __restrict__ qe,
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<
         cov[q] = 0;
         return;
     }
-    const GridContig c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
+    const GridContig<S> c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
     uint32_t a_u, r_qs, r_qe, ls;
     grid_two_ranks(gs, c1, e, ge, c2, s, a_u, r_qs);
     grid_two_ranks(ge, c2, e, gs, c1, s, r_qe, ls);
@@ -297,7 +302,8 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
     for (int r = 0; r < R; ++r) {
         const int64_t q = base + r * kWarp;
         uint32_t upper;
-        const int64_t x = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, pieces != 0, &work->err, lane, upper);
+        const int64_t x = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, pieces != 0, &work->err, lane,
+                                      upper);
         if (q < nq) su[q] = upper;
         int64_t inc = x;
 #pragma unroll
@@ -575,10 +581,11 @@ int64_t grid_t1_words(const int64_t* seg, int G, uint32_t* base) {
 
 template <typename S>
 cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G, const uint32_t* d_base,
-                              int64_t t1_words, GridContig* c, uint32_t* t1, uint32_t* t2, cudaStream_t st) {
+                              int64_t t1_words, GridContig<S>* c, uint32_t* t1, uint32_t* t2, uint16_t* lo,
+                              cudaStream_t st) {
     k_grid_params<S><<<blocks_for(G), kThreads, 0, st>>>(arr, seg, G, d_base, c);
-    k_grid_fill<S><<<blocks_for(t1_words), kThreads, 0, st>>>(arr, G, d_base, c, (uint32_t)t1_words, t1);
-    k_grid_sub<S><<<blocks_for(n), kThreads, 0, st>>>(arr, seg, G, n, c, t1, t2);
+    k_grid_fill<S><<<blocks_for(t1_words), kThreads, 0, st>>>(arr, seg, G, d_base, c, (uint32_t)t1_words, t1);
+    k_grid_sub<S><<<blocks_for(n), kThreads, 0, st>>>(arr, seg, G, n, c, t1, t2, lo);
     note_launch(3);
     return cudaGetLastError();
 }
@@ -705,7 +712,7 @@ cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32
 
 #define SIG_RINST(S)                                                                                            \
     template cudaError_t launch_grid_build<S>(const S*, int64_t, const int64_t*, int, const uint32_t*, int64_t,  \
-                                              GridContig*, uint32_t*, uint32_t*, cudaStream_t);                  \
+                                              GridContig<S>*, uint32_t*, uint32_t*, uint16_t*, cudaStream_t);       \
     template cudaError_t launch_rank_count<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, uint32_t*, int*, \
                                               cudaStream_t);                                                     \
     template cudaError_t launch_rank_scan<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, bool, uint32_t*,  \

@@ -11,7 +11,12 @@
 // the bucket's first position, so that no second index is needed (a bucket of n entries uses at
 // most n/4 + 1 words).  Any bucket still crowded after that is searched by halving: the answer is
 // exact for every distribution, only the number of reads changes.
-// Memory: 2.5 bytes per entry and array (t1 1, t2 1.5), beside 4 or 8 for the coordinates.
+// Inside buckets at most 65536 wide the entries are compared by their 16-bit offsets from the bucket's
+// first coordinate, eight to a 16-byte read (four packed compares), not by halving over the coordinates:
+// the usual bucket is one read instead of two or three dependent ones, and the tables and offsets of
+// an 8 M-interval index, starts and ends, are 58 MB, which the L2 keeps; the coordinates alone are
+// 64 MB of 32 bits, 128 MB of 64.
+// Memory: at most 4.5 bytes per entry and array (t1 1, t2 1.5, offsets 2), beside 4 or 8 for the coordinates.
 #pragma once
 #include "si_internal.cuh"
 
@@ -21,35 +26,40 @@ constexpr uint32_t kGridFill = 4;    // at most n / kGridFill buckets: 4-8 entri
 constexpr uint32_t kGridDense = 32;  // entries from which a bucket has its own table (>= 24: see above)
 constexpr int kGridSubBits = 10;     // at most 1024 words of t2 per bucket
 
-struct alignas(32) GridContig {
-    int64_t k0;       // smallest key of the contig
-    uint32_t lo, hi;  // its positions
-    uint32_t base;    // its first word in t1 (nb + 1 words: the last one is hi)
-    uint32_t nb;      // buckets (0: empty contig)
-    uint32_t shift;   // bucket width 2^shift
-    uint32_t pad;
+// A contig's buckets.  Its first position is t1[base], its end t1[base + nb].
+template <typename S>
+struct GridContig;
+template <>
+struct alignas(16) GridContig<int32_t> {
+    int32_t k0;      // smallest key
+    uint32_t base;   // first word in t1 (nb + 1 words)
+    uint32_t nb;     // buckets (0: empty contig)
+    uint32_t shift;  // bucket width 2^shift (offsets are kept up to 16)
+};
+template <>
+struct alignas(16) GridContig<int64_t> {
+    int64_t k0;
+    uint32_t base, nb, shift, pad[3];
 };
 
 template <typename S>
 struct RankGrid {
     const S* arr = nullptr;          // ascending inside each contig
-    const GridContig* c = nullptr;
-    const uint32_t* t1 = nullptr;
+    const GridContig<S>* c = nullptr;
+    const uint32_t* t1 = nullptr;    // per bucket: its first position (then the contig's end)
     const uint32_t* t2 = nullptr;
+    const uint16_t* lo = nullptr;    // offsets inside buckets of contigs with shift <= 16
 };
 
-__device__ __forceinline__ GridContig load_contig(const GridContig* __restrict__ p) {
-    const int4* q = reinterpret_cast<const int4*>(p);
-    const int4 a = __ldg(q), b = __ldg(q + 1);
-    GridContig c;
-    c.k0 = (int64_t)(((uint64_t)(uint32_t)a.y << 32) | (uint32_t)a.x);
-    c.lo = (uint32_t)a.z;
-    c.hi = (uint32_t)a.w;
-    c.base = (uint32_t)b.x;
-    c.nb = (uint32_t)b.y;
-    c.shift = (uint32_t)b.z;
-    c.pad = 0;
-    return c;
+template <typename S>
+__device__ __forceinline__ GridContig<S> load_contig(const GridContig<S>* __restrict__ p) {
+    union {
+        GridContig<S> c;
+        int4 q[sizeof(GridContig<S>) / 16];
+    } u;
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(GridContig<S>) / 16); ++k) u.q[k] = reinterpret_cast<const int4*>(p)[k];
+    return u.c;
 }
 
 // log2 of the sub-buckets of a bucket holding cnt >= kGridDense entries
@@ -60,25 +70,19 @@ __device__ __forceinline__ int grid_sub_bits(uint32_t cnt, uint32_t shift) {
 __device__ __forceinline__ uint32_t grid_sub_base(uint32_t first) { return (uint32_t)((3ull * first + 7) >> 3); }
 
 // The positions [a, a + len) among which the first entry >= v of the contig lies (a + len when none
-// of them is): len is 0 where the tables alone give the answer.
+// of them is): len is 0 where the tables alone give the answer.  off: v's offset in its bucket.
 template <typename S>
-__device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridContig& c, S v, uint32_t& a,
-                                             uint32_t& len) {
-    a = c.lo;
-    len = 0;
-    if (c.nb == 0 || (int64_t)v <= c.k0) return;
-    const uint64_t d = (uint64_t)(int64_t)v - (uint64_t)c.k0;
+__device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridContig<S>& c, S v, uint32_t& a,
+                                             uint32_t& len, uint32_t& off) {
+    const uint64_t d = (uint64_t)(int64_t)v - (uint64_t)(int64_t)c.k0;
     const uint64_t b = d >> c.shift;
-    if (b >= c.nb) {
-        a = c.hi;
-        return;
-    }
-    const uint32_t* t = R.t1 + c.base + (uint32_t)b;
-    a = __ldg(t);
-    const uint32_t cnt = __ldg(t + 1) - a;
-    len = cnt;
-    if (cnt >= kGridDense) {
-        const int k = grid_sub_bits(cnt, c.shift);
+    const bool before = v <= c.k0, in = !before && b < c.nb;
+    const uint32_t* t1 = R.t1 + c.base + (before ? 0u : in ? (uint32_t)b : c.nb);
+    a = __ldg(t1);
+    len = in ? __ldg(t1 + 1) - a : 0u;
+    off = (uint32_t)d & ((1u << min(c.shift, 16u)) - 1u);
+    if (len >= kGridDense) {
+        const int k = grid_sub_bits(len, c.shift);
         const int ss = (int)c.shift - k;
         const uint32_t r = (uint32_t)(d >> ss) & ((1u << k) - 1u);
         const uint32_t* t2 = R.t2 + grid_sub_base(a) + r;
@@ -88,54 +92,77 @@ __device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridCon
     }
 }
 
-// First position of the contig with arr >= v (its end when none).
+// Entries of v's bucket among the eight from `at` (a multiple of 8) on that lie in [a, a + len) and
+// below v (offset off): one 16-byte read and four packed compares.
+__device__ __forceinline__ uint32_t grid_block8(const uint16_t* __restrict__ lo, uint32_t at, uint32_t a, uint32_t len,
+                                                uint32_t off2) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(lo + at));
+    uint32_t below = (__vcmpltu2(x.x, off2) & 0x00010001u) | (__vcmpltu2(x.y, off2) & 0x00020002u) |
+                     (__vcmpltu2(x.z, off2) & 0x00040004u) | (__vcmpltu2(x.w, off2) & 0x00080008u);
+    // bits 0-3: entries 0, 2, 4, 6; bits 16-19: entries 1, 3, 5, 7
+    const int f = (int)(a - at), l = (int)(a + len - at);  // [f, l) of the block counts
+    const uint32_t from = f <= 0 ? 0u : (uint32_t)f, to = l >= 8 ? 8u : (uint32_t)l;
+    const uint32_t even = ((1u << ((to + 1) >> 1)) - 1u) & ~((1u << ((from + 1) >> 1)) - 1u);
+    const uint32_t odd = ((1u << (to >> 1)) - 1u) & ~((1u << (from >> 1)) - 1u);
+    below &= even | (odd << 16);
+    return (uint32_t)__popc(below);
+}
+
+// The first of the positions [a, a + len) of v's bucket whose entry is >= v (a + len when none).
 template <typename S>
-__device__ __forceinline__ uint32_t grid_first_geq(const RankGrid<S>& R, const GridContig& c, S v) {
-    uint32_t a, len;
-    grid_bracket(R, c, v, a, len);
-    while (len > 0) {
-        const uint32_t half = len >> 1;
-        const bool below = __ldg(R.arr + a + half) < v;
-        a = below ? a + half + 1 : a;
-        len = below ? len - half - 1 : half;
+__device__ __forceinline__ uint32_t grid_inside(const RankGrid<S>& R, const GridContig<S>& c, S v, uint32_t a,
+                                                uint32_t len, uint32_t off) {
+    if (c.shift <= 16) {
+        while (len > 8) {
+            const uint32_t half = len >> 1;
+            const bool below = (uint32_t)__ldg(R.lo + a + half) < off;
+            a = below ? a + half + 1 : a;
+            len = below ? len - half - 1 : half;
+        }
+        if (len > 0) {
+            const uint32_t at = a & ~7u, off2 = off | (off << 16);
+            uint32_t n = grid_block8(R.lo, at, a, len, off2);
+            if (a + len > at + 8) n += grid_block8(R.lo, at + 8, a, len, off2);
+            a += n;
+        }
+    } else {
+        while (len > 0) {
+            const uint32_t half = len >> 1;
+            const bool below = __ldg(R.arr + a + half) < v;
+            a = below ? a + half + 1 : a;
+            len = below ? len - half - 1 : half;
+        }
     }
     return a;
 }
 
-// First position with arr > v.
+// First position of the contig with arr >= v (its end when none).
 template <typename S>
-__device__ __forceinline__ uint32_t grid_first_gt(const RankGrid<S>& R, const GridContig& c, S v) {
-    return v == Lim<S>::hi ? c.hi : grid_first_geq<S>(R, c, (S)(v + 1));
+__device__ __forceinline__ uint32_t grid_first_geq(const RankGrid<S>& R, const GridContig<S>& c, S v) {
+    uint32_t a, len, off;
+    grid_bracket(R, c, v, a, len, off);
+    return grid_inside(R, c, v, a, len, off);
 }
 
-// first_gt(v1) in one array and first_geq(v2) in another, their reads side by side.
+// First position with arr > v.
 template <typename S>
-__device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const GridContig& c1, S v1,
-                                               const RankGrid<S>& R2, const GridContig& c2, S v2, uint32_t& r1,
+__device__ __forceinline__ uint32_t grid_first_gt(const RankGrid<S>& R, const GridContig<S>& c, S v) {
+    return v == Lim<S>::hi ? __ldg(R.t1 + c.base + c.nb) : grid_first_geq<S>(R, c, (S)(v + 1));
+}
+
+// first_gt(v1) in one array and first_geq(v2) in another, their table reads side by side.
+template <typename S>
+__device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const GridContig<S>& c1, S v1,
+                                               const RankGrid<S>& R2, const GridContig<S>& c2, S v2, uint32_t& r1,
                                                uint32_t& r2) {
-    uint32_t a1, l1, a2, l2;
+    uint32_t a1, l1, o1, a2, l2, o2;
     const bool top = v1 == Lim<S>::hi;
     const S w1 = top ? v1 : (S)(v1 + 1);
-    grid_bracket(R1, c1, w1, a1, l1);
-    grid_bracket(R2, c2, v2, a2, l2);
-    while ((l1 | l2) != 0u) {
-        const uint32_t h1 = l1 >> 1, h2 = l2 >> 1;
-        S x1 = Lim<S>::hi, x2 = Lim<S>::hi;
-        if (l1) x1 = __ldg(R1.arr + a1 + h1);
-        if (l2) x2 = __ldg(R2.arr + a2 + h2);
-        if (l1) {
-            const bool below = x1 < w1;
-            a1 = below ? a1 + h1 + 1 : a1;
-            l1 = below ? l1 - h1 - 1 : h1;
-        }
-        if (l2) {
-            const bool below = x2 < v2;
-            a2 = below ? a2 + h2 + 1 : a2;
-            l2 = below ? l2 - h2 - 1 : h2;
-        }
-    }
-    r1 = top ? c1.hi : a1;
-    r2 = a2;
+    grid_bracket(R1, c1, w1, a1, l1, o1);
+    grid_bracket(R2, c2, v2, a2, l2, o2);
+    r1 = grid_inside(R1, c1, w1, a1, l1, o1);
+    r2 = grid_inside(R2, c2, v2, a2, l2, o2);
+    if (top) r1 = __ldg(R1.t1 + c1.base + c1.nb);
 }
 
 // ---------------------------------------------------------------- launchers (si_rank.cu)
@@ -145,7 +172,8 @@ inline int64_t grid_t2_words(int64_t n) { return (3 * n + 7) / 8 + 8; }
 // Builds the tables over arr (ascending inside each contig): d_base holds grid_t1_words' bases.
 template <typename S>
 cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G, const uint32_t* d_base,
-                              int64_t t1_words, GridContig* c, uint32_t* t1, uint32_t* t2, cudaStream_t st);
+                              int64_t t1_words, GridContig<S>* c, uint32_t* t1, uint32_t* t2, uint16_t* lo,
+                              cudaStream_t st);
 
 // Counts of a batch in its own order, for an index without intervals with start > end.
 template <typename S>

@@ -106,6 +106,28 @@ def test_ranks_match_numpy(api, kind, n, dt):
     idx.close()
 
 
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+@pytest.mark.parametrize("width", [1, 2, 7, 8, 15, 16, 17])
+def test_offsets_inside_buckets(api, width, dt):
+    """Buckets of 2^width coordinates with 0 to 40 entries each, at every alignment in the 8-entry
+    blocks, keys on both bucket edges; widths on both sides of what a 16-bit offset holds."""
+    rng = np.random.default_rng(width)
+    n, nb = 4096, 1024
+    first = np.sort(np.repeat(np.arange(nb), rng.integers(0, 41, nb))[:n - 2])
+    first = np.concatenate([first, np.full(n - 2 - len(first), nb // 2)]).astype(np.int64)
+    inside = rng.choice(np.array([0, 1, (1 << width) // 2, (1 << width) - 1]), n - 2)
+    s = np.concatenate([[0, (nb << width) - 1], (first << width) + np.minimum(inside, (1 << width) - 1)]) - 77
+    e = s + rng.integers(0, 3 << width, n)
+    qe = np.concatenate([s, s - 1, s + 1])
+    qs = qe - rng.integers(0, 2 << width, len(qe))
+    cnt = np.searchsorted(np.sort(s), qe, side="right") - np.searchsorted(np.sort(e), qs, side="left")
+    idx = api.GpuIndex(np.dtype(dt).itemsize * 8)
+    idx.add_arrays(s.astype(dt), e.astype(dt))
+    idx.build()
+    assert np.array_equal(idx.count(qs.astype(dt), qe.astype(dt)), cnt)
+    idx.close()
+
+
 def _uncovered(s, e, lo, hi):
     """Stretches of [lo, hi] that no interval [s, e] covers, as exact Python ints."""
     out, cur = [], lo
