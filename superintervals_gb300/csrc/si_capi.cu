@@ -185,6 +185,9 @@ struct gSuperIntervals {
     // that the emit of one chunk overlaps the device-to-host copy of the previous one
     DevBuf w_out2;
     cudaStream_t copy_st = nullptr;
+    void* land = nullptr;       // pinned host bytes that small results land in (landing())
+    DevBuf w_small;             // a small host batch, its work record, offsets and values (search_small)
+    cudaEvent_t ev_work = nullptr;
     cudaEvent_t ev_emitted[2] = {nullptr, nullptr}, ev_copied[2] = {nullptr, nullptr};
     sig::BatchedWorkspace bws;
     // set operations: hit lists, staged pieces, and whether some interval has start > end
@@ -599,13 +602,27 @@ int dev_status(const gSuperIntervals* si, int e) {
     return SI_OK;
 }
 
+// Pinned host bytes, kept with the handle, that a call's status and small results are copied to: a copy
+// to pageable memory is staged by the driver and waited for at once, some 8 us each.  Null when the
+// host has no pinned memory left; callers then copy to pageable memory.
+constexpr size_t kLandBytes = 65536;
+char* landing(gSuperIntervals* si) {
+    if (!si->land && cudaHostAlloc(&si->land, kLandBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        si->land = nullptr;
+    }
+    return static_cast<char*>(si->land);
+}
+
 // Reads the device error word after the work queued on `st` (the handle's stream by default).
 int read_dev_err(gSuperIntervals* si, cudaStream_t st = nullptr) {
     if (!st) st = si->st;
-    int e = 0;
-    SI_CK(cudaMemcpyAsync(&e, si->w_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int here = 0;
+    char* land = landing(si);
+    int* e = land ? reinterpret_cast<int*>(land) : &here;
+    SI_CK(cudaMemcpyAsync(e, si->w_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
-    return dev_status(si, e);
+    return dev_status(si, *e);
 }
 
 // The automatic choice: the batched path for batches of 4096+ queries; for smaller ones the plain
@@ -682,35 +699,40 @@ int run_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, co
 
 // ---- searches over ranks (rank_search): counts and offsets in one kernel, then, knowing the result
 // size, either the direct emit or the sorted tiles.
-// The hit count and the error word of launch_rank_scan, in one copy.
+// The error word, then the hit count, of a work record.
+struct RankResult {
+    int err, inv;
+    unsigned long long total;
+};
+static_assert(offsetof(sig::RankWork, err) == 0 && offsetof(sig::RankWork, total) == 8, "read back in one copy");
+
+// Reads them after the work queued on `st`.  With `then`, work to be queued behind the copy (which the
+// host does not wait for), waits by an event.
+template <typename Then>
+int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err, Then then) {
+    RankResult here{}, *h = &here;
+    if (char* land = landing(si)) h = reinterpret_cast<RankResult*>(land);
+    SI_CK(cudaMemcpyAsync(h, si->w_err.p, sizeof(*h), cudaMemcpyDeviceToHost, st));
+    if (!si->ev_work) SI_CK(cudaEventCreateWithFlags(&si->ev_work, cudaEventDisableTiming));
+    SI_CK(cudaEventRecord(si->ev_work, st));
+    SI_TRY(then());
+    SI_CK(cudaEventSynchronize(si->ev_work));
+    *P = (int64_t)h->total;
+    *err = h->err;
+    return SI_OK;
+}
 int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err) {
-    struct {
-        int err, inv;
-        unsigned long long total;
-    } h;
-    static_assert(offsetof(sig::RankWork, total) == 8, "read back in one copy");
-    SI_CK(cudaMemcpyAsync(&h, si->w_err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    RankResult here{}, *h = &here;
+    if (char* land = landing(si)) h = reinterpret_cast<RankResult*>(land);
+    SI_CK(cudaMemcpyAsync(h, si->w_err.p, sizeof(*h), cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
-    *P = (int64_t)h.total;
-    *err = h.err;
+    *P = (int64_t)h->total;
+    *err = h->err;
     return SI_OK;
 }
 
-// Queues counts, upper bounds (w_upper) and offsets; waits for the hit count and the error word.
-template <typename S>
-int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, cudaStream_t st,
-                 int64_t* P, int* err) {
-    SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
-    SI_TRY(si->w_upper.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
-    {
-        PhaseTimer pt(si, 0, st);
-        SI_CK(sig::launch_rank_scan<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, pieces,
-                                       si->w_upper.as<uint32_t>(), d_off, si->w_err.as<sig::RankWork>(), st));
-    }
-    return read_rank_work(si, st, P, err);
-}
-
-// The direct emit's lanes per query for a batch of nq queries and P hits, 0 for the sorted tiles.
+// The direct emit's lanes per query for a batch of nq queries and P hits, 0 for the sorted tiles
+// (sig::rank_lanes, whose far_below this is: long intervals are most of the hits below it).
 // The tiles cost some 75 us (sort, records, tile set-up), 0.19 ns a query and 20 ps an interval (each
 // is gathered by some tile) more than the direct emit; that costs 11 ps a hit more, or 20 where most
 // hits are long intervals lying far apart, each a step of the walk.  Measured (whole calls of 3 M
@@ -722,13 +744,64 @@ int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int
 // few lanes waste less on queries whose hits are few or far apart (3 M queries with 10 far hits: 569
 // us at 2 lanes, 1097 at 8, 2589 at 32), while dense hits want wider chunks (25 hits: 1403, 1317;
 // 300 k queries with 79 hits: 803, 468, 375).
+int64_t far_below(const gSuperIntervals* si, int64_t nq) {
+    return (int64_t)std::ceil(std::min(2.0 * si->long_depth * (double)nq, 4e18));
+}
 int direct_lanes(const gSuperIntervals* si, int64_t nq, int64_t P) {
-    if (si->path != SI_PATH_AUTO) return 0;
-    const bool far = si->long_depth * (double)nq > 0.5 * (double)P;
-    if (far ? P > 4000000 + 10 * nq + si->n || P > 160 * nq : P > 7000000 + 17 * nq + 9 * si->n / 5) return 0;
-    if (nq <= (far ? 4096 : P > 30 * nq ? 524288 : 32768)) return 32;
-    if (nq <= 262144) return 8;
-    return !far && P > 16 * nq ? 8 : 2;
+    return si->path != SI_PATH_AUTO ? 0 : sig::rank_lanes(si->n, far_below(si, nq), nq, P);
+}
+
+// The lanes of the direct emit to queue behind the offsets (EmitGate), before the hit count is known, 0
+// for none: those that sparse hits take.  When the count says otherwise the launch ends at once, some 3
+// us of a call that then takes hundreds; above two million queries the wait that it saves is below 5%
+// of the sparsest call (keys of 2 M queries 249 -> 234 us, 100 k searches 60 -> 45 us).
+int gated_lanes(const gSuperIntervals* si, int64_t nq) {
+    if (si->path != SI_PATH_AUTO || si->prof || nq == 0 || nq > (int64_t)1 << 21) return 0;
+    if (nq <= (si->long_depth < 1.0 ? 32768 : 4096)) return 32;
+    return nq <= 262144 ? 8 : 2;
+}
+
+// What an emit writes: field `what` (a RankOut) to d, which holds `room` results, in `order`.
+template <typename S>
+struct EmitTo {
+    int what = sig::kOutIdx, order = 0;
+    sig::RankDest<S> d;
+    int64_t room = 0;
+};
+
+// Queues counts, upper bounds (w_upper) and offsets and, gated, the direct emit to `to` (*lanes, or 0).
+template <typename S>
+int queue_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, sig::RankWork* work,
+                  bool cleared, const EmitTo<S>& to, cudaStream_t st, int* lanes) {
+    *lanes = 0;
+    SI_TRY(si->w_upper.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
+    {
+        PhaseTimer pt(si, 0, st);
+        SI_CK(sig::launch_rank_scan<S>(view<S>(si), rank_grid<S>(si, 0), rank_grid<S>(si, 1), q, pieces,
+                                       si->w_upper.as<uint32_t>(), d_off, work, st, cleared));
+    }
+    if (to.room > 0 && (*lanes = gated_lanes(si, q.nq)))
+        SI_CK(sig::launch_rank_emit<S>(view<S>(si), q, si->w_upper.as<uint32_t>(), d_off, 0, to.order, to.what, to.d,
+                                       *lanes, &work->err, st, {work, to.room, si->n, far_below(si, q.nq)}));
+    return SI_OK;
+}
+
+// Whether the emit queued with `lanes` found its gate open.
+bool emitted(const gSuperIntervals* si, int64_t nq, int64_t room, int lanes, int64_t P, int err) {
+    return lanes && !err && P > 0 && P <= room && direct_lanes(si, nq, P) == lanes;
+}
+
+// Offsets and the gated emit; waits for the hit count and the error word.  *done: the results are
+// written.
+template <typename S>
+int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, const EmitTo<S>& to,
+                 cudaStream_t st, int64_t* P, int* err, bool* done) {
+    int lanes = 0;
+    SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
+    SI_TRY(queue_offsets<S>(si, q, pieces, d_off, si->w_err.as<sig::RankWork>(), false, to, st, &lanes));
+    SI_TRY(read_rank_work(si, st, P, err));
+    *done = emitted(si, q.nq, to.room, lanes, *P, *err);
+    return SI_OK;
 }
 
 // Sorts the batch into tiles when `lanes` says so; the emits of its parts follow.
@@ -789,10 +862,16 @@ int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool
         return search_device_counted<S>(si, q, order, values, d_offsets, d_out, cap, total, st);
     int64_t P = 0;
     int err = 0;
-    SI_TRY(rank_offsets<S>(si, q, false, d_offsets, st, &P, &err));
+    bool done = false;
+    EmitTo<S> to;
+    to.what = values ? sig::kOutValue : sig::kOutIdx;
+    to.order = order;
+    to.d.i32 = d_out;
+    to.room = d_out ? (int64_t)std::min<size_t>(cap, INT64_MAX) : 0;
+    SI_TRY(rank_offsets<S>(si, q, false, d_offsets, to, st, &P, &err, &done));
     if (total) *total = (size_t)P;
     if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
-    if (err || P == 0) return dev_status(si, err);
+    if (err || P == 0 || done) return dev_status(si, err);
     const int lanes = direct_lanes(si, q.nq, P);
     SI_TRY(rank_prepare<S>(si, q, lanes, st));
     SI_TRY(rank_emit<S>(si, q, 0, d_offsets, 0, order, values, d_out, lanes, P, st));
@@ -822,6 +901,60 @@ int upload_queries(gSuperIntervals* si, const S* qs, const S* qe, const int32_t*
     return SI_OK;
 }
 
+// A small host batch: its queries and a cleared work record go over in one copy, and the record, the
+// offsets and the values come back in one, both through pinned memory.  One lookup of a region: 85 us
+// with a copy per array, a wait for the hit count and one for the values, 49 us so.
+constexpr size_t kSmallQueries = 1024;
+constexpr int64_t kSmallValues = 4096;
+struct SmallBatch {
+    const int64_t* off = nullptr;     // host offsets; null: not such a batch, nothing was done
+    const int32_t* values = nullptr;  // host values; null: not written (P or another emit)
+    int64_t P = 0;
+    int err = 0;
+    int64_t* d_off = nullptr;         // device offsets
+    sig::QueryBatch q;                // device queries
+};
+template <typename S>
+int search_small(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int order, bool values,
+                 size_t cap, SmallBatch* b) {
+    if (nq == 0 || nq > kSmallQueries || !qs || !qe || !rank_search(si, (int64_t)nq) || !gated_lanes(si, (int64_t)nq))
+        return SI_OK;
+    const auto up = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    const size_t at_e = up(sizeof(S) * nq), at_c = at_e + up(sizeof(S) * nq);
+    const size_t at_work = at_c + up(qc ? sizeof(int32_t) * nq : 0);
+    const size_t at_off = at_work + up(sig::rank_work_bytes((int64_t)nq)), at_val = at_off + up(sizeof(int64_t) * (nq + 1));
+    const int64_t room = (int64_t)std::min<size_t>(cap, (size_t)kSmallValues);
+    const size_t end = at_val + sizeof(int32_t) * (size_t)room;
+    static_assert(kSmallQueries * 28 + kSmallValues * 4 + 1024 <= kLandBytes, "a small batch fits the landing");
+    char* land = landing(si);
+    if (!land || si->w_small.reserve(kLandBytes) != SI_OK) return SI_OK;
+    char* dev = si->w_small.as<char>();
+    cudaStream_t st = si->st;
+    memcpy(land, qs, sizeof(S) * nq);
+    memcpy(land + at_e, qe, sizeof(S) * nq);
+    if (qc) memcpy(land + at_c, qc, sizeof(int32_t) * nq);
+    memset(land + at_work, 0, at_off - at_work);
+    SI_CK(cudaMemcpyAsync(dev, land, at_off, cudaMemcpyHostToDevice, st));
+    b->q = {dev, dev + at_e, qc ? reinterpret_cast<int32_t*>(dev + at_c) : nullptr, (int64_t)nq};
+    b->d_off = reinterpret_cast<int64_t*>(dev + at_off);
+    EmitTo<S> to;
+    to.what = values ? sig::kOutValue : sig::kOutIdx;
+    to.order = order;
+    to.d.i32 = reinterpret_cast<int32_t*>(dev + at_val);
+    to.room = room;
+    int lanes = 0;
+    SI_TRY(queue_offsets<S>(si, b->q, false, b->d_off, reinterpret_cast<sig::RankWork*>(dev + at_work), true, to, st,
+                            &lanes));
+    SI_CK(cudaMemcpyAsync(land + at_work, dev + at_work, end - at_work, cudaMemcpyDeviceToHost, st));
+    SI_CK(cudaStreamSynchronize(st));
+    const sig::RankWork* w = reinterpret_cast<const sig::RankWork*>(land + at_work);
+    b->P = (int64_t)w->total;
+    b->err = w->err;
+    b->off = reinterpret_cast<const int64_t*>(land + at_off);
+    if (emitted(si, (int64_t)nq, room, lanes, b->P, b->err)) b->values = reinterpret_cast<const int32_t*>(land + at_val);
+    return SI_OK;
+}
+
 // host queries -> host CSR; result grown when `grow` is set, else caller buffers
 template <typename S>
 int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int order,
@@ -842,15 +975,45 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         grow->size = 0;
     }
     sig::QueryBatch q;
-    SI_TRY(upload_queries<S>(si, qs, qe, qc, nq, q));
-    SI_TRY(si->w_offsets.reserve(sizeof(int64_t) * (nq + 1)));
-    int64_t* d_off = si->w_offsets.as<int64_t>();
-    const bool ranks = rank_search(si, q.nq);
+    const bool ranks = rank_search(si, (int64_t)nq);
     int64_t P = 0;
     int err = 0;
-    if (ranks) {
-        SI_TRY(rank_offsets<S>(si, q, false, d_off, st, &P, &err));
-        SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
+    bool done = false;  // the results are in w_out
+    int64_t* d_off = nullptr;
+    SmallBatch small;
+    SI_TRY(search_small<S>(si, qs, qe, qc, nq, order, values, grow || h_out ? (grow ? SIZE_MAX : cap) : 0, &small));
+    if (small.off) {
+        q = small.q;
+        d_off = small.d_off;
+        P = small.P;
+        err = small.err;
+        memcpy(h_off, small.off, sizeof(int64_t) * (nq + 1));
+    } else {
+        SI_TRY(upload_queries<S>(si, qs, qe, qc, nq, q));
+        SI_TRY(si->w_offsets.reserve(sizeof(int64_t) * (nq + 1)));
+        d_off = si->w_offsets.as<int64_t>();
+    }
+    if (small.off) {
+    } else if (ranks) {
+        // the gated emit writes to the output buffer as it stands (a first one of up to 1 MB)
+        const int64_t most = std::max<int64_t>((int64_t)(si->out_budget / sizeof(int32_t)), 1 << 20);
+        if (!si->w_out.p && gated_lanes(si, q.nq) && (grow || cap))
+            si->w_out.reserve(sizeof(int32_t) * (grow ? 262144 : std::min<size_t>(cap, 262144)));
+        EmitTo<S> to;
+        to.what = values ? sig::kOutValue : sig::kOutIdx;
+        to.order = order;
+        to.d.i32 = si->w_out.as<int32_t>();
+        to.room = std::min<int64_t>((int64_t)(si->w_out.bytes / sizeof(int32_t)), most);
+        if (!grow) to.room = (int64_t)std::min<size_t>((size_t)to.room, cap);
+        int lanes = 0;
+        SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
+        SI_TRY(queue_offsets<S>(si, q, false, d_off, si->w_err.as<sig::RankWork>(), false, to, st, &lanes));
+        // the offsets follow behind the hit count, which the host waits for
+        SI_TRY(read_rank_work(si, st, &P, &err, [&]() -> int {
+            SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
+            return SI_OK;
+        }));
+        done = emitted(si, q.nq, to.room, lanes, P, err);
     } else {
         SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<size_t>(nq, 1)));
         SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
@@ -877,9 +1040,23 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         if (ranks) SI_CK(cudaStreamSynchronize(st));  // the offsets are the caller's
         return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
     }
+    if (small.off && (P == 0 || err)) return dev_status(si, err);
     if (P == 0 || err) {
         SI_TRY(read_dev_err(si));  // waits for the offsets too
         return dev_status(si, err);
+    }
+    if (small.values) {
+        memcpy(h_out, small.values, sizeof(int32_t) * P);
+        return SI_OK;
+    }
+    if (done) {
+        SI_CK(cudaMemcpyAsync(h_out, si->w_out.p, sizeof(int32_t) * P, cudaMemcpyDeviceToHost, st));
+        SI_CK(cudaStreamSynchronize(st));
+        return SI_OK;
+    }
+    if (small.off) {  // its error word was another one
+        SI_TRY(si->w_err.reserve(2 * sizeof(int)));
+        SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
     }
     const int lanes = ranks ? direct_lanes(si, q.nq, P) : 0;
     if (ranks) SI_TRY(rank_prepare<S>(si, q, lanes, st));
@@ -1081,6 +1258,8 @@ void destroySuperIntervalsGpu(gSuperIntervals* si) {
         cudaStreamSynchronize(si->copy_st);
         cudaStreamDestroy(si->copy_st);
     }
+    if (si->ev_work) cudaEventDestroy(si->ev_work);
+    if (si->land) cudaFreeHost(si->land);
     for (int b = 0; b < 2; ++b) {
         if (si->ev_emitted[b]) cudaEventDestroy(si->ev_emitted[b]);
         if (si->ev_copied[b]) cudaEventDestroy(si->ev_copied[b]);
@@ -1911,8 +2090,13 @@ int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStre
     if (rank_search(si, q.nq)) {
         int64_t P = 0;
         int err = 0;
-        SI_TRY(rank_offsets<S>(si, q, false, si->so_hoff.as<int64_t>(), st, &P, &err));
-        if (err) return dev_status(si, err);
+        bool done = false;
+        EmitTo<S> to;
+        to.order = order;
+        to.d.i32 = si->so_hits.as<int32_t>();
+        to.room = (int64_t)(si->so_hits.bytes / sizeof(int32_t));
+        SI_TRY(rank_offsets<S>(si, q, false, si->so_hoff.as<int64_t>(), to, st, &P, &err, &done));
+        if (err || done) return dev_status(si, err);
         SI_TRY(si->so_hits.reserve(sizeof(int32_t) * std::max<int64_t>(P, 1)));
         if (P == 0) return SI_OK;
         const int lanes = direct_lanes(si, q.nq, P);
@@ -1936,12 +2120,17 @@ int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStre
 
 // Intersections and keys of a rank search: every hit gives one piece (a query with start > end none),
 // or one key, so the hits' offsets are the result's, and the emit writes the fields itself instead of
-// a hit list for a second pass.  Queues offsets and bounds; waits for the total.
+// a hit list for a second pass.  Queues offsets, bounds and the gated emit; waits for the total.
 template <typename S>
-int field_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool keys, int64_t* d_off, cudaStream_t st,
-                  int64_t* P) {
+int field_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool keys, int64_t* d_off,
+                  sig::RankDest<S> d, size_t cap, cudaStream_t st, int64_t* P, bool* done) {
     int err = 0;
-    SI_TRY(rank_offsets<S>(si, q, !keys, d_off, st, P, &err));
+    EmitTo<S> to;
+    to.what = keys ? sig::kOutKeys : sig::kOutPieces;
+    to.order = order;
+    to.d = d;
+    to.room = d.s && d.e && (keys || d.i32) ? (int64_t)std::min<size_t>(cap, INT64_MAX) : 0;
+    SI_TRY(rank_offsets<S>(si, q, !keys, d_off, to, st, P, &err, done));
     return dev_status(si, err);
 }
 
@@ -2014,26 +2203,33 @@ sig::RankGrid<S> gap_grid(const gSuperIntervals* si, int which) {
     return grid_view<S>(si->gap_grid, si->gaps.as<S>() + (which ? si->n_gaps : 0), which);
 }
 
-// Difference from the gaps: the pieces of a query are the gaps it meets, so their number is a
-// difference of two ranks, as a search's hits.  Queues offsets and bounds; waits for the total.
 template <typename S>
-int gap_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int64_t* d_off, size_t* total, cudaStream_t st) {
+int gap_emit(gSuperIntervals* si, const sig::QueryBatch& q, const int64_t* d_off, S* os, S* oe, cudaStream_t st,
+             sig::EmitGate gate = sig::EmitGate()) {
+    const S* a0 = si->gaps.as<S>();
+    SI_CK(sig::launch_gap_emit<S>(a0, a0 + si->n_gaps, q, si->w_upper.as<uint32_t>(), d_off, os, oe, st,
+                                  gate));
+    return SI_OK;
+}
+
+// Difference from the gaps: the pieces of a query are the gaps it meets, so their number is a
+// difference of two ranks, as a search's hits.  Queues offsets and bounds and the emit, gated by the
+// room for `cap` pieces; waits for the total.
+template <typename S>
+int gap_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int64_t* d_off, S* os, S* oe, size_t cap,
+                size_t* total, cudaStream_t st) {
     SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
     SI_TRY(si->w_upper.reserve(sizeof(uint32_t) * std::max<int64_t>(q.nq, 1)));
     SI_CK(sig::launch_rank_scan<S>(view<S>(si), gap_grid<S>(si, 0), gap_grid<S>(si, 1), q, true,
                                    si->w_upper.as<uint32_t>(), d_off, si->w_err.as<sig::RankWork>(), st));
+    if (os && oe && cap)
+        SI_TRY(gap_emit<S>(si, q, d_off, os, oe, st,
+                           {si->w_err.as<sig::RankWork>(), (int64_t)std::min<size_t>(cap, INT64_MAX), 0, 0}));
     int64_t T = 0;
     int err = 0;
     SI_TRY(read_rank_work(si, st, &T, &err));
     SI_TRY(dev_status(si, err));
     *total = (size_t)T;
-    return SI_OK;
-}
-
-template <typename S>
-int gap_emit(gSuperIntervals* si, const sig::QueryBatch& q, const int64_t* d_off, S* os, S* oe, cudaStream_t st) {
-    const S* a0 = si->gaps.as<S>();
-    SI_CK(sig::launch_gap_emit<S>(a0, a0 + si->n_gaps, q, si->w_upper.as<uint32_t>(), d_off, os, oe, st));
     return SI_OK;
 }
 
@@ -2053,20 +2249,19 @@ int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int orde
     }
     if (op == 1 && use_ranks(si, q.nq) && make_gaps<S>(si, st) == SI_OK) {
         size_t T = 0;
-        SI_TRY(gap_offsets<S>(si, q, d_off, &T, st));
+        SI_TRY(gap_offsets<S>(si, q, d_off, d_os, d_oe, cap, &T, st));  // and the pieces, where they fit
         if (total) *total = T;
         if (T > cap) return fail(SI_ERR_CAPACITY, "output needs %zu pieces, capacity %zu", T, cap);
-        if (T == 0) return SI_OK;
-        if (!d_os || !d_oe) return fail(SI_ERR_INVALID, "null output buffer");
-        SI_TRY(gap_emit<S>(si, q, d_off, d_os, d_oe, st));
-        return read_dev_err(si, st);
+        if (T > 0 && (!d_os || !d_oe)) return fail(SI_ERR_INVALID, "null output buffer");
+        return SI_OK;
     }
     if (op == 0 && rank_search(si, q.nq)) {
         int64_t P = 0;
-        SI_TRY(field_offsets<S>(si, q, false, d_off, st, &P));
+        bool done = false;
+        SI_TRY(field_offsets<S>(si, q, order, false, d_off, {d_ob, d_os, d_oe}, cap, st, &P, &done));
         if (total) *total = (size_t)P;
         if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld pieces, capacity %zu", (long long)P, cap);
-        if (P == 0) return SI_OK;
+        if (P == 0 || done) return SI_OK;
         if (!d_os || !d_oe || !d_ob) return fail(SI_ERR_INVALID, "null output buffer");
         SI_TRY(field_emit<S>(si, q, order, false, d_off, {d_ob, d_os, d_oe}, P, st));
         return read_dev_err(si, st);
@@ -2289,10 +2484,11 @@ int keys_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_
     }
     int64_t P = 0;
     if (rank_search(si, q.nq)) {
-        SI_TRY(field_offsets<S>(si, q, true, d_off, st, &P));
+        bool done = false;
+        SI_TRY(field_offsets<S>(si, q, order, true, d_off, {d_d, d_s, d_e}, cap, st, &P, &done));
         if (total) *total = (size_t)P;
         if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld keys, capacity %zu", (long long)P, cap);
-        if (P == 0) return SI_OK;
+        if (P == 0 || done) return SI_OK;
         if (!d_s || !d_e) return fail(SI_ERR_INVALID, "null output buffer");
         SI_TRY(field_emit<S>(si, q, order, true, d_off, {d_d, d_s, d_e}, P, st));
         return read_dev_err(si, st);

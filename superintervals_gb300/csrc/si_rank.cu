@@ -375,14 +375,18 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
 // Right for sparse results: a tile of queries far apart shares nothing, and sorting the batch
 // costs more than the hits.  Bound by the dependent reads of the walk (about 12-16 ps a hit with the
 // device full; lanes per query: see direct_lanes).  Whole calls, before (sorted tiles) and after:
-// 100 k queries with 0.7 hits each 205 -> 57 us, 3 M with 2.7 hits 1290 -> 289 us, 3 M with 33 hits
+// 100 k queries with 0.7 hits each 205 -> 45 us, 3 M with 2.7 hits 1290 -> 289 us, 3 M with 33 hits
 // 1418 -> 1130 us; 3 M with 126 hits would go 2306 -> 5551 us.
 template <typename S, int W, int OUT>
 __global__ void __launch_bounds__(kThreads) k_rank_emit(MapView<S> m, const S* __restrict__ qs,
                                                         const S* __restrict__ qe, const int32_t* __restrict__ qc,
                                                         int64_t nq, const uint32_t* __restrict__ su,
                                                         const int64_t* __restrict__ off, int64_t out_base, int order,
-                                                        RankDest<S> dst, int* d_err) {
+                                                        RankDest<S> dst, int* d_err, EmitGate gate) {
+    if (gate.work) {
+        const int64_t P = (int64_t)gate.work->total;
+        if (gate.work->err || P > gate.room || rank_lanes(gate.n, gate.far_below, nq, P) != W) return;
+    }
     const int lane = threadIdx.x & 31, sub = lane & (W - 1);
     const unsigned gmask = W == 32 ? kFull : ((1u << (W & 31)) - 1u) << (lane & ~(W - 1));
     const int64_t q = ((int64_t)blockIdx.x * kThreads + threadIdx.x) / W;
@@ -524,14 +528,15 @@ __global__ void __launch_bounds__(kThreads) k_gap_write(MapView<S> m, int64_t sl
 // One warp writes the pieces of 32 neighbouring queries, which lie one after another in the output:
 // lane l takes every 32nd piece of the warp's stretch and finds its query among the 32 by halving
 // over their offsets (shuffles), so writes coalesce and a query of many pieces is shared by all lanes.
-// 5 M queries against 5 M intervals: the whole call 1856 us with hit lists swept per query, 300 us
+// 5 M queries against 5 M intervals: the whole call 1856 us with hit lists swept per query, 283 us
 // from the gaps.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_gap_emit(const S* __restrict__ gs, const S* __restrict__ ge,
                                                        const S* __restrict__ qs, const S* __restrict__ qe, int64_t nq,
                                                        const uint32_t* __restrict__ su,
                                                        const int64_t* __restrict__ off, S* __restrict__ os,
-                                                       S* __restrict__ oe) {
+                                                       S* __restrict__ oe, EmitGate gate) {
+    if (gate.work && (gate.work->err || (int64_t)gate.work->total > gate.room)) return;
     const int lane = threadIdx.x & 31;
     const int64_t q = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const bool live = q < nq;
@@ -611,9 +616,11 @@ size_t rank_work_bytes(int64_t nq) {
 
 template <typename S>
 cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, bool pieces, uint32_t* su,
-                             int64_t* off, RankWork* work, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(work, 0, rank_work_bytes(q.nq), st);
-    if (e != cudaSuccess) return e;
+                             int64_t* off, RankWork* work, cudaStream_t st, bool cleared) {
+    if (!cleared) {
+        cudaError_t e = cudaMemsetAsync(work, 0, rank_work_bytes(q.nq), st);
+        if (e != cudaSuccess) return e;
+    }
     if (q.nq <= 0) return cudaMemsetAsync(off, 0, sizeof(int64_t), st);
     const S* qs = static_cast<const S*>(q.qs);
     const S* qe = static_cast<const S*>(q.qe);
@@ -628,22 +635,22 @@ cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, Query
 
 template <typename S, int W>
 static cudaError_t rank_emit_w(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
-                               int order, int what, RankDest<S> d, int* d_err, cudaStream_t st) {
+                               int order, int what, RankDest<S> d, int* d_err, cudaStream_t st, EmitGate gate) {
     const unsigned blocks = blocks_for(q.nq * W);
     const S* qs = static_cast<const S*>(q.qs);
     const S* qe = static_cast<const S*>(q.qe);
     switch (what) {
         case kOutIdx:
-            k_rank_emit<S, W, kOutIdx><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            k_rank_emit<S, W, kOutIdx><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err, gate);
             break;
         case kOutValue:
-            k_rank_emit<S, W, kOutValue><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            k_rank_emit<S, W, kOutValue><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err, gate);
             break;
         case kOutKeys:
-            k_rank_emit<S, W, kOutKeys><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            k_rank_emit<S, W, kOutKeys><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err, gate);
             break;
         default:
-            k_rank_emit<S, W, kOutPieces><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err);
+            k_rank_emit<S, W, kOutPieces><<<blocks, kThreads, 0, st>>>(m, qs, qe, q.qc, q.nq, su, off, out_base, order, d, d_err, gate);
     }
     note_launch();
     return cudaGetLastError();
@@ -651,11 +658,12 @@ static cudaError_t rank_emit_w(MapView<S> m, QueryBatch q, const uint32_t* su, c
 
 template <typename S>
 cudaError_t launch_rank_emit(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
-                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st) {
+                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st,
+                             EmitGate gate) {
     if (q.nq <= 0) return cudaSuccess;
-    if (lanes == 2) return rank_emit_w<S, 2>(m, q, su, off, out_base, order, what, d, d_err, st);
-    if (lanes == 8) return rank_emit_w<S, 8>(m, q, su, off, out_base, order, what, d, d_err, st);
-    return rank_emit_w<S, 32>(m, q, su, off, out_base, order, what, d, d_err, st);
+    if (lanes == 2) return rank_emit_w<S, 2>(m, q, su, off, out_base, order, what, d, d_err, st, gate);
+    if (lanes == 8) return rank_emit_w<S, 8>(m, q, su, off, out_base, order, what, d, d_err, st, gate);
+    return rank_emit_w<S, 32>(m, q, su, off, out_base, order, what, d, d_err, st, gate);
 }
 
 template <typename S>
@@ -702,10 +710,10 @@ cudaError_t launch_gap_write(MapView<S> m, const uint32_t* flags, const int64_t*
 
 template <typename S>
 cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32_t* su, const int64_t* off, S* os,
-                            S* oe, cudaStream_t st) {
+                            S* oe, cudaStream_t st, EmitGate gate) {
     if (q.nq <= 0) return cudaSuccess;
     k_gap_emit<S><<<blocks_for(q.nq), kThreads, 0, st>>>(gs, ge, static_cast<const S*>(q.qs),
-                                                         static_cast<const S*>(q.qe), q.nq, su, off, os, oe);
+                                                         static_cast<const S*>(q.qe), q.nq, su, off, os, oe, gate);
     note_launch();
     return cudaGetLastError();
 }
@@ -716,9 +724,9 @@ cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32
     template cudaError_t launch_rank_count<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, uint32_t*, int*, \
                                               cudaStream_t);                                                     \
     template cudaError_t launch_rank_scan<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, bool, uint32_t*,  \
-                                             int64_t*, RankWork*, cudaStream_t);                                 \
+                                             int64_t*, RankWork*, cudaStream_t, bool);                           \
     template cudaError_t launch_rank_emit<S>(MapView<S>, QueryBatch, const uint32_t*, const int64_t*, int64_t,   \
-                                             int, int, RankDest<S>, int, int*, cudaStream_t);                    \
+                                             int, int, RankDest<S>, int, int*, cudaStream_t, EmitGate);          \
     template cudaError_t launch_rank_ub<S>(RankGrid<S>, int, const void*, const int32_t*, int64_t, int32_t*,     \
                                            int*, cudaStream_t);                                                  \
     template cudaError_t launch_rank_coverage<S>(RankGrid<S>, RankGrid<S>, int, QueryBatch, const uint64_t*,     \
@@ -727,7 +735,7 @@ cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32
     template cudaError_t launch_gap_flags<S>(MapView<S>, uint32_t*, cudaStream_t);                            \
     template cudaError_t launch_gap_write<S>(MapView<S>, const uint32_t*, const int64_t*, S*, S*, cudaStream_t); \
     template cudaError_t launch_gap_emit<S>(const S*, const S*, QueryBatch, const uint32_t*, const int64_t*, S*, \
-                                            S*, cudaStream_t);
+                                            S*, cudaStream_t, EmitGate);
 SIG_GINST(int32_t)
 SIG_GINST(int64_t)
 SIG_RINST(int32_t)

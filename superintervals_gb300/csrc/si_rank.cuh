@@ -181,7 +181,8 @@ cudaError_t launch_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, Quer
                               int* d_err, cudaStream_t st);
 // Counts and their exclusive prefix sums (off, n + 1 entries) in one pass, and each query's upper
 // bound (su: the first position whose start exceeds the query's end, 0 when no start of its contig
-// is at or below it or the contig is outside [0, G)).  work: rank_work_bytes(nq), zeroed by the call.
+// is at or below it or the contig is outside [0, G)).  work: rank_work_bytes(nq), zeroed by the call
+// unless it is `cleared`.
 // With pieces, a query with start > end counts nothing (it gives no piece of an intersection).
 struct RankWork {
     int err;                   // device error word
@@ -193,7 +194,25 @@ struct RankWork {
 size_t rank_work_bytes(int64_t nq);
 template <typename S>
 cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, bool pieces, uint32_t* su,
-                             int64_t* off, RankWork* work, cudaStream_t st);
+                             int64_t* off, RankWork* work, cudaStream_t st, bool cleared = false);
+// The direct emit's lanes per query for a batch of nq queries and P hits over n intervals, 0 for the
+// sorted tiles; below far_below hits most of them are long intervals lying far apart (see direct_lanes).
+__host__ __device__ inline int rank_lanes(int64_t n, int64_t far_below, int64_t nq, int64_t P) {
+    const bool far = P < far_below;
+    if (far ? P > 4000000 + 10 * nq + n || P > 160 * nq : P > 7000000 + 17 * nq + 9 * n / 5) return 0;
+    if (nq <= (far ? 4096 : P > 30 * nq ? 524288 : 32768)) return 32;
+    if (nq <= 262144) return 8;
+    return !far && P > 16 * nq ? 8 : 2;
+}
+// An emit queued behind launch_rank_scan before the host knows the hit count: every block reads the
+// count and leaves when the batch failed, when the output has no room or when rank_lanes names
+// another kernel; the host, which reads the same record after both, then goes that other way.  It
+// saves the wait between the two kernels: 100 k searches with 0.7 hits each 60 -> 45 us.
+struct EmitGate {
+    const RankWork* work = nullptr;    // null: emit
+    int64_t room = 0;                  // results that the output holds
+    int64_t n = 0, far_below = 0;      // rank_lanes
+};
 // What the direct emit writes for each hit.
 enum RankOut : int { kOutIdx = 0, kOutValue = 1, kOutKeys = 2, kOutPieces = 3 };
 template <typename S>
@@ -205,7 +224,8 @@ struct RankDest {
 // Writes every query's hits at off[q] - out_base, by groups of `lanes` (2, 8 or 32) lanes per query.
 template <typename S>
 cudaError_t launch_rank_emit(MapView<S> m, QueryBatch q, const uint32_t* su, const int64_t* off, int64_t out_base,
-                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st);
+                             int order, int what, RankDest<S> d, int lanes, int* d_err, cudaStream_t st,
+                             EmitGate gate = EmitGate());
 
 // Gaps: the stretches of each contig's coordinate range that no interval covers (no interval has
 // start > end).  Slots: contig g's positions, then one after its last; flags mark those with a gap
@@ -218,7 +238,7 @@ cudaError_t launch_gap_write(MapView<S> m, const uint32_t* flags, const int64_t*
 // The gaps that each query meets, clipped to it: the off[q + 1] - off[q] gaps before su[q].
 template <typename S>
 cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32_t* su, const int64_t* off, S* os,
-                            S* oe, cudaStream_t st);
+                            S* oe, cudaStream_t st, EmitGate gate = EmitGate());
 
 // Contig-local upper bounds (-1: none) of every query end.
 template <typename S>

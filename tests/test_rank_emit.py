@@ -90,3 +90,67 @@ def test_direct_emit_matches_oracle(api, oracle, kind, nq, dt):
     off, out = idx.search(qs, qe, qc)
     assert np.array_equal(off, want_off) and np.array_equal(out, want)
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("nq,hits", [(1, 3), (1, 4096), (1, 4097), (1024, 2), (1024, 4), (1024, 9), (1025, 4),
+                                     (40_000, 5), (40_000, 70)])
+def test_emit_queued_before_the_count(api, bits, nq, hits):
+    """Host and device searches whose emit is queued before the host knows the hit count: batches and
+    results on both sides of what a small batch's buffer holds, an exact capacity, one short of it
+    (nothing but offsets written), another emit than the queued one, a contig outside the index."""
+    import ctypes as C
+
+    dt = np.int32 if bits == 32 else np.int64
+    rng = np.random.default_rng(nq + hits)
+    n = 30_000
+    s = (np.arange(n) * 10).astype(dt)
+    e = s + 9
+    data = rng.integers(-9, 9, n).astype(np.int32)
+    first = rng.integers(0, n - hits, nq)
+    qs, qe = (first * 10).astype(dt), ((first + hits) * 10 - 1).astype(dt)
+    qc = np.zeros(nq, np.int32)
+    P = nq * hits
+    want = (first[:, None] + np.arange(hits)[::-1]).ravel().astype(np.int32)
+    want_off = np.arange(nq + 1, dtype=np.int64) * hits
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s, e, data)
+    idx.build()
+    lib, p = idx.lib, lambda a: C.c_void_p(a.ctypes.data)
+    total = C.c_size_t(0)
+    bad = qc.copy()
+    bad[nq // 2] = 1
+    for values, expect in ((0, want), (1, data[want])):
+        for _ in range(2):                                   # cold and kept workspaces
+            off, out = np.full(nq + 1, -1, np.int64), np.full(P + 8, -7, np.int32)
+            args = (p(qs), p(qe), p(qc), nq, api.ORDER_DESC, values, p(off), p(out))
+            api.check(lib.searchBatchIntoGpu(idx.h, *args, P, C.byref(total)))
+            assert total.value == P and np.array_equal(off, want_off)
+            assert np.array_equal(out[:P], expect) and (out[P:] == -7).all()
+            out[:], off[:] = -7, -1
+            assert lib.searchBatchIntoGpu(idx.h, *args, P - 1, C.byref(total)) == api._capi.SI_ERR_CAPACITY
+            assert total.value == P and np.array_equal(off, want_off) and (out == -7).all()
+            assert lib.searchBatchIntoGpu(idx.h, p(qs), p(qe), p(bad), *args[3:], P, C.byref(total)) == \
+                api._capi.SI_ERR_INVALID
+            assert (out == -7).all()
+    dev = []
+    for a in (qs, qe, qc, bad, np.zeros(nq + 1, np.int64), np.full(P + 8, -7, np.int32)):
+        d = C.c_void_p()
+        api.check(lib.deviceMallocGpu(C.byref(d), a.nbytes))
+        api.check(lib.memcpyGpu(d, p(a), a.nbytes, idx.stream))
+        dev.append(d)
+    got = np.empty(P + 8, np.int32)
+
+    def device(contigs, cap):
+        st = lib.searchDeviceGpu(idx.h, dev[0], dev[1], contigs, nq, api.ORDER_DESC, 0, dev[4], dev[5], cap,
+                                 C.byref(total), None)
+        api.check(lib.memcpyGpu(p(got), dev[5], got.nbytes, idx.stream))
+        api.check(lib.streamSynchronizeGpu(idx.stream))
+        return st
+
+    assert device(dev[2], P - 1) == api._capi.SI_ERR_CAPACITY and total.value == P and (got == -7).all()
+    assert device(dev[3], P) == api._capi.SI_ERR_INVALID and (got == -7).all()
+    assert device(dev[2], P) == 0 and np.array_equal(got[:P], want) and (got[P:] == -7).all()
+    for d in dev:
+        lib.deviceFreeGpu(d)
+    idx.close()
