@@ -130,11 +130,11 @@ void dev_release(void** p, size_t* bytes) {
 }
 }  // namespace sig
 
-// Rank grids over one or two arrays of the same contigs: per array the contig records, t1 and t2
+// Rank grids over one or two arrays of the same contigs: per array the contig records, bucket records, t2
 // words and offsets (si_rank.cuh), in one allocation.
 struct GridSet {
     DevBuf buf;
-    size_t at[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};  // byte offsets of [array][contigs, t1, t2, offsets]
+    size_t at[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};  // byte offsets of [array][contigs, records, t2, offsets]
 };
 
 struct gSuperIntervals {
@@ -362,7 +362,7 @@ sig::RankGrid<S> grid_view(const GridSet& g, const S* arr, int which) {
     sig::RankGrid<S> R;
     R.arr = arr;
     R.c = reinterpret_cast<const sig::GridContig<S>*>(p + g.at[which][0]);
-    R.t1 = reinterpret_cast<const uint32_t*>(p + g.at[which][1]);
+    R.rec = reinterpret_cast<const uint4*>(p + g.at[which][1]);
     R.t2 = reinterpret_cast<const uint32_t*>(p + g.at[which][2]);
     R.lo = reinterpret_cast<const uint16_t*>(p + g.at[which][3]);
     return R;
@@ -381,9 +381,9 @@ int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vect
                 const int64_t* d_seg, std::vector<uint32_t>& base, cudaStream_t st) {
     const int G = (int)segv.size() - 1;
     base.resize(G);
-    const int64_t w1 = sig::grid_t1_words(segv.data(), G, base.data()), w2 = sig::grid_t2_words(n);
+    const int64_t w1 = sig::grid_records(segv.data(), G, base.data()), w2 = sig::grid_t2_words(n);
     size_t at = (sizeof(uint32_t) * (size_t)G + 255) & ~(size_t)255;
-    const size_t parts[4] = {sizeof(sig::GridContig<S>) * (size_t)G, sizeof(uint32_t) * (size_t)w1,
+    const size_t parts[4] = {sizeof(sig::GridContig<S>) * (size_t)G, sizeof(uint4) * (size_t)w1,
                              sizeof(uint32_t) * (size_t)w2, sizeof(uint16_t) * (size_t)(n + 16)};
     for (int a = 0; a < (a1 ? 2 : 1); ++a)
         for (int k = 0; k < 4; ++k) {
@@ -396,7 +396,7 @@ int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vect
     for (int a = 0; a < (a1 ? 2 : 1); ++a)
         SI_CK(sig::launch_grid_build<S>(a ? a1 : a0, n, d_seg, G, reinterpret_cast<uint32_t*>(p), w1,
                                         reinterpret_cast<sig::GridContig<S>*>(p + g.at[a][0]),
-                                        reinterpret_cast<uint32_t*>(p + g.at[a][1]),
+                                        reinterpret_cast<uint4*>(p + g.at[a][1]),
                                         reinterpret_cast<uint32_t*>(p + g.at[a][2]),
                                         reinterpret_cast<uint16_t*>(p + g.at[a][3]), st));
     return SI_OK;

@@ -22,11 +22,13 @@ __device__ __forceinline__ int owner(const uint32_t* __restrict__ base, int G, u
 }
 
 // buckets a contig of n entries may have (two at least, so that any span fits with a shift below
-// 64); its words in t1 are one more
+// 64); its records are one more
 __host__ __device__ __forceinline__ uint32_t grid_cap(int64_t n) {
     const int64_t c = n / kGridFill;
     return (uint32_t)(c > 2 ? c : 2);
 }
+
+constexpr int kSamples = 64;
 
 template <typename S>
 __global__ void k_grid_params(const S* __restrict__ arr, const int64_t* __restrict__ seg, int G,
@@ -39,7 +41,18 @@ __global__ void k_grid_params(const S* __restrict__ arr, const int64_t* __restri
     if (hi > lo) {
         c.k0 = arr[lo];
         const uint64_t span = (uint64_t)(int64_t)arr[hi - 1] - (uint64_t)(int64_t)arr[lo];
-        const uint32_t cap = grid_cap(hi - lo);
+        // records for the entries outside the crowded stretches: the others, at least four times as
+        // dense as the whole, get sub-tables, and a smaller table stays closer (gaps of 5 M intervals,
+        // 5 M differences: 270 us with a record per four gaps throughout, 257 so)
+        int spread = 0;
+        S from = c.k0;
+#pragma unroll 8
+        for (int k = 1; k <= kSamples; ++k) {
+            const S to = arr[lo + (hi - lo - 1) * k / kSamples];
+            spread += (uint64_t)(int64_t)to - (uint64_t)(int64_t)from >= span / (4 * kSamples) ? 1 : 0;
+            from = to;
+        }
+        const uint32_t cap = grid_cap((hi - lo) * spread / kSamples);
         uint32_t sh = 0;
         while ((span >> sh) >= cap) ++sh;  // at most 63: span >> 63 is below cap
         c.shift = sh;
@@ -61,21 +74,43 @@ __device__ __forceinline__ uint32_t first_off(const S* __restrict__ arr, uint32_
     return a;
 }
 
-// t1: one thread per bucket word, a halving search each.  Neighbouring threads search for
-// neighbouring keys, so their reads fall on the same lines.
+// Records: one thread each, a halving search for the bucket's first position (neighbouring threads
+// search for neighbouring keys, so their reads fall on the same lines), then its entries' codes.  A
+// block's last thread only finds the end of the one before.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ arr, const int64_t* __restrict__ seg,
                                                         int G, const uint32_t* __restrict__ base,
-                                                        const GridContig<S>* __restrict__ cs, uint32_t words,
-                                                        uint32_t* __restrict__ t1) {
-    const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= words) return;
-    const int g = owner(base, G, i);
-    const GridContig<S> c = cs[g];
-    const uint32_t j = i - c.base;
-    if (j > c.nb) return;
-    const uint32_t lo = (uint32_t)seg[g], hi = (uint32_t)seg[g + 1];
-    t1[i] = j == 0 ? lo : j == c.nb ? hi : first_off(arr, lo, hi, c.k0, (uint64_t)j << c.shift);
+                                                        const GridContig<S>* __restrict__ cs, uint32_t records,
+                                                        uint4* __restrict__ rec) {
+    __shared__ uint32_t s_at[kThreads];
+    const uint32_t i = blockIdx.x * (kThreads - 1) + threadIdx.x;
+    uint32_t at = 0, j = 0;
+    GridContig<S> c{};
+    if (i < records) {
+        const int g = owner(base, G, i);
+        c = cs[g];
+        j = i - c.base;
+        const uint32_t lo = (uint32_t)seg[g], hi = (uint32_t)seg[g + 1];
+        at = j == 0 ? lo : j >= c.nb ? hi : first_off(arr, lo, hi, c.k0, (uint64_t)j << c.shift);
+    }
+    s_at[threadIdx.x] = at;
+    __syncthreads();
+    if (threadIdx.x == kThreads - 1 || i >= records || j > c.nb) return;
+    const uint32_t cnt = j < c.nb ? s_at[threadIdx.x + 1] - at : 0u;
+    uint4 x = make_uint4(at, ~0u, ~0u, ~0u);
+    if (cnt > kGridSlots) {
+        x = make_uint4(at | kGridMany, cnt, 0u, 0u);
+    } else {
+        uint32_t w[3] = {~0u, ~0u, ~0u};
+#pragma unroll
+        for (uint32_t k = 0; k < kGridSlots; ++k)
+            if (k < cnt) {
+                const uint32_t code = grid_code((uint64_t)(int64_t)arr[at + k] - (uint64_t)(int64_t)c.k0, c.shift);
+                w[k >> 2] ^= (code ^ 0xffu) << (8 * (k & 3));
+            }
+        x = make_uint4(at, w[0], w[1], w[2]);
+    }
+    rec[i] = x;
 }
 
 // Offsets and t2: one thread per position.  A position of a crowded bucket writes itself to the words of the
@@ -85,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ ar
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr, const int64_t* __restrict__ seg,
                                                        int G, int64_t n, const GridContig<S>* __restrict__ cs,
-                                                       const uint32_t* __restrict__ t1, uint32_t* __restrict__ t2,
+                                                       const uint4* __restrict__ rec, uint32_t* __restrict__ t2,
                                                        uint16_t* __restrict__ lo) {
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
@@ -98,9 +133,9 @@ __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr
     const GridContig<S> c = cs[g];
     const uint64_t d = (uint64_t)(int64_t)arr[i] - (uint64_t)(int64_t)c.k0;
     lo[i] = (uint16_t)((uint32_t)d & ((1u << min(c.shift, 16u)) - 1u));
-    const uint32_t* t = t1 + c.base + (uint32_t)(d >> c.shift);
-    const uint32_t a = t[0], e = t[1], cnt = e - a;
-    if (cnt < kGridDense) return;
+    const uint4 x = rec[c.base + (uint32_t)(d >> c.shift)];
+    if (x.x < kGridMany || x.y < kGridDense) return;
+    const uint32_t a = x.x & ~kGridMany, cnt = x.y, e = a + cnt;
     const int k = grid_sub_bits(cnt, c.shift), ss = (int)c.shift - k;
     const uint32_t nsub = 1u << k, last = nsub - 1u;
     const uint32_t r = (uint32_t)(d >> ss) & last;
@@ -187,10 +222,10 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
 // walked by their warp.
 // Bound by random sector reads (ncu at 12.5 M x 12.5 M int32: L2 75%, DRAM 63% of peak, 5.0 TB/s;
 // issue 23%).  One query per thread keeps 92% of the warps resident to cover the four dependent
-// reads.  12.5 M random queries: 267 us (371 us halving over the coordinates instead of packed
-// offsets); 990 us through the sorted batch (sort, gather and scattered count write).  2-4 or 8-16
-// entries a bucket instead of 4-8: 296 and 287 us.  A word pair per bucket, so that both table words
-// come in one read: 319 us (twice the table).  Contig records in shared memory: 352 us.
+// reads.  12.5 M random queries: 226 us; 990 us through the sorted batch (sort, gather and scattered
+// count write).  With first positions in one table and the offsets in another 267 us (halving over
+// the coordinates instead: 371), with a record per 3 or 6 entries 220 and 256 us.  Contig records in
+// shared memory cost 20 us.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
                                                          const S* __restrict__ qs, const S* __restrict__ qe,
@@ -202,7 +237,8 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
     if (q < nq) counts[q] = cnt;
 }
 
-// 20 M random 64-bit queries over 20 M keys, 70% of both in hotspots: 218 us; 2.31 ms through the
+// 20 M random 64-bit queries over 20 M keys, 70% of both in hotspots: 241 us (218 with a table of first
+// positions, whose words are four times as close in the hotspots); 2.31 ms through the
 // sorted batch, whose search windows a hotspot overflows.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, const S* __restrict__ qe,
@@ -218,7 +254,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, con
     }
     const GridContig<S> c = load_contig(gs.c + g);
     const uint32_t r = grid_first_gt<S>(gs, c, qe[q]);
-    out[q] = (int32_t)(r - (qc ? __ldg(gs.t1 + c.base) : 0u)) - 1;  // without contig ids: contig 0
+    out[q] = (int32_t)(r - (qc ? grid_first_of(gs.rec + c.base) : 0u)) - 1;  // without contig ids: contig 0
 }
 
 // Coverage of a query with qs <= qe, over the hits {start <= qe} minus {end < qs}:
@@ -228,7 +264,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, con
 // with a_u the first start > qe, r_qs / r_qe the first sorted ends >= qs / > qe, ls the first
 // start >= qs, and PS / PE the exclusive prefix sums (mod 2^64) of the starts and of the sorted
 // ends.  The coverage, sum min - sum max, wraps as the coordinate type does.
-// 5 M x 5 M: 288 us for the call; 853 us through the sorted batch and three block searches.
+// 5 M x 5 M: 236 us for the call; 853 us through the sorted batch and three block searches.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<S> ge, int G,
                                                        const S* __restrict__ qs, const S* __restrict__ qe,
@@ -528,7 +564,7 @@ __global__ void __launch_bounds__(kThreads) k_gap_write(MapView<S> m, int64_t sl
 // One warp writes the pieces of 32 neighbouring queries, which lie one after another in the output:
 // lane l takes every 32nd piece of the warp's stretch and finds its query among the 32 by halving
 // over their offsets (shuffles), so writes coalesce and a query of many pieces is shared by all lanes.
-// 5 M queries against 5 M intervals: the whole call 1856 us with hit lists swept per query, 283 us
+// 5 M queries against 5 M intervals: the whole call 1856 us with hit lists swept per query, 257 us
 // from the gaps.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_gap_emit(const S* __restrict__ gs, const S* __restrict__ ge,
@@ -575,7 +611,7 @@ inline unsigned blocks_for(int64_t n) { return (unsigned)std::max<int64_t>(1, ce
 
 }  // namespace
 
-int64_t grid_t1_words(const int64_t* seg, int G, uint32_t* base) {
+int64_t grid_records(const int64_t* seg, int G, uint32_t* base) {
     int64_t w = 0;
     for (int g = 0; g < G; ++g) {
         base[g] = (uint32_t)w;
@@ -586,11 +622,12 @@ int64_t grid_t1_words(const int64_t* seg, int G, uint32_t* base) {
 
 template <typename S>
 cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G, const uint32_t* d_base,
-                              int64_t t1_words, GridContig<S>* c, uint32_t* t1, uint32_t* t2, uint16_t* lo,
+                              int64_t records, GridContig<S>* c, uint4* rec, uint32_t* t2, uint16_t* lo,
                               cudaStream_t st) {
     k_grid_params<S><<<blocks_for(G), kThreads, 0, st>>>(arr, seg, G, d_base, c);
-    k_grid_fill<S><<<blocks_for(t1_words), kThreads, 0, st>>>(arr, seg, G, d_base, c, (uint32_t)t1_words, t1);
-    k_grid_sub<S><<<blocks_for(n), kThreads, 0, st>>>(arr, seg, G, n, c, t1, t2, lo);
+    k_grid_fill<S><<<(unsigned)ceil_div(records, (int64_t)kThreads - 1), kThreads, 0, st>>>(arr, seg, G, d_base, c,
+                                                                                           (uint32_t)records, rec);
+    k_grid_sub<S><<<blocks_for(n), kThreads, 0, st>>>(arr, seg, G, n, c, rec, t2, lo);
     note_launch(3);
     return cudaGetLastError();
 }
@@ -720,7 +757,7 @@ cudaError_t launch_gap_emit(const S* gs, const S* ge, QueryBatch q, const uint32
 
 #define SIG_RINST(S)                                                                                            \
     template cudaError_t launch_grid_build<S>(const S*, int64_t, const int64_t*, int, const uint32_t*, int64_t,  \
-                                              GridContig<S>*, uint32_t*, uint32_t*, uint16_t*, cudaStream_t);       \
+                                              GridContig<S>*, uint4*, uint32_t*, uint16_t*, cudaStream_t);          \
     template cudaError_t launch_rank_count<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, uint32_t*, int*, \
                                               cudaStream_t);                                                     \
     template cudaError_t launch_rank_scan<S>(MapView<S>, RankGrid<S>, RankGrid<S>, QueryBatch, bool, uint32_t*,  \

@@ -5,34 +5,38 @@
 // key).  A halving search makes log2(n) dependent reads per rank, and sorting the batch first, so
 // that neighbours share a search window, costs three radix passes, a gather and a scattered write.
 // The grid cuts each contig's coordinate range into power-of-two wide buckets, 4-8 entries each on
-// average (table t1: first position of every bucket), so that a rank is one read of two adjacent
-// table words and a search over the few entries between them.  Where coordinates crowd, a bucket of
-// kGridDense entries or more is cut again, by its own count, in table t2; its words sit at 3/8 of
-// the bucket's first position, so that no second index is needed (a bucket of n entries uses at
-// most n/4 + 1 words).  Any bucket still crowded after that is searched by halving: the answer is
-// exact for every distribution, only the number of reads changes.
-// Inside buckets at most 65536 wide the entries are compared by their 16-bit offsets from the bucket's
-// first coordinate, eight to a 16-byte read (four packed compares), not by halving over the coordinates:
-// the usual bucket is one read instead of two or three dependent ones, and the tables and offsets of
-// an 8 M-interval index, starts and ends, are 58 MB, which the L2 keeps; the coordinates alone are
-// 64 MB of 32 bits, 128 MB of 64.
-// Memory: at most 4.5 bytes per entry and array (t1 1, t2 1.5, offsets 2), beside 4 or 8 for the coordinates.
+// average, with a 16-byte record each: the bucket's first position and, of up to 12 entries, the top
+// seven bits of their offsets from the bucket's first coordinate.  A rank is then one 16-byte read and
+// a packed compare of the key's own seven bits; only where an entry shares them with the key (1 in 20
+// ranks) are those entries compared in full.  Where coordinates crowd, the record of a bucket of more
+// entries holds their number; one of kGridDense or more is cut again, by its own count, in table t2;
+// its words sit at 3/8 of the bucket's first position, so that no second index is needed (a bucket of
+// n entries uses at most n/4 + 1 words).  Any bucket still crowded after that is searched by halving:
+// the answer is exact for every distribution, only the number of reads changes.
+// Full compares take 16-bit offsets inside buckets at most 65536 wide, eight to a 16-byte read, and
+// the coordinates elsewhere.  What bounds it is sectors from the L2 (some 9 TB/s of them): the tables
+// and offsets of an 8 M-interval index, starts and ends, are some 100 MB, but a rank reads one sector,
+// not the two or three of a table of first positions with the offsets beside it.
+// Memory: at most 7.5 bytes per entry and array (records 4, t2 1.5, offsets 2), beside 4 or 8 for the
+// coordinates.
 #pragma once
 #include "si_internal.cuh"
 
 namespace sig {
 
 constexpr uint32_t kGridFill = 4;    // at most n / kGridFill buckets: 4-8 entries a bucket
-constexpr uint32_t kGridDense = 32;  // entries from which a bucket has its own table (>= 24: see above)
+constexpr uint32_t kGridSlots = 12;  // entries whose codes a record holds
+constexpr uint32_t kGridMany = 0x80000000u;
+constexpr uint32_t kGridDense = 20;  // entries from which a bucket has its own table (>= 13: see above)
 constexpr int kGridSubBits = 10;     // at most 1024 words of t2 per bucket
 
-// A contig's buckets.  Its first position is t1[base], its end t1[base + nb].
+// A contig's buckets.  Its first position is in rec[base], its end in rec[base + nb].
 template <typename S>
 struct GridContig;
 template <>
 struct alignas(16) GridContig<int32_t> {
     int32_t k0;      // smallest key
-    uint32_t base;   // first word in t1 (nb + 1 words)
+    uint32_t base;   // first record (nb + 1 of them)
     uint32_t nb;     // buckets (0: empty contig)
     uint32_t shift;  // bucket width 2^shift (offsets are kept up to 16)
 };
@@ -46,7 +50,9 @@ template <typename S>
 struct RankGrid {
     const S* arr = nullptr;          // ascending inside each contig
     const GridContig<S>* c = nullptr;
-    const uint32_t* t1 = nullptr;    // per bucket: its first position (then the contig's end)
+    // per bucket (then one for the contig's end): x its first position, y to w a byte per entry, unused
+    // ones 0xff; of a bucket with more entries x has kGridMany set and y is their number
+    const uint4* rec = nullptr;
     const uint32_t* t2 = nullptr;
     const uint16_t* lo = nullptr;    // offsets inside buckets of contigs with shift <= 16
 };
@@ -69,6 +75,15 @@ __device__ __forceinline__ int grid_sub_bits(uint32_t cnt, uint32_t shift) {
 }
 __device__ __forceinline__ uint32_t grid_sub_base(uint32_t first) { return (uint32_t)((3ull * first + 7) >> 3); }
 
+// Top seven bits of an offset in a bucket 2^shift wide (all of them up to 2^7).
+__device__ __forceinline__ uint32_t grid_code(uint64_t d, uint32_t shift) {
+    return shift > 7 ? (uint32_t)(d >> (shift - 7)) & 127u : (uint32_t)d & ((1u << shift) - 1u);
+}
+
+__device__ __forceinline__ uint32_t grid_first_of(const uint4* __restrict__ rec) {
+    return __ldg(reinterpret_cast<const uint32_t*>(rec)) & ~kGridMany;
+}
+
 // The positions [a, a + len) among which the first entry >= v of the contig lies (a + len when none
 // of them is): len is 0 where the tables alone give the answer.  off: v's offset in its bucket.
 template <typename S>
@@ -77,10 +92,27 @@ __device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridCon
     const uint64_t d = (uint64_t)(int64_t)v - (uint64_t)(int64_t)c.k0;
     const uint64_t b = d >> c.shift;
     const bool before = v <= c.k0, in = !before && b < c.nb;
-    const uint32_t* t1 = R.t1 + c.base + (before ? 0u : in ? (uint32_t)b : c.nb);
-    a = __ldg(t1);
-    len = in ? __ldg(t1 + 1) - a : 0u;
+    const uint4 x = __ldg(R.rec + c.base + (before ? 0u : in ? (uint32_t)b : c.nb));
+    a = x.x & ~kGridMany;
+    len = 0;
     off = (uint32_t)d & ((1u << min(c.shift, 16u)) - 1u);
+    if (!in) return;
+    if (x.x < kGridMany) {
+        // bytes with the top bit set are >= the code (codes have seven bits, so no borrow leaves a
+        // byte); taking one more away leaves it where they are above the code
+        constexpr uint32_t H = 0x80808080u, one = 0x01010101u;
+        const uint32_t q = grid_code(d, c.shift) * one;
+        const uint32_t y = (x.y | H) - q, z = (x.z | H) - q, w = (x.w | H) - q;
+        const uint32_t lt = (~y & H) | ((~z & H) >> 1) | ((~w & H) >> 2);
+        const uint32_t n = (uint32_t)__popc(lt);
+        if (c.shift > 7) {
+            const uint32_t le = (~(y - one) & ~x.y & H) | ((~(z - one) & ~x.z & H) >> 1) | ((~(w - one) & ~x.w & H) >> 2);
+            len = (uint32_t)__popc(le) - n;
+        }
+        a += n;
+        return;
+    }
+    len = x.y;
     if (len >= kGridDense) {
         const int k = grid_sub_bits(len, c.shift);
         const int ss = (int)c.shift - k;
@@ -147,7 +179,7 @@ __device__ __forceinline__ uint32_t grid_first_geq(const RankGrid<S>& R, const G
 // First position with arr > v.
 template <typename S>
 __device__ __forceinline__ uint32_t grid_first_gt(const RankGrid<S>& R, const GridContig<S>& c, S v) {
-    return v == Lim<S>::hi ? __ldg(R.t1 + c.base + c.nb) : grid_first_geq<S>(R, c, (S)(v + 1));
+    return v == Lim<S>::hi ? grid_first_of(R.rec + c.base + c.nb) : grid_first_geq<S>(R, c, (S)(v + 1));
 }
 
 // first_gt(v1) in one array and first_geq(v2) in another, their table reads side by side.
@@ -162,17 +194,17 @@ __device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const Grid
     grid_bracket(R2, c2, v2, a2, l2, o2);
     r1 = grid_inside(R1, c1, w1, a1, l1, o1);
     r2 = grid_inside(R2, c2, v2, a2, l2, o2);
-    if (top) r1 = __ldg(R1.t1 + c1.base + c1.nb);
+    if (top) r1 = grid_first_of(R1.rec + c1.base + c1.nb);
 }
 
 // ---------------------------------------------------------------- launchers (si_rank.cu)
-// Words of t1 for contigs of these sizes (fills base[g]), and of t2 for n entries.
-int64_t grid_t1_words(const int64_t* seg, int G, uint32_t* base);
+// Records for contigs of these sizes (fills base[g]), and words of t2 for n entries.
+int64_t grid_records(const int64_t* seg, int G, uint32_t* base);
 inline int64_t grid_t2_words(int64_t n) { return (3 * n + 7) / 8 + 8; }
-// Builds the tables over arr (ascending inside each contig): d_base holds grid_t1_words' bases.
+// Builds the tables over arr (ascending inside each contig): d_base holds grid_records' bases.
 template <typename S>
 cudaError_t launch_grid_build(const S* arr, int64_t n, const int64_t* seg, int G, const uint32_t* d_base,
-                              int64_t t1_words, GridContig<S>* c, uint32_t* t1, uint32_t* t2, uint16_t* lo,
+                              int64_t records, GridContig<S>* c, uint4* rec, uint32_t* t2, uint16_t* lo,
                               cudaStream_t st);
 
 // Counts of a batch in its own order, for an index without intervals with start > end.
