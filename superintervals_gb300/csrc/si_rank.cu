@@ -173,37 +173,53 @@ __device__ uint32_t warp_walk_count(const MapView<S>& m, int64_t lo, int64_t top
     return cnt;
 }
 
-// One query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
+// One query and the records of its two ranks (g < 0: none, or a contig outside the index).
+template <typename S>
+struct RankQuery {
+    int g = -1;
+    S s = 0, e = 0;
+    uint4 x1, x2;
+};
+template <typename S>
+__device__ __forceinline__ void rank_load(const MapView<S>& m, const S* __restrict__ qs, const S* __restrict__ qe,
+                                          const int32_t* __restrict__ qc, int64_t q, int64_t nq, int* d_err,
+                                          RankQuery<S>& Q) {
+    if (q >= nq) return;
+    const int g = qc ? qc[q] : 0;
+    Q.s = qs[q];
+    Q.e = qe[q];
+    if (g >= 0 && g < m.G) Q.g = g;
+    else atomicCAS(d_err, kDevOk, kDevBadContig);
+}
+template <typename S>
+__device__ __forceinline__ void rank_probe(const RankGrid<S>& gs, const RankGrid<S>& ge, RankQuery<S>& Q) {
+    const int g = max(Q.g, 0);
+    Q.x1 = __ldg(gs.rec + grid_slot(load_contig(gs.c + g), grid_after(Q.e)));
+    Q.x2 = __ldg(ge.rec + grid_slot(load_contig(ge.c + g), Q.s));
+}
+
+// The query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
 // walked by the whole warp, so every lane of the warp calls it.
 template <typename S>
 __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid<S>& gs, const RankGrid<S>& ge,
-                                             const S* __restrict__ qs, const S* __restrict__ qe,
-                                             const int32_t* __restrict__ qc, int64_t q, bool live, bool pieces,
-                                             int* d_err, int lane, uint32_t& upper) {
+                                             const RankQuery<S>& Q, bool pieces, int lane, uint32_t& upper) {
     bool walk = false;
     uint32_t cnt = 0, lo = 0, top = 0;
-    S s = 0;
+    const S s = Q.s, e = Q.e;
     upper = 0;
-    if (live) {
-        const int g = qc ? qc[q] : 0;
-        if (g < 0 || g >= m.G) {
-            atomicCAS(d_err, kDevOk, kDevBadContig);
+    if (Q.g >= 0) {
+        const GridContig<S> c1 = load_contig(gs.c + Q.g);
+        const bool any = c1.nb != 0 && e >= c1.k0;  // some start at or below the query's end
+        if (s <= e) {
+            uint32_t r2;
+            grid_two_ranks(gs, c1, e, Q.x1, ge, load_contig(ge.c + Q.g), s, Q.x2, top, r2);
+            cnt = top > r2 ? top - r2 : 0u;
         } else {
-            s = qs[q];
-            const S e = qe[q];
-            const GridContig<S> c1 = load_contig(gs.c + g);
-            const bool any = c1.nb != 0 && e >= c1.k0;  // some start at or below the query's end
-            if (s <= e) {
-                uint32_t r2;
-                grid_two_ranks(gs, c1, e, ge, load_contig(ge.c + g), s, top, r2);
-                cnt = top > r2 ? top - r2 : 0u;
-            } else {
-                top = grid_first_gt<S>(gs, c1, e);
-                walk = !pieces && any;
-                lo = walk ? (uint32_t)m.seg[g] : 0u;
-            }
-            upper = any && (s <= e || !pieces) ? top : 0u;
+            top = grid_first_gt<S>(gs, c1, e);
+            walk = !pieces && any;
+            lo = walk ? (uint32_t)m.seg[Q.g] : 0u;
         }
+        upper = any && (s <= e || !pieces) ? top : 0u;
     }
     unsigned todo = __ballot_sync(kFull, walk);
     while (todo) {
@@ -220,12 +236,13 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
 // Counts: no interval has start > end, so an interval that ends before qs starts before qe, and
 // count = #(start <= qe) - #(end < qs) for every query with qs <= qe.  The others (qs > qe) are
 // walked by their warp.
-// Bound by random sector reads (ncu at 12.5 M x 12.5 M int32: L2 75%, DRAM 63% of peak, 5.0 TB/s;
-// issue 23%).  One query per thread keeps 92% of the warps resident to cover the four dependent
-// reads.  12.5 M random queries: 226 us; 990 us through the sorted batch (sort, gather and scattered
-// count write).  With first positions in one table and the offsets in another 267 us (halving over
-// the coordinates instead: 371), with a record per 3 or 6 entries 220 and 256 us.  Contig records in
-// shared memory cost 20 us.
+// Bound by random sector reads (ncu at 12.5 M x 12.5 M int32: 5 L2 sectors a query, two of them the
+// records, which come from DRAM for the larger part: 1.08 GB, 61% of its peak; issue 46%).  One query
+// per thread keeps 84% of the warps resident.  12.5 M random queries: 205 us, with both records read
+// before either is used (226 else); 990 us through the sorted batch (sort, gather and scattered count
+// write).  With first positions in one table and the offsets in another 267 us (halving over the
+// coordinates instead: 371), with a record per 3 or 6 entries 3% less and 13% more.  Contig records
+// in shared memory cost 20 us.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
                                                          const S* __restrict__ qs, const S* __restrict__ qe,
@@ -233,7 +250,10 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
                                                          uint32_t* __restrict__ counts, int* d_err) {
     const int64_t q = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     uint32_t upper;
-    const uint32_t cnt = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, false, d_err, threadIdx.x & 31, upper);
+    RankQuery<S> Q;
+    rank_load(m, qs, qe, qc, q, nq, d_err, Q);
+    rank_probe(gs, ge, Q);
+    const uint32_t cnt = rank_one<S>(m, gs, ge, Q, false, threadIdx.x & 31, upper);
     if (q < nq) counts[q] = cnt;
 }
 
@@ -264,7 +284,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_ub(RankGrid<S> gs, int G, con
 // with a_u the first start > qe, r_qs / r_qe the first sorted ends >= qs / > qe, ls the first
 // start >= qs, and PS / PE the exclusive prefix sums (mod 2^64) of the starts and of the sorted
 // ends.  The coverage, sum min - sum max, wraps as the coordinate type does.
-// 5 M x 5 M: 236 us for the call; 853 us through the sorted batch and three block searches.
+// 5 M x 5 M: 225 us for the call; 853 us through the sorted batch and three block searches.
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<S> ge, int G,
                                                        const S* __restrict__ qs, const S* __restrict__ qe,
@@ -286,8 +306,11 @@ __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<
     }
     const GridContig<S> c1 = load_contig(gs.c + g), c2 = load_contig(ge.c + g);
     uint32_t a_u, r_qs, r_qe, ls;
-    grid_two_ranks(gs, c1, e, ge, c2, s, a_u, r_qs);
-    grid_two_ranks(ge, c2, e, gs, c1, s, r_qe, ls);
+    const S after = grid_after(e);
+    grid_two_ranks(gs, c1, e, __ldg(gs.rec + grid_slot(c1, after)), ge, c2, s, __ldg(ge.rec + grid_slot(c2, s)), a_u,
+                   r_qs);
+    grid_two_ranks(ge, c2, e, __ldg(ge.rec + grid_slot(c2, after)), gs, c1, s, __ldg(gs.rec + grid_slot(c1, s)), r_qe,
+                   ls);
     const uint64_t qe64 = (uint64_t)(int64_t)e, qs64 = (uint64_t)(int64_t)s;
     const uint64_t smin = ps_end[r_qe] - ps_end[r_qs] + qe64 * ((uint64_t)a_u - (uint64_t)r_qe);
     const uint64_t smax = ps_start[a_u] - ps_start[ls] + qs64 * ((uint64_t)ls - (uint64_t)r_qs);
@@ -338,8 +361,10 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
     for (int r = 0; r < R; ++r) {
         const int64_t q = base + r * kWarp;
         uint32_t upper;
-        const int64_t x = rank_one<S>(m, gs, ge, qs, qe, qc, q, q < nq, pieces != 0, &work->err, lane,
-                                      upper);
+        RankQuery<S> Q;
+        rank_load(m, qs, qe, qc, q, nq, &work->err, Q);
+        rank_probe(gs, ge, Q);
+        const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, lane, upper);
         if (q < nq) su[q] = upper;
         int64_t inc = x;
 #pragma unroll

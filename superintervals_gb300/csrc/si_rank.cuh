@@ -84,15 +84,21 @@ __device__ __forceinline__ uint32_t grid_first_of(const uint4* __restrict__ rec)
     return __ldg(reinterpret_cast<const uint32_t*>(rec)) & ~kGridMany;
 }
 
-// The positions [a, a + len) among which the first entry >= v of the contig lies (a + len when none
-// of them is): len is 0 where the tables alone give the answer.  off: v's offset in its bucket.
+// The record of v's bucket (before the contig: its first one's, behind it: the end's).
 template <typename S>
-__device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridContig<S>& c, S v, uint32_t& a,
+__device__ __forceinline__ uint32_t grid_slot(const GridContig<S>& c, S v) {
+    const uint64_t b = ((uint64_t)(int64_t)v - (uint64_t)(int64_t)c.k0) >> c.shift;
+    return c.base + (v <= c.k0 ? 0u : b < c.nb ? (uint32_t)b : c.nb);
+}
+
+// The positions [a, a + len) among which the first entry >= v of the contig lies (a + len when none
+// of them is), x being v's record: len is 0 where the tables alone give the answer.  off: v's offset
+// in its bucket.
+template <typename S>
+__device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridContig<S>& c, S v, uint4 x, uint32_t& a,
                                              uint32_t& len, uint32_t& off) {
     const uint64_t d = (uint64_t)(int64_t)v - (uint64_t)(int64_t)c.k0;
-    const uint64_t b = d >> c.shift;
-    const bool before = v <= c.k0, in = !before && b < c.nb;
-    const uint4 x = __ldg(R.rec + c.base + (before ? 0u : in ? (uint32_t)b : c.nb));
+    const bool in = v > c.k0 && (d >> c.shift) < c.nb;
     a = x.x & ~kGridMany;
     len = 0;
     off = (uint32_t)d & ((1u << min(c.shift, 16u)) - 1u);
@@ -172,7 +178,7 @@ __device__ __forceinline__ uint32_t grid_inside(const RankGrid<S>& R, const Grid
 template <typename S>
 __device__ __forceinline__ uint32_t grid_first_geq(const RankGrid<S>& R, const GridContig<S>& c, S v) {
     uint32_t a, len, off;
-    grid_bracket(R, c, v, a, len, off);
+    grid_bracket(R, c, v, __ldg(R.rec + grid_slot(c, v)), a, len, off);
     return grid_inside(R, c, v, a, len, off);
 }
 
@@ -182,22 +188,27 @@ __device__ __forceinline__ uint32_t grid_first_gt(const RankGrid<S>& R, const Gr
     return v == Lim<S>::hi ? grid_first_of(R.rec + c.base + c.nb) : grid_first_geq<S>(R, c, (S)(v + 1));
 }
 
-// first_gt(v1) in one array and first_geq(v2) in another, their table reads side by side.
+// The key whose first_geq is v's first_gt, where there is one.
 template <typename S>
-__device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const GridContig<S>& c1, S v1,
-                                               const RankGrid<S>& R2, const GridContig<S>& c2, S v2, uint32_t& r1,
-                                               uint32_t& r2) {
-    uint32_t a1, l1, o1, a2, l2, o2;
-    const bool top = v1 == Lim<S>::hi;
-    const S w1 = top ? v1 : (S)(v1 + 1);
-    grid_bracket(R1, c1, w1, a1, l1, o1);
-    grid_bracket(R2, c2, v2, a2, l2, o2);
-    r1 = grid_inside(R1, c1, w1, a1, l1, o1);
-    r2 = grid_inside(R2, c2, v2, a2, l2, o2);
-    if (top) r1 = grid_first_of(R1.rec + c1.base + c1.nb);
+__device__ __forceinline__ S grid_after(S v) {
+    return v == Lim<S>::hi ? v : (S)(v + 1);
 }
 
-// ---------------------------------------------------------------- launchers (si_rank.cu)
+// first_gt(v1) in one array and first_geq(v2) in another, x1 and x2 being the records of
+// grid_after(v1) and v2.
+template <typename S>
+__device__ __forceinline__ void grid_two_ranks(const RankGrid<S>& R1, const GridContig<S>& c1, S v1, uint4 x1,
+                                               const RankGrid<S>& R2, const GridContig<S>& c2, S v2, uint4 x2,
+                                               uint32_t& r1, uint32_t& r2) {
+    uint32_t a1, l1, o1, a2, l2, o2;
+    const S w1 = grid_after(v1);
+    grid_bracket(R1, c1, w1, x1, a1, l1, o1);
+    grid_bracket(R2, c2, v2, x2, a2, l2, o2);
+    r1 = grid_inside(R1, c1, w1, a1, l1, o1);
+    r2 = grid_inside(R2, c2, v2, a2, l2, o2);
+    if (v1 == Lim<S>::hi) r1 = grid_first_of(R1.rec + c1.base + c1.nb);
+}
+
 // Records for contigs of these sizes (fills base[g]), and words of t2 for n entries.
 int64_t grid_records(const int64_t* seg, int G, uint32_t* base);
 inline int64_t grid_t2_words(int64_t n) { return (3 * n + 7) / 8 + 8; }
