@@ -50,9 +50,9 @@ extern "C" {
 #define SI_ORDER_DESC 1       /* search_values (hpp:551-579) and C searchIdxs (c_superintervals.h:610-643) */
 
 /* ---- query paths -------------------------------------------------------- */
-#define SI_PATH_AUTO 0        /* library choice */
+#define SI_PATH_AUTO 0        /* library choice: ranks, a direct emit or sorted tiles */
 #define SI_PATH_PLAIN 1       /* one query per thread, reference walk */
-#define SI_PATH_BATCHED 2     /* sorted-query tiles sharing one candidate walk */
+#define SI_PATH_BATCHED 2     /* sorted-query tiles sharing their candidates */
 
 /* ---- upper-bound search modes -------------------------------------------- */
 #define SI_UB_BINARY 0        /* branch-free halving search (superintervals.hpp:501-516) */
@@ -163,7 +163,8 @@ int setBatchedParamsGpu(gSuperIntervals* si, int tile_queries, int tile_candidat
 int getBatchedParamsGpu(const gSuperIntervals* si, int* tile_queries, int* tile_candidates,
                         int64_t* long_query_len, int64_t* split_len);
 /* Further tunables of the batched path (no reference counterpart); results never depend on
- * them.  SI_OPT_EMIT_COPY: 1 writes the section of a tile's long candidates that comes from
+ * them.  SI_OPT_EMIT_COPY (batches counted by the tiles, i.e. an index with start > end
+ * intervals, and graph capture): 1 writes the section of a tile's long candidates that comes from
  * the long-interval list (intervals at least 32768 long) as copied runs between its few
  * misses, 0 (default) checks every candidate.  SI_OPT_EYTZ_DEPTH: levels of the Eytzinger
  * tree (1-13, 0 automatic), resampled at once when it is the current provider.
