@@ -3128,6 +3128,18 @@ int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>
     return SI_OK;
 }
 
+// Allows a kernel all the dynamic shared memory that a block may have.  The limit belongs to the
+// kernel, not to a handle: set to one launch's size, it would refuse another handle's larger launch.
+static cudaError_t allow_smem(const void* fn, int dev) {
+    cudaFuncAttributes at;
+    int most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&at, fn);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    return e;
+}
+
 // Tile size: the largest of 256, 128, 64, 32 queries whose expected candidates, tile * (intervals
 // per query) + hits per query, fill at most 3/4 of the candidate slots (a tile that overflows them
 // emits its queries one by one).
@@ -3204,7 +3216,7 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
         int dev = 0, nsm = 152, per_sm = 1;
         SI_CU(cudaGetDevice(&dev));
         SI_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        SI_CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        SI_CU(allow_smem(reinterpret_cast<const void*>(fn), dev));
         SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, sm));
         ws.occ_blocks[e] = nsm * std::max(per_sm, 1);
         ws.occ_smem[e] = sm;
@@ -3273,10 +3285,10 @@ static int run_tiles(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, int
         SI_CU(cudaGetDevice(&dev));
         SI_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         if (emit) {
-            SI_CU(cudaFuncSetAttribute(k_tiles<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            SI_CU(allow_smem(reinterpret_cast<const void*>(&k_tiles<S, true>), dev));
             SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tiles<S, true>, kThreads, sm));
         } else {
-            SI_CU(cudaFuncSetAttribute(k_tiles<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            SI_CU(allow_smem(reinterpret_cast<const void*>(&k_tiles<S, false>), dev));
             SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tiles<S, false>, kThreads, sm));
         }
         ws.occ_blocks[e] = nsm * std::max(per_sm, 1);

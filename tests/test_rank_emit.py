@@ -154,3 +154,28 @@ def test_emit_queued_before_the_count(api, bits, nq, hits):
     for d in dev:
         lib.deviceFreeGpu(d)
     idx.close()
+
+
+def test_tiles_of_two_handles_with_different_shared_memory(api, oracle):
+    """A dense batch's tiles need more shared memory than a sparse one's: a search of one handle
+    between two of another leaves the second as the first."""
+    rng = np.random.default_rng(5)
+    n, nq = 40_000, 5_000
+    made = []
+    for span, longest in ((n, 300), (400 * n, 50)):
+        s = np.sort(rng.integers(0, span, n))
+        e = s + rng.integers(0, longest, n)
+        qs = rng.integers(0, span, nq)
+        qe = qs + rng.integers(0, longest, nq)
+        idx = api.GpuIndex(64)
+        idx.add_arrays(s, e)
+        idx.build()
+        idx.set_path(api.PATH_BATCHED)
+        m = oracle.build(s, e, np.zeros(n, np.int32), seg=np.array([0, n]))
+        made.append((idx, qs, qe, oracle.search_batch(m, qs, qe, None, order=1, nthreads=4)))
+    for k in (0, 1, 0, 1, 0):
+        idx, qs, qe, (want_off, want) = made[k]
+        off, out = idx.search(qs, qe, order=1)
+        assert np.array_equal(off, want_off) and np.array_equal(out, want)
+    for idx, *_ in made:
+        idx.close()
