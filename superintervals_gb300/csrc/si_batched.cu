@@ -297,7 +297,8 @@ __device__ void block_excl_scan(int32_t* v, int n, int* s_wsum, int* s_sum) {
 // order into (cpos, cend), one level of the max pyramid per round: every warp expands frontier
 // nodes (one coalesced 32-child load + ballot each), a block scan places the surviving children
 // in order.  Frontier lists ping-pong between cpos and lst.  Returns |C|, or -1 when a frontier
-// or C would exceed `cap`.  Block-uniform.
+// or C would exceed `cap`.  Block-uniform; no warp is still reading the scratch when another one
+// returns, so that a gather may follow at once.
 template <typename S>
 __device__ int gather_bfs(const Pyr<S>& P, int64_t lo, int64_t umax, S L, int cap, int32_t* cpos, S* cend,
                           int32_t* lst, int32_t* cnt, uint32_t* msk, int* s_wsum, int* s_n, int* s_sum,
@@ -326,6 +327,7 @@ __device__ int gather_bfs(const Pyr<S>& P, int64_t lo, int64_t umax, S L, int ca
     }
     __syncthreads();
     int nf = *s_n;
+    if (H == 0 || nf < 0) __syncthreads();  // nothing else separates the read of *s_n from the return
     if (nf < 0) return -1;
     for (int h = H; h >= 1; --h) {
         const S* A = (h == 1) ? P.ends : P.m[h - 2];
@@ -360,7 +362,10 @@ __device__ int gather_bfs(const Pyr<S>& P, int64_t lo, int64_t umax, S L, int ca
         __syncthreads();
         block_excl_scan(cnt, nf, s_wsum, s_sum);
         const int total = *s_sum;
-        if (total > cap) return -1;
+        if (total > cap) {
+            __syncthreads();
+            return -1;
+        }
         for (int f = warp; f < nf; f += kWarpsPerCta) {
             const unsigned m = msk[f];
             if ((m >> lane) & 1u) {
