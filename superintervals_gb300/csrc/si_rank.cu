@@ -151,12 +151,17 @@ __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr
 }
 
 // The positions of one query with start > end that hit, by one warp: the reference's walk 32
-// positions at a time (from a miss it goes on at the smallest branch of the chunk's misses).
+// positions at a time (from a miss it goes on at the smallest branch of the chunk's misses).  A walk
+// is as long as its hits are many; it counts every kBeatChunks chunks in *walked (null: nobody waits
+// for the warp).
+constexpr uint32_t kBeatChunks = 256;
 template <typename S>
-__device__ uint32_t warp_walk_count(const MapView<S>& m, int64_t lo, int64_t top, S s, int lane) {
-    uint32_t cnt = 0;
+__device__ uint32_t warp_walk_count(const MapView<S>& m, int64_t lo, int64_t top, S s, int lane,
+                                    unsigned int* walked) {
+    uint32_t cnt = 0, chunks = 0;
     int64_t i = top;
     while (i >= lo) {
+        if (++chunks % kBeatChunks == 0 && walked && lane == 0) atomicAdd(walked, 1u);
         const int64_t k = i - lane;
         const bool valid = k >= lo;
         S e = 0;
@@ -199,10 +204,11 @@ __device__ __forceinline__ void rank_probe(const RankGrid<S>& gs, const RankGrid
 }
 
 // The query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
-// walked by the whole warp, so every lane of the warp calls it.
+// walked by the whole warp, so every lane of the warp calls it (walked: see warp_walk_count).
 template <typename S>
 __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid<S>& gs, const RankGrid<S>& ge,
-                                             const RankQuery<S>& Q, bool pieces, int lane, uint32_t& upper) {
+                                             const RankQuery<S>& Q, bool pieces, int lane, uint32_t& upper,
+                                             unsigned int* walked) {
     bool walk = false;
     uint32_t cnt = 0, lo = 0, top = 0;
     const S s = Q.s, e = Q.e;
@@ -227,7 +233,7 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
         todo &= todo - 1;
         const uint32_t r = warp_walk_count<S>(m, (int64_t)__shfl_sync(kFull, lo, src),
                                               (int64_t)__shfl_sync(kFull, top, src) - 1, __shfl_sync(kFull, s, src),
-                                              lane);
+                                              lane, walked);
         if (lane == src) cnt = r;
     }
     return cnt;
@@ -253,7 +259,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
     RankQuery<S> Q;
     rank_load(m, qs, qe, qc, q, nq, d_err, Q);
     rank_probe(gs, ge, Q);
-    const uint32_t cnt = rank_one<S>(m, gs, ge, Q, false, threadIdx.x & 31, upper);
+    const uint32_t cnt = rank_one<S>(m, gs, ge, Q, false, threadIdx.x & 31, upper, nullptr);
     if (q < nq) counts[q] = cnt;
 }
 
@@ -322,7 +328,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_cov(RankGrid<S> gs, RankGrid<
 constexpr unsigned long long kTileAgg = 1ull << 62;  // the tile's own total
 constexpr unsigned long long kTilePre = 2ull << 62;  // the total of this and all earlier tiles
 constexpr unsigned long long kTileVal = (1ull << 62) - 1ull;
-constexpr int kSpinLimit = 1 << 22;                  // polls of one window before giving up
+constexpr int kSpinLimit = 1 << 22;                  // polls of one window without progress before giving up
 
 __device__ __forceinline__ void st_tile(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -332,13 +338,20 @@ __device__ __forceinline__ unsigned long long ld_tile(const unsigned long long* 
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned int ld_walked(const unsigned int* p) {
+    unsigned int v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Counts and offsets in one pass: a block takes the next tile of kThreads * R queries from an atomic
 // counter, counts them, publishes the tile's total, and its first warp looks back over the earlier
-// tiles' published totals, 32 at a time, until an inclusive prefix (decoupled look-back; a window
-// that stays unpublished for kSpinLimit polls records kDevTimeout and the walk ends, so the kernel
-// always ends).  Against the count kernel and a scan it saves a launch, a cleared buffer and the
-// counts' way through memory.
+// tiles' published totals, 32 at a time, until an inclusive prefix (decoupled look-back).  A tile of
+// queries with start > end publishes only when it has walked their hits (1024 queries of 4 M hits
+// each: seconds), so a window that stays unpublished for kSpinLimit polls is given up, with
+// kDevTimeout, only when no walk of the launch went on meanwhile; a walk ends at its contig's first
+// position, so the kernel always ends.  Against the count kernel and a scan it saves a launch, a
+// cleared buffer and the counts' way through memory.
 template <typename S, int R>
 __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
                                                         const S* __restrict__ qs, const S* __restrict__ qe,
@@ -364,7 +377,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         RankQuery<S> Q;
         rank_load(m, qs, qe, qc, q, nq, &work->err, Q);
         rank_probe(gs, ge, Q);
-        const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, lane, upper);
+        const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, lane, upper, &work->walked);
         if (q < nq) su[q] = upper;
         int64_t inc = x;
 #pragma unroll
@@ -386,14 +399,20 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         if (t > 0) {
             int64_t top = t - 1;
             int spins = 0;
+            unsigned int walked = 0;
             while (true) {
                 const int64_t p = top - lane;
                 const unsigned long long s = p >= 0 ? ld_tile(status + p) : kTilePre;
                 const unsigned long long f = s & ~kTileVal;
                 if (__any_sync(kFull, f == 0ull)) {
                     if (++spins > kSpinLimit) {
-                        if (lane == 0) atomicCAS(&work->err, kDevOk, kDevTimeout);
-                        break;
+                        const unsigned int now = __shfl_sync(kFull, ld_walked(&work->walked), 0);
+                        if (now == walked) {
+                            if (lane == 0) atomicCAS(&work->err, kDevOk, kDevTimeout);
+                            break;
+                        }
+                        walked = now;
+                        spins = 0;
                     }
                     __nanosleep(32);
                     continue;

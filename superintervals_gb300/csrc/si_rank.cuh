@@ -232,7 +232,8 @@ struct RankWork {
     int inv;                   // free for the caller
     unsigned long long total;  // hits of the batch
     unsigned int tiles;        // tile counter
-    unsigned int pad[11];
+    unsigned int walked;       // progress of the walks of queries with start > end
+    unsigned int pad[10];
 };
 size_t rank_work_bytes(int64_t nq);
 template <typename S>

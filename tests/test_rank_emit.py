@@ -179,3 +179,26 @@ def test_tiles_of_two_handles_with_different_shared_memory(api, oracle):
         assert np.array_equal(off, want_off) and np.array_equal(out, want)
     for idx, *_ in made:
         idx.close()
+
+
+def test_walks_longer_than_a_wait(api):
+    """Queries with start > end that hit everything: a tile's walks (8 warps of 128 queries, 3 M
+    positions each) take longer than later tiles poll for its total, which they do not give up while
+    the walks go on."""
+    import ctypes as C
+
+    n, walks = 3_000_000, 1024
+    nq = 152 * 2048 + walks                                   # four queries a thread from here on
+    idx = api.GpuIndex(32)
+    idx.add_arrays(np.arange(n, dtype=np.int32), np.full(n, 10_000_000, np.int32))
+    idx.build()
+    qs = np.full(nq, 20_000_000, np.int32)                    # behind everything
+    qe = qs.copy()
+    qs[:walks], qe[:walks] = 9_000_000, 5_000_000
+    off, total = np.empty(nq + 1, np.int64), C.c_size_t(0)
+    st = idx.lib.searchBatchIntoGpu(idx.h, C.c_void_p(qs.ctypes.data), C.c_void_p(qe.ctypes.data), None, nq,
+                                    api.ORDER_DESC, 0, C.c_void_p(off.ctypes.data), None, 0, C.byref(total))
+    assert st == api._capi.SI_ERR_CAPACITY
+    assert total.value == walks * n
+    assert np.array_equal(off, np.minimum(np.arange(nq + 1), walks) * n)
+    idx.close()
