@@ -3135,13 +3135,15 @@ int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>
 
 // Allows a kernel all the dynamic shared memory that a block may have.  The limit belongs to the
 // kernel, not to a handle: set to one launch's size, it would refuse another handle's larger launch.
-static cudaError_t allow_smem(const void* fn, int dev) {
+// room: that size.
+static cudaError_t allow_smem(const void* fn, int dev, size_t* room = nullptr) {
     cudaFuncAttributes at;
     int most = 0;
     cudaError_t e = cudaFuncGetAttributes(&at, fn);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    most -= (int)at.sharedSizeBytes;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (room) *room = (size_t)most;
     return e;
 }
 
@@ -3206,22 +3208,35 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
     a.dst = dst;
     a.d_err = d_err;
     const bool pieces = what == kOutPieces;
-    // (the padding: a last slice of candidates may read 31 past its list's end)
-    a.at_rec = (int)(2 * sizeof(Cand<S>) * a.cap + 31 * sizeof(Cand<S>) + 15) & ~15;
-    a.at_start = a.at_rec + (int)sizeof(QRec<S>) * a.tile_q;
-    a.at_class = a.at_start + (int)sizeof(S) * (a.cap + 32);
-    const size_t sm = (size_t)a.at_class + 4 * (size_t)a.tile_q;
-    const int five = sizeof(S) == 4 && sm + 4096 <= kSmemPerSm / 5 ? 1 : 0;  // 4 KB: static and reserved
     using Kernel = void (*)(EmitArgs<S>);
     const Kernel fns[2][2] = {{&k_emit_tiles<S, kOutIdx, 4>, &k_emit_tiles<S, kOutIdx, 5>},
                               {&k_emit_tiles<S, kOutPieces, 4>, &k_emit_tiles<S, kOutPieces, 5>}};
-    const Kernel fn = fns[pieces][five];
     const int e = 2 + (pieces ? 1 : 0);
+    int dev = 0;
+    SI_CU(cudaGetDevice(&dev));
+    if (!ws.smem_room[pieces])
+        for (const Kernel fn : fns[pieces]) {  // of both, what the one with less has
+            size_t room = 0;
+            SI_CU(allow_smem(reinterpret_cast<const void*>(fn), dev, &room));
+            ws.smem_room[pieces] = ws.smem_room[pieces] ? std::min(ws.smem_room[pieces], room) : room;
+        }
+    // 40 bytes a slot with 64-bit coordinates and 52 a query: the largest tunables ask for more than a
+    // block may have (6656 slots and 256 queries: 239,344 bytes of some 230,000).  Fewer slots then: a
+    // tile that overflows them emits its queries one by one.
+    size_t sm;
+    for (;; a.cap -= 256) {
+        // (the padding: a last slice of candidates may read 31 past its list's end)
+        a.at_rec = (int)(2 * sizeof(Cand<S>) * a.cap + 31 * sizeof(Cand<S>) + 15) & ~15;
+        a.at_start = a.at_rec + (int)sizeof(QRec<S>) * a.tile_q;
+        a.at_class = a.at_start + (int)sizeof(S) * (a.cap + 32);
+        sm = (size_t)a.at_class + 4 * (size_t)a.tile_q;
+        if (sm <= ws.smem_room[pieces] || a.cap <= 256) break;
+    }
+    const int five = sizeof(S) == 4 && sm + 4096 <= kSmemPerSm / 5 ? 1 : 0;  // 4 KB: static and reserved
+    const Kernel fn = fns[pieces][five];
     if (ws.occ_smem[e] != sm) {
-        int dev = 0, nsm = 152, per_sm = 1;
-        SI_CU(cudaGetDevice(&dev));
+        int nsm = 152, per_sm = 1;
         SI_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        SI_CU(allow_smem(reinterpret_cast<const void*>(fn), dev));
         SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, sm));
         ws.occ_blocks[e] = nsm * std::max(per_sm, 1);
         ws.occ_smem[e] = sm;

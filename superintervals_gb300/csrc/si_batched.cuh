@@ -87,6 +87,7 @@ struct BatchedWorkspace {
     // resident blocks on the device at that size
     size_t occ_smem[4] = {0, 0, 0, 0};  // count, emit, ranked emit, ranked pieces
     int occ_blocks[4] = {0, 0, 0, 0};
+    size_t smem_room[2] = {0, 0};       // dynamic shared memory that a ranked emit (pieces) may have
     // long-interval list: global positions, starts and ends of the intervals at least long_split long,
     // in position order, its max pyramid (long_H levels) and each contig's first list index
     const void* long_ends = nullptr;

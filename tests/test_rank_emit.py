@@ -202,3 +202,31 @@ def test_walks_longer_than_a_wait(api):
     assert total.value == walks * n
     assert np.array_equal(off, np.minimum(np.arange(nq + 1), walks) * n)
     idx.close()
+
+
+@pytest.mark.parametrize("tile_q,cap", [(32, 6912), (256, 5632), (256, 6656), (1024, 4608), (1024, 5376)])
+def test_large_tunables_with_64_bit_coordinates(api, oracle, tile_q, cap):
+    """Dense batches with 64-bit coordinates at the tile sizes that the shared memory of a block only
+    just holds, or would not hold with a start beside every candidate."""
+    rng = np.random.default_rng(cap)
+    n, nq = 40_000, 5_000
+    s = np.sort(rng.integers(0, n, n))
+    e = s + rng.integers(0, 300, n)
+    qs = rng.integers(0, n, nq)
+    qe = qs + rng.integers(0, 300, nq)
+    idx = api.GpuIndex(64)
+    idx.add_arrays(s, e)
+    idx.build()
+    idx.set_path(api.PATH_BATCHED)
+    api.check(idx.lib.setBatchedParamsGpu(idx.h, tile_q, cap, 0, -1))
+    m = oracle.build(s, e, np.zeros(n, np.int32), seg=np.array([0, n]))
+    want_off, want = oracle.search_batch(m, qs, qe, None, order=1, nthreads=8)
+    off, out = idx.search(qs, qe, order=1)
+    assert np.array_equal(off, want_off) and np.array_equal(out, want)
+    off, ps, pe, ph = idx.intersect(qs, qe, order=1)
+    assert np.array_equal(off, want_off) and np.array_equal(ph, want)
+    sorted_s, sorted_e, _, _ = idx.arrays()
+    owner = np.repeat(np.arange(nq), np.diff(want_off))
+    assert np.array_equal(ps, np.maximum(qs[owner], sorted_s[want]))
+    assert np.array_equal(pe, np.minimum(qe[owner], sorted_e[want]))
+    idx.close()
