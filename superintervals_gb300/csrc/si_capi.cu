@@ -30,6 +30,8 @@ std::atomic<size_t> g_used{0};
 // buffers may have moved is captured again
 std::atomic<unsigned long long> g_alloc_gen{0};
 std::atomic<size_t> g_budget{0};
+// a device allocation of this thread found no room (with_room)
+thread_local bool g_no_room = false;
 
 int fail(int code, const char* fmt, ...) {
     char buf[512];
@@ -77,6 +79,7 @@ struct DevBuf {
         if (b == 0) b = 256;
         b = (b + 255) & ~(size_t)255;
         const size_t cap = g_budget.load();
+        g_no_room = true;
         if (cap && g_used.load() + b > cap)
             return fail(SI_ERR_OOM, "device budget exceeded: %zu in use + %zu requested > %zu", g_used.load(),
                         b, cap);
@@ -86,6 +89,7 @@ struct DevBuf {
             p = nullptr;
             return fail(SI_ERR_OOM, "cudaMalloc(%zu) failed: %s", b, cudaGetErrorString(e));
         }
+        g_no_room = false;
         bytes = b;
         g_used += b;
         ++g_alloc_gen;
@@ -106,6 +110,7 @@ int dev_reserve(void** p, size_t* bytes, size_t need) {
     if (need == 0) need = 256;
     need = (need + 255) & ~(size_t)255;
     const size_t cap = g_budget.load();
+    g_no_room = true;
     if (cap && g_used.load() + need > cap)
         return fail(SI_ERR_OOM, "device budget exceeded: %zu in use + %zu requested > %zu", g_used.load(), need, cap);
     cudaError_t e = cudaMalloc(p, need);
@@ -114,6 +119,7 @@ int dev_reserve(void** p, size_t* bytes, size_t need) {
         *p = nullptr;
         return fail(SI_ERR_OOM, "cudaMalloc(%zu) failed: %s", need, cudaGetErrorString(e));
     }
+    g_no_room = false;
     *bytes = need;
     g_used += need;
     ++g_alloc_gen;
@@ -217,6 +223,27 @@ struct gSuperIntervals {
 namespace {
 
 size_t staged(const gSuperIntervals* si) { return si->hdata.size(); }
+
+// Gives up what calls can do without: the rank grids, the gaps and what only calls over ranks use.
+// Says whether that freed anything.  (A release waits for the device, so nothing queued still reads
+// them.)
+bool drop_optional(gSuperIntervals* si) {
+    const size_t before = g_used.load();
+    si->grid_starts = si->grid_ends = si->gaps_ready = false;
+    for (DevBuf* b : {&si->grid.buf, &si->gap_grid.buf, &si->gaps, &si->gap_seg, &si->w_upper, &si->w_small})
+        b->release();
+    sig::dev_release(&si->bws.tile_recs.p, &si->bws.tile_recs.bytes);
+    return g_used.load() != before;
+}
+
+// A call that finds no room on the device is made again without the optional tables, in the way that
+// needs none of them: they never take the room of something required.
+template <typename F>
+int with_room(gSuperIntervals* si, F call) {
+    g_no_room = false;
+    const int r = call();
+    return r == SI_ERR_OOM && g_no_room && drop_optional(si) ? call() : r;
+}
 
 // Brackets one pipeline phase with CUDA events when profiling is on.
 struct PhaseTimer {
@@ -402,8 +429,10 @@ int build_grids(GridSet& g, const S* a0, const S* a1, int64_t n, const std::vect
     return SI_OK;
 }
 
+// tight: one stage's temporaries at a time, each freed before the next, and the optional grids
+// only from what is left at the end.
 template <typename S>
-int build_impl(gSuperIntervals* si) {
+int build_impl(gSuperIntervals* si, bool tight) {
     SI_TRY(set_dev(si));
     cudaStream_t st = si->st;
     const int64_t n = (int64_t)staged(si);
@@ -446,25 +475,34 @@ int build_impl(gSuperIntervals* si) {
     // Every temporary of the build in one allocation, cut anew for each stage: the stages run one
     // after the other on the stream, so a stage may overwrite what the one before left.  (One
     // cudaMalloc / cudaFree instead of some twenty, and no wait between stages to free by: 200 k
-    // intervals built in 1.58 ms before.)
+    // intervals built in 1.58 ms before.)  A tight build takes the input and each stage by itself.
     const int K = sig::key_words<S>(G), Ke = sig::end_key_words<S>(G);
     const size_t tb = sig::radix_temp_bytes(n, K), tbe = sig::radix_temp_bytes(n, Ke);
     const size_t words = TempArena::room(sizeof(uint32_t) * n);
-    const size_t in_bytes = 2 * TempArena::room(sizeof(S) * n) + words + 2 * TempArena::room(256);
+    const size_t in_bytes = 2 * TempArena::room(sizeof(S) * n) + words;
     const size_t stages[4] = {
-        in_bytes + (2 * (size_t)K + 2) * words + TempArena::room(tb),
-        in_bytes + TempArena::room(sig::branch_temp_bytes(n_pad)),
-        in_bytes + words + TempArena::room(sizeof(int64_t) * (n + 1)) + TempArena::room(sig::scan_temp_bytes(n)) +
+        (2 * (size_t)K + 2) * words + TempArena::room(tb),
+        TempArena::room(sig::branch_temp_bytes(n_pad)),
+        words + TempArena::room(sizeof(int64_t) * (n + 1)) + TempArena::room(sig::scan_temp_bytes(n)) +
             TempArena::room(256),
-        in_bytes + (2 * (size_t)Ke + 2) * words + TempArena::room(tbe)};
-    TempArena arena;
-    SI_TRY(arena.buf.reserve(*std::max_element(stages, stages + 4)));
-    int* berr = arena.take<int>(256);  // bounded waits of the one-sweep sorts and scans
-    int* flag = arena.take<int>(256);
-    S* s_in = arena.take<S>(sizeof(S) * n);
-    S* e_in = arena.take<S>(sizeof(S) * n);
-    int32_t* d_in = arena.take<int32_t>(sizeof(int32_t) * n);
-    const size_t stage0 = arena.at;
+        (2 * (size_t)Ke + 2) * words + TempArena::room(tbe)};
+    TempArena input, own;
+    TempArena& arena = tight ? own : input;
+    SI_TRY(input.buf.reserve(in_bytes + (tight ? 0 : *std::max_element(stages, stages + 4))));
+    S* s_in = input.take<S>(sizeof(S) * n);
+    S* e_in = input.take<S>(sizeof(S) * n);
+    int32_t* d_in = input.take<int32_t>(sizeof(int32_t) * n);
+    const size_t stage0 = tight ? 0 : input.at;
+    auto begin_stage = [&](int k) -> int {
+        arena.at = stage0;
+        if (!tight) return SI_OK;
+        SI_CK(cudaStreamSynchronize(st));
+        own.buf.release();
+        return own.buf.reserve(stages[k]);
+    };
+    SI_TRY(si->w_err.reserve(512));
+    int* berr = si->w_err.as<int>();  // bounded waits of the one-sweep sorts and scans
+    int* flag = berr + 64;
     SI_CK(cudaMemsetAsync(berr, 0, sizeof(int), st));
     SI_CK(cudaMemcpyAsync(s_in, hs<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
     SI_CK(cudaMemcpyAsync(e_in, he<S>(si).data(), sizeof(S) * n, cudaMemcpyHostToDevice, st));
@@ -481,6 +519,7 @@ int build_impl(gSuperIntervals* si) {
         SI_CK(sig::launch_copy_pad<S>(s_in, e_in, d_in, n, n_pad, si->starts.as<S>(), si->ends.as<S>(),
                                       si->data.as<int32_t>(), st));
     } else {
+        SI_TRY(begin_stage(0));
         for (int k = 0; k < K; ++k) {
             kp[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
             ka[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
@@ -498,14 +537,15 @@ int build_impl(gSuperIntervals* si) {
     S* lp[sig::kMaxLevels];
     for (int h = 0; h < sig::kMaxLevels; ++h) lp[h] = si->lvl[h].as<S>();
     SI_CK(sig::launch_pyramid<S>(ends, si->lvl_sizes, si->H, lp, st));
-    arena.at = stage0;
+    SI_TRY(begin_stage(1));
+    if (tight) input.buf.release();  // decoded
     SI_CK(sig::launch_branch<S>(ends, n, n_pad, levels<S>(si), si->H, si->seg.as<int64_t>(), G,
                                 si->branch.as<int32_t>(), st, arena.take<char>(sig::branch_temp_bytes(n_pad)), berr));
     // long-interval list of the batched path: intervals at least kLongIntervalSplit long, in
     // position order, with their own max pyramid (a tile reaches them without visiting the
     // positions in between); and whether some interval has start > end
     {
-        arena.at = stage0;
+        SI_TRY(begin_stage(2));
         uint32_t* flags = arena.take<uint32_t>(sizeof(uint32_t) * n);
         int64_t* offs = arena.take<int64_t>(sizeof(int64_t) * (n + 1));
         void* tmp = arena.take<char>(sig::scan_temp_bytes(n));
@@ -551,7 +591,7 @@ int build_impl(gSuperIntervals* si) {
     // without intervals with start > end: each contig's ends in ascending order, from which the
     // batched path counts short queries (two ranks per query)
     if (si->inverted == 0) {
-        arena.at = stage0;
+        SI_TRY(begin_stage(3));
         for (int k = 0; k < Ke; ++k) {
             kp[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
             ka[k] = arena.take<uint32_t>(sizeof(uint32_t) * n);
@@ -567,6 +607,12 @@ int build_impl(gSuperIntervals* si) {
         SI_CK(sig::launch_end_decode<S>(in_alt ? ka : kp, n, n_pad, si->end_sorted.as<S>(), st));
         si->bws.end_sorted = si->end_sorted.p;
     }
+    if (tight) {
+        SI_CK(cudaStreamSynchronize(st));
+        own.buf.release();
+    }
+    SI_TRY(sig::batched_prepare<S>(si->bws, view<S>(si), levels<S>(si), si->H, si->lvl_sizes,
+                                   si->ub_mode, st));
     std::vector<uint32_t> grid_base;
     const bool two = si->inverted == 0;
     // no room for them is no error: the index then works without
@@ -575,8 +621,6 @@ int build_impl(gSuperIntervals* si) {
     if (gr != SI_OK && gr != SI_ERR_OOM) return gr;
     si->grid_starts = gr == SI_OK;
     si->grid_ends = gr == SI_OK && two;
-    SI_TRY(sig::batched_prepare<S>(si->bws, view<S>(si), levels<S>(si), si->H, si->lvl_sizes,
-                                   si->ub_mode, st));
     SI_CK(cudaStreamSynchronize(st));
     SI_CK(cudaGetLastError());
     {
@@ -586,6 +630,15 @@ int build_impl(gSuperIntervals* si) {
     }
     si->built = true;
     return SI_OK;
+}
+
+template <typename S>
+int build_index(gSuperIntervals* si) {
+    g_no_room = false;
+    const int r = build_impl<S>(si, false);
+    if (r != SI_ERR_OOM || !g_no_room) return r;
+    drop_optional(si);
+    return build_impl<S>(si, true);
 }
 
 int check_built(const gSuperIntervals* si) {
@@ -649,7 +702,7 @@ bool rank_search(const gSuperIntervals* si, int64_t nq) {
 
 // count into d_counts (device) for device-resident queries
 template <typename S>
-int run_count(gSuperIntervals* si, const sig::QueryBatch& q, uint32_t* d_counts, cudaStream_t st,
+int run_count_once(gSuperIntervals* si, const sig::QueryBatch& q, uint32_t* d_counts, cudaStream_t st,
               bool for_emit = false) {
     SI_TRY(si->w_err.reserve(2 * sizeof(int)));
     SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
@@ -677,6 +730,11 @@ int run_count(gSuperIntervals* si, const sig::QueryBatch& q, uint32_t* d_counts,
         SI_CK(sig::launch_count_plain<S>(view<S>(si), q, d_counts, si->w_err.as<int>(), st));
     }
     return SI_OK;
+}
+
+template <typename S, typename... A>
+int run_count(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return run_count_once<S>(si, a...); });
 }
 
 // q may be a slice starting at query q_offset of the batch counted last.
@@ -854,7 +912,7 @@ int search_device_counted(gSuperIntervals* si, const sig::QueryBatch& q, int ord
 
 // device-resident queries and outputs
 template <typename S>
-int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool values,
+int search_device_once(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool values,
                   int64_t* d_offsets, int32_t* d_out, size_t cap, size_t* total, cudaStream_t st) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
@@ -876,6 +934,11 @@ int search_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool
     SI_TRY(rank_prepare<S>(si, q, lanes, st));
     SI_TRY(rank_emit<S>(si, q, 0, d_offsets, 0, order, values, d_out, lanes, P, st));
     return read_dev_err(si, st);
+}
+
+template <typename S, typename... A>
+int search_device(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return search_device_once<S>(si, a...); });
 }
 
 template <typename S>
@@ -957,7 +1020,7 @@ int search_small(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* q
 
 // host queries -> host CSR; result grown when `grow` is set, else caller buffers
 template <typename S>
-int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int order,
+int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int order,
                 bool values, cCsrResult* grow, int64_t* h_off, int32_t* h_out, size_t cap, size_t* total) {
     SI_TRY(check_width<S>(si));
     SI_TRY(check_built(si));
@@ -1037,7 +1100,6 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
         h_out = grow->values;
         grow->size = (size_t)P;
     } else if ((size_t)P > cap) {
-        if (ranks) SI_CK(cudaStreamSynchronize(st));  // the offsets are the caller's
         return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
     }
     if (small.off && (P == 0 || err)) return dev_status(si, err);
@@ -1138,8 +1200,16 @@ int search_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc
     return read_dev_err(si);
 }
 
+template <typename S, typename... A>
+int search_host(gSuperIntervals* si, A... a) {
+    const int r = with_room(si, [&] { return search_host_once<S>(si, a...); });
+    // a failed call leaves no copy to the caller's buffers behind
+    if (r != SI_OK && si && si->st) cudaStreamSynchronize(si->st);
+    return r;
+}
+
 template <typename S>
-int count_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, uint32_t* counts) {
+int count_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, uint32_t* counts) {
     SI_TRY(check_width<S>(si));
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
@@ -1152,8 +1222,13 @@ int count_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc,
     return read_dev_err(si);
 }
 
+template <typename S, typename... A>
+int count_host(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return count_host_once<S>(si, a...); });
+}
+
 template <typename S>
-int any_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, uint8_t* out) {
+int any_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, uint8_t* out) {
     SI_TRY(check_width<S>(si));
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
@@ -1171,6 +1246,11 @@ int any_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, s
     SI_CK(sig::launch_any_plain<S>(view<S>(si), q, si->w_out.as<uint8_t>(), si->w_err.as<int>(), si->st));
     if (nq) SI_CK(cudaMemcpyAsync(out, si->w_out.p, nq, cudaMemcpyDeviceToHost, si->st));
     return read_dev_err(si);
+}
+
+template <typename S, typename... A>
+int any_host(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return any_host_once<S>(si, a...); });
 }
 
 template <typename S>
@@ -1322,7 +1402,7 @@ size_t numContigsGpu(const gSuperIntervals* si) {
 
 int indexSuperIntervalsGpu(gSuperIntervals* si) {
     if (!si) return fail(SI_ERR_INVALID, "null handle");
-    return si->bits == 64 ? build_impl<int64_t>(si) : build_impl<int32_t>(si);
+    return si->bits == 64 ? build_index<int64_t>(si) : build_index<int32_t>(si);
 }
 
 int getIndexArraysGpu(const gSuperIntervals* si, void* s, void* e, int32_t* d, int64_t* br) {
@@ -1344,11 +1424,13 @@ int setUpperBoundModeGpu(gSuperIntervals* si, int mode) {
     si->ub_mode = mode;
     if (si->built) {
         SI_TRY(set_dev(si));
-        int r = si->bits == 64
-                    ? sig::batched_prepare<int64_t>(si->bws, view<int64_t>(si), levels<int64_t>(si), si->H,
-                                                    si->lvl_sizes, mode, si->st)
-                    : sig::batched_prepare<int32_t>(si->bws, view<int32_t>(si), levels<int32_t>(si), si->H,
-                                                    si->lvl_sizes, mode, si->st);
+        const int r = with_room(si, [&] {
+            return si->bits == 64
+                       ? sig::batched_prepare<int64_t>(si->bws, view<int64_t>(si), levels<int64_t>(si), si->H,
+                                                       si->lvl_sizes, mode, si->st)
+                       : sig::batched_prepare<int32_t>(si->bws, view<int32_t>(si), levels<int32_t>(si), si->H,
+                                                       si->lvl_sizes, mode, si->st);
+        });
         if (r != SI_OK) return r;
         SI_CK(cudaStreamSynchronize(si->st));
     }
@@ -1598,11 +1680,13 @@ extern "C" int upperBoundDeviceGpu(gSuperIntervals* si, const void* d_qe, const 
     }
     // the batched query path sorts the ends first (same answers): see setQueryPathGpu
     const bool sorted = use_batched(si, (int64_t)nq);
-    int r = si->bits == 64
-                ? sig::upper_bounds<int64_t>(si->bws, view<int64_t>(si), q, mode, d_out, si->w_err.as<int>(), st,
-                                             sorted)
-                : sig::upper_bounds<int32_t>(si->bws, view<int32_t>(si), q, mode, d_out, si->w_err.as<int>(), st,
-                                             sorted);
+    const int r = with_room(si, [&] {
+        return si->bits == 64
+                   ? sig::upper_bounds<int64_t>(si->bws, view<int64_t>(si), q, mode, d_out, si->w_err.as<int>(), st,
+                                                sorted)
+                   : sig::upper_bounds<int32_t>(si->bws, view<int32_t>(si), q, mode, d_out, si->w_err.as<int>(), st,
+                                                sorted);
+    });
     if (r != SI_OK) return fail(r, "upper-bound kernel failed");
     return SI_OK;
 }
@@ -1836,7 +1920,7 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
             return r;
         }
         P = t;
-        int rr = out.reserve(sizeof(int32_t) * std::max<size_t>(P, 1));
+        int rr = with_room(si, [&] { return out.reserve(sizeof(int32_t) * std::max<size_t>(P, 1)); });
         if (rr != SI_OK) {
             si->path = saved_path;
             return rr;
@@ -2037,9 +2121,11 @@ extern "C" int searchDeviceGraphGpu(gSuperIntervals* si, const void* d_qs, const
         return SI_OK;
     }
     // workspace first: nothing may be allocated while a capture is open
-    SI_TRY(si->w_err.reserve(2 * sizeof(int)));
-    SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * nq));
-    SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
+    SI_TRY(with_room(si, [&]() -> int {
+        SI_TRY(si->w_err.reserve(2 * sizeof(int)));
+        SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * nq));
+        return si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq));
+    }));
     // batched when the handle would take it for this batch and the key packs on the device
     const bool batched = use_batched(si, (int64_t)nq, true) && si->bits == 32 && sig::query_code_bits(si->G) <= 8 &&
                          nq < (size_t)INT32_MAX;
@@ -2051,7 +2137,8 @@ extern "C" int searchDeviceGraphGpu(gSuperIntervals* si, const void* d_qs, const
     if (!same) {
         sig::QueryBatch q{d_qs, d_qe, d_qc, (int64_t)nq};
         int r;
-        if (batched) r = capture_batched<int32_t>(si, q, order, d_offsets, d_values, capacity, st);
+        if (batched)
+            r = with_room(si, [&] { return capture_batched<int32_t>(si, q, order, d_offsets, d_values, capacity, st); });
         else if (si->bits == 64) r = capture_plain<int64_t>(si, q, order, d_offsets, d_values, capacity, st);
         else r = capture_plain<int32_t>(si, q, order, d_offsets, d_values, capacity, st);
         if (r != SI_OK) return r;
@@ -2236,7 +2323,7 @@ int gap_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int64_t* d_off, S
 // op 0: intersection (order = the hit order), op 1: difference.  Pieces go to caller device
 // buffers when they hold `cap` pieces; `total` always receives the piece count.
 template <typename S>
-int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int order, int64_t* d_off, S* d_os,
+int setop_device_once(gSuperIntervals* si, const sig::QueryBatch& q, int op, int order, int64_t* d_off, S* d_os,
                  S* d_oe, int32_t* d_ob, size_t cap, size_t* total, cudaStream_t st) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
@@ -2340,8 +2427,13 @@ int setop_device(gSuperIntervals* si, const sig::QueryBatch& q, int op, int orde
     return read_dev_err(si, st);
 }
 
+template <typename S, typename... A>
+int setop_device(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return setop_device_once<S>(si, a...); });
+}
+
 template <typename S>
-int setop_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int op, int order,
+int setop_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc, size_t nq, int op, int order,
                int64_t* h_off, S* h_os, S* h_oe, int32_t* h_ob, size_t cap, size_t* total) {
     SI_TRY(check_width<S>(si));
     SI_TRY(check_built(si));
@@ -2386,6 +2478,11 @@ int setop_host(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* qc,
     if (op == 0) SI_CK(cudaMemcpyAsync(h_ob, si->so_ob.p, sizeof(int32_t) * T, cudaMemcpyDeviceToHost, si->st));
     SI_CK(cudaStreamSynchronize(si->st));
     return SI_OK;
+}
+
+template <typename S, typename... A>
+int setop_host(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return setop_host_once<S>(si, a...); });
 }
 
 int check_order(int order) {
@@ -2470,7 +2567,7 @@ int lists_or_empty(gSuperIntervals* si, const sig::QueryBatch& q, int order, cud
 }
 
 template <typename S>
-int keys_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_t* d_off, S* d_s, S* d_e,
+int keys_device_once(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_t* d_off, S* d_s, S* d_e,
                 int32_t* d_d, size_t cap, size_t* total, cudaStream_t st) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
@@ -2512,6 +2609,11 @@ int keys_device(gSuperIntervals* si, const sig::QueryBatch& q, int order, int64_
     return SI_OK;
 }
 
+template <typename S, typename... A>
+int keys_device(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return keys_device_once<S>(si, a...); });
+}
+
 // Prefix sums of the starts and of the sorted ends, made on the first coverage call after a build.
 template <typename S>
 int cov_sums(gSuperIntervals* si, cudaStream_t st) {
@@ -2537,7 +2639,7 @@ int cov_sums(gSuperIntervals* si, cudaStream_t st) {
 }
 
 template <typename S>
-int coverage_device(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t* d_count, S* d_cov, cudaStream_t st) {
+int coverage_device_once(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t* d_count, S* d_cov, cudaStream_t st) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
     if (q.nq && (!q.qs || !q.qe || !d_count || !d_cov)) return fail(SI_ERR_INVALID, "null device buffer");
@@ -2584,6 +2686,11 @@ int coverage_device(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t* d_c
     return SI_OK;
 }
 
+template <typename S, typename... A>
+int coverage_device(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return coverage_device_once<S>(si, a...); });
+}
+
 }  // namespace
 
 extern "C" int searchKeysDeviceGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe, const int32_t* d_qc,
@@ -2599,9 +2706,9 @@ extern "C" int searchKeysDeviceGpu(gSuperIntervals* si, const void* d_qs, const 
                                 total, st);
 }
 
-extern "C" int searchKeysBatchGpu(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
-                                  int order, int64_t* offsets, void* starts, void* ends, int32_t* data,
-                                  size_t capacity, size_t* total) {
+static int keys_batch(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
+                      int order, int64_t* offsets, void* starts, void* ends, int32_t* data,
+                      size_t capacity, size_t* total) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
     if (!offsets) return fail(SI_ERR_INVALID, "null offsets");
@@ -2656,6 +2763,14 @@ extern "C" int searchKeysBatchGpu(gSuperIntervals* si, const void* qs, const voi
     return SI_OK;
 }
 
+extern "C" int searchKeysBatchGpu(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
+                                  int order, int64_t* offsets, void* starts, void* ends, int32_t* data,
+                                  size_t capacity, size_t* total) {
+    return with_room(si, [&] {
+        return keys_batch(si, qs, qe, qc, nq, order, offsets, starts, ends, data, capacity, total);
+    });
+}
+
 extern "C" int coverageDeviceGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe, const int32_t* d_qc,
                                  size_t nq, uint64_t* d_count, void* d_cov, void* stream) {
     SI_TRY(check_built(si));
@@ -2665,8 +2780,8 @@ extern "C" int coverageDeviceGpu(gSuperIntervals* si, const void* d_qs, const vo
     return coverage_device<int32_t>(si, q, d_count, (int32_t*)d_cov, st);
 }
 
-extern "C" int coverageBatchGpu(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
-                                uint64_t* count, void* cov) {
+static int coverage_batch(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
+                          uint64_t* count, void* cov) {
     SI_TRY(check_built(si));
     SI_TRY(set_dev(si));
     if (nq && (!count || !cov)) return fail(SI_ERR_INVALID, "null output");
@@ -2685,6 +2800,11 @@ extern "C" int coverageBatchGpu(gSuperIntervals* si, const void* qs, const void*
     SI_CK(cudaMemcpyAsync(cov, si->so_os.p, sb * nq, cudaMemcpyDeviceToHost, si->st));
     SI_CK(cudaStreamSynchronize(si->st));
     return SI_OK;
+}
+
+extern "C" int coverageBatchGpu(gSuperIntervals* si, const void* qs, const void* qe, const int32_t* qc, size_t nq,
+                                uint64_t* count, void* cov) {
+    return with_room(si, [&] { return coverage_batch(si, qs, qe, qc, nq, count, cov); });
 }
 
 // =====================================================================================
@@ -2763,10 +2883,10 @@ int deserialize_impl(gSuperIntervals* si, const ImageHeader& h, const unsigned c
     if (G > 1) si->hseg.assign(seg, seg + G + 1);
     si->contig_names = names;
     si->built = false;
-    SI_TRY(build_impl<S>(si));
+    SI_TRY(build_index<S>(si));
     if (n == 0) return SI_OK;
     DevBuf tmp, flag;
-    SI_TRY(tmp.reserve(4 * n));
+    SI_TRY(with_room(si, [&] { return tmp.reserve(4 * n); }));
     SI_TRY(flag.reserve(sizeof(int)));
     SI_CK(cudaMemcpyAsync(tmp.p, br, 4 * n, cudaMemcpyHostToDevice, si->st));
     SI_CK(sig::launch_differs_i32(tmp.as<int32_t>(), si->branch.as<int32_t>(), (int64_t)n, flag.as<int>(), si->st));
@@ -2976,7 +3096,7 @@ int bed_records(gSuperIntervals* si, const char* text, size_t len, int options, 
 }
 
 template <typename S>
-int bed_ingest(gSuperIntervals* si, const char* text, size_t len, int options, cBedStats* stats) {
+int bed_ingest_once(gSuperIntervals* si, const char* text, size_t len, int options, cBedStats* stats) {
     cudaStream_t st = si->st;
     BedRecords B;
     SI_TRY(bed_records(si, text, len, options, B, stats));
@@ -3100,8 +3220,13 @@ int bed_ingest(gSuperIntervals* si, const char* text, size_t len, int options, c
     return SI_OK;
 }
 
+template <typename S, typename... A>
+int bed_ingest(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return bed_ingest_once<S>(si, a...); });
+}
+
 template <typename S>
-int bed_queries(gSuperIntervals* si, const char* text, size_t len, int options, S* qs, S* qe, int32_t* qc,
+int bed_queries_once(gSuperIntervals* si, const char* text, size_t len, int options, S* qs, S* qe, int32_t* qc,
                 int64_t* line, size_t cap, size_t* n_out, cBedStats* stats) {
     cudaStream_t st = si->st;
     const int G = (int)si->contig_names.size();
@@ -3172,6 +3297,11 @@ int bed_queries(gSuperIntervals* si, const char* text, size_t len, int options, 
     if (line) SI_CK(cudaMemcpyAsync(line, dl.p, 8 * k, cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
     return SI_OK;
+}
+
+template <typename S, typename... A>
+int bed_queries(gSuperIntervals* si, A... a) {
+    return with_room(si, [&] { return bed_queries_once<S>(si, a...); });
 }
 
 }  // namespace
