@@ -2249,9 +2249,9 @@ int field_emit(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool ke
 }
 
 // The gaps of each contig (no interval has start > end), made on the first difference after a build.
+// Without room for them (SI_ERR_OOM) or positions (SI_ERR_TOO_LARGE) differences come from hit lists.
 template <typename S>
-int make_gaps(gSuperIntervals* si, cudaStream_t st) {
-    if (si->gaps_ready) return SI_OK;
+int find_gaps(gSuperIntervals* si, cudaStream_t st) {
     const int64_t slots = si->n + si->G;
     if (slots >= (int64_t)INT32_MAX) return SI_ERR_TOO_LARGE;
     TempArena tmp;
@@ -2283,6 +2283,14 @@ int make_gaps(gSuperIntervals* si, cudaStream_t st) {
     si->n_gaps = M;
     si->gaps_ready = true;
     return SI_OK;
+}
+template <typename S>
+int make_gaps(gSuperIntervals* si, cudaStream_t st) {
+    if (si->gaps_ready) return SI_OK;
+    const int r = find_gaps<S>(si, st);
+    if (r != SI_OK)
+        for (DevBuf* b : {&si->gaps, &si->gap_seg, &si->gap_grid.buf}) b->release();
+    return r;
 }
 
 template <typename S>
@@ -2334,7 +2342,9 @@ int setop_device_once(gSuperIntervals* si, const sig::QueryBatch& q, int op, int
         SI_CK(cudaStreamSynchronize(st));
         return SI_OK;
     }
-    if (op == 1 && use_ranks(si, q.nq) && make_gaps<S>(si, st) == SI_OK) {
+    const int gaps = op == 1 && use_ranks(si, q.nq) ? make_gaps<S>(si, st) : SI_ERR_OOM;
+    if (gaps != SI_OK && gaps != SI_ERR_OOM && gaps != SI_ERR_TOO_LARGE) return gaps;
+    if (gaps == SI_OK) {
         size_t T = 0;
         SI_TRY(gap_offsets<S>(si, q, d_off, d_os, d_oe, cap, &T, st));  // and the pieces, where they fit
         if (total) *total = T;
@@ -2614,14 +2624,19 @@ int keys_device(gSuperIntervals* si, A... a) {
     return with_room(si, [&] { return keys_device_once<S>(si, a...); });
 }
 
-// Prefix sums of the starts and of the sorted ends, made on the first coverage call after a build.
+// Prefix sums of the starts and of the sorted ends, made on the first coverage call after a build;
+// without room for them (SI_ERR_OOM) coverage comes from hit lists.
 template <typename S>
 int cov_sums(gSuperIntervals* si, cudaStream_t st) {
     if (si->cov_ready) return SI_OK;
-    SI_TRY(si->ps_start.reserve(sizeof(uint64_t) * (si->n + 1)));
-    SI_TRY(si->ps_end.reserve(sizeof(uint64_t) * (si->n + 1)));
     DevBuf tmp;
-    SI_TRY(tmp.reserve(sig::scan_temp_bytes(si->n)));
+    if (si->ps_start.reserve(sizeof(uint64_t) * (si->n + 1)) != SI_OK ||
+        si->ps_end.reserve(sizeof(uint64_t) * (si->n + 1)) != SI_OK ||
+        tmp.reserve(sig::scan_temp_bytes(si->n)) != SI_OK) {
+        si->ps_start.release();
+        si->ps_end.release();
+        return SI_ERR_OOM;
+    }
     if (sizeof(S) == 4) {
         SI_CK(sig::exclusive_scan_i32_to_u64((const int32_t*)si->starts.p, si->ps_start.as<uint64_t>(), si->n, tmp.p,
                                              st));
@@ -2644,7 +2659,9 @@ int coverage_device_once(gSuperIntervals* si, const sig::QueryBatch& q, uint64_t
     SI_TRY(set_dev(si));
     if (q.nq && (!q.qs || !q.qe || !d_count || !d_cov)) return fail(SI_ERR_INVALID, "null device buffer");
     if (q.nq == 0) return SI_OK;
-    if (si->n > 0 && si->inverted == 0 && si->bws.end_sorted && cov_sums<S>(si, st) == SI_OK) {
+    const int sums = si->n > 0 && si->inverted == 0 && si->bws.end_sorted ? cov_sums<S>(si, st) : SI_ERR_OOM;
+    if (sums != SI_OK && sums != SI_ERR_OOM) return sums;
+    if (sums == SI_OK) {
         // no interval has start > end: when no query has start > end either, the coverage comes
         // from ranks and prefix sums, without hit lists
         SI_TRY(si->w_err.reserve(2 * sizeof(int)));

@@ -109,3 +109,34 @@ def test_calls_in_the_room_of_the_required(api, budget, first, bits):
         assert all(np.array_equal(a, b) for a, b in zip(got, want[k])), k
         budget(0)
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("call", ["difference", "coverage", "keys", "intersect"])
+def test_calls_at_every_budget(api, budget, call, bits):
+    """Between no room at all and room for everything a call is refused for want of it or exact, and
+    what it could not finish holds nothing."""
+    n = 500_000
+    s, e, seg = _intervals(n, bits, 3, False)
+    qc = np.repeat(np.arange(3), np.diff(seg))[::50].astype(np.int32)
+    run = _calls(api, s[::50], e[::50], qc)[call]
+    want, served = None, 0
+    for room in [None] + [k << 20 for k in range(-8, 40, 3)]:
+        idx = api.GpuIndex(bits)
+        idx.add_arrays(s, e, seg=seg)
+        idx.build()
+        if room is not None:
+            budget(idx.lib.deviceBytesInUseGpu() + room)
+        try:
+            got = [np.array(a) for a in run(idx)]
+        except api.SIError as ex:
+            assert room is not None and ex.status == api._capi.SI_ERR_OOM
+            budget(0)
+            got = [np.array(a) for a in run(idx)]
+        else:
+            served += 1
+        budget(0)
+        want = want or got
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)), room
+        idx.close()
+    assert served > 2
