@@ -187,6 +187,7 @@ struct gSuperIntervals {
     DevBuf wq_s, wq_e, wq_c, w_counts, w_offsets, w_out, w_tmp;
     DevBuf w_err;    // device error word; the rank searches' whole work record (sig::RankWork)
     DevBuf w_upper;  // rank searches: each query's upper bound
+    uint32_t w_longest = 0;  // the most results of a query of the batch that field_offsets counted last
     // host-buffer searches of several chunks: a second result buffer and a copy stream, so
     // that the emit of one chunk overlaps the device-to-host copy of the previous one
     DevBuf w_out2;
@@ -757,35 +758,36 @@ int run_emit(gSuperIntervals* si, const sig::QueryBatch& q, int64_t q_offset, co
 
 // ---- searches over ranks (rank_search): counts and offsets in one kernel, then, knowing the result
 // size, either the direct emit or the sorted tiles.
-// The error word, then the hit count, of a work record.
+// The error word, the hit count and the longest query's of a work record.
 struct RankResult {
-    int err, inv;
-    unsigned long long total;
+    int err = 0, inv = 0;
+    unsigned long long total = 0;
+    unsigned int longest = 0, pad = 0;
 };
-static_assert(offsetof(sig::RankWork, err) == 0 && offsetof(sig::RankWork, total) == 8, "read back in one copy");
+static_assert(offsetof(sig::RankWork, err) == 0 && offsetof(sig::RankWork, total) == 8 &&
+                  offsetof(sig::RankWork, longest) == 16,
+              "read back in one copy");
 
 // Reads them after the work queued on `st`.  With `then`, work to be queued behind the copy (which the
 // host does not wait for), waits by an event.
 template <typename Then>
-int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err, Then then) {
-    RankResult here{}, *h = &here;
+int read_rank_work(gSuperIntervals* si, cudaStream_t st, RankResult* r, Then then) {
+    RankResult here, *h = &here;
     if (char* land = landing(si)) h = reinterpret_cast<RankResult*>(land);
     SI_CK(cudaMemcpyAsync(h, si->w_err.p, sizeof(*h), cudaMemcpyDeviceToHost, st));
     if (!si->ev_work) SI_CK(cudaEventCreateWithFlags(&si->ev_work, cudaEventDisableTiming));
     SI_CK(cudaEventRecord(si->ev_work, st));
     SI_TRY(then());
     SI_CK(cudaEventSynchronize(si->ev_work));
-    *P = (int64_t)h->total;
-    *err = h->err;
+    *r = *h;
     return SI_OK;
 }
-int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err) {
-    RankResult here{}, *h = &here;
+int read_rank_work(gSuperIntervals* si, cudaStream_t st, RankResult* r) {
+    RankResult here, *h = &here;
     if (char* land = landing(si)) h = reinterpret_cast<RankResult*>(land);
     SI_CK(cudaMemcpyAsync(h, si->w_err.p, sizeof(*h), cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
-    *P = (int64_t)h->total;
-    *err = h->err;
+    *r = *h;
     return SI_OK;
 }
 
@@ -805,8 +807,10 @@ int read_rank_work(gSuperIntervals* si, cudaStream_t st, int64_t* P, int* err) {
 int64_t far_below(const gSuperIntervals* si, int64_t nq) {
     return (int64_t)std::ceil(std::min(2.0 * si->long_depth * (double)nq, 4e18));
 }
-int direct_lanes(const gSuperIntervals* si, int64_t nq, int64_t P) {
-    return si->path != SI_PATH_AUTO ? 0 : sig::rank_lanes(si->n, far_below(si, nq), nq, P);
+int direct_lanes(const gSuperIntervals* si, int64_t nq, const RankResult& r) {
+    return si->path != SI_PATH_AUTO
+               ? 0
+               : sig::rank_lanes(si->n, far_below(si, nq), nq, (int64_t)r.total, (int64_t)r.longest);
 }
 
 // The lanes of the direct emit to queue behind the offsets (EmitGate), before the hit count is known, 0
@@ -845,20 +849,20 @@ int queue_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, in
 }
 
 // Whether the emit queued with `lanes` found its gate open.
-bool emitted(const gSuperIntervals* si, int64_t nq, int64_t room, int lanes, int64_t P, int err) {
-    return lanes && !err && P > 0 && P <= room && direct_lanes(si, nq, P) == lanes;
+bool emitted(const gSuperIntervals* si, int64_t nq, int64_t room, int lanes, const RankResult& r) {
+    return lanes && !r.err && r.total > 0 && (int64_t)r.total <= room && direct_lanes(si, nq, r) == lanes;
 }
 
 // Offsets and the gated emit; waits for the hit count and the error word.  *done: the results are
 // written.
 template <typename S>
 int rank_offsets(gSuperIntervals* si, const sig::QueryBatch& q, bool pieces, int64_t* d_off, const EmitTo<S>& to,
-                 cudaStream_t st, int64_t* P, int* err, bool* done) {
+                 cudaStream_t st, RankResult* r, bool* done) {
     int lanes = 0;
     SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
     SI_TRY(queue_offsets<S>(si, q, pieces, d_off, si->w_err.as<sig::RankWork>(), false, to, st, &lanes));
-    SI_TRY(read_rank_work(si, st, P, err));
-    *done = emitted(si, q.nq, to.room, lanes, *P, *err);
+    SI_TRY(read_rank_work(si, st, r));
+    *done = emitted(si, q.nq, to.room, lanes, *r);
     return SI_OK;
 }
 
@@ -918,19 +922,19 @@ int search_device_once(gSuperIntervals* si, const sig::QueryBatch& q, int order,
     SI_TRY(set_dev(si));
     if (!rank_search(si, q.nq))
         return search_device_counted<S>(si, q, order, values, d_offsets, d_out, cap, total, st);
-    int64_t P = 0;
-    int err = 0;
+    RankResult res;
     bool done = false;
     EmitTo<S> to;
     to.what = values ? sig::kOutValue : sig::kOutIdx;
     to.order = order;
     to.d.i32 = d_out;
     to.room = d_out ? (int64_t)std::min<size_t>(cap, INT64_MAX) : 0;
-    SI_TRY(rank_offsets<S>(si, q, false, d_offsets, to, st, &P, &err, &done));
+    SI_TRY(rank_offsets<S>(si, q, false, d_offsets, to, st, &res, &done));
+    const int64_t P = (int64_t)res.total;
     if (total) *total = (size_t)P;
     if ((size_t)P > cap) return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
-    if (err || P == 0 || done) return dev_status(si, err);
-    const int lanes = direct_lanes(si, q.nq, P);
+    if (res.err || P == 0 || done) return dev_status(si, res.err);
+    const int lanes = direct_lanes(si, q.nq, res);
     SI_TRY(rank_prepare<S>(si, q, lanes, st));
     SI_TRY(rank_emit<S>(si, q, 0, d_offsets, 0, order, values, d_out, lanes, P, st));
     return read_dev_err(si, st);
@@ -972,8 +976,7 @@ constexpr int64_t kSmallValues = 4096;
 struct SmallBatch {
     const int64_t* off = nullptr;     // host offsets; null: not such a batch, nothing was done
     const int32_t* values = nullptr;  // host values; null: not written (P or another emit)
-    int64_t P = 0;
-    int err = 0;
+    RankResult res;
     int64_t* d_off = nullptr;         // device offsets
     sig::QueryBatch q;                // device queries
 };
@@ -1010,11 +1013,9 @@ int search_small(gSuperIntervals* si, const S* qs, const S* qe, const int32_t* q
                             &lanes));
     SI_CK(cudaMemcpyAsync(land + at_work, dev + at_work, end - at_work, cudaMemcpyDeviceToHost, st));
     SI_CK(cudaStreamSynchronize(st));
-    const sig::RankWork* w = reinterpret_cast<const sig::RankWork*>(land + at_work);
-    b->P = (int64_t)w->total;
-    b->err = w->err;
+    b->res = *reinterpret_cast<const RankResult*>(land + at_work);
     b->off = reinterpret_cast<const int64_t*>(land + at_off);
-    if (emitted(si, (int64_t)nq, room, lanes, b->P, b->err)) b->values = reinterpret_cast<const int32_t*>(land + at_val);
+    if (emitted(si, (int64_t)nq, room, lanes, b->res)) b->values = reinterpret_cast<const int32_t*>(land + at_val);
     return SI_OK;
 }
 
@@ -1039,8 +1040,7 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
     }
     sig::QueryBatch q;
     const bool ranks = rank_search(si, (int64_t)nq);
-    int64_t P = 0;
-    int err = 0;
+    RankResult res;
     bool done = false;  // the results are in w_out
     int64_t* d_off = nullptr;
     SmallBatch small;
@@ -1048,8 +1048,7 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
     if (small.off) {
         q = small.q;
         d_off = small.d_off;
-        P = small.P;
-        err = small.err;
+        res = small.res;
         memcpy(h_off, small.off, sizeof(int64_t) * (nq + 1));
     } else {
         SI_TRY(upload_queries<S>(si, qs, qe, qc, nq, q));
@@ -1072,11 +1071,11 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
         SI_TRY(si->w_err.reserve(sig::rank_work_bytes(q.nq)));
         SI_TRY(queue_offsets<S>(si, q, false, d_off, si->w_err.as<sig::RankWork>(), false, to, st, &lanes));
         // the offsets follow behind the hit count, which the host waits for
-        SI_TRY(read_rank_work(si, st, &P, &err, [&]() -> int {
+        SI_TRY(read_rank_work(si, st, &res, [&]() -> int {
             SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
             return SI_OK;
         }));
-        done = emitted(si, q.nq, to.room, lanes, P, err);
+        done = emitted(si, q.nq, to.room, lanes, res);
     } else {
         SI_TRY(si->w_counts.reserve(sizeof(uint32_t) * std::max<size_t>(nq, 1)));
         SI_TRY(si->w_tmp.reserve(sig::scan_temp_bytes((int64_t)nq)));
@@ -1087,8 +1086,9 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
         }
         SI_CK(cudaMemcpyAsync(h_off, d_off, sizeof(int64_t) * (nq + 1), cudaMemcpyDeviceToHost, st));
         SI_CK(cudaStreamSynchronize(st));
-        P = h_off[nq];
+        res.total = (unsigned long long)h_off[nq];
     }
+    const int64_t P = (int64_t)res.total;
     if (total) *total = (size_t)P;
     if (grow) {
         if (grow->capacity < (size_t)P) {
@@ -1102,10 +1102,10 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
     } else if ((size_t)P > cap) {
         return fail(SI_ERR_CAPACITY, "output needs %lld values, capacity %zu", (long long)P, cap);
     }
-    if (small.off && (P == 0 || err)) return dev_status(si, err);
-    if (P == 0 || err) {
+    if (small.off && (P == 0 || res.err)) return dev_status(si, res.err);
+    if (P == 0 || res.err) {
         SI_TRY(read_dev_err(si));  // waits for the offsets too
-        return dev_status(si, err);
+        return dev_status(si, res.err);
     }
     if (small.values) {
         memcpy(h_out, small.values, sizeof(int32_t) * P);
@@ -1120,7 +1120,7 @@ int search_host_once(gSuperIntervals* si, const S* qs, const S* qe, const int32_
         SI_TRY(si->w_err.reserve(2 * sizeof(int)));
         SI_CK(cudaMemsetAsync(si->w_err.p, 0, sizeof(int), st));
     }
-    const int lanes = ranks ? direct_lanes(si, q.nq, P) : 0;
+    const int lanes = ranks ? direct_lanes(si, q.nq, res) : 0;
     if (ranks) SI_TRY(rank_prepare<S>(si, q, lanes, st));
     // Results are staged in device memory and copied in bulk: the emit writes every query's
     // list at a scattered place, and such writes over the host link run several times slower
@@ -2175,18 +2175,18 @@ template <typename S>
 int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStream_t st) {
     SI_TRY(si->so_hoff.reserve(sizeof(int64_t) * (q.nq + 1)));
     if (rank_search(si, q.nq)) {
-        int64_t P = 0;
-        int err = 0;
+        RankResult res;
         bool done = false;
         EmitTo<S> to;
         to.order = order;
         to.d.i32 = si->so_hits.as<int32_t>();
         to.room = (int64_t)(si->so_hits.bytes / sizeof(int32_t));
-        SI_TRY(rank_offsets<S>(si, q, false, si->so_hoff.as<int64_t>(), to, st, &P, &err, &done));
-        if (err || done) return dev_status(si, err);
+        SI_TRY(rank_offsets<S>(si, q, false, si->so_hoff.as<int64_t>(), to, st, &res, &done));
+        if (res.err || done) return dev_status(si, res.err);
+        const int64_t P = (int64_t)res.total;
         SI_TRY(si->so_hits.reserve(sizeof(int32_t) * std::max<int64_t>(P, 1)));
         if (P == 0) return SI_OK;
-        const int lanes = direct_lanes(si, q.nq, P);
+        const int lanes = direct_lanes(si, q.nq, res);
         SI_TRY(rank_prepare<S>(si, q, lanes, st));
         SI_TRY(rank_emit<S>(si, q, 0, si->so_hoff.as<int64_t>(), 0, order, false, si->so_hits.as<int32_t>(), lanes, P,
                             st));
@@ -2211,14 +2211,16 @@ int hit_lists(gSuperIntervals* si, const sig::QueryBatch& q, int order, cudaStre
 template <typename S>
 int field_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool keys, int64_t* d_off,
                   sig::RankDest<S> d, size_t cap, cudaStream_t st, int64_t* P, bool* done) {
-    int err = 0;
+    RankResult res;
     EmitTo<S> to;
     to.what = keys ? sig::kOutKeys : sig::kOutPieces;
     to.order = order;
     to.d = d;
     to.room = d.s && d.e && (keys || d.i32) ? (int64_t)std::min<size_t>(cap, INT64_MAX) : 0;
-    SI_TRY(rank_offsets<S>(si, q, !keys, d_off, to, st, P, &err, done));
-    return dev_status(si, err);
+    SI_TRY(rank_offsets<S>(si, q, !keys, d_off, to, st, &res, done));
+    *P = (int64_t)res.total;
+    si->w_longest = res.longest;
+    return dev_status(si, res.err);
 }
 
 // The P pieces or keys of the batch counted last by field_offsets.  Dense keys go through hit lists:
@@ -2226,7 +2228,10 @@ int field_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool
 template <typename S>
 int field_emit(gSuperIntervals* si, const sig::QueryBatch& q, int order, bool keys, const int64_t* d_off,
                sig::RankDest<S> d, int64_t P, cudaStream_t st) {
-    const int lanes = direct_lanes(si, q.nq, P);
+    RankResult res;
+    res.total = (unsigned long long)P;
+    res.longest = si->w_longest;
+    const int lanes = direct_lanes(si, q.nq, res);
     const uint32_t* su = si->w_upper.as<uint32_t>();
     int* err = si->w_err.as<int>();
     if (lanes) {
@@ -2320,11 +2325,10 @@ int gap_offsets(gSuperIntervals* si, const sig::QueryBatch& q, int64_t* d_off, S
     if (os && oe && cap)
         SI_TRY(gap_emit<S>(si, q, d_off, os, oe, st,
                            {si->w_err.as<sig::RankWork>(), (int64_t)std::min<size_t>(cap, INT64_MAX), 0, 0}));
-    int64_t T = 0;
-    int err = 0;
-    SI_TRY(read_rank_work(si, st, &T, &err));
-    SI_TRY(dev_status(si, err));
-    *total = (size_t)T;
+    RankResult res;
+    SI_TRY(read_rank_work(si, st, &res));
+    SI_TRY(dev_status(si, res.err));
+    *total = (size_t)res.total;
     return SI_OK;
 }
 

@@ -338,7 +338,7 @@ __device__ __forceinline__ unsigned long long ld_tile(const unsigned long long* 
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned int ld_walked(const unsigned int* p) {
+__device__ __forceinline__ unsigned int ld_word(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
                                                         RankWork* __restrict__ work) {
     constexpr int kWarps = kThreads / kWarp;
     __shared__ int64_t s_warp[kWarps];
+    __shared__ unsigned int s_most[kWarps];
     __shared__ int64_t s_prefix;
     __shared__ unsigned int s_t;
     unsigned long long* status = reinterpret_cast<unsigned long long*>(work + 1);
@@ -370,6 +371,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
     const int64_t base = t * (kThreads * R) + (int64_t)w * (R * kWarp) + lane;
     int64_t v[R];
     int64_t carry = 0;
+    unsigned int most = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int64_t q = base + r * kWarp;
@@ -379,6 +381,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         rank_probe(gs, ge, Q);
         const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, lane, upper, &work->walked);
         if (q < nq) su[q] = upper;
+        most = max(most, (unsigned int)x);
         int64_t inc = x;
 #pragma unroll
         for (int d = 1; d < kWarp; d <<= 1) {
@@ -388,12 +391,20 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         v[r] = carry + inc - x;
         carry += __shfl_sync(kFull, inc, 31);
     }
-    if (lane == 0) s_warp[w] = carry;
+    most = __reduce_max_sync(kFull, most);
+    if (lane == 0) {
+        s_warp[w] = carry;
+        s_most[w] = most;
+    }
     __syncthreads();
     if (w == 0) {
         int64_t total = 0;
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) total += s_warp[k];
+        for (int k = 0; k < kWarps; ++k) {
+            total += s_warp[k];
+            most = max(most, s_most[k]);
+        }
+        if (lane == 0 && most > ld_word(&work->longest)) atomicMax(&work->longest, most);
         if (lane == 0) st_tile(status + t, (t == 0 ? kTilePre : kTileAgg) | (unsigned long long)total);
         int64_t excl = 0;
         if (t > 0) {
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
                 const unsigned long long f = s & ~kTileVal;
                 if (__any_sync(kFull, f == 0ull)) {
                     if (++spins > kSpinLimit) {
-                        const unsigned int now = __shfl_sync(kFull, ld_walked(&work->walked), 0);
+                        const unsigned int now = __shfl_sync(kFull, ld_word(&work->walked), 0);
                         if (now == walked) {
                             if (lane == 0) atomicCAS(&work->err, kDevOk, kDevTimeout);
                             break;
@@ -465,7 +476,9 @@ __global__ void __launch_bounds__(kThreads) k_rank_emit(MapView<S> m, const S* _
                                                         RankDest<S> dst, int* d_err, EmitGate gate) {
     if (gate.work) {
         const int64_t P = (int64_t)gate.work->total;
-        if (gate.work->err || P > gate.room || rank_lanes(gate.n, gate.far_below, nq, P) != W) return;
+        if (gate.work->err || P > gate.room ||
+            rank_lanes(gate.n, gate.far_below, nq, P, gate.work->longest) != W)
+            return;
     }
     const int lane = threadIdx.x & 31, sub = lane & (W - 1);
     const unsigned gmask = W == 32 ? kFull : ((1u << (W & 31)) - 1u) << (lane & ~(W - 1));

@@ -231,22 +231,30 @@ struct RankWork {
     int err;                   // device error word
     int inv;                   // free for the caller
     unsigned long long total;  // hits of the batch
+    unsigned int longest;      // hits of its query with the most
     unsigned int tiles;        // tile counter
     unsigned int walked;       // progress of the walks of queries with start > end
-    unsigned int pad[10];
+    unsigned int pad[9];
 };
 size_t rank_work_bytes(int64_t nq);
 template <typename S>
 cudaError_t launch_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge, QueryBatch q, bool pieces, uint32_t* su,
                              int64_t* off, RankWork* work, cudaStream_t st, bool cleared = false);
-// The direct emit's lanes per query for a batch of nq queries and P hits over n intervals, 0 for the
-// sorted tiles; below far_below hits most of them are long intervals lying far apart (see direct_lanes).
-__host__ __device__ inline int rank_lanes(int64_t n, int64_t far_below, int64_t nq, int64_t P) {
+// The direct emit's lanes per query for a batch of nq queries and P hits, `longest` of them of one query,
+// over n intervals, 0 for the sorted tiles; below far_below hits most of them are long intervals lying
+// far apart (see direct_lanes).  A query's walk is a chain of dependent reads: some 400 ns a chunk of
+// `lanes` positions, 600 ns a far hit, however many other queries there are.  The tiles, which write
+// such a query's hits by stretches, take 77 us, 190 ps a query, 20 ps an interval and 11 ps a hit in all; the
+// direct emit is left to batches whose longest walk ends sooner (1 M queries over 5 M intervals with
+// 3 hits each: 0.2 ms, and 54 ms when one of them had 400 k).
+__host__ __device__ inline int rank_lanes(int64_t n, int64_t far_below, int64_t nq, int64_t P, int64_t longest) {
     const bool far = P < far_below;
     if (far ? P > 4000000 + 10 * nq + n || P > 160 * nq : P > 7000000 + 17 * nq + 9 * n / 5) return 0;
-    if (nq <= (far ? 4096 : P > 30 * nq ? 524288 : 32768)) return 32;
-    if (nq <= 262144) return 8;
-    return !far && P > 16 * nq ? 8 : 2;
+    const int lanes = nq <= (far ? 4096 : P > 30 * nq ? 524288 : 32768) ? 32
+                      : nq <= 262144 || (!far && P > 16 * nq)           ? 8
+                                                                        : 2;
+    const int64_t walk_ps = far ? 600000 * longest : 400000 / lanes * longest;
+    return walk_ps > 77000000 + 190 * nq + 20 * n + 11 * P ? 0 : lanes;
 }
 // An emit queued behind launch_rank_scan before the host knows the hit count: every block reads the
 // count and leaves when the batch failed, when the output has no room or when rank_lanes names

@@ -230,3 +230,48 @@ def test_large_tunables_with_64_bit_coordinates(api, oracle, tile_q, cap):
     assert np.array_equal(ps, np.maximum(qs[owner], sorted_s[want]))
     assert np.array_equal(pe, np.minimum(qe[owner], sorted_e[want]))
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("nq,longest", [(1, None), (1, 1 << 20), (900, None), (900, 1 << 20), (30_001, None),
+                                        (200_000, None), (300_001, None), (300_001, 1 << 20)])
+def test_one_query_with_most_of_the_hits(api, bits, nq, longest):
+    """A batch of short queries and one long one, on both sides of the line from which its walk would
+    outlast the tiles, and far above it, where a walk by 2 to 32 lanes takes 20 to 130 ms."""
+    import time
+
+    dt = np.int32 if bits == 32 else np.int64
+    n = (1 << 20) + 5
+    s = (np.arange(n) * 10).astype(dt)
+    e = s + 9
+    data = np.random.default_rng(nq).integers(-9, 9, n).astype(np.int32)
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s, e, data)
+    idx.build()
+    first = np.random.default_rng(nq + 1).integers(0, n - 2, nq)
+    hits = np.full(nq, 2)
+    lanes = 32 if nq <= 32768 else 8 if nq <= 262144 else 2
+    line = lanes * (77_000_000 + 190 * nq + 20 * n + 22 * nq) // 400_000
+    for most in ([longest] if longest else [min(line - 50, n), min(line + 500, n)]):
+        first[nq // 2], hits[nq // 2] = (n - most) // 2, most
+        qs, qe = (first * 10).astype(dt), ((first + hits) * 10 - 1).astype(dt)
+        want_off = np.concatenate([[0], np.cumsum(hits)])
+        last = np.repeat(first + hits - 1, hits)
+        want = (last - (np.arange(want_off[-1]) - np.repeat(want_off[:-1], hits))).astype(np.int32)
+        for values, expect in ((False, want), (True, data[want])):
+            off, out = idx.search(qs, qe, order=api.ORDER_DESC, values=values)
+            assert np.array_equal(off, want_off) and np.array_equal(out, expect)
+        off, ks, ke, kd = idx.search_keys(qs, qe, order=api.ORDER_DESC, with_data=True)
+        assert np.array_equal(off, want_off) and np.array_equal(kd, data[want])
+        assert np.array_equal(ks, s[want]) and np.array_equal(ke, e[want])
+        off, ps, pe, ph = idx.intersect(qs, qe, order=api.ORDER_DESC)
+        assert np.array_equal(off, want_off) and np.array_equal(ph, want)
+        assert np.array_equal(ps, s[want]) and np.array_equal(pe, e[want])
+    if longest:
+        best = 1.0
+        for _ in range(3):
+            t = time.perf_counter()
+            idx.search(qs, qe, order=api.ORDER_DESC)
+            best = min(best, time.perf_counter() - t)
+        assert best < 0.015
+    idx.close()
