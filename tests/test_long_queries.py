@@ -1,4 +1,5 @@
-"""Queries longer than a tile's (emit_alone): run lengths on both sides of what a round writes."""
+"""Queries longer than a tile's (emit_alone): run lengths on both sides of what a round writes, and windows
+of the long-interval list that one contig-long interval makes as long as the list."""
 import ctypes as C
 import time
 
@@ -12,6 +13,12 @@ pytestmark = pytest.mark.gpu
 def api():
     from superintervals_gb300 import interval_map
     return interval_map
+
+
+@pytest.fixture(scope="module")
+def oracle():
+    from oracle.oracle import Oracle
+    return Oracle()
 
 
 @pytest.mark.parametrize("bits", [32, 64])
@@ -82,3 +89,60 @@ def test_payloads_of_a_long_run_cost_little_more_than_positions(api):
     assert d.ms(1) < 7 * d.ms(0)
     d.close()
     idx.close()
+
+
+def _reads(n, nq, span, far, rng, whole):
+    """A tenth of the intervals and of the queries 10-50 kb, the others 150; `whole`: one interval over
+    everything."""
+    def lengths(k):
+        return np.where(rng.random(k) < far, rng.integers(10_000, 50_000, k), 150)
+    s, qs = rng.integers(0, span, n), rng.integers(0, span, nq)
+    e, qe = s + lengths(n), qs + lengths(nq)
+    if whole:
+        s[0], e[0] = 0, span
+    return s, e, qs, qe
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("span", [3_000_000, 60_000_000, 1_500_000_000])
+def test_one_interval_over_everything(api, oracle, span, bits):
+    dt = np.int32 if bits == 32 else np.int64
+    rng = np.random.default_rng(span)
+    s, e, qs, qe = (a.astype(dt) for a in _reads(30_000, 6_000, span, 0.3, rng, True))
+    data = rng.integers(-5, 1 << 30, len(s)).astype(np.int32)
+    m = oracle.build(s, e, data, seg=np.array([0, len(s)]))
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s, e, data)
+    idx.build()
+    ss, se, sd, _ = idx.arrays()
+    for path in (api.PATH_AUTO, api.PATH_BATCHED):
+        idx.set_path(path)
+        for order in (0, 1):
+            want_off, want = oracle.search_batch(m, qs, qe, None, order=order, nthreads=8)
+            off, out = idx.search(qs, qe, order=order)
+            assert np.array_equal(off, want_off) and np.array_equal(out, want)
+            off, out = idx.search(qs, qe, order=order, values=True)
+            assert np.array_equal(off, want_off) and np.array_equal(out, sd[want])
+            owner = np.repeat(np.arange(len(qs)), np.diff(want_off))
+            off, ps, pe, ph = idx.intersect(qs, qe, order=order)
+            assert np.array_equal(off, want_off) and np.array_equal(ph, want)
+            assert np.array_equal(ps, np.maximum(ss[want], qs[owner]))
+            assert np.array_equal(pe, np.minimum(se[want], qe[owner]))
+    idx.close()
+
+
+def test_one_interval_over_everything_costs_little(api):
+    """1 M reads against 1 M: with one contig-long interval every long query's window was the whole list of
+    long intervals before it, and the call took 6.8 times as long; 1.3 times now."""
+    ms = []
+    for whole in (False, True):
+        s, e, qs, qe = (a.astype(np.int32) for a in _reads(1_000_000, 1_000_000, 249_000_000, 0.1,
+                                                           np.random.default_rng(3), whole))
+        idx = api.GpuIndex(32)
+        idx.add_arrays(s, e)
+        idx.build()
+        d = _Device(api, idx, qs, qe, 40_000_000)
+        ms.append(d.ms(1))
+        d.close()
+        idx.close()
+    assert ms[1] < 2.5 * ms[0]
