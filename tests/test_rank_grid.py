@@ -179,3 +179,58 @@ def test_count_paths_agree(api):
         idx.set_path(path)
         assert np.array_equal(idx.count(qs, qe, qc), cnt)
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("nq", [1, 2, 31, 33, 257, 2431, 2433, 4865, 155_649])
+def test_few_queries_with_many_gaps(api, nq, bits):
+    """Stretches of pieces shared by 64 warps down to one each, empty queries among them."""
+    dt = np.int32 if bits == 32 else np.int64
+    n = 5000 if nq > 300 else 40_000
+    s = (np.arange(n) * 10).astype(dt)                        # a gap of 4 behind each interval
+    rng = np.random.default_rng(nq)
+    lo = np.sort(rng.integers(0, n - 1, (2, nq)), axis=0)
+    if nq > 3000:
+        lo[1] = np.minimum(lo[0] + rng.integers(0, 40, nq), n - 1)
+    qs, qe = (lo[0] * 10 + 7).astype(dt), (lo[1] * 10 + 8).astype(dt)
+    none = rng.random(nq) < 0.2
+    qs[none], qe[none] = lo[0][none] * 10, lo[0][none] * 10 + 5
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s, s + 5)
+    idx.build()
+    off, ps, pe = idx.difference(qs, qe)
+    cnt = np.where(none, 0, lo[1] - lo[0] + 1)
+    want_off = np.concatenate([[0], np.cumsum(cnt)])
+    assert np.array_equal(off, want_off)
+    gap = np.repeat(lo[0], cnt) + np.arange(want_off[-1]) - np.repeat(want_off[:-1], cnt)
+    assert np.array_equal(ps, np.maximum(gap * 10 + 6, np.repeat(qs, cnt)))
+    assert np.array_equal(pe, np.minimum(gap * 10 + 9, np.repeat(qe, cnt)))
+    idx.close()
+
+
+def test_few_long_differences_take_the_device(api):
+    """300 differences of 20 k pieces each: 4.2 ms by ten warps."""
+    import time
+
+    n, nq = 20_000, 300
+    s = np.arange(n, dtype=np.int32) * 10
+    idx = api.GpuIndex(32)
+    idx.add_arrays(s, s + 5)
+    idx.build()
+    lib, cap, best = idx.lib, n * nq + 1000, 1.0
+    bufs = [C.c_void_p() for _ in range(5)]
+    for b, size in zip(bufs, (4 * nq, 4 * nq, 8 * (nq + 1), 4 * cap, 4 * cap)):
+        api.check(lib.deviceMallocGpu(C.byref(b), size))
+    ends = np.full(nq, 10 * n, np.int32)
+    for b, a in zip(bufs, (np.zeros(nq, np.int32), ends)):
+        api.check(lib.memcpyGpu(b, C.c_void_p(a.ctypes.data), a.nbytes, idx.stream))
+    total = C.c_size_t(0)
+    for _ in range(6):
+        t = time.perf_counter()
+        api.check(lib.differenceDeviceGpu(idx.h, bufs[0], bufs[1], None, nq, bufs[2], bufs[3], bufs[4], cap,
+                                          C.byref(total), None))
+        best = min(best, time.perf_counter() - t)
+    assert total.value == n * nq and best < 0.0015
+    for b in bufs:
+        lib.deviceFreeGpu(b)
+    idx.close()
