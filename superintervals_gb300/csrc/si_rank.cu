@@ -203,6 +203,8 @@ __device__ __forceinline__ void rank_probe(const RankGrid<S>& gs, const RankGrid
     Q.x2 = __ldg(ge.rec + grid_slot(load_contig(ge.c + g), Q.s));
 }
 
+constexpr int kOwnSteps = 64;
+
 // The query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
 // walked by the whole warp, so every lane of the warp calls it (walked: see warp_walk_count).
 template <typename S>
@@ -228,13 +230,27 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
         upper = any && (s <= e || !pieces) ? top : 0u;
     }
     unsigned todo = __ballot_sync(kFull, walk);
+    if (__popc(todo) > 2) {
+        // several at once: each lane walks its own a little way, which ends most of them (a warp's 32 one
+        // after another: 1000 such queries over 1 M intervals 104 us, 26 so), the warp the rest
+        int64_t i = (int64_t)top - 1;
+        for (int k = 0; k < kOwnSteps && walk; ++k) {
+            const bool hit = s <= m.ends[i];
+            const int32_t br = m.branch[i];
+            cnt += hit ? 1u : 0u;
+            i = hit ? i - 1 : (int64_t)br;
+            walk = i >= (int64_t)lo;
+        }
+        top = (uint32_t)(i + 1);
+        todo = __ballot_sync(kFull, walk);
+    }
     while (todo) {
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;
         const uint32_t r = warp_walk_count<S>(m, (int64_t)__shfl_sync(kFull, lo, src),
                                               (int64_t)__shfl_sync(kFull, top, src) - 1, __shfl_sync(kFull, s, src),
                                               lane, walked);
-        if (lane == src) cnt = r;
+        if (lane == src) cnt += r;
     }
     return cnt;
 }

@@ -275,3 +275,80 @@ def test_one_query_with_most_of_the_hits(api, bits, nq, longest):
             best = min(best, time.perf_counter() - t)
         assert best < 0.015
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("nq", [1, 2, 3, 33, 1000, 40_000, 320_000])
+def test_batches_of_start_above_end(api, nq, bits):
+    """Queries with start > end: walks of none to thousands of hits in one warp, alone and many."""
+    dt = np.int32 if bits == 32 else np.int64
+    rng = np.random.default_rng(nq)
+    n = 20_000
+    s = rng.integers(0, 400_000, n)
+    ln = rng.integers(1, 60, n)
+    ln[rng.random(n) < 0.01] = 100_000
+    e = s + ln
+    e[:40] = 10_000_000
+    s[-3000:], e[-3000:] = np.arange(700_000, 703_000), 900_000   # behind 800,000 all of them hit
+    seg = np.array([0, 0, 9000, 9001, n], np.int64)
+    qc = rng.integers(0, 4, nq).astype(np.int32)
+    qe = rng.integers(0, 420_000, nq)
+    qs = qe + rng.integers(1, 2000, nq)
+    far = rng.random(nq) < (1.0 if nq < 4 else 0.02)
+    qe[far], qs[far], qc[far] = 800_000, 850_000, 3
+    if nq > 300:                                              # a warp without any, one with one
+        qs[64:96], qs[97:128] = qe[64:96], qe[97:128]
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s.astype(dt), e.astype(dt), seg=seg)
+    idx.build()
+    ss, se, _, branch = idx.arrays()
+    # the reference's walk: from the last start at or below the query's end, on a miss to the branch
+    sample = np.unique(np.concatenate([np.flatnonzero(far)[:3], np.arange(min(nq, 140))]))
+    got = idx.count(qs.astype(dt), qe.astype(dt), qc)
+    off, hits = idx.search(qs.astype(dt), qe.astype(dt), qc, order=api.ORDER_DESC)
+    assert np.array_equal(np.diff(off), got)
+    for q in sample:
+        a, b = seg[qc[q]], seg[qc[q] + 1]
+        i, want = int(np.searchsorted(ss[a:b], qe[q], side="right")) - 1, []
+        while i >= 0:
+            if se[a + i] >= qs[q]:
+                want.append(i)
+                i -= 1
+            else:
+                i = int(branch[a + i])
+        assert got[q] == len(want) and hits[off[q]:off[q + 1]].tolist() == want
+    idx.set_path(api.PATH_PLAIN)
+    assert np.array_equal(idx.count(qs.astype(dt), qe.astype(dt), qc), got)
+    idx.close()
+
+
+def test_a_warp_of_start_above_end_walks_at_once(api):
+    """1000 counts with start > end and some ten far hits each: 104 us a call when a warp walked its 32
+    queries one after another."""
+    import ctypes as C
+    import time
+
+    rng = np.random.default_rng(8)
+    n, nq, span = 1_000_000, 1000, 3_000_000_000
+    s = rng.integers(0, span, n)
+    e = s + np.where(rng.random(n) < 0.01, rng.integers(1_000_000, 5_000_000, n), 300)
+    idx = api.GpuIndex(64)
+    idx.add_arrays(s, e)
+    idx.build()
+    mid = rng.integers(0, span, nq)
+    lib, bufs = idx.lib, [C.c_void_p() for _ in range(3)]
+    for b, a in zip(bufs, (mid + 1, mid - 1, np.zeros(nq, np.uint32))):
+        api.check(lib.deviceMallocGpu(C.byref(b), a.nbytes))
+        api.check(lib.memcpyGpu(b, C.c_void_p(a.ctypes.data), a.nbytes, idx.stream))
+    best = 1.0
+    for _ in range(5):
+        api.check(lib.streamSynchronizeGpu(idx.stream))
+        t = time.perf_counter()
+        for _ in range(40):
+            api.check(lib.countOverlapsDeviceGpu(idx.h, bufs[0], bufs[1], None, nq, bufs[2], None))
+        api.check(lib.streamSynchronizeGpu(idx.stream))
+        best = min(best, (time.perf_counter() - t) / 40)
+    assert best < 60e-6
+    for b in bufs:
+        lib.deviceFreeGpu(b)
+    idx.close()
