@@ -98,7 +98,16 @@ __global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ ar
     if (threadIdx.x == kThreads - 1 || i >= records || j > c.nb) return;
     const uint32_t cnt = j < c.nb ? s_at[threadIdx.x + 1] - at : 0u;
     uint4 x = make_uint4(at, ~0u, ~0u, ~0u);
-    if (cnt > kGridSlots) {
+    if (cnt >= kGridDense) {
+        // as many sub-buckets as a quarter of the entries, or fewer, over the entries' own range
+        const uint64_t in_bucket = (1ull << c.shift) - 1ull;
+        const uint64_t first = ((uint64_t)(int64_t)arr[at] - (uint64_t)(int64_t)c.k0) & in_bucket;
+        const uint64_t last = ((uint64_t)(int64_t)arr[at + cnt - 1] - (uint64_t)(int64_t)c.k0) & in_bucket;
+        const uint32_t bits = 31 - __clz(cnt >> 2);
+        uint32_t ss = 0;
+        while (((last - first) >> ss) >> bits) ++ss;
+        x = make_uint4(at | kGridMany, kGridOwn | bits << 8 | ss, (uint32_t)first, (uint32_t)(first >> 32));
+    } else if (cnt > kGridSlots) {
         x = make_uint4(at | kGridMany, cnt, 0u, 0u);
     } else {
         uint32_t w[3] = {~0u, ~0u, ~0u};
@@ -113,41 +122,62 @@ __global__ void __launch_bounds__(kThreads) k_grid_fill(const S* __restrict__ ar
     rec[i] = x;
 }
 
-// Offsets and t2: one thread per position.  A position of a crowded bucket writes itself to the words of the
-// sub-buckets after its predecessor's up to its own (at most 1024), the bucket's last position also
-// the rest.  Coalesced reads and no search: 20 M clustered 64-bit keys took 7.6 ms with a warp per
-// bucket searching every word.
+// Offsets and t2: one thread per position.  A position of a bucket with its own table writes itself to
+// the words of the sub-buckets after its predecessor's up to its own, the bucket's last position also
+// the rest; stretches of more than kOwnWords words (a gap in a large bucket) are written by the block.
+// Coalesced reads and no search: 20 M clustered 64-bit keys took 7.6 ms with a warp per bucket
+// searching every word.
+constexpr uint32_t kOwnWords = 64;
 template <typename S>
 __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr, const int64_t* __restrict__ seg,
                                                        int G, int64_t n, const GridContig<S>* __restrict__ cs,
                                                        const uint4* __restrict__ rec, uint32_t* __restrict__ t2,
                                                        uint16_t* __restrict__ lo) {
+    __shared__ uint32_t s_from[2 * kThreads], s_len[2 * kThreads], s_val[2 * kThreads];
+    __shared__ unsigned int s_n;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    int g = 0;
-    for (int hi = G - 1; g < hi;) {  // largest g with seg[g] <= i
-        const int mid = (g + hi + 1) >> 1;
-        if (seg[mid] <= i) g = mid;
-        else hi = mid - 1;
+    auto fill = [&](uint32_t at, uint32_t len, uint32_t val) {
+        if (len <= kOwnWords) {
+            for (uint32_t j = 0; j < len; ++j) t2[at + j] = val;
+        } else {
+            const unsigned int k = atomicAdd(&s_n, 1u);  // a thread has two stretches at most
+            s_from[k] = at;
+            s_len[k] = len;
+            s_val[k] = val;
+        }
+    };
+    if (i < n) {
+        int g = 0;
+        for (int hi = G - 1; g < hi;) {  // largest g with seg[g] <= i
+            const int mid = (g + hi + 1) >> 1;
+            if (seg[mid] <= i) g = mid;
+            else hi = mid - 1;
+        }
+        const GridContig<S> c = cs[g];
+        const uint64_t d = (uint64_t)(int64_t)arr[i] - (uint64_t)(int64_t)c.k0;
+        lo[i] = (uint16_t)((uint32_t)d & ((1u << min(c.shift, 16u)) - 1u));
+        const uint32_t at = c.base + (uint32_t)(d >> c.shift);
+        const uint4 x = rec[at];
+        if (x.x >= kGridMany && x.y >= kGridOwn) {
+            const uint32_t a = x.x & ~kGridMany, e = rec[at + 1].x & ~kGridMany;  // the bucket [a, e)
+            const uint32_t ss = x.y & 63u, nsub = 1u << ((x.y >> 8) & 31u);
+            const uint64_t in_bucket = (1ull << c.shift) - 1ull, first = (uint64_t)x.w << 32 | x.z;
+            const uint32_t r = (uint32_t)(((d & in_bucket) - first) >> ss);
+            uint32_t from = 0;
+            if ((uint32_t)i > a) {
+                const uint64_t dp = (uint64_t)(int64_t)arr[i - 1] - (uint64_t)(int64_t)c.k0;
+                from = (uint32_t)(((dp & in_bucket) - first) >> ss) + 1u;
+            }
+            const uint32_t w = grid_sub_base(a);
+            if (from <= r) fill(w + from, r + 1u - from, (uint32_t)i);
+            if ((uint32_t)i == e - 1u) fill(w + r + 1u, nsub - r, e);
+        }
     }
-    const GridContig<S> c = cs[g];
-    const uint64_t d = (uint64_t)(int64_t)arr[i] - (uint64_t)(int64_t)c.k0;
-    lo[i] = (uint16_t)((uint32_t)d & ((1u << min(c.shift, 16u)) - 1u));
-    const uint4 x = rec[c.base + (uint32_t)(d >> c.shift)];
-    if (x.x < kGridMany || x.y < kGridDense) return;
-    const uint32_t a = x.x & ~kGridMany, cnt = x.y, e = a + cnt;
-    const int k = grid_sub_bits(cnt, c.shift), ss = (int)c.shift - k;
-    const uint32_t nsub = 1u << k, last = nsub - 1u;
-    const uint32_t r = (uint32_t)(d >> ss) & last;
-    uint32_t from = 0;
-    if ((uint32_t)i > a) {
-        const uint64_t dp = (uint64_t)(int64_t)arr[i - 1] - (uint64_t)(int64_t)c.k0;
-        from = ((uint32_t)(dp >> ss) & last) + 1u;
-    }
-    uint32_t* __restrict__ w = t2 + grid_sub_base(a);
-    for (uint32_t j = from; j <= r; ++j) w[j] = (uint32_t)i;
-    if ((uint32_t)i == e - 1u)
-        for (uint32_t j = r + 1u; j <= nsub; ++j) w[j] = e;
+    __syncthreads();
+    for (unsigned int k = 0; k < s_n; ++k)
+        for (uint32_t j = threadIdx.x; j < s_len[k]; j += kThreads) t2[s_from[k] + j] = s_val[k];
 }
 
 // The positions of one query with start > end that hit, by one warp: the reference's walk 32

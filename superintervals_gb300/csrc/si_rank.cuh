@@ -9,10 +9,12 @@
 // seven bits of their offsets from the bucket's first coordinate.  A rank is then one 16-byte read and
 // a packed compare of the key's own seven bits; only where an entry shares them with the key (1 in 20
 // ranks) are those entries compared in full.  Where coordinates crowd, the record of a bucket of more
-// entries holds their number; one of kGridDense or more is cut again, by its own count, in table t2;
-// its words sit at 3/8 of the bucket's first position, so that no second index is needed (a bucket of
-// n entries uses at most n/4 + 1 words).  Any bucket still crowded after that is searched by halving:
-// the answer is exact for every distribution, only the number of reads changes.
+// entries holds their number; one of kGridDense or more is cut again, by its own count and over its own
+// entries' range, in table t2 (by the bucket's range, one outlying coordinate in a 64-bit contig, which
+// leaves all others in one bucket, left them in one sub-bucket as well: 12 M counts 1851 us, 467 so).
+// Its words sit at 3/8 of the bucket's first position, so that no second index is needed (a bucket of
+// n entries uses at most n/4 + 1 words).  Any sub-bucket still crowded is searched by halving: the
+// answer is exact for every distribution, only the number of reads changes.
 // Full compares take 16-bit offsets inside buckets at most 65536 wide, eight to a 16-byte read, and
 // the coordinates elsewhere.  What bounds it is sectors from the L2 (some 9 TB/s of them): the tables
 // and offsets of an 8 M-interval index, starts and ends, are some 100 MB, but a rank reads one sector,
@@ -27,8 +29,8 @@ namespace sig {
 constexpr uint32_t kGridFill = 4;    // at most n / kGridFill buckets: 4-8 entries a bucket
 constexpr uint32_t kGridSlots = 12;  // entries whose codes a record holds
 constexpr uint32_t kGridMany = 0x80000000u;
+constexpr uint32_t kGridOwn = 0x80000000u;
 constexpr uint32_t kGridDense = 20;  // entries from which a bucket has its own table (>= 13: see above)
-constexpr int kGridSubBits = 10;     // at most 1024 words of t2 per bucket
 
 // A contig's buckets.  Its first position is in rec[base], its end in rec[base + nb].
 template <typename S>
@@ -51,7 +53,9 @@ struct RankGrid {
     const S* arr = nullptr;          // ascending inside each contig
     const GridContig<S>* c = nullptr;
     // per bucket (then one for the contig's end): x its first position, y to w a byte per entry, unused
-    // ones 0xff; of a bucket with more entries x has kGridMany set and y is their number
+    // ones 0xff; of a bucket with more entries x has kGridMany set and y is their number or, with its own
+    // table, kGridOwn | log2 of its sub-buckets << 8 | log2 of their width, z and w the offset of its first
+    // entry, where they begin
     const uint4* rec = nullptr;
     const uint32_t* t2 = nullptr;
     const uint16_t* lo = nullptr;    // offsets inside buckets of contigs with shift <= 16
@@ -68,11 +72,6 @@ __device__ __forceinline__ GridContig<S> load_contig(const GridContig<S>* __rest
     return u.c;
 }
 
-// log2 of the sub-buckets of a bucket holding cnt >= kGridDense entries
-__device__ __forceinline__ int grid_sub_bits(uint32_t cnt, uint32_t shift) {
-    const int k = 31 - __clz(cnt >> 2);
-    return min(min(k, (int)shift), kGridSubBits);
-}
 __device__ __forceinline__ uint32_t grid_sub_base(uint32_t first) { return (uint32_t)((3ull * first + 7) >> 3); }
 
 // Top seven bits of an offset in a bucket 2^shift wide (all of them up to 2^7).
@@ -118,16 +117,19 @@ __device__ __forceinline__ void grid_bracket(const RankGrid<S>& R, const GridCon
         a += n;
         return;
     }
-    len = x.y;
-    if (len >= kGridDense) {
-        const int k = grid_sub_bits(len, c.shift);
-        const int ss = (int)c.shift - k;
-        const uint32_t r = (uint32_t)(d >> ss) & ((1u << k) - 1u);
-        const uint32_t* t2 = R.t2 + grid_sub_base(a) + r;
-        a = __ldg(t2);
-        len = __ldg(t2 + 1) - a;
-        if (ss == 0) len = 0;  // one coordinate wide: every entry equals v, the first one is the answer
+    if (x.y < kGridOwn) {
+        len = x.y;
+        return;
     }
+    const uint64_t in_bucket = d & ((1ull << c.shift) - 1ull), first = (uint64_t)x.w << 32 | x.z;
+    if (in_bucket <= first) return;
+    const uint64_t r = (in_bucket - first) >> (x.y & 63u);
+    const uint32_t nsub = 1u << ((x.y >> 8) & 31u);
+    const uint32_t* t2 = R.t2 + grid_sub_base(a) + (r < nsub ? (uint32_t)r : nsub);
+    a = __ldg(t2);
+    // (behind the last sub-bucket the bucket's end is the answer, and where one is a coordinate wide every
+    // entry of v's equals v)
+    if (r < nsub && (x.y & 63u) != 0u) len = __ldg(t2 + 1) - a;
 }
 
 // Entries of v's bucket among the eight from `at` (a multiple of 8) on that lie in [a, a + len) and

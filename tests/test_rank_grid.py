@@ -234,3 +234,80 @@ def test_few_long_differences_take_the_device(api):
     for b in bufs:
         lib.deviceFreeGpu(b)
     idx.close()
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+@pytest.mark.parametrize("n", [25, 300, 5000, 300_000])
+@pytest.mark.parametrize("shape", ["outlier", "low", "two", "ladder", "steps", "equal"])
+def test_crowded_buckets(api, shape, n, dt):
+    """Buckets with their own tables over their entries' range: nearly all entries in one bucket, a cluster
+    at each end of a bucket, clusters of every width, long stretches of one table between two entries, and
+    buckets of equal entries."""
+    info = np.iinfo(dt)
+    rng = np.random.default_rng(n)
+    top = int(info.max) - 3000
+    s = rng.integers(0, 40 * n, n)
+    if shape == "outlier":
+        s[0] = top
+    elif shape == "low":
+        s[0] = info.min + 5
+    elif shape == "two":
+        s[: n // 2] += top // 2
+    elif shape == "ladder":                                   # a cluster around every power of two
+        s = (1 << rng.integers(0, int(info.bits) - 2, n)) + rng.integers(0, 50, n)
+    elif shape == "steps":                                    # pairs far apart inside a crowded bucket
+        s = np.sort(rng.integers(0, 30, n)) * (top // 64) + rng.choice([0, 1, 9_000_000], n)
+        s[0] = info.min // 2
+    else:
+        s = rng.choice([7, 8, 5000, top // 3], n)
+    e = s + rng.integers(0, 90, n)
+    s, e = s.astype(dt), e.astype(dt)
+    near = rng.choice(np.concatenate([s, e]), 20_000).astype(object)
+    qs = np.array([min(max(v + d, int(info.min)), int(info.max) - 200) for v, d in
+                   zip(near, rng.integers(-3, 4, len(near)).tolist())]).astype(dt)
+    qe = qs + rng.choice(np.array([0, 1, 100], dt), len(qs))
+    qs[:100] = info.min
+    qe[100:200] = info.max
+    cnt = np.searchsorted(np.sort(s), qe, side="right") - np.searchsorted(np.sort(e), qs, side="left")
+    idx = api.GpuIndex(np.dtype(dt).itemsize * 8)
+    idx.add_arrays(s, e)
+    idx.build()
+    assert np.array_equal(idx.count(qs, qe), cnt)
+    got = idx.coverage(qs, qe)
+    idx.set_path(api.PATH_BATCHED)
+    for a, b in zip(got, idx.coverage(qs, qe)):
+        assert np.array_equal(a, b)
+    idx.close()
+
+
+def test_one_outlying_coordinate_costs_little(api):
+    """5 M counts over 5 M intervals with 64-bit coordinates: 6.7 times as long with one interval far behind
+    the others, which then all lay in one bucket and one sub-bucket; 1.9 times now."""
+    import time
+
+    rng = np.random.default_rng(2)
+    n, ms = 5_000_000, []
+    for far in (False, True):
+        s = rng.integers(0, 249_000_000, n)
+        if far:
+            s[0] = 1 << 62
+        idx = api.GpuIndex(64)
+        idx.add_arrays(s, s + 800)
+        idx.build()
+        qs = rng.integers(0, 249_000_000, n)
+        lib, bufs = idx.lib, [C.c_void_p() for _ in range(3)]
+        for b, a in zip(bufs, (qs, qs + 800, np.zeros(n, np.uint32))):
+            api.check(lib.deviceMallocGpu(C.byref(b), a.nbytes))
+            api.check(lib.memcpyGpu(b, C.c_void_p(a.ctypes.data), a.nbytes, idx.stream))
+        best = 1e9
+        for _ in range(6):
+            api.check(lib.streamSynchronizeGpu(idx.stream))
+            t = time.perf_counter()
+            api.check(lib.countOverlapsDeviceGpu(idx.h, bufs[0], bufs[1], None, n, bufs[2], None))
+            api.check(lib.streamSynchronizeGpu(idx.stream))
+            best = min(best, 1e3 * (time.perf_counter() - t))
+        ms.append(best)
+        for b in bufs:
+            lib.deviceFreeGpu(b)
+        idx.close()
+    assert ms[1] < 3.5 * ms[0]
