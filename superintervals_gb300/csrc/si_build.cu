@@ -180,8 +180,33 @@ __global__ void k_differs_i32(const int32_t* __restrict__ a, const int32_t* __re
     if (__any_sync(kFull, d) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
 }
 
-// out[0] += total length of the intervals at least X long; out[1] += the contigs' extents (last
-// start - first start + 1 over the sorted starts).  Their ratio is the depth of long intervals.
+// Last start - first start of a contig's n sorted starts, without what a few outlying ones add: no eighth
+// of the entries counts for more than four times the median eighth.  (With one 64-bit start far behind
+// the others the mean density was nothing, the tiles' lists as short as they get, and a search of 12 M
+// genes wrote most queries one by one: 10.9 ms, 6.9 so.)
+template <typename S>
+__device__ unsigned long long typical_extent(const S* __restrict__ starts, int64_t n) {
+    constexpr int K = 8;
+    unsigned long long w[K], sum = 0;
+    S from = starts[0];
+    for (int k = 0; k < K; ++k) {
+        const S to = starts[(n - 1) / K * (k + 1) + (n - 1) % K * (k + 1) / K];
+        const unsigned long long x = (unsigned long long)(int64_t)to - (unsigned long long)(int64_t)from;
+        from = to;
+        sum += x;
+        int j = k;
+        for (; j > 0 && w[j - 1] > x; --j) w[j] = w[j - 1];
+        w[j] = x;
+    }
+    if (n < 4 * K) return sum;
+    const unsigned long long most = w[K / 2] < ~0ull / 4 ? 4 * w[K / 2] : ~0ull;
+    sum = 0;
+    for (int k = 0; k < K; ++k) sum += w[k] < most ? w[k] : most;
+    return sum;
+}
+
+// out[0] += total length of the intervals at least X long; out[1] += the contigs' extents
+// (typical_extent + 1).  Their ratio is the depth of long intervals.
 // Integer sums (a length is clamped to 2^40, which leaves room for 2^23 such intervals per
 // block before the 64-bit total could wrap; the ratio only steers a path choice).  out[2] = the
 // largest end - start of an interval with start <= end.
@@ -202,8 +227,7 @@ __global__ void __launch_bounds__(kThreads) k_long_depth(const S* __restrict__ s
     }
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G; g += stride)
         if (seg[g + 1] > seg[g]) {
-            const unsigned long long d =
-                (unsigned long long)(int64_t)starts[seg[g + 1] - 1] - (unsigned long long)(int64_t)starts[seg[g]];
+            const unsigned long long d = typical_extent(starts + seg[g], seg[g + 1] - seg[g]);
             b += d < kClamp ? d + 1ull : kClamp;
         }
     for (int k = 0; k < 2; ++k) {

@@ -206,7 +206,8 @@ cudaError_t launch_end_keys(const S* ends, int64_t n, const int64_t* seg, int G,
                             cudaStream_t st);
 template <typename S>
 cudaError_t launch_end_decode(const uint32_t* const* kw, int64_t n, int64_t n_pad, S* out, cudaStream_t st);
-// out[0] = total length of intervals at least X long, out[1] = total contig extent (sorted starts),
+// out[0] = total length of intervals at least X long, out[1] = total contig extent (sorted starts,
+// without what a few outlying ones add),
 // out[2] = the largest end - start
 template <typename S>
 cudaError_t launch_long_depth(const S* starts, const S* ends, int64_t n, const int64_t* seg, int G, int64_t X,

@@ -10,7 +10,7 @@ import subprocess
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SOURCE = os.path.join(ROOT, "superintervals_gb300", "csrc", "si_batched.cu")
+CSRC = os.path.join(ROOT, "superintervals_gb300", "csrc")
 
 SHIM = r"""
 #include <algorithm>
@@ -120,9 +120,9 @@ int main(int argc, char** argv) {
 """
 
 
-def device_function(name):
-    """The text of a __device__ function of si_batched.cu, its template line included."""
-    text = open(SOURCE).read()
+def device_function(name, source="si_batched.cu"):
+    """The text of a __device__ function, its template line included."""
+    text = open(os.path.join(CSRC, source)).read()
     m = re.search(r"^(template <[^\n]*>\n)?__device__ [^\n]*\b%s\(.*?^\}\n" % name, text, re.S | re.M)
     assert m, name
     return m.group(0)
