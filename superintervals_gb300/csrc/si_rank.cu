@@ -180,30 +180,55 @@ __global__ void __launch_bounds__(kThreads) k_grid_sub(const S* __restrict__ arr
         for (uint32_t j = threadIdx.x; j < s_len[k]; j += kThreads) t2[s_from[k] + j] = s_val[k];
 }
 
-// The positions of one query with start > end that hit, by one warp: the reference's walk 32
-// positions at a time (from a miss it goes on at the smallest branch of the chunk's misses).  A walk
-// is as long as its hits are many; it counts every kBeatChunks chunks in *walked (null: nobody waits
-// for the warp).
+// The positions of a warp's queries with start > end (walk) that hit, from top - 1 down to lo.  Several
+// at once: each lane walks its own a little way, which ends most of them (a warp's 32 one after another:
+// 1000 such queries over 1 M intervals 104 us, 26 so).  What is left the warp walks together, one query
+// after the other: the reference's walk 32 positions at a time (from a miss it goes on at the smallest
+// branch of the chunk's misses).  A walk is as long as its hits are many; it counts every kBeatChunks
+// chunks in *walked (null: nobody waits for the warp).  A function of its own: inlined, the rare walks
+// cost the scan kernel up to eight registers a thread.
+constexpr int kOwnSteps = 64;
 constexpr uint32_t kBeatChunks = 256;
 template <typename S>
-__device__ uint32_t warp_walk_count(const MapView<S>& m, int64_t lo, int64_t top, S s, int lane,
-                                    unsigned int* walked) {
-    uint32_t cnt = 0, chunks = 0;
-    int64_t i = top;
-    while (i >= lo) {
-        if (++chunks % kBeatChunks == 0 && walked && lane == 0) atomicAdd(walked, 1u);
-        const int64_t k = i - lane;
-        const bool valid = k >= lo;
-        S e = 0;
-        int32_t br = 0;
-        if (valid) {
-            e = m.ends[k];
-            br = m.branch[k];
+__device__ __noinline__ uint32_t warp_walks(const S* __restrict__ ends, const int32_t* __restrict__ branch, uint32_t lo,
+                                            uint32_t top, S s, bool walk, unsigned int* walked) {
+    const int lane = threadIdx.x & 31;
+    uint32_t cnt = 0;
+    unsigned todo = __ballot_sync(kFull, walk);
+    if (__popc(todo) > 2) {
+        int64_t i = (int64_t)top - 1;
+        for (int k = 0; k < kOwnSteps && walk; ++k) {
+            const bool hit = s <= ends[i];
+            const int32_t br = branch[i];
+            cnt += hit ? 1u : 0u;
+            i = hit ? i - 1 : (int64_t)br;
+            walk = i >= (int64_t)lo;
         }
-        const bool hit = valid && s <= e;
-        cnt += (uint32_t)__popc(__ballot_sync(kFull, hit));
-        const int b = __reduce_min_sync(kFull, valid && !hit ? br : INT32_MAX);
-        i = (int64_t)b < i - 32 ? (int64_t)b : i - 32;
+        top = (uint32_t)(i + 1);
+        todo = __ballot_sync(kFull, walk);
+    }
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int64_t last = __shfl_sync(kFull, lo, src);
+        const S key = __shfl_sync(kFull, s, src);
+        uint32_t r = 0, chunks = 0;
+        for (int64_t i = (int64_t)__shfl_sync(kFull, top, src) - 1; i >= last;) {
+            if (++chunks % kBeatChunks == 0 && walked && lane == 0) atomicAdd(walked, 1u);
+            const int64_t k = i - lane;
+            const bool valid = k >= last;
+            S e = 0;
+            int32_t br = 0;
+            if (valid) {
+                e = ends[k];
+                br = branch[k];
+            }
+            const bool hit = valid && key <= e;
+            r += (uint32_t)__popc(__ballot_sync(kFull, hit));
+            const int b = __reduce_min_sync(kFull, valid && !hit ? br : INT32_MAX);
+            i = (int64_t)b < i - 32 ? (int64_t)b : i - 32;
+        }
+        if (lane == src) cnt += r;
     }
     return cnt;
 }
@@ -233,13 +258,11 @@ __device__ __forceinline__ void rank_probe(const RankGrid<S>& gs, const RankGrid
     Q.x2 = __ldg(ge.rec + grid_slot(load_contig(ge.c + g), Q.s));
 }
 
-constexpr int kOwnSteps = 64;
-
 // The query's count (see k_rank_count) and upper bound; the warp's queries with start > end are
-// walked by the whole warp, so every lane of the warp calls it (walked: see warp_walk_count).
+// walked by the whole warp, so every lane of the warp calls it (walked: see warp_walks).
 template <typename S>
 __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid<S>& gs, const RankGrid<S>& ge,
-                                             const RankQuery<S>& Q, bool pieces, int lane, uint32_t& upper,
+                                             const RankQuery<S>& Q, bool pieces, uint32_t& upper,
                                              unsigned int* walked) {
     bool walk = false;
     uint32_t cnt = 0, lo = 0, top = 0;
@@ -259,29 +282,7 @@ __device__ __forceinline__ uint32_t rank_one(const MapView<S>& m, const RankGrid
         }
         upper = any && (s <= e || !pieces) ? top : 0u;
     }
-    unsigned todo = __ballot_sync(kFull, walk);
-    if (__popc(todo) > 2) {
-        // several at once: each lane walks its own a little way, which ends most of them (a warp's 32 one
-        // after another: 1000 such queries over 1 M intervals 104 us, 26 so), the warp the rest
-        int64_t i = (int64_t)top - 1;
-        for (int k = 0; k < kOwnSteps && walk; ++k) {
-            const bool hit = s <= m.ends[i];
-            const int32_t br = m.branch[i];
-            cnt += hit ? 1u : 0u;
-            i = hit ? i - 1 : (int64_t)br;
-            walk = i >= (int64_t)lo;
-        }
-        top = (uint32_t)(i + 1);
-        todo = __ballot_sync(kFull, walk);
-    }
-    while (todo) {
-        const int src = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const uint32_t r = warp_walk_count<S>(m, (int64_t)__shfl_sync(kFull, lo, src),
-                                              (int64_t)__shfl_sync(kFull, top, src) - 1, __shfl_sync(kFull, s, src),
-                                              lane, walked);
-        if (lane == src) cnt += r;
-    }
+    if (__any_sync(kFull, walk)) cnt += warp_walks<S>(m.ends, m.branch, lo, top, s, walk, walked);
     return cnt;
 }
 
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_count(MapView<S> m, RankGrid<
     RankQuery<S> Q;
     rank_load(m, qs, qe, qc, q, nq, d_err, Q);
     rank_probe(gs, ge, Q);
-    const uint32_t cnt = rank_one<S>(m, gs, ge, Q, false, threadIdx.x & 31, upper, nullptr);
+    const uint32_t cnt = rank_one<S>(m, gs, ge, Q, false, upper, nullptr);
     if (q < nq) counts[q] = cnt;
 }
 
@@ -397,9 +398,10 @@ __device__ __forceinline__ unsigned int ld_word(const unsigned int* p) {
 // each: seconds), so a window that stays unpublished for kSpinLimit polls is given up, with
 // kDevTimeout, only when no walk of the launch went on meanwhile; a walk ends at its contig's first
 // position, so the kernel always ends.  Against the count kernel and a scan it saves a launch, a
-// cleared buffer and the counts' way through memory.
+// cleared buffer and the counts' way through memory.  (The bounds on the registers, 32, 40 and 48, are what
+// the kernel takes without the call to the walks.)
 template <typename S, int R>
-__global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
+__global__ void __launch_bounds__(kThreads, R == 1 ? 8 : sizeof(S) == 4 ? 6 : 5) k_rank_scan(MapView<S> m, RankGrid<S> gs, RankGrid<S> ge,
                                                         const S* __restrict__ qs, const S* __restrict__ qe,
                                                         const int32_t* __restrict__ qc, int64_t nq, int pieces,
                                                         uint32_t* __restrict__ su, int64_t* __restrict__ off,
@@ -425,9 +427,9 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         RankQuery<S> Q;
         rank_load(m, qs, qe, qc, q, nq, &work->err, Q);
         rank_probe(gs, ge, Q);
-        const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, lane, upper, &work->walked);
+        const int64_t x = rank_one<S>(m, gs, ge, Q, pieces != 0, upper, &work->walked);
         if (q < nq) su[q] = upper;
-        most = max(most, (unsigned int)x);
+        most = max(most, __reduce_max_sync(kFull, (unsigned int)x));
         int64_t inc = x;
 #pragma unroll
         for (int d = 1; d < kWarp; d <<= 1) {
@@ -437,7 +439,6 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
         v[r] = carry + inc - x;
         carry += __shfl_sync(kFull, inc, 31);
     }
-    most = __reduce_max_sync(kFull, most);
     if (lane == 0) {
         s_warp[w] = carry;
         s_most[w] = most;
@@ -450,7 +451,6 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
             total += s_warp[k];
             most = max(most, s_most[k]);
         }
-        if (lane == 0 && most > ld_word(&work->longest)) atomicMax(&work->longest, most);
         if (lane == 0) st_tile(status + t, (t == 0 ? kTilePre : kTileAgg) | (unsigned long long)total);
         int64_t excl = 0;
         if (t > 0) {
@@ -492,6 +492,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_scan(MapView<S> m, RankGrid<S
                 off[nq] = excl + total;
                 work->total = (unsigned long long)(excl + total);
             }
+            atomicMax(&work->longest, most);  // nobody waits for it
         }
     }
     __syncthreads();
@@ -520,11 +521,15 @@ __global__ void __launch_bounds__(kThreads) k_rank_emit(MapView<S> m, const S* _
                                                         int64_t nq, const uint32_t* __restrict__ su,
                                                         const int64_t* __restrict__ off, int64_t out_base, int order,
                                                         RankDest<S> dst, int* d_err, EmitGate gate) {
-    if (gate.work) {
-        const int64_t P = (int64_t)gate.work->total;
-        if (gate.work->err || P > gate.room ||
-            rank_lanes(gate.n, gate.far_below, nq, P, gate.work->longest) != W)
-            return;
+    __shared__ int s_open;
+    if (gate.work) {  // by one thread, not by every warp
+        if (threadIdx.x == 0) {
+            const int64_t P = (int64_t)gate.work->total;
+            s_open = !gate.work->err && P <= gate.room &&
+                     rank_lanes(gate.n, gate.far_below, nq, P, gate.work->longest) == W;
+        }
+        __syncthreads();
+        if (!s_open) return;
     }
     const int lane = threadIdx.x & 31, sub = lane & (W - 1);
     const unsigned gmask = W == 32 ? kFull : ((1u << (W & 31)) - 1u) << (lane & ~(W - 1));
