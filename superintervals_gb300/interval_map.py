@@ -190,10 +190,13 @@ class GpuIndex:
         return qs, qe, qc
 
     @staticmethod
-    def _first_capacity(nq: int) -> int:
+    def _first_capacity(nq: int, arrays: int = 1) -> int:
         """Result slots offered to the first call: a sparse result then takes one call of the
-        library, a larger one a second call with the size that the first one reported."""
-        return 4 * nq + 1024
+        library, a larger one a second call with the size that the first one reported.  Arrays much
+        larger than their result, or held while the right ones are made, cost fresh pages in every
+        call, more than the first call saves: with four slots a query, differences of 1 M queries
+        2.4 ms, 0.39 with one, keys of 300 k queries 3.8 instead of 2.8 ms."""
+        return 4 * nq + 1024 if arrays == 1 or nq <= 1 << 17 else nq + 1024
 
     def count(self, qs, qe, qc=None) -> np.ndarray:
         qs, qe, qc = self._queries(qs, qe, qc)
@@ -225,6 +228,7 @@ class GpuIndex:
                                              C.byref(total))
             if st == _capi.SI_ERR_CAPACITY:
                 cap = int(total.value)
+                out = None
                 out = np.empty(max(cap, 1), np.int32)
                 continue
             check(st)
@@ -236,7 +240,7 @@ class GpuIndex:
         nq = qs.shape[0]
         off = np.empty(nq + 1, np.int64)
         total = C.c_size_t(0)
-        cap = self._first_capacity(nq)
+        cap = self._first_capacity(nq, 3)
         bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
         for _ in range(2):
             args = [self.h, _p(qs), _p(qe), _p(qc), nq, *extra, _p(off), _p(bufs[0]), _p(bufs[1])]
@@ -245,6 +249,7 @@ class GpuIndex:
             st = fn(*args, cap, C.byref(total))
             if st == _capi.SI_ERR_CAPACITY:
                 cap = int(total.value)
+                bufs = None
                 bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
                 continue
             check(st)
@@ -259,7 +264,7 @@ class GpuIndex:
         nq = qs.shape[0]
         off = np.empty(nq + 1, np.int64)
         total = C.c_size_t(0)
-        cap = self._first_capacity(nq)
+        cap = self._first_capacity(nq, 3)
         bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
         for _ in range(2):
             st = self.lib.searchKeysBatchGpu(self.h, _p(qs), _p(qe), _p(qc), nq, int(order), _p(off), _p(bufs[0]),
@@ -267,6 +272,7 @@ class GpuIndex:
                                              C.byref(total))
             if st == _capi.SI_ERR_CAPACITY:
                 cap = int(total.value)
+                bufs = None
                 bufs = (np.empty(cap, self.dtype), np.empty(cap, self.dtype), np.empty(cap, np.int32))
                 continue
             check(st)
