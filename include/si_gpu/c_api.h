@@ -180,7 +180,9 @@ int getBatchedOptionGpu(const gSuperIntervals* si, int option, int64_t* value);
  * and keeps the fastest upper-bound provider,
  * tile size, candidate capacity and length split (coordinate descent from the
  * current values).  flags & SI_TUNE_KEEP_UPPER_BOUND keeps the current upper-bound
- * provider.  The choice stays set on the handle and is also written to `report`
+ * provider.  The provider and SI_OPT_EMIT_COPY, which searches over ranks do not use,
+ * are timed where they act (the counted search: graph replays, an index with start > end
+ * intervals).  The choice stays set on the handle and is also written to `report`
  * as a JSON object (may be NULL).  Results never depend on it. */
 #define SI_TUNE_KEEP_UPPER_BOUND 1
 int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe,

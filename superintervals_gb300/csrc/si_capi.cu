@@ -15,6 +15,7 @@
 #include <iterator>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "si_gpu/c_api.h"
@@ -1870,6 +1871,8 @@ extern "C" long long getLaunchCountGpu(void) { return g_launches.load(); }
 // Autotuner for the batched path: times full searches (count -> scan -> emit) on a sample of
 // the caller's own device-resident queries and keeps the fastest upper-bound provider, tile
 // size, candidate capacity and length split, by coordinate descent from the current values.
+// A search over ranks uses neither the provider nor SI_OPT_EMIT_COPY: those are timed on the
+// counted search, where graph replays and indexes with start > end intervals use them.
 // The chosen values stay set on the handle; `report` receives them as one JSON object.
 // =====================================================================================
 extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe, const int32_t* d_qc,
@@ -1885,7 +1888,7 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
     SI_TRY(off.reserve(sizeof(int64_t) * (ns + 1)));
     sig::QueryBatch q{d_qs, d_qe, d_qc, (int64_t)ns};
     size_t P = 0;
-    auto run = [&](int& status) -> double {
+    auto run = [&](int& status, bool counted = false) -> double {
         cudaEvent_t a, b;
         cudaEventCreate(&a);
         cudaEventCreate(&b);
@@ -1893,10 +1896,14 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
         for (int rep = 0; rep < 2; ++rep) {
             size_t t = 0;
             cudaEventRecord(a, st);
-            status = si->bits == 64 ? search_device<int64_t>(si, q, SI_ORDER_IDXS_CPP, false, off.as<int64_t>(),
-                                                              out.as<int32_t>(), out.bytes / 4, &t, st)
-                                    : search_device<int32_t>(si, q, SI_ORDER_IDXS_CPP, false, off.as<int64_t>(),
-                                                              out.as<int32_t>(), out.bytes / 4, &t, st);
+            auto search = [&](auto* one) -> int {
+                using S = std::remove_pointer_t<decltype(one)>;
+                return counted ? search_device_counted<S>(si, q, SI_ORDER_IDXS_CPP, false, off.as<int64_t>(),
+                                                          out.as<int32_t>(), out.bytes / 4, &t, st)
+                               : search_device<S>(si, q, SI_ORDER_IDXS_CPP, false, off.as<int64_t>(),
+                                                  out.as<int32_t>(), out.bytes / 4, &t, st);
+            };
+            status = si->bits == 64 ? search((int64_t*)nullptr) : search((int32_t*)nullptr);
             cudaEventRecord(b, st);
             cudaEventSynchronize(b);
             float ms = 0;
@@ -1930,11 +1937,13 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
     int best_ub = si->ub_mode;
     int status = SI_OK;
     double best_ms = run(status);
+    const bool ranks = rank_search(si, (int64_t)ns);
+    double counted_ms = status == SI_OK && ranks ? run(status, true) : best_ms;
     if (status != SI_OK) {
         si->path = saved_path;
         return status;
     }
-    int trials = 1;
+    int trials = ranks ? 2 : 1;
     // set parameters and provider; the provider's structure is rebuilt when the provider or the
     // Eytzinger depth changes
     auto apply = [&](const sig::BatchedParams& p, int ub) -> bool {
@@ -1942,7 +1951,8 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
         si->bws.prm = p;
         return !rebuild || setUpperBoundModeGpu(si, ub) == SI_OK;
     };
-    auto try_params = [&](const sig::BatchedParams& p, int ub) {
+    auto try_params = [&](const sig::BatchedParams& p, int ub, bool counted = false) {
+        double& best_of = counted && ranks ? counted_ms : best_ms;
         const sig::BatchedParams keep = si->bws.prm;
         const int keep_ub = si->ub_mode;
         if (!apply(p, ub)) {
@@ -1950,12 +1960,12 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
             return;
         }
         int s = SI_OK;
-        const double ms = run(s);
+        const double ms = run(s, counted && ranks);
         ++trials;
         // a trial replaces the current choice only when 2% faster, so that timing noise does
         // not trade a good setting for one that measured better once
-        if (s == SI_OK && ms < 0.98 * best_ms) {
-            best_ms = ms;
+        if (s == SI_OK && ms < 0.98 * best_of) {
+            best_of = ms;
             best = p;
             best_ub = ub;
         } else {
@@ -1964,7 +1974,7 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
     };
     if (!(flags & SI_TUNE_KEEP_UPPER_BOUND))
         for (int ub : {SI_UB_BINARY, SI_UB_EYTZINGER, SI_UB_LEARNED})
-            if (ub != best_ub) try_params(best, ub);
+            if (ub != best_ub) try_params(best, ub, true);
     for (int t : {128, 256, 384, 512})
         if (t != best.tile_q || best.auto_tile) {
             sig::BatchedParams p = best;
@@ -1987,14 +1997,14 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
     {  // how the emit writes the long-interval list's section of part B
         sig::BatchedParams p = best;
         p.emit_copy = !best.emit_copy;
-        try_params(p, best_ub);
+        try_params(p, best_ub, true);
     }
     if (best_ub == SI_UB_EYTZINGER)  // depth of the Eytzinger tree (the shared-memory top levels)
         for (int dpt : {7, 10, 13})
             if (dpt != si->bws.ub.eytz_depth) {
                 sig::BatchedParams p = best;
                 p.eytz_depth = dpt;
-                try_params(p, best_ub);
+                try_params(p, best_ub, true);
             }
     if (!apply(best, best_ub)) return fail(SI_ERR_CUDA, "autotune: restoring the chosen provider failed");
     si->path = saved_path;
@@ -2002,9 +2012,10 @@ extern "C" int autotuneBatchedGpu(gSuperIntervals* si, const void* d_qs, const v
         snprintf(report, report_len,
                  "{\"upper_bound\": %d, \"tile_queries\": %d, \"tile_auto\": %d, \"tile_candidates\": %d, "
                  "\"split_len\": %lld, \"long_query_len\": %lld, \"emit_copy\": %d, \"eytz_depth\": %d, "
-                 "\"sample_queries\": %zu, \"sample_ms\": %.4f, \"trials\": %d}",
+                 "\"sample_queries\": %zu, \"sample_ms\": %.4f, \"counted_ms\": %.4f, \"trials\": %d}",
                  best_ub, best.tile_q, best.auto_tile ? 1 : 0, best.cap, (long long)best.split_len,
-                 (long long)best.long_len, best.emit_copy ? 1 : 0, best.eytz_depth, ns, best_ms, trials);
+                 (long long)best.long_len, best.emit_copy ? 1 : 0, best.eytz_depth, ns, best_ms,
+                 ranks ? counted_ms : best_ms, trials);
     }
     return SI_OK;
 }

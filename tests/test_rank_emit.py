@@ -352,3 +352,36 @@ def test_a_warp_of_start_above_end_walks_at_once(api):
     for b in bufs:
         lib.deviceFreeGpu(b)
     idx.close()
+
+
+@pytest.mark.parametrize("inverted", [False, True])
+def test_autotuner_times_what_a_setting_changes(api, inverted):
+    """Searches over ranks use neither the upper-bound provider nor the copied sections: those are timed on
+    the counted search, which is slower on the same batch; an index with a start > end interval has that
+    search only."""
+    import ctypes as C
+    import json
+
+    rng = np.random.default_rng(4)
+    n = 300_000
+    s = rng.integers(0, 60_000_000, n).astype(np.int32)
+    e = s + rng.integers(0, 3000, n).astype(np.int32)
+    if inverted:
+        s[0], e[0] = 500, 3
+    idx = api.GpuIndex(32)
+    idx.add_arrays(s, e)
+    idx.build()
+    bufs = [C.c_void_p() for _ in range(2)]
+    for b, a in zip(bufs, (s, e + 2000)):
+        api.check(idx.lib.deviceMallocGpu(C.byref(b), a.nbytes))
+        api.check(idx.lib.memcpyGpu(b, C.c_void_p(a.ctypes.data), a.nbytes, idx.stream))
+    rep = C.create_string_buffer(512)
+    api.check(idx.lib.autotuneBatchedGpu(idx.h, bufs[0], bufs[1], None, n, 0, 0, rep, 512))
+    tuned = json.loads(rep.value.decode())
+    if inverted:
+        assert tuned["counted_ms"] == tuned["sample_ms"]
+    else:
+        assert tuned["counted_ms"] > 1.1 * tuned["sample_ms"]
+    for b in bufs:
+        idx.lib.deviceFreeGpu(b)
+    idx.close()
