@@ -617,9 +617,12 @@ int build_impl(gSuperIntervals* si, bool tight) {
                                    si->ub_mode, st));
     std::vector<uint32_t> grid_base;
     const bool two = si->inverted == 0;
-    // no room for them is no error: the index then works without
-    const int gr = build_grids<S>(si->grid, si->starts.as<S>(), two ? si->end_sorted.as<S>() : nullptr, n, segv,
-                                  si->seg.as<int64_t>(), grid_base, st);
+    // no room for them is no error: the index then works without.  (Nor do more contigs have them than
+    // the ranked tiles' sort keys, position >> shift + contig in 30 bits, leave room for.)
+    const int gr = G > 1 << 28
+                       ? SI_ERR_OOM
+                       : build_grids<S>(si->grid, si->starts.as<S>(), two ? si->end_sorted.as<S>() : nullptr, n, segv,
+                                        si->seg.as<int64_t>(), grid_base, st);
     if (gr != SI_OK && gr != SI_ERR_OOM) return gr;
     si->grid_starts = gr == SI_OK;
     si->grid_ends = gr == SI_OK && two;
