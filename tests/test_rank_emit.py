@@ -385,3 +385,33 @@ def test_autotuner_times_what_a_setting_changes(api, inverted):
     for b in bufs:
         idx.lib.deviceFreeGpu(b)
     idx.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("nq", [311_296, 311_297, 1_048_576, 1_048_577])
+def test_batches_around_the_pass_limits(api, nq, bits):
+    """Four queries a thread above 311,296 queries, and three passes of the tiles' sort above 1,048,576."""
+    dt = np.int32 if bits == 32 else np.int64
+    rng = np.random.default_rng(nq)
+    n = 50_000
+    s = np.sort(rng.integers(0, 2_000_000, n))
+    seg = np.array([0, 20_000, 20_000, n], np.int64)
+    s[20_000:] -= s[20_000] - 5
+    e = s + np.where(rng.random(n) < 0.01, 40_000, rng.integers(1, 90, n))
+    data = rng.integers(-9, 9, n).astype(np.int32)
+    qs = rng.integers(-50, 1_300_000, nq)
+    qe = qs + rng.integers(0, 100, nq)
+    qc = rng.integers(0, 3, nq).astype(np.int32)
+    idx = api.GpuIndex(bits)
+    idx.add_arrays(s.astype(dt), e.astype(dt), data, seg=seg)
+    idx.build()
+    got = []
+    for path in (api.PATH_AUTO, api.PATH_BATCHED, api.PATH_PLAIN):
+        idx.set_path(path)
+        off, out = idx.search(qs.astype(dt), qe.astype(dt), qc, order=api.ORDER_IDXS_CPP)
+        _, val = idx.search(qs.astype(dt), qe.astype(dt), qc, order=api.ORDER_DESC, values=True)
+        got.append((off, out, val))
+    for a, b, c in zip(*got):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+    assert np.array_equal(np.diff(got[0][0]), idx.count(qs.astype(dt), qe.astype(dt), qc))
+    idx.close()

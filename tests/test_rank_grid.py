@@ -311,3 +311,62 @@ def test_one_outlying_coordinate_costs_little(api):
             lib.deviceFreeGpu(b)
         idx.close()
     assert ms[1] < 3.5 * ms[0]
+
+
+def _grid_shift(keys):
+    """log2 of the bucket width that the grid takes for these ascending keys (k_grid_params)."""
+    n, span = len(keys), int(keys[-1]) - int(keys[0])
+    at = [int(keys[(n - 1) * k // 64]) for k in range(65)]
+    spread = sum(b - a >= span // 256 for a, b in zip(at, at[1:]))
+    cap, shift = max(2, n * spread // 64 // 4), 0
+    while span >> shift >= cap:
+        shift += 1
+    return shift
+
+
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+@pytest.mark.parametrize("width", [0, 1, 6, 7, 8, 9, 15, 16, 17, 20, 33])
+def test_bucket_widths(api, width, dt):
+    """Starts and ends in buckets of exactly 2^width coordinates, on both sides of what a record's seven-bit
+    code and a 16-bit offset hold, with records of all codes (up to 12 entries), counts only (13-19) and
+    tables of their own (20 and more), entries on both bucket edges and equal ones among them."""
+    if width > 20 and dt is np.int32:
+        pytest.skip("1000 buckets of 2^33 pass the 32-bit range")
+    rng = np.random.default_rng(width)
+    n, nb = 4096, 1000
+    per = rng.choice([0, 1, 2, 3, 4, 5, 6, 7, 8, 12], nb, p=[.1, .1, .15, .2, .15, .1, .08, .05, .05, .02])
+    per[10::50] = rng.integers(20, 41, len(per[10::50]))
+    per[35::50] = rng.integers(13, 20, len(per[35::50]))
+    while per.sum() != n:                                     # to exactly n, in buckets of few entries
+        k = rng.integers(1, nb - 1)
+        if per[k] < 12:
+            per[k] = min(max(per[k] + np.sign(n - per.sum()), 0), 11)
+    per[0], per[1], per[-2], per[-1] = 1, per[:2].sum() - 1, per[-2:].sum() - 1, 1
+    b = np.repeat(np.arange(nb), per)
+    w = 1 << width
+    inside = rng.integers(0, w, n) if width < 6 else np.where(rng.random(n) < 0.3, rng.choice([0, 1, w // 2, w - 1], n),
+                                                               rng.integers(0, w, n))
+    inside[0], inside[-1] = 0, w - 1
+    s = np.sort((b << width) + inside) - 77
+    e = s + 5 * w + 1
+    assert _grid_shift(s) == width and _grid_shift(e) == width
+    got = np.bincount((s - s[0]) >> width)
+    assert (got > 20).any() and ((got >= 13) & (got < 20)).any() and (got == 12).any()
+    edges = ((np.arange(nb + 1) << width) - 77)
+    qe = np.concatenate([s, s - 1, s + 1, edges, edges - 1, edges + w // 2])
+    qs = rng.permutation(np.concatenate([e, e - 1, e + 1, edges + 5 * w + 1, edges + 5 * w, edges + 5 * w + w // 2]))
+    qs = np.minimum(qs, qe)
+    near = np.arange(len(qe)) % 2 == 0                        # the end's rank from a key of its own
+    qs[near] = qe[near] - rng.integers(0, 6 * w, near.sum())
+    info = np.iinfo(dt)
+    assert s[0] > info.min and e[-1] + w < info.max
+    cnt = np.searchsorted(s, qe, side="right") - np.searchsorted(e, qs, side="left")
+    idx = api.GpuIndex(np.dtype(dt).itemsize * 8)
+    idx.add_arrays(s.astype(dt), e.astype(dt))
+    idx.build()
+    assert np.array_equal(idx.count(qs.astype(dt), qe.astype(dt)), cnt)
+    got = idx.coverage(qs.astype(dt), qe.astype(dt))
+    idx.set_path(api.PATH_PLAIN)
+    for x, y in zip(got, idx.coverage(qs.astype(dt), qe.astype(dt))):
+        assert np.array_equal(x, y)
+    idx.close()
