@@ -3105,13 +3105,12 @@ int batched_prepare_queries(BatchedWorkspace& ws, MapView<S> m, const QueryBatch
     ws.launches += 2 + (packed ? 1 : 2) + passes + 1;
     ws.prepared_qs = q.qs;
     ws.prepared_nq = nq;
-    ws.prepared_mode = ub_mode;
     return SI_OK;
 }
 
 template <typename S>
 int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>& gs, const QueryBatch& q,
-                           const uint32_t* su, int* d_err, int ub_mode, cudaStream_t st) {
+                           const uint32_t* su, int* d_err, cudaStream_t st) {
     const int64_t nq = q.nq;
     ws.prepared_nq = -1;
     if (nq <= 0) return SI_OK;
@@ -3158,7 +3157,6 @@ int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>
     ws.launches += 2 + passes + 1;
     ws.prepared_qs = q.qs;
     ws.prepared_nq = nq;
-    ws.prepared_mode = ub_mode;
     ws.n_heads = 0;       // no head runs and no candidate lists are kept: batched_emit_ranked only
     ws.cache_ok = false;
     return SI_OK;
@@ -3240,8 +3238,10 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
     a.d_err = d_err;
     const bool pieces = what == kOutPieces;
     using Kernel = void (*)(EmitArgs<S>);
-    const Kernel fns[2][2] = {{&k_emit_tiles<S, kOutIdx, 4>, &k_emit_tiles<S, kOutIdx, 5>},
-                              {&k_emit_tiles<S, kOutPieces, 4>, &k_emit_tiles<S, kOutPieces, 5>}};
+    // [pieces][five blocks per SM]; 64-bit lists take too much shared memory for five
+    constexpr int kMost = sizeof(S) == 4 ? 5 : 4;
+    const Kernel fns[2][2] = {{&k_emit_tiles<S, kOutIdx, 4>, &k_emit_tiles<S, kOutIdx, kMost>},
+                              {&k_emit_tiles<S, kOutPieces, 4>, &k_emit_tiles<S, kOutPieces, kMost>}};
     const int e = 2 + (pieces ? 1 : 0);
     int dev = 0;
     SI_CU(cudaGetDevice(&dev));
@@ -3263,7 +3263,7 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
         sm = (size_t)a.at_class + 4 * (size_t)a.tile_q;
         if (sm <= ws.smem_room[pieces] || a.cap <= 256) break;
     }
-    const int five = sizeof(S) == 4 && sm + 4096 <= kSmemPerSm / 5 ? 1 : 0;  // 4 KB: static and reserved
+    const int five = kMost == 5 && sm + 4096 <= kSmemPerSm / 5 ? 1 : 0;  // 4 KB: static and reserved
     const Kernel fn = fns[pieces][five];
     if (ws.occ_smem[e] != sm) {
         int nsm = 152, per_sm = 1;
@@ -3468,7 +3468,7 @@ int batched_coverage(BatchedWorkspace& ws, MapView<S> m, const QueryBatch& q, co
     template int batched_prepare_queries<S>(BatchedWorkspace&, MapView<S>, const QueryBatch&, int*, int,          \
                                             cudaStream_t, uint32_t*, bool);                                                \
     template int batched_prepare_ranked<S>(BatchedWorkspace&, MapView<S>, const RankGrid<S>&, const QueryBatch&,  \
-                                           const uint32_t*, int*, int, cudaStream_t);                            \
+                                           const uint32_t*, int*, cudaStream_t);                                 \
     template int batched_emit_ranked<S>(BatchedWorkspace&, MapView<S>, Levels<S>, int, const RankGrid<S>&,         \
                                         const QueryBatch&, int64_t, const int64_t*, int64_t, int, int,            \
                                         RankDest<S>, int*, cudaStream_t, int64_t);                               \

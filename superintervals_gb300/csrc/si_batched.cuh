@@ -75,7 +75,6 @@ struct BatchedWorkspace {
     // identity of the batch the sorted records belong to
     const void* prepared_qs = nullptr;
     int64_t prepared_nq = -1;
-    int prepared_mode = -1;
     int64_t n_heads = 0;
     long long launches = 0;      // kernels launched by this path
     // candidate lists of every tile, written by the count pass, read by the emit pass
@@ -134,7 +133,7 @@ int batched_prepare_queries(BatchedWorkspace& ws, MapView<S> m, const QueryBatch
 // position), without a host round trip.  The batch is counted already; emit it next.
 template <typename S>
 int batched_prepare_ranked(BatchedWorkspace& ws, MapView<S> m, const RankGrid<S>& gs, const QueryBatch& q,
-                           const uint32_t* su, int* d_err, int ub_mode, cudaStream_t st);
+                           const uint32_t* su, int* d_err, cudaStream_t st);
 // Emits queries [q_offset, q_offset + q.nq) of the batch prepared last by batched_prepare_ranked;
 // `what` is a RankOut other than keys.
 template <typename S>

@@ -876,7 +876,7 @@ int rank_prepare(gSuperIntervals* si, const sig::QueryBatch& q, int lanes, cudaS
     if (lanes) return SI_OK;
     PhaseTimer pt(si, 3, st);
     const int r = sig::batched_prepare_ranked<S>(si->bws, view<S>(si), rank_grid<S>(si, 0), q,
-                                                 si->w_upper.as<uint32_t>(), si->w_err.as<int>(), si->ub_mode, st);
+                                                 si->w_upper.as<uint32_t>(), si->w_err.as<int>(), st);
     return r == SI_OK ? SI_OK : fail(r, "batched query preparation failed (status %d)", r);
 }
 
