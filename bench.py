@@ -305,23 +305,6 @@ def run_gpu(args, rank, world, dist):
     n4 = (C.c_int64 * 4)()
     _capi.check(lib.getPhaseTimesGpu(idx.h, ms4, n4))
     res["phase_ms"] = [ms4[k] / max(1, n4[k]) for k in range(4)]
-    if path == _capi.PATH_BATCHED:
-        # the emit in each of its two modes for the long-interval list's section of part B
-        # (copied around its misses / filtered), the tuned mode restored afterwards
-        cur = C.c_int64(1)
-        _capi.check(lib.getBatchedOptionGpu(idx.h, _capi.OPT_EMIT_COPY, C.byref(cur)))
-        res["emit_mode_ms"] = {}
-        for mode, name in ((1, "copy"), (0, "filter")):
-            _capi.check(lib.setProfilingGpu(idx.h, 0))
-            _capi.check(lib.setProfilingGpu(idx.h, 1))
-            _capi.check(lib.setBatchedOptionGpu(idx.h, _capi.OPT_EMIT_COPY, mode))
-            for _ in range(max(1, min(3, args.steps))):
-                _capi.check(lib.flushL2Gpu(st))
-                step()
-            _capi.check(lib.getPhaseTimesGpu(idx.h, ms4, n4))
-            res["emit_mode_ms"][name] = ms4[2] / max(1, n4[2])
-        _capi.check(lib.setBatchedOptionGpu(idx.h, _capi.OPT_EMIT_COPY, cur.value))
-        res["emit_copy_tuned"] = int(cur.value)
     _capi.check(lib.setProfilingGpu(idx.h, 0))
 
     # the plain one-query-per-thread GPU path on the same inputs (the 1.0x baseline)
@@ -401,7 +384,7 @@ def run_gpu(args, rank, world, dist):
         f_cnt = lib.countOverlapsBatchGpu_i64 if s_bytes == 8 else lib.countOverlapsBatchGpu
         lat = {"count": [], "search_idxs": []}
         saved = path
-        idx.set_path(_capi.PATH_AUTO)     # one query takes the plain path
+        idx.set_path(_capi.PATH_AUTO)
         for _ in range(220):
             t0 = time.perf_counter()
             _capi.check(f_cnt(idx.h, C.c_void_p(one_s.ctypes.data), C.c_void_p(one_e.ctypes.data),
@@ -939,7 +922,7 @@ def run_serving(args, rank, world, dist):
 
     res = {"wl": wl, "build_s": build_s, "nreq": nreq, "nq": nq_all, "sizes": sizes, "qs": qs, "qe": qe, "qc": qc}
     with ClockSampler(int(os.environ.get("LOCAL_RANK", "0"))) as clk:
-        # the library picks the batched path for batches of 4096+ queries and the plain one below
+        # the library's choice: ranks, then a direct emit or sorted tiles by the hits they find
         serve(_capi.PATH_AUTO, _capi.UB_LEARNED, True)               # warm-up
         res["batched_sat"] = serve(_capi.PATH_AUTO, _capi.UB_LEARNED, True)
         res["batched_rate"] = serve(_capi.PATH_AUTO, _capi.UB_LEARNED, False)
@@ -964,7 +947,7 @@ def serving_line(args, res, world):
                                    f"({res['nq']} queries, sizes log-uniform), offered {args.rate}/s",
                        "n_intervals": wl.n, "requests": res["nreq"], "queries": res["nq"],
                        "op": "search_idxs (C++ order) per request batch",
-                       "path": "auto (batched for 4096+ queries, else plain) + learned upper bound",
+                       "path": "auto (ranks, then a direct emit or sorted tiles)",
                        "inputs": "queries from pinned host memory; results to pinned host memory"},
             "latency_ms": {"offered_rate_per_s": args.rate, "p50": br["p50_ms"], "p99": br["p99_ms"],
                            "queries_per_s": br["queries_per_s"], "batches": br["batches"]},
@@ -1215,18 +1198,19 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "int32" if s == 4 else "int64", "data": "synthetic (seeded)",
             "config": dict(workload_desc(cfg, wl), path=args.path, upper_bound=args.ub,
-                           autotuned=res.get("tuned")),
+                           bounds="ranks of the starts and sorted ends; no provider is read in the step"
+                           if args.path == "batched" else "the provider", autotuned=res.get("tuned")),
             "pairs_per_s": pps, "result_pairs_per_step": P,
             "build_s": res["build_s"], "clocks": res["clocks"]}
     if args.profile_only:
         print(json.dumps(line), flush=True)
         return
     # roofline of the dominant kernel (emit) with the algorithmic bytes
-    # B = Q*(2s+8) + P*(s+4): query read, offset read, one end read and one index
-    # write per result pair
+    # B = Q*(2s+8) + 4P: query read, offset read, one index write per result pair (a tile's
+    # queries share the reads of their candidates)
     ph = res.get("phase_ms", [0, 0, 0, 0])
     emit_ms = ph[2] if ph[2] > 0 else ms
-    algo = nq * (2 * s + 8) + P * (s + 4)
+    algo = nq * (2 * s + 8) + P * 4
     achieved = algo / (emit_ms / 1000.0) / 1e9
     traffic = (EMIT_DRAM_WRITE_PER_PAIR * P + EMIT_DRAM_READ_PER_QUERY * nq
                if cfg == "config3" and args.path == "batched" else None)
@@ -1237,7 +1221,6 @@ def main():
                         "traffic_frac": (traffic / (emit_ms / 1000.0) / 1e9 / peak) if traffic else None,
                         "peak_kind": peak_kind, "algorithmic_bytes": algo,
                         "phase_ms": {"count": ph[0], "scan": ph[1], "emit": ph[2], "prepare": ph[3]},
-                        "emit_ms_by_mode": res.get("emit_mode_ms"),
                         "whole_step_frac": (algo / (ms / 1000.0) / 1e9) / peak}
     line["gpu_launches"] = res["launches"]
     if "single_query_us" in res:

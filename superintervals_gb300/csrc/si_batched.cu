@@ -1304,6 +1304,7 @@ constexpr int kDirectBlocks = 128;  // 32-slot blocks of a tile's direct gather
 constexpr int kMaxMiss = 31;        // possible misses up to which a section has versions
 constexpr int kMinSection = 96;     // and its length from which they pay
 constexpr size_t kSmemPerSm = 228 * 1024;
+constexpr size_t kSmemAlways = 192 * 1024;  // dynamic shared memory that a tile emit surely may have
 
 // First index in [a, b) of an ascending list whose entry is >= key (b when none).
 __device__ __forceinline__ int64_t first_at_least(const int32_t* __restrict__ arr, int64_t a, int64_t b, int32_t key) {
@@ -3245,12 +3246,6 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
     const int e = 2 + (pieces ? 1 : 0);
     int dev = 0;
     SI_CU(cudaGetDevice(&dev));
-    if (!ws.smem_room[pieces])
-        for (const Kernel fn : fns[pieces]) {  // of both, what the one with less has
-            size_t room = 0;
-            SI_CU(allow_smem(reinterpret_cast<const void*>(fn), dev, &room));
-            ws.smem_room[pieces] = ws.smem_room[pieces] ? std::min(ws.smem_room[pieces], room) : room;
-        }
     // 40 bytes a slot with 64-bit coordinates and 52 a query: the largest tunables ask for more than a
     // block may have (6656 slots and 256 queries: 239,344 bytes of some 230,000).  Fewer slots then: a
     // tile that overflows them emits its queries one by one.
@@ -3261,13 +3256,17 @@ int batched_emit_ranked(BatchedWorkspace& ws, MapView<S> m, Levels<S> L, int H, 
         a.at_start = a.at_rec + (int)sizeof(QRec<S>) * a.tile_q;
         a.at_class = a.at_start + (int)sizeof(S) * (a.cap + 32);
         sm = (size_t)a.at_class + 4 * (size_t)a.tile_q;
-        if (sm <= ws.smem_room[pieces] || a.cap <= 256) break;
+        if (sm <= kSmemAlways || a.cap <= 256) break;
+        if (!ws.smem_room[pieces])
+            SI_CU(allow_smem(reinterpret_cast<const void*>(fns[pieces][0]), dev, &ws.smem_room[pieces]));
+        if (sm <= ws.smem_room[pieces]) break;
     }
     const int five = kMost == 5 && sm + 4096 <= kSmemPerSm / 5 ? 1 : 0;  // 4 KB: static and reserved
     const Kernel fn = fns[pieces][five];
     if (ws.occ_smem[e] != sm) {
         int nsm = 152, per_sm = 1;
         SI_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        SI_CU(allow_smem(reinterpret_cast<const void*>(fn), dev));
         SI_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, sm));
         ws.occ_blocks[e] = nsm * std::max(per_sm, 1);
         ws.occ_smem[e] = sm;
