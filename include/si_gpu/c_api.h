@@ -271,16 +271,19 @@ int searchIdxsNoAllocGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe
 
 /* Upper bound of every query end: contig-local position of the last interval
  * whose start <= qe, or -1.  upperBound (c_superintervals.h:195, 537-568) /
- * IntervalMap::upper_bound (superintervals.hpp:501-516), computed with the
- * provider `mode` (SI_UB_*), which must be the handle's current mode or
- * SI_UB_BINARY.  Device buffers. */
+ * IntervalMap::upper_bound (superintervals.hpp:501-516).  `mode` (SI_UB_*) must be
+ * the handle's current mode or SI_UB_BINARY.  On the automatic path an index with rank
+ * grids answers from those; the provider `mode` answers where there are none and on
+ * the paths that setQueryPathGpu names.  Device buffers. */
 int upperBoundDeviceGpu(gSuperIntervals* si, const void* d_qe, const int32_t* d_qcontig, size_t nq,
                         int mode, int32_t* d_out, void* stream);
 
 /* Same result as searchDeviceGpu (values_not_idxs = 0, plain path), replayed from a CUDA
  * graph: count -> scan -> emit are captured on the first call of a given shape (buffers,
- * size, order, capacity, stream) and replayed by later calls with that shape -- for
- * repeated small batches, where launch overhead dominates.  Never writes past `capacity`;
+ * size, order, capacity, stream) and replayed by later calls with that shape.  A replay
+ * does the counted search's work: over an index with start > end intervals, where
+ * searchDeviceGpu does the same, it saves launches; elsewhere searchDeviceGpu searches
+ * by ranks and is faster.  Never writes past `capacity`;
  * a larger result returns SI_ERR_CAPACITY with *total set. */
 int searchDeviceGraphGpu(gSuperIntervals* si, const void* d_qs, const void* d_qe,
                          const int32_t* d_qcontig, size_t nq, int order, int64_t* d_offsets,

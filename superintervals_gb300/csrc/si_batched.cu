@@ -1624,7 +1624,7 @@ __device__ __forceinline__ void st_if(bool p, int32_t* addr, int32_t v) {
 
 // What bounds it (two chromosomes at the full density, 7.95 M queries with 511 hits each, 16.3 GB
 // written): 3.7 ms, 4.4 TB/s of scattered 2 KB lists, against 5.4 ms with every candidate checked
-// (595 warp instructions a query, now 403 at 78% issue).  Set-up takes 18 us of a tile's 89 us, its
+// (595 warp instructions a query, now 399 at 78% issue).  Set-up takes 18 us of a tile's 89 us, its
 // queries 62.  BLOCKS resident per SM: five where the lists fit (1280 slots: 35 KB; four: 4606 against
 // 4512 us for the call), else four with the registers that leaves.
 template <typename S, int OUT, int BLOCKS>

@@ -1,5 +1,5 @@
-// si_rank.cuh -- rank grid: the rank of a key in each contig's ascending coordinates in about four
-// dependent reads, for queries in any order.
+// si_rank.cuh -- rank grid: the rank of a key in each contig's ascending coordinates in one or two
+// dependent reads (three to five where coordinates crowd), for queries in any order.
 //
 // Counts, upper bounds and coverage need only ranks (how many starts / sorted ends lie below a
 // key).  A halving search makes log2(n) dependent reads per rank, and sorting the batch first, so
@@ -299,7 +299,7 @@ template <typename S>
 cudaError_t launch_rank_ub(RankGrid<S> gs, int G, const void* qe, const int32_t* qc, int64_t nq, int32_t* out,
                            int* d_err, cudaStream_t st);
 // Coverage from ranks and prefix sums (see launch site); *d_inv is set when a query has start > end
-// (its answer is not written).
+// (it is answered 0 and 0, and the caller computes the batch another way).
 template <typename S>
 cudaError_t launch_rank_coverage(RankGrid<S> gs, RankGrid<S> ge, int G, QueryBatch q, const uint64_t* ps_start,
                                  const uint64_t* ps_end, uint64_t* count, S* cov, int* d_err, int* d_inv,
