@@ -1355,31 +1355,40 @@ __device__ void emit_alone(const EmitArgs<S>& a, S qs, S qe, int64_t u, int g, i
 #pragma unroll 8
             for (int r = lane; r < h; r += 32) d[r] = first + step * r - (int32_t)lo;
         } else {
-            for (int r0 = lane; r0 < h; r0 += 32 * U) {
-                S st[U], e[U];
-                int32_t v[U];
-#pragma unroll
-                for (int k = 0; k < U; ++k) {
-                    const int32_t pos = first + step * min(r0 + 32 * k, h - 1);
-                    if constexpr (OUT == kOutPieces) {
-                        st[k] = a.starts[pos];
-                        e[k] = ends[pos];
-                    } else {
-                        v[k] = a.data[pos];
-                    }
+            // Whole groups of U rounds, then the rest round by round: a run shorter than a group, as most
+            // are, makes no reads for the rounds that it has not, and groups carry no checks (pieces of 300
+            // queries with 200 k hits 9.26 -> 6.87 ms, payloads 2.85 -> 2.69).
+            S st[U], e[U];
+            int32_t v[U];
+            auto fetch = [&](int r, int k) {
+                const int32_t pos = first + step * r;
+                if constexpr (OUT == kOutPieces) {
+                    st[k] = a.starts[pos];
+                    e[k] = ends[pos];
+                } else {
+                    v[k] = a.data[pos];
                 }
-#pragma unroll
-                for (int k = 0; k < U; ++k) {
-                    const int r = r0 + 32 * k;
-                    if (r >= h) continue;
-                    if constexpr (OUT == kOutPieces) {
-                        d[r] = first + step * r - (int32_t)lo;
-                        (a.dst.s + out_off)[r] = st[k] > qs ? st[k] : qs;
-                        (a.dst.e + out_off)[r] = e[k] < qe ? e[k] : qe;
-                    } else {
-                        d[r] = v[k];
-                    }
+            };
+            auto store = [&](int r, int k) {
+                if constexpr (OUT == kOutPieces) {
+                    d[r] = first + step * r - (int32_t)lo;
+                    (a.dst.s + out_off)[r] = st[k] > qs ? st[k] : qs;
+                    (a.dst.e + out_off)[r] = e[k] < qe ? e[k] : qe;
+                } else {
+                    d[r] = v[k];
                 }
+            };
+            int r0 = 0;
+            for (; r0 + 32 * U <= h; r0 += 32 * U) {
+#pragma unroll
+                for (int k = 0; k < U; ++k) fetch(r0 + 32 * k + lane, k);
+#pragma unroll
+                for (int k = 0; k < U; ++k) store(r0 + 32 * k + lane, k);
+            }
+#pragma unroll 1
+            for (int r = r0 + lane; r < h; r += 32) {
+                fetch(r, 0);
+                store(r, 0);
             }
         }
     }
